@@ -585,8 +585,10 @@ __device__ __forceinline__ float gn_value(const GroupNormParams& p, size_t t, in
 constexpr int GN_CACHE = 8;
 
 // ONE_PLANE: the gate's sums are finished, so a thread asks for everything it needs before it uses the first value.
+// The launch bound holds the block form to the registers that its largest block (1,024 threads: a part of 2,048 and more
+// elements in a step of few tokens) finds on an SM.
 template <typename TO, bool WARP, bool ONE_PLANE>
-__global__ void group_gate_norm_kernel(const GroupNormParams p, TO* __restrict__ out) {
+__global__ void __launch_bounds__(WARP ? 128 : 1024) group_gate_norm_kernel(const GroupNormParams p, TO* __restrict__ out) {
     pdl_launch_dependents();
     pdl_wait();
     __shared__ float scratch[32];

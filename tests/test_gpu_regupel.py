@@ -425,6 +425,18 @@ def test_linear_attention_with_a_decay_per_head_in_portions(heads, dim, vdim):
         torch.testing.assert_close(out.float().cpu().double(), wanted, atol=1e-4 if store == torch.float32 else 3e-2, rtol=1e-2)
 
 
+@pytest.mark.parametrize("splits", [1, 3])
+@pytest.mark.parametrize("tokens, width", [(1, 2048), (3, 4096), (255, 2050), (1, 8193)])
+def test_norm_and_gate_of_wide_rows_in_short_steps(tokens, width, splits):
+    """Rows that take a block of 1,024 threads."""
+    torch.manual_seed(width + splits)
+    o, gate, weight = torch.randn(tokens, width), torch.randn(splits, tokens, width), torch.randn(width) * 0.2 + 1.0
+    wanted = plain.rms_divide(o.double(), 1e-5) * weight.double() * torch.sigmoid(gate.double().sum(0))
+    out = torch.empty(tokens, width, device=DEV)
+    kernels.group_gate_norm(o.to(DEV), weight.to(DEV), 1e-5, out, proj=GemmOut(gate.to(DEV)), at_gate=0)
+    torch.testing.assert_close(out.cpu().double(), wanted, atol=1e-4, rtol=1e-2)
+
+
 def test_a_write_to_the_state_survives_hundreds_of_tokens():
     """With a decay of 1 the first token's key and value are read back by a query 600 tokens later; with a decay of 0.99
     they arrive times 0.99^599; with a decay of 0 only the query's own token answers."""
