@@ -1,7 +1,6 @@
 // C[M, N] = A[M, K] * W[N, K]^T with float accumulation on the FMA pipe, for any sizes and for
-// float or bfloat16 inputs.  This is the whole 32-bit path's matrix product (true float: no
-// tensor cores, no reduced-precision mode; sums blocked over K in three levels) and the bfloat16 path's choice for shapes the
-// tensor-core kernel refuses.  Counterpart in luozoupi/Qwen-Triton: kernels/matmul.py:52-97.
+// float or bfloat16 inputs (true float: no tensor cores, no reduced-precision mode; sums blocked over K in three levels): what
+// neither gemm_f32.cu (float rows of whole 16-byte pieces) nor the tensor-core kernels take.  Counterpart in luozoupi/Qwen-Triton: kernels/matmul.py:52-97.
 #include "common.cuh"
 
 using namespace qt;

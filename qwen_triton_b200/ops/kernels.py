@@ -129,6 +129,9 @@ _SIGNATURES = {
         "qt_attention_prefill_tc": [_c_ptr, _c_ptr, _c_ptr, _c_ptr, _c_int, _c_int, _c_ptr, _c_int, _c_ptr, _c_ptr, _c_int,
                                     _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_float, _c_ptr, _c_ptr, _c_int, _c_int, _c_int, _c_ptr, _c_float, _c_int, _c_ptr, _c_ptr],
     },
+    "gemm_f32": {
+        "qt_gemm_f32": [_c_ptr, _c_ptr, _c_ptr, _c_int, _c_int, _c_int, _c_ptr],
+    },
     "gemm_simt": {
         "qt_gemm_simt": [_c_ptr, _c_ptr, _c_int, _c_ptr, _c_int, _c_int, _c_int, _c_int, _c_ptr],
     },
@@ -1360,6 +1363,21 @@ def gemm_simt(a: torch.Tensor, w: torch.Tensor, out: GemmOut) -> None:
           a.shape[0], w.shape[0], a.shape[1], _stream())
 
 
+def gemm_f32_supported(a: torch.Tensor, w: torch.Tensor, out: GemmOut) -> bool:
+    return (a.dtype == w.dtype == out.tensor.dtype == torch.float32 and a.shape[1] % 4 == 0 and a.data_ptr() % 16 == 0
+            and w.data_ptr() % 16 == 0)
+
+
+def gemm_f32(a: torch.Tensor, w: torch.Tensor, out: GemmOut) -> None:
+    """out = a [M, K] @ w [N, K]^T in true float on the FMA pipe; K a multiple of 4, 16-byte aligned operands."""
+    _need(a, "a", torch.float32)
+    _need(w, "w", torch.float32)
+    if a.shape[1] != w.shape[1] or out.n_splits != 1 or (out.rows, out.cols) != (a.shape[0], w.shape[0]):
+        raise KernelError(f"gemm: a {tuple(a.shape)}, w {tuple(w.shape)}, out {tuple(out.tensor.shape)} do not fit")
+    _need(out.tensor, "out", torch.float32)
+    _call("gemm_f32", "qt_gemm_f32", _ptr(a), _ptr(w), _ptr(out.tensor), a.shape[0], w.shape[0], a.shape[1], _stream())
+
+
 # ----------------------------------------------------------------------------- sampling
 def argmax(logits: torch.Tensor, out: torch.Tensor) -> None:
     _need(logits, "logits", torch.float32)
@@ -1561,14 +1579,18 @@ def gemm_uses_pairs(a: torch.Tensor, w: torch.Tensor) -> bool:
 
 def gemm(a: torch.Tensor, w: torch.Tensor, out: GemmOut, bias: torch.Tensor | None = None) -> None:
     """out = a @ w^T (+ ``bias`` [N], float, for float results) with the kernel that fits the element type and shape (a static choice):
-    tensor cores for bfloat16 with 16-byte aligned rows, the FMA kernel for float32 and the rest."""
+    tensor cores for bfloat16 with 16-byte aligned rows; on the FMA pipe the packed float32 kernels, and the plain one for what is left
+    (float32 rows that are not 16-byte aligned, bfloat16 that the tensor cores' loads cannot take)."""
     if gemm_tc_supported(a, w):
         if gemm_uses_pairs(a, w):
             gemm_tc_pair(a, w, out, bias=bias)         # more tokens than one block's tile: pairs of blocks, a third less operand traffic
         else:
             gemm_tc(a, w, out, bias=bias)
     elif out.n_splits == 1:
-        gemm_simt(a, w, out)
+        if gemm_f32_supported(a, w, out):
+            gemm_f32(a, w, out)
+        else:
+            gemm_simt(a, w, out)
         if bias is not None and out.rows:
             add_bias(out.tensor[0], bias)
     else:

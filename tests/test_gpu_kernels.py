@@ -200,6 +200,19 @@ def test_gemm_simt(dtype, m, n, k):
         close(out[0], expected, out_dtype, f"{m}x{n}x{k}")
 
 
+@pytest.mark.parametrize("m", [1, 2, 3, 4, 5, 8, 9, 16, 17, 32, 33, 64, 65, 200])
+@pytest.mark.parametrize("n, k", [(1, 4), (37, 28), (127, 128), (128, 32), (129, 36), (503, 1000), (1024, 3072), (4100, 260)])
+def test_gemm_f32(m, n, k):
+    """Rows kernel and tiles, alone and cut over K: every result within the rounding of its longest chain of additions (16 products
+    of a slice's even or odd k, their halves, the slices, the ranks; a row's lanes have shorter ones)."""
+    a, w = rand(m, k, seed=14, dtype=torch.float32), rand(n, k, seed=15, scale=0.1, dtype=torch.float32)
+    out = torch.full((1, m + 1, n), 7.0, device=DEV)                      # one row behind the result that must stay as it is
+    kernels.gemm_f32(a, w, GemmOut(out[:, :m]))
+    bound = (a.double().abs() @ w.double().abs().T) * 2.0 ** -24 * (18 + -(-k // 32) + 8)
+    assert bool(((out[0, :m].double() - a.double() @ w.double().T).abs() <= bound).all())
+    assert bool((out[0, m] == 7.0).all())
+
+
 def test_gemm_float32_is_true_float32():
     """Inputs that a reduced-precision matrix mode would round away: 1 + 2^-12 squared keeps the 2^-11 term."""
     a = torch.full((4, 64), 1.0 + 2.0 ** -12, device=DEV)
