@@ -49,37 +49,7 @@ __device__ __forceinline__ float la_raw(const LinAttnParams& p, size_t index) {
 }
 __device__ __forceinline__ float la_act(const LinAttnParams& p, float x) { return p.act ? x / (1.f + expf(-x)) : x; }
 
-// out[t, c] = SiLU(sum_s proj[s][t, c]) (or the sum itself) for the first `cols` columns of every row: q, k and v of a
-// step, summed and activated once where every block of the recurrence would otherwise activate its head's q and k again.
-__global__ void linear_attention_prepare_kernel(const float* __restrict__ proj, int n_splits, size_t split_stride, int proj_cols, int cols,
-                                                float* __restrict__ out, long long total, int act) {
-    pdl_launch_dependents();
-    pdl_wait();
-    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
-        const size_t at = (size_t)(i / cols) * proj_cols + (size_t)(i % cols);
-        float x = proj[at];
-        for (int s = 1; s < n_splits; ++s) x += proj[at + (size_t)s * split_stride];
-        out[i] = act ? x / (1.f + expf(-x)) : x;
-    }
-}
-
-extern "C" int qt_linear_attention_prepare(const float* proj, int n_splits, long long split_stride, int proj_cols, int cols, float* out, int n_tokens,
-                                           int act, void* stream) {
-    QT_REQUIRE(n_tokens >= 0 && cols > 0 && cols <= proj_cols && n_splits >= 1, "linear_attention_prepare: %d of %d columns", cols, proj_cols);
-    if (n_tokens == 0) return QT_OK;
-    const long long total = (long long)n_tokens * cols;
-    long long blocks = (total + 255) / 256;
-    if (blocks > (long long)sm_count() * 16) blocks = (long long)sm_count() * 16;
-    launch_kernel(linear_attention_prepare_kernel, dim3((unsigned)blocks), dim3(256), 0, (cudaStream_t)stream, proj, n_splits, (size_t)split_stride, proj_cols,
-                  cols, out, total, act);
-    QT_CHECK_LAUNCH("linear_attention_prepare");
-    return QT_OK;
-}
-
-// The same sums for rows whose first `heads` runs of `dim` columns (q heads, then k heads) are rotated by the token's position: in
-// each, element i < rd / 2 turns together with element i + rd / 2 by the angle whose cos and sin the table row of the position
-// holds (cos | sin, rd columns); the other columns pass.  A thread takes V neighbouring pairs, or V neighbouring columns that
-// do not turn; grid (blocks of a row's items, tokens).
+// V neighbouring floats of a row: their sums over the planes, and their store.
 template <int V> struct RotPack { float v[V]; };
 template <int V> __device__ __forceinline__ RotPack<V> rot_sum(const float* p, int n_splits, size_t stride) {
     RotPack<V> r;
@@ -101,6 +71,44 @@ template <int V> __device__ __forceinline__ void rot_put(float* p, const RotPack
     else *p = r.v[0];
 }
 
+// out[t, c] = SiLU(sum_s proj[s][t, c]) (or the sum itself) for the first `cols` columns of every row: q, k and v of a
+// step, summed and activated once where every block of the recurrence would otherwise activate its head's q and k again.
+// Bound by the bytes it moves.  A thread takes V neighbouring columns (16-byte accesses where the rows allow) of row blockIdx.y, + gridDim.y, ..;
+// 1,999 rows of 6,144 columns: 19 us, 38 us with single floats whose place was divided out of one running index.
+template <int V>
+__global__ void __launch_bounds__(256) linear_attention_prepare_kernel(const float* __restrict__ proj, int n_splits, size_t split_stride, int proj_cols, int cols,
+                                                                       float* __restrict__ out, int n_tokens, int act) {
+    pdl_launch_dependents();
+    pdl_wait();
+    const int c = (blockIdx.x * 256 + threadIdx.x) * V;
+    if (c >= cols) return;
+    for (int t = blockIdx.y; t < n_tokens; t += gridDim.y) {
+        RotPack<V> x = rot_sum<V>(proj + (size_t)t * proj_cols + c, n_splits, split_stride);
+        if (act) {
+#pragma unroll
+            for (int i = 0; i < V; ++i) x.v[i] = x.v[i] / (1.f + expf(-x.v[i]));
+        }
+        rot_put<V>(out + (size_t)t * cols + c, x);
+    }
+}
+
+extern "C" int qt_linear_attention_prepare(const float* proj, int n_splits, long long split_stride, int proj_cols, int cols, float* out, int n_tokens,
+                                           int act, void* stream) {
+    QT_REQUIRE(n_tokens >= 0 && cols > 0 && cols <= proj_cols && n_splits >= 1, "linear_attention_prepare: %d of %d columns", cols, proj_cols);
+    if (n_tokens == 0) return QT_OK;
+    const bool wide = cols % 4 == 0 && proj_cols % 4 == 0 && (n_splits == 1 || split_stride % 4 == 0) && (uintptr_t)proj % 16 == 0 && (uintptr_t)out % 16 == 0;
+    const int per_block = 256 * (wide ? 4 : 1);
+    const dim3 grid((unsigned)((cols + per_block - 1) / per_block), (unsigned)(n_tokens < 65535 ? n_tokens : 65535));
+    if (wide) launch_kernel(linear_attention_prepare_kernel<4>, grid, dim3(256), 0, (cudaStream_t)stream, proj, n_splits, (size_t)split_stride, proj_cols, cols, out, n_tokens, act);
+    else launch_kernel(linear_attention_prepare_kernel<1>, grid, dim3(256), 0, (cudaStream_t)stream, proj, n_splits, (size_t)split_stride, proj_cols, cols, out, n_tokens, act);
+    QT_CHECK_LAUNCH("linear_attention_prepare");
+    return QT_OK;
+}
+
+// The same sums for rows whose first `heads` runs of `dim` columns (q heads, then k heads) are rotated by the token's position: in
+// each, element i < rd / 2 turns together with element i + rd / 2 by the angle whose cos and sin the table row of the position
+// holds (cos | sin, rd columns); the other columns pass.  A thread takes V neighbouring pairs, or V neighbouring columns that
+// do not turn; grid (blocks of a row's items, tokens).
 template <int V>
 __global__ void __launch_bounds__(256) linear_attention_rotate_kernel(const float* __restrict__ proj, int n_splits, size_t split_stride, int proj_cols, int cols,
                                                                       float* __restrict__ out, int heads, int dim, int rd, const float* __restrict__ cos_sin,

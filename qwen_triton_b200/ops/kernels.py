@@ -843,6 +843,17 @@ def decay_scratch(max_step_tokens: int, heads: int, dim: int, vdim: int, per_cha
             "q_from": max_step_tokens * heads * wide, "k_to": max_step_tokens * heads * wide}
 
 
+def decay_chunks_pay(ctx, tokens: int, dim: int, max_step_tokens: int) -> bool:
+    """Whether a recurrence with a constant decay per head runs in chunks: from a longest portion of 64 tokens on (1,024 for up to 64 key
+    channels), where the scratch for ``max_step_tokens`` holds the step's chunks.  Token by token a step takes a time that grows
+    with its longest portion and a column's rows, in chunks it is four kernels whatever the length.  16 heads of 128 x 128, token
+    by token / in chunks: 2,048 tokens 763 / 117 us, 200 tokens 79 / 48, 100 tokens 42 / 51, 5 x 90 tokens 85 / 61, 32 x 64 tokens
+    218 / 128, 32 x 24 tokens 96 / 101; error against 64 bits at 64 tokens 3.1e-7 / 2.3e-7, at 2,048 7.5e-7 / 2.7e-7.  8 heads of
+    64 x 128: 2,048 tokens 453 / 55 us and 2.4e-7 / 2.3e-7; 400 tokens 92 / 40 us, but 2.0e-7 / 2.2e-7: eight rows a lane and a
+    short walk round less than two sums over 64."""
+    return ctx.max_q_len >= (64 if dim > 64 else 1024) and tokens // DECAY_CHUNK + ctx.n_seqs <= decay_chunks(max_step_tokens)
+
+
 def decayed_attention(rows: GemmOut, at_q: int, at_k: int, at_v: int, log_decay: torch.Tensor, state: torch.Tensor, out: torch.Tensor, ctx,
                       dim: int, scratch: dict[str, torch.Tensor] | None, heads_per_key: int = 1, v_scale: torch.Tensor | None = None,
                       out_scale: float = 1.0, impl: str | None = None) -> None:

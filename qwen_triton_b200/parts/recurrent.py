@@ -175,6 +175,24 @@ class GatedDeltaRule:
         return DeferredProduct(self.o, normed) if self.o.fusable(tokens) else self.o(normed)
 
 
+def _declare_decay_scratch(mixer, per_channel: bool) -> None:
+    """Scratch of the chunked recurrence, shared by the layers."""
+    sizes = kernels.decay_scratch(mixer.runtime.max_step_tokens, mixer.heads, mixer.dim, mixer.vdim, per_channel)
+    mixer.scratch_sizes = {f"decayed.{name}": numel for name, numel in sizes.items()}
+    for name, numel in mixer.scratch_sizes.items():
+        mixer.runtime.workspace.declare(name, numel, torch.float32)
+
+
+def _decay_scratch_views(mixer) -> dict:
+    return {name.split(".", 1)[1]: mixer.runtime.workspace.view(name, numel) for name, numel in mixer.scratch_sizes.items()}
+
+
+def _log_decays(values: list[float], runtime: Runtime) -> torch.Tensor:
+    """[tokens of a step, heads]: the logarithms of decays that are the same for every token, formed in double."""
+    logs = torch.tensor(values, dtype=torch.float64).log().to(torch.float32)
+    return logs.to(runtime.device).expand(runtime.max_step_tokens, len(values)).contiguous()
+
+
 @register_mixer("linear_attention")
 class LinearAttention:
     """Linear attention with a constant decay per head ("lightning attention"):
@@ -186,7 +204,7 @@ class LinearAttention:
     elements, ``eps`` inside the root) with a weight of that size, multiplied by sigmoid(W_g h) (``gate``) and projected by
     W_o.  Per sequence the mixer keeps the states, float, zero for a new sequence, in the cache's per-slot state rows
     (stored transposed, [heads, vdim, dim]).  The four projections of h run as one product with float sums; SiLU, the
-    recurrence, the norm and the gate are float (``csrc/linear_attention.cu``).
+    recurrence, the norm and the gate are float (``csrc/linear_attention.cu``, ``csrc/linear_attention_chunk.cu``).
 
     Parameters: ``hidden_size``, ``num_heads``, ``head_dim``, ``v_head_dim``, ``decay`` (one number per head), ``eps``,
     ``activation``, ``gate``, ``float_out``, ``init_std``, and the tensor-name pieces ``q``, ``k``, ``v``, ``g``, ``o``, ``norm``,
@@ -226,7 +244,11 @@ class LinearAttention:
         ws.declare("linattn.read", runtime.max_step_tokens * self.heads * self.vdim, torch.float32)
         ws.declare("linattn.qkv", runtime.max_step_tokens * self.at_gate, torch.float32)
         ws.declare("linattn.normed", runtime.max_step_tokens * self.heads * self.vdim, runtime.dtype)
-        self.norm = None
+        # long portions run in chunks, which work with the decays' logarithms: decays above 0 and at most 1
+        self.chunked = all(0.0 < d <= 1.0 for d in decay)
+        if self.chunked:
+            _declare_decay_scratch(self, per_channel=False)
+        self.norm = self.log_decay = None
 
     @staticmethod
     def _names(params, prefix: str) -> dict[str, str]:
@@ -259,6 +281,8 @@ class LinearAttention:
         self.o.set_weight(source(n["o"]))
         self.norm = to_device(source(n["norm"]), torch.float32, device)
         self.decay = torch.tensor(self.decay_values, dtype=torch.float32, device=device)
+        if self.chunked:
+            self.log_decay = _log_decays(self.decay_values, self.runtime)
 
     def cache_request(self):
         return StateRequest((self.heads, self.vdim, self.dim), torch.float32)
@@ -272,7 +296,11 @@ class LinearAttention:
         read = ws.view("linattn.read", tokens, self.heads, self.vdim)
         # q, k and v are summed and activated once, not by every block of the recurrence that reads them
         ready = kernels.linear_attention_prepare(proj, self.at_gate, ws.view("linattn.qkv", tokens, self.at_gate), self.act)
-        kernels.linear_attention_scan(ready, 0, self.at_k, self.at_v, self.decay, cache.state, read, ctx, self.dim, False)
+        if self.chunked and kernels.decay_chunks_pay(ctx, tokens, self.dim, self.runtime.max_step_tokens):
+            kernels.decayed_attention(ready, 0, self.at_k, self.at_v, self.log_decay[:tokens], cache.state, read, ctx, self.dim,
+                                      _decay_scratch_views(self), impl="chunks")
+        else:
+            kernels.linear_attention_scan(ready, 0, self.at_k, self.at_v, self.decay, cache.state, read, ctx, self.dim, False)
         normed = ws.view("linattn.normed", tokens, self.heads * self.vdim)
         kernels.group_gate_norm(read.view(tokens, self.heads * self.vdim), self.norm, self.eps, normed, proj=proj if self.gated else None, at_gate=self.at_gate)
         return self.o(normed)
@@ -285,14 +313,9 @@ class _DecayedMixer:
 
     def _declare_scratch(self, per_channel: bool) -> None:
         ws, tokens = self.runtime.workspace, self.runtime.max_step_tokens
-        self._scratch = {f"decayed.{name}": numel for name, numel in kernels.decay_scratch(tokens, self.heads, self.dim, self.vdim, per_channel).items()}
-        for name, numel in self._scratch.items():
-            ws.declare(name, numel, torch.float32)
+        _declare_decay_scratch(self, per_channel)
         ws.declare("decayed.read", tokens * self.heads * self.vdim, torch.float32)
         ws.declare("decayed.normed", tokens * self.heads * self.vdim, self.runtime.dtype)
-
-    def _scratch_views(self) -> dict:
-        return {name.split(".", 1)[1]: self.runtime.workspace.view(name, numel) for name, numel in self._scratch.items()}
 
     def _check(self, states) -> None:
         if not states.writable:
@@ -394,7 +417,7 @@ class GatedLinearAttention(_DecayedMixer):
         # split sums are added once, not by every block of the recurrence that reads them
         rows = proj if proj.n_splits == 1 else kernels.linear_attention_prepare(proj, self.at_gate, ws.view("gla.qkv", tokens, self.at_gate), False)
         read = ws.view("decayed.read", tokens, self.heads, self.vdim)
-        kernels.decayed_attention(rows, 0, self.at_k, self.at_v, decay, cache.state, read, ctx, self.dim, self._scratch_views(),
+        kernels.decayed_attention(rows, 0, self.at_k, self.at_v, decay, cache.state, read, ctx, self.dim, _decay_scratch_views(self),
                                   out_scale=self.dim ** -0.5)
         normed = ws.view("decayed.normed", tokens, width)
         kernels.group_gate_norm(read.view(tokens, width), self.norm, self.eps, normed, groups=self.heads, proj=proj, at_gate=self.at_gate, gate="silu")
@@ -472,9 +495,7 @@ class Retention(_DecayedMixer):
         self.proj.set_weight(torch.cat(rows, dim=0))
         self.o.set_weight(source(n["o"]))
         self.norm = torch.ones(self.vdim, dtype=torch.float32, device=device)
-        # the logarithms, formed in double, for as many tokens as a step may have
-        logs = torch.tensor(self.decay_values, dtype=torch.float64).log().to(torch.float32)
-        self.log_decay = logs.to(device).expand(self.runtime.max_step_tokens, self.heads).contiguous()
+        self.log_decay = _log_decays(self.decay_values, self.runtime)
         tables = self.runtime.options.setdefault("position_tables", {})
         key = self.position.key() + (self.runtime.max_positions,)
         if key not in tables:
@@ -495,7 +516,7 @@ class Retention(_DecayedMixer):
         else:
             rows = proj if proj.n_splits == 1 else kernels.linear_attention_prepare(proj, self.at_gate, ws.view("retention.qkv", tokens, self.at_gate), False)
         read = ws.view("decayed.read", tokens, self.heads, self.vdim)
-        kernels.decayed_attention(rows, 0, self.at_k, self.at_v, self.log_decay[:tokens], cache.state, read, ctx, self.dim, self._scratch_views(),
+        kernels.decayed_attention(rows, 0, self.at_k, self.at_v, self.log_decay[:tokens], cache.state, read, ctx, self.dim, _decay_scratch_views(self),
                                   out_scale=self.dim ** -0.5)
         normed = ws.view("decayed.normed", tokens, width)
         kernels.group_gate_norm(read.view(tokens, width), self.norm, self.eps, normed, groups=self.heads, proj=proj, at_gate=self.at_gate, gate="silu")
@@ -599,7 +620,7 @@ class StateSpace(_DecayedMixer):
         read = ws.view("decayed.read", tokens, self.heads, self.vdim)
         at_b, at_c = self.inner, self.inner + self.groups * self.dim
         kernels.decayed_attention(GemmOut(mixed.view(1, tokens, self.channels)), at_c, at_b, 0, decay, states.state, read, ctx, self.dim,
-                                  self._scratch_views(), heads_per_key=self.heads // self.groups, v_scale=step)
+                                  _decay_scratch_views(self), heads_per_key=self.heads // self.groups, v_scale=step)
         normed = ws.view("decayed.normed", tokens, self.inner)
         kernels.group_gate_norm(read.view(tokens, self.inner), self.norm, self.eps, normed, groups=self.norm_groups, proj=proj, at_gate=0, gate="silu",
                                 gate_first=True, x=mixed, at_x=0, skip=self.skip)

@@ -425,6 +425,40 @@ def test_linear_attention_with_a_decay_per_head_in_portions(heads, dim, vdim):
         torch.testing.assert_close(out.float().cpu().double(), wanted, atol=1e-4 if store == torch.float32 else 3e-2, rtol=1e-2)
 
 
+@pytest.mark.parametrize("heads, dim, vdim, decay", [(3, 64, 40, [0.5, 1.0, 0.9961]), (2, 36, 33, [1e-30, 0.25]), (2, 128, 128, [0.999, 0.0])])
+def test_long_portions_in_chunks_follow_the_token_by_token_walk(heads, dim, vdim, decay):
+    """The mixer at and around the length from which it runs in chunks (64 tokens, 1,024 of up to 64 key channels; never with a decay of 0), with
+    sequences that end on, before and behind a chunk's edge and a state left by the portion before, against 64 bits: both forms round
+    in 32 bits, so nothing may be off by more than 2e-5 of the largest value (a few hundred additions of 2^-24 each)."""
+    from qwen_triton_b200.parts.base import Runtime, Workspace
+    from qwen_triton_b200.parts.recurrent import LinearAttention
+    torch.manual_seed(dim)
+    runtime = Runtime(device=torch.device(DEV), dtype=torch.float32, max_step_tokens=2048, max_positions=64, workspace=Workspace(torch.device(DEV)))
+    mixer = LinearAttention({"hidden_size": 32, "num_heads": heads, "head_dim": dim, "v_head_dim": vdim, "decay": decay, "gate": False}, "m", runtime)
+    tensors = {name: torch.randn(*spec.shape) * 0.3 for name, spec in LinearAttention.expected_tensors(mixer.params, "m").items()}
+    tensors["m.norm"] = torch.ones(heads * vdim)
+    mixer.load(lambda name: tensors[name])
+    runtime.workspace.allocate()
+    assert mixer.chunked == (min(decay) > 0)
+    edge = 64 if dim > 64 else 1024
+    cache = type("View", (), {})()
+    cache.writable, cache.state = True, torch.zeros(4, heads, vdim, dim, device=DEV)
+    portions = ([edge, 64, 1], [edge - 1, 65, 127], [2, edge + 63, 128])
+    xs = [torch.randn(sum(p[s] for p in portions), 32) for s in range(3)]
+    want = []
+    for x in xs:
+        q, k, v = (plain.silu(x.double() @ tensors[f"m.{n}.weight"].double().T).view(len(x), heads, -1) for n in ("q", "k", "v"))
+        o = plain.decayed_linear_attention(q, k, v, torch.tensor(decay).double()).reshape(len(x), -1)
+        want.append(plain.rms_divide(o, 1e-6) @ tensors["m.o.weight"].double().T)
+    done = [0, 0, 0]
+    for counts in portions:
+        step = _Step(counts, done, [2, 0, 1])
+        got = mixer.forward(torch.cat([x[d:d + c] for x, d, c in zip(xs, done, counts)]).to(DEV), step, cache).value().cpu().double()
+        wanted = torch.cat([w[d:d + c] for w, d, c in zip(want, done, counts)])
+        assert float((got - wanted).abs().max()) < 2e-5 * float(wanted.abs().max())
+        done = [d + c for d, c in zip(done, counts)]
+
+
 @pytest.mark.parametrize("splits", [1, 3])
 @pytest.mark.parametrize("tokens, width", [(1, 2048), (3, 4096), (255, 2050), (1, 8193)])
 def test_norm_and_gate_of_wide_rows_in_short_steps(tokens, width, splits):
