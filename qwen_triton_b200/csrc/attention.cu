@@ -69,7 +69,7 @@ template <typename T, int DMAX>
 __global__ void __launch_bounds__(PF_WARPS * 32) attention_prefill_kernel(const AttnParams p) {
     pdl_launch_dependents();
     pdl_wait();
-    extern __shared__ float smem[];
+    extern __shared__ __align__(16) float smem[];
     const int d = p.d, dv = p.dv;
     const int kstride = d + 1;
     float* qs = smem;                         // [PF_BQ][d]
@@ -196,6 +196,230 @@ static int launch_prefill(const AttnParams& p, int max_q_len, cudaStream_t strea
     return QT_OK;
 }
 
+// ----------------------------------------------------------------------------- many tokens per sequence, 32-bit rows of whole 16-byte pieces
+// Heads of up to 128 elements, d, dv and value rows multiples of 4, 16-byte aligned operands; everything else as above.
+// grid (tiles of 32 queries, heads, sequences), the longest tiles first; 128 threads, tiles of 64 keys, two blocks an SM.
+// Bound by the FMA pipe and by reads of shared memory.  A warp owns 8 query rows in both products: in q k^T lane (half, t) holds rows
+// 2 warp + half + 8 i against keys t + 16 j (16 results, fma.rn.f32x2 along d, rows 4 floats apart so that neither operand's reads collide), in
+// P V it holds four value columns of all 8 rows.  So the softmax and P stay within the warp, and the block meets only where a
+// tile's keys or values change: the next keys arrive (cp.async) under P V, the next values under q k^T.
+// Prompts of 333 and 216 tokens, 16 heads of 128 on 8 key heads: 69 us against 202 us of the kernel above, which reads
+// shared memory once per multiply-add.
+constexpr int AF_BQ = 32, AF_BK = 64, AF_THREADS = 128;
+
+__device__ __forceinline__ unsigned long long af_fma2(unsigned long long a, unsigned long long b, unsigned long long c) {
+    unsigned long long r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+__device__ __forceinline__ unsigned long long af_pair(float a, float b) {
+    unsigned long long r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ float2 af_halves(unsigned long long v) {
+    float2 r;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+    return r;
+}
+__device__ __forceinline__ void af_copy16(float* to, const float* from, bool there) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(to)), "l"(from), "r"(there ? 16 : 0) : "memory");
+}
+
+__global__ void __launch_bounds__(AF_THREADS, 2) attention_prefill_f32_kernel(const AttnParams p) {
+    pdl_launch_dependents();
+    pdl_wait();
+    extern __shared__ __align__(16) float smem[];
+    const int d = p.d, dv = p.dv, row = d + 4;
+    float* qs = smem;                         // [AF_BQ][row]
+    float* ks = qs + AF_BQ * row;             // [AF_BK][row]
+    float* vs = ks + AF_BK * row;             // [AF_BK][dv]
+    float* ps = vs + AF_BK * dv;              // [AF_BQ][AF_BK + 4]
+    constexpr int PROW = AF_BK + 4;
+
+    const int seq = blockIdx.z, head = blockIdx.y;
+    const int q_begin = p.seq_start[seq], q_len = p.seq_start[seq + 1] - q_begin;
+    const int q0 = (gridDim.x - 1 - blockIdx.x) * AF_BQ;
+    if (q0 >= q_len) return;
+    const int rows = min(AF_BQ, q_len - q0), past = p.seq_past[seq];
+    const int kvh = head / (p.nq / p.nkv), vh = kvh % p.nv;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, half = lane >> 4, tk = lane & 15;
+    const int* table = p.block_table + (size_t)seq * p.max_blocks;
+    const float* q = (const float*)p.q;
+    const float* kc = (const float*)p.k_cache;
+    const float* vc = (const float*)p.v_cache;
+    const bool penalised = p.r1 != nullptr;
+    const float r1 = penalised ? p.r1[head] : 0.f, r2 = penalised ? (p.r2 ? p.r2[head] : -1.f) : 0.f;
+
+    const int p_first = past + q0, p_last = past + q0 + rows - 1;
+    int key_lo = p.window > 0 ? max(0, p_first - p.window + 1) : 0;
+    if (p.chunk > 0) key_lo = max(key_lo, p_first / p.chunk * p.chunk);
+    // two ranges of keys: the kept first ones that lie before the window of the block's first row, then the window
+    const int keep_end = (p.window > 0 && p.keep_first > 0) ? min(p.keep_first, key_lo) : 0;
+    const int kept_tiles = (keep_end + AF_BK - 1) / AF_BK, tiles = kept_tiles + (p_last + 1 - key_lo + AF_BK - 1) / AF_BK;
+    auto tile_first = [&](int t) { return t < kept_tiles ? t * AF_BK : key_lo + (t - kept_tiles) * AF_BK; };
+    auto tile_end = [&](int t) { return t < kept_tiles ? keep_end : p_last + 1; };
+    auto fetch = [&](int t, const float* cache, float* to, int to_row, int width, int row_elems, int heads, int h) {
+        // a warp copies rows warp, warp + 4, ..; their places are looked up side by side, one a lane, and handed round
+        constexpr int PER = AF_BK / (AF_THREADS / 32);
+        const int k0 = tile_first(t) + warp, hi = tile_end(t), pieces = width >> 2;
+        unsigned long long place = 0;
+        if (lane < PER && k0 + 4 * lane < hi) place = cache_offset(table, k0 + 4 * lane, p.ring_tokens, p.page_tokens, heads, h, row_elems);
+#pragma unroll
+        for (int i = 0; i < PER; ++i) {
+            const float* from = cache + __shfl_sync(0xffffffffu, place, i);
+            const bool there = k0 + 4 * i < hi;
+            if (lane < pieces) af_copy16(to + (warp + 4 * i) * to_row + 4 * lane, from + (there ? 4 * lane : 0), there);
+        }
+    };
+    auto fetch_k = [&](int t) { if (t < tiles) fetch(t, kc, ks, row, d, d, p.nkv, kvh); asm volatile("cp.async.commit_group;" ::: "memory"); };
+    auto fetch_v = [&](int t) { if (t < tiles) fetch(t, vc, vs, dv, dv, p.v_row, p.nv, vh); asm volatile("cp.async.commit_group;" ::: "memory"); };
+    fetch_k(0);
+    fetch_v(0);
+    for (int r = warp; r < AF_BQ; r += AF_THREADS / 32)
+        for (int c = lane; c < d; c += 32) qs[r * row + c] = r < rows ? q[((size_t)(q_begin + q0 + r) * p.nq + head) * d + c] * p.scale : 0.f;
+
+    // row i of this thread's four: 2 warp + half + 8 i; row (h, i) of the warp's eight in P V: 2 warp + h + 8 i
+    float m[4], l[4];
+    unsigned long long acc[8][2];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) { m[i] = -INFINITY; l[i] = 0.f; }
+#pragma unroll
+    for (int i = 0; i < 8; ++i) acc[i][0] = acc[i][1] = 0ull;
+
+    for (int t = 0; t < tiles; ++t) {
+        const int k0 = tile_first(t), hi = tile_end(t);
+        asm volatile("cp.async.wait_group 1;" ::: "memory");               // this tile's keys
+        __syncthreads();
+        unsigned long long part[4][4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+            for (int j = 0; j < 4; ++j) part[i][j] = 0ull;
+        const float* qr = qs + (2 * warp + half) * row;
+        const float* kr = ks + tk * row;
+#pragma unroll 2
+        for (int c = 0; c < d; c += 4) {
+            ulonglong2 a[4], b[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) a[i] = *reinterpret_cast<const ulonglong2*>(qr + 8 * i * row + c);
+#pragma unroll
+            for (int j = 0; j < 4; ++j) b[j] = *reinterpret_cast<const ulonglong2*>(kr + 16 * j * row + c);
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+#pragma unroll
+                for (int j = 0; j < 4; ++j) part[i][j] = af_fma2(a[i].y, b[j].y, af_fma2(a[i].x, b[j].x, part[i][j]));
+        }
+        float alpha[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const int r = 2 * warp + half + 8 * i, pos = past + q0 + r;
+            float s[4];
+            float top = -INFINITY;
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const int key = k0 + tk + 16 * j;
+                const float2 both = af_halves(part[i][j]);
+                float x = both.x + both.y;
+                if (p.softcap > 0.f) x = p.softcap * tanhf(x / p.softcap);
+                const bool visible = r < rows && key < hi && key <= pos && (p.window <= 0 || key > pos - p.window || key < p.keep_first) &&
+                                     (p.chunk <= 0 || key >= pos / p.chunk * p.chunk);
+                if (penalised && visible) x -= distance_penalty(r1, r2, pos - key);
+                s[j] = visible ? x : -INFINITY;
+                top = fmaxf(top, s[j]);
+            }
+#pragma unroll
+            for (int off = 8; off > 0; off >>= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, off));
+            const float m_new = fmaxf(m[i], top), m_use = m_new == -INFINITY ? 0.f : m_new;
+            float sum = 0.f;
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const float e = s[j] == -INFINITY ? 0.f : expf(s[j] - m_use);
+                sum += e;
+                ps[r * PROW + tk + 16 * j] = e;
+            }
+#pragma unroll
+            for (int off = 8; off > 0; off >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, off);
+            alpha[i] = expf(m[i] - m_use);                                  // m[i] = -inf gives 0, and nothing is accumulated yet
+            l[i] = l[i] * alpha[i] + sum;
+            m[i] = m_new;
+        }
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const float f = __shfl_sync(0xffffffffu, alpha[i], h * 16);
+                const unsigned long long ff = af_pair(f, f);
+                acc[4 * h + i][0] = af_fma2(acc[4 * h + i][0], ff, 0ull);
+                acc[4 * h + i][1] = af_fma2(acc[4 * h + i][1], ff, 0ull);
+            }
+        __syncthreads();                                                    // the keys are read
+        fetch_k(t + 1);
+        asm volatile("cp.async.wait_group 1;" ::: "memory");               // this tile's values
+        __syncthreads();
+        if (4 * lane < dv) {
+            const int keys = min(AF_BK, (hi - k0 + 3) & ~3);                // whole fours; what lies behind has weight 0 and value 0
+            for (int kk = 0; kk < keys; kk += 4) {
+                ulonglong2 v[4];
+#pragma unroll
+                for (int u = 0; u < 4; ++u) v[u] = *reinterpret_cast<const ulonglong2*>(vs + (kk + u) * dv + 4 * lane);
+#pragma unroll
+                for (int h = 0; h < 2; ++h)
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) {
+                        const float4 w = *reinterpret_cast<const float4*>(ps + (2 * warp + h + 8 * i) * PROW + kk);
+                        const float wv[4] = {w.x, w.y, w.z, w.w};
+#pragma unroll
+                        for (int u = 0; u < 4; ++u) {
+                            const unsigned long long ww = af_pair(wv[u], wv[u]);
+                            acc[4 * h + i][0] = af_fma2(ww, v[u].x, acc[4 * h + i][0]);
+                            acc[4 * h + i][1] = af_fma2(ww, v[u].y, acc[4 * h + i][1]);
+                        }
+                    }
+            }
+        }
+        __syncthreads();                                                    // the values are read
+        fetch_v(t + 1);
+    }
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    float* out = (float*)p.out;
+    float inv[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        float factor = 1.f;
+        if (p.sink) with_sink(m[i], l[i], factor, p.sinks ? p.sinks[head] : 0.f);
+        inv[i] = factor / l[i];
+    }
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const float f = __shfl_sync(0xffffffffu, inv[i], h * 16);
+            const int r = 2 * warp + h + 8 * i;
+            const float2 a = af_halves(acc[4 * h + i][0]), b = af_halves(acc[4 * h + i][1]);
+            if (r < rows && 4 * lane < dv)
+                *reinterpret_cast<float4*>(out + ((size_t)(q_begin + q0 + r) * p.nq + head) * dv + 4 * lane) = make_float4(a.x * f, a.y * f, b.x * f, b.y * f);
+        }
+}
+
+static bool prefill_f32_fits(const AttnParams& p) {
+    return p.d <= 128 && p.dv <= 128 && p.d % 4 == 0 && p.dv % 4 == 0 && p.v_row % 4 == 0 &&
+           (((uintptr_t)p.k_cache | (uintptr_t)p.v_cache | (uintptr_t)p.out) & 15) == 0;
+}
+
+static int launch_prefill_f32(const AttnParams& p, int max_q_len, cudaStream_t stream) {
+    const size_t smem = ((size_t)(AF_BQ + AF_BK) * (p.d + 4) + (size_t)AF_BK * p.dv + (size_t)AF_BQ * (AF_BK + 4)) * sizeof(float);
+    static bool configured = false;
+    if (!configured) {
+        cudaError_t err = cudaFuncSetAttribute(attention_prefill_f32_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 100 * 1024);
+        if (err != cudaSuccess) QT_FAIL(QT_ERR_LAUNCH, "attention_prefill: cannot raise shared memory: %s", cudaGetErrorString(err));
+        configured = true;
+    }
+    launch_kernel(attention_prefill_f32_kernel, dim3((max_q_len + AF_BQ - 1) / AF_BQ, p.nq, p.n_seqs), dim3(AF_THREADS), smem, stream, p);
+    QT_CHECK_LAUNCH("attention_prefill");
+    return QT_OK;
+}
+
 static int check_common(const char* name, int n_seqs, int nq, int nkv, int d, int dv, const float* r1, const float* r2, int page_tokens,
                         int ring_tokens, int window, int chunk, int nv, int keep_first, int v_row) {
     QT_REQUIRE(keep_first >= 0 && (keep_first == 0 || ring_tokens == 0), "%s: kept first keys (%d) do not go with a ring of %d tokens", name, keep_first, ring_tokens);
@@ -224,6 +448,7 @@ extern "C" int qt_attention_prefill(const void* q, const void* k_cache, const vo
     AttnParams p{q, k_cache, v_cache, out, block_table, max_blocks, seq_start, seq_past, n_seqs, nq, nkv, d, page_tokens, ring_tokens, window, scale,
                  dv, r1, r2, chunk, nv, keep_first, sink, v_row, sinks, softcap};
     cudaStream_t s = (cudaStream_t)stream;
+    if (dtype == QT_F32 && prefill_f32_fits(p)) return launch_prefill_f32(p, max_q_len, s);
     return QT_DISPATCH_DTYPE(dtype, "attention_prefill", {
         if (dv <= 64) return launch_prefill<T, 64>(p, max_q_len, s);
         if (dv <= 128) return launch_prefill<T, 128>(p, max_q_len, s);
@@ -237,7 +462,9 @@ extern "C" int qt_attention_prefill(const void* q, const void* k_cache, const vo
 // kv head over the keys [lo + split * chunk, lo + (split + 1) * chunk) of its sequence, where
 // [lo, len) is the visible range.  QK: one key per lane.  PV: one column group per lane.
 // The partial result (max, sum, unnormalised accumulator) goes to scratch; the combine kernel
-// merges the splits.  With one split the block writes the output itself.
+// merges the splits.  With one split the block writes the output itself.  Bound by the latency of its loads: a lane asks for eight
+// pieces of its key, and the warp for eight keys' values, before it uses the first (2 sequences of 333 and 216 tokens, 16 heads of 128
+// in 32 bits: 36 us with one element of a key and one value's place looked up at a time, 20 us so).
 constexpr int DEC_WARPS = 4;
 
 struct DecodeParams {
@@ -246,14 +473,22 @@ struct DecodeParams {
     int n_splits;
     float* part_acc;      // [B, nq, n_splits, dv]
     float* part_ml;       // [B, nq, n_splits, 2]
+    int fours;            // keys are read four elements at a time: d a multiple of 4, the cache 16-byte aligned
 };
+
+__device__ __forceinline__ float4 load_four(const float* p) { return *reinterpret_cast<const float4*>(p); }
+__device__ __forceinline__ float4 load_four(const __nv_bfloat16* p) {
+    const uint2 raw = *reinterpret_cast<const uint2*>(p);
+    const __nv_bfloat162 a = reinterpret_cast<const __nv_bfloat162&>(raw.x), b = reinterpret_cast<const __nv_bfloat162&>(raw.y);
+    return make_float4(__low2float(a), __high2float(a), __low2float(b), __high2float(b));
+}
 
 template <typename T, int DMAX, int DEC_HEADS>
 __global__ void __launch_bounds__(DEC_WARPS * 32) attention_decode_kernel(const DecodeParams dp) {
     pdl_launch_dependents();
     pdl_wait();
     const AttnParams& p = dp.a;
-    extern __shared__ float smem[];
+    extern __shared__ __align__(16) float smem[];
     const int d = p.d, dv = p.dv;
     const int group = p.nq / p.nkv;
     const int chunks_per_kv = (group + DEC_HEADS - 1) / DEC_HEADS;
@@ -313,10 +548,29 @@ __global__ void __launch_bounds__(DEC_WARPS * 32) attention_decode_kernel(const 
         for (int h = 0; h < DEC_HEADS; ++h) s[h] = 0.f;
         if (valid) {
             const T* krow = kc + cache_offset(table, key, p.ring_tokens, p.page_tokens, p.nkv, kvh, d);
-            for (int c = 0; c < d; ++c) {
-                const float kv = to_float(krow[c]);
+            if (dp.fours) {
+                constexpr int AHEAD = 8;                    // pieces of the key asked for before the first is used
+                for (int c0 = 0; c0 < d; c0 += 4 * AHEAD) {
+                    float4 kv[AHEAD];
 #pragma unroll
-                for (int h = 0; h < DEC_HEADS; ++h) s[h] += qs[h * d + c] * kv;
+                    for (int u = 0; u < AHEAD; ++u)
+                        if (c0 + 4 * u < d) kv[u] = load_four(krow + c0 + 4 * u);
+#pragma unroll
+                    for (int u = 0; u < AHEAD; ++u)
+                        if (c0 + 4 * u < d) {
+#pragma unroll
+                            for (int h = 0; h < DEC_HEADS; ++h) {
+                                const float4 x = *reinterpret_cast<const float4*>(qs + h * d + c0 + 4 * u);
+                                s[h] += x.x * kv[u].x; s[h] += x.y * kv[u].y; s[h] += x.z * kv[u].z; s[h] += x.w * kv[u].w;
+                            }
+                        }
+                }
+            } else {
+                for (int c = 0; c < d; ++c) {
+                    const float kv = to_float(krow[c]);
+#pragma unroll
+                    for (int h = 0; h < DEC_HEADS; ++h) s[h] += qs[h * d + c] * kv;
+                }
             }
             if (p.softcap > 0.f) {
 #pragma unroll
@@ -339,21 +593,29 @@ __global__ void __launch_bounds__(DEC_WARPS * 32) attention_decode_kernel(const 
 #pragma unroll
             for (int j = 0; j < DMAX / 32; ++j) acc[h][j] *= alpha;
         }
+        // every lane knows where its key's value lies; VALUES_AHEAD of them are asked for before the first is used
         const int n_keys = min(32, k_end - k0);
-        for (int kk = 0; kk < n_keys; ++kk) {
-            const T* vrow = vc + cache_offset(table, k0 + kk < keep_end ? k0 + kk : k0 + kk + gap, p.ring_tokens, p.page_tokens, p.nv, vh, p.v_row);
-            float v[DMAX / 32];
+        const unsigned long long mine = valid ? cache_offset(table, key, p.ring_tokens, p.page_tokens, p.nv, vh, p.v_row) : 0;
+        constexpr int VALUES_AHEAD = DMAX <= 128 ? 8 : DMAX <= 256 ? 4 : 1;
+        for (int kk = 0; kk < n_keys; kk += VALUES_AHEAD) {
+            float v[VALUES_AHEAD][DMAX / 32];
 #pragma unroll
-            for (int j = 0; j < DMAX / 32; ++j) {
-                const int c = lane + 32 * j;
-                v[j] = c < dv ? to_float(vrow[c]) : 0.f;
+            for (int u = 0; u < VALUES_AHEAD; ++u) {
+                const T* vrow = vc + __shfl_sync(0xffffffffu, mine, kk + u);
+#pragma unroll
+                for (int j = 0; j < DMAX / 32; ++j) {
+                    const int c = lane + 32 * j;
+                    v[u][j] = c < dv && kk + u < n_keys ? to_float(vrow[c]) : 0.f;
+                }
             }
 #pragma unroll
-            for (int h = 0; h < DEC_HEADS; ++h) {
-                const float w = __shfl_sync(0xffffffffu, e[h], kk);
+            for (int u = 0; u < VALUES_AHEAD; ++u)
 #pragma unroll
-                for (int j = 0; j < DMAX / 32; ++j) acc[h][j] += w * v[j];
-            }
+                for (int h = 0; h < DEC_HEADS; ++h) {
+                    const float w = __shfl_sync(0xffffffffu, e[h], kk + u);    // 0 for keys beyond the range
+#pragma unroll
+                    for (int j = 0; j < DMAX / 32; ++j) acc[h][j] += w * v[u][j];
+                }
         }
     }
 
@@ -465,7 +727,7 @@ extern "C" int qt_attention_decode(const void* q, const void* k_cache, const voi
     QT_REQUIRE(n_seqs <= 65535, "attention_decode: too many sequences for one launch");
     DecodeParams dp{{q, k_cache, v_cache, out, block_table, max_blocks, nullptr, nullptr, n_seqs, nq, nkv, d, page_tokens, ring_tokens, window, scale,
                      dv, r1, r2, chunk, nv, keep_first, sink, v_row, sinks, softcap},
-                    seq_len, n_splits, part_acc, part_ml};
+                    seq_len, n_splits, part_acc, part_ml, d % 4 == 0 && ((uintptr_t)k_cache & 15) == 0};
     cudaStream_t s = (cudaStream_t)stream;
     return QT_DISPATCH_DTYPE(dtype, "attention_decode", {
         if (dv <= 64) return launch_decode<T, 64>(dp, s);

@@ -258,6 +258,54 @@ def test_attention_prefill(dtype, nq, nkv, d, window, ring):
             start += n
 
 
+@pytest.mark.parametrize("d, dv, nq, nkv, nv", [(4, 4, 2, 1, 1), (36, 128, 4, 2, 1), (128, 60, 3, 3, 3), (128, 128, 8, 2, 2), (132, 64, 2, 2, 2), (30, 30, 2, 1, 1)])
+@pytest.mark.parametrize("window, keep_first, chunk, options", [(None, 0, None, ""), (40, 0, None, "sinks"), (33, 70, None, "penalty"), (None, 0, 50, "softcap")])
+def test_attention_prefill_float32_at_the_edges_of_its_tiles(d, dv, nq, nkv, nv, window, keep_first, chunk, options):
+    """Tiles of 32 queries and 64 keys: lengths on, before and behind both, with and without keys from before, every mask and score
+    option; heads that the tiled kernel takes and (132, 30) that it does not.  Bound: exponents and sums of up to 200 terms of the values'
+    size round to about 1e-6; 1e-5 with the logarithm and the hyperbolic tangent."""
+    q_lens, past = [1, 31, 32, 33, 64, 65, 129], [0, 33, 0, 31, 64, 0, 63]
+    totals = [p + n for p, n in zip(past, q_lens)]
+    k = [rand(t, nkv, d, seed=120 + i).cpu() for i, t in enumerate(totals)]
+    v = [rand(t, nv, dv, seed=130 + i).cpu() for i, t in enumerate(totals)]
+    width = -(-max(totals) // PAGE)
+    order = torch.randperm(width * len(totals), generator=gen(9)).view(len(totals), width)
+    k_cache, v_cache = torch.full((order.numel(), nkv, PAGE, d), 1e4), torch.full((order.numel(), nv, PAGE, dv), -1e4)
+    for i, t in enumerate(totals):
+        for at in range(t):
+            k_cache[order[i, at // PAGE], :, at % PAGE], v_cache[order[i, at // PAGE], :, at % PAGE] = k[i][at], v[i][at]
+    q = rand(sum(q_lens), nq, d, seed=140)
+    sinks, penalty = rand(nq, seed=141), (rand(nq, seed=142).abs() * 0.3, rand(nq, seed=143).abs())
+    out = torch.full((sum(q_lens), nq, dv), float("nan"), device=DEV)
+    as_int = lambda values: torch.tensor(values, dtype=torch.int32, device=DEV)
+    kernels.attention_prefill(q, k_cache.to(DEV), v_cache.to(DEV), out, order.int().to(DEV), as_int([sum(q_lens[:i]) for i in range(len(q_lens) + 1)]), as_int(past),
+                              max(q_lens), nkv, PAGE, 0, window, d ** -0.5, chunk=chunk, keep_first=keep_first, v_dim=dv,
+                              sink=options == "sinks", sinks=sinks if options == "sinks" else None, penalty=penalty if options == "penalty" else None,
+                              softcap=2.0 if options == "softcap" else None)
+    start = 0
+    for i, n in enumerate(q_lens):
+        pos, key = torch.arange(past[i], totals[i])[:, None], torch.arange(totals[i])[None]
+        seen = key <= pos
+        if window:
+            seen &= (key > pos - window) | (key < keep_first)
+        if chunk:
+            seen &= key // chunk == pos // chunk
+        keys, values = k[i].double().repeat_interleave(nq // nkv, 1), v[i].double()[:, torch.arange(nkv) % nv].repeat_interleave(nq // nkv, 1)
+        score = torch.einsum("qhd,khd->hqk", q[start:start + n].cpu().double(), keys) * d ** -0.5
+        if options == "softcap":
+            score = 2.0 * torch.tanh(score / 2.0)
+        if options == "penalty":
+            r1, r2 = (t.cpu().double()[:, None, None] for t in penalty)
+            score = score - r1 * torch.log1p(r2 * (pos - key).clamp(min=0))
+        score = score.masked_fill(~seen, float("-inf"))
+        if options == "sinks":
+            score = torch.cat((score, sinks.cpu().double()[:, None, None].expand(nq, n, 1)), dim=-1)
+        weight = score.softmax(-1)[..., :totals[i]]
+        want = torch.einsum("hqk,khd->qhd", weight, values)
+        torch.testing.assert_close(out[start:start + n].cpu().double(), want, atol=1e-5, rtol=1e-5, msg=lambda m: f"sequence {i}: {m}")
+        start += n
+
+
 @pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("nq, nkv, d, window, ring, splits", [
     (6, 2, 80, None, 0, 1), (6, 2, 80, None, 0, 5), (4, 4, 16, 40, 128, 2), (16, 1, 128, None, 0, 3),
