@@ -46,52 +46,25 @@ __device__ __forceinline__ int expert_of(const ExpertParams& p, int t, int k) {
     return e < 0 ? 0 : (e >= p.experts ? p.experts - 1 : e);          // never read outside the weights
 }
 
-// Eight consecutive elements of a weight row as floats, by 16-byte loads (rows that start on 16-byte boundaries).
-__device__ __forceinline__ void load8(const float* src, float (&v)[8]) {
-    const float4 a = reinterpret_cast<const float4*>(src)[0], b = reinterpret_cast<const float4*>(src)[1];
-    v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
-}
-__device__ __forceinline__ void load8(const __nv_bfloat16* src, float (&v)[8]) {
-    const uint4 raw = *reinterpret_cast<const uint4*>(src);
-    const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&raw);
-#pragma unroll
-    for (int j = 0; j < 4; ++j) { v[2 * j] = __low2float(h[j]); v[2 * j + 1] = __high2float(h[j]); }
-}
-
 // EV_FEATS dot products of consecutive weight rows (`stride` apart, `n` elements each) with a vector in shared memory,
-// summed over the warp.  VEC: n is a multiple of 8 and the rows start on 16-byte boundaries; every lane then loads 16
-// bytes of each row per turn, all rows' loads of a turn ahead of its arithmetic.
-template <typename T, bool VEC>
+// summed over the warp, for rows that do not lie on 16-byte boundaries.
+template <typename T>
 __device__ __forceinline__ void warp_dots(const T* __restrict__ w, size_t stride, int rows, int n, const float* __restrict__ xs, int lane,
                                           float (&acc)[EV_FEATS]) {
 #pragma unroll
     for (int j = 0; j < EV_FEATS; ++j) acc[j] = 0.f;
-    if (VEC) {
-        for (int i = lane * 8; i < n; i += 256) {
-            float wv[EV_FEATS][8];
+    for (int i = lane; i < n; i += 32) {
+        const float xv = xs[i];
 #pragma unroll
-            for (int j = 0; j < EV_FEATS; ++j) load8(w + (size_t)(j < rows ? j : 0) * stride + i, wv[j]);
-            const float4 xa = *reinterpret_cast<const float4*>(xs + i), xb = *reinterpret_cast<const float4*>(xs + i + 4);
-            const float xv[8] = {xa.x, xa.y, xa.z, xa.w, xb.x, xb.y, xb.z, xb.w};
-#pragma unroll
-            for (int j = 0; j < EV_FEATS; ++j)
-#pragma unroll
-                for (int e = 0; e < 8; ++e) acc[j] += wv[j][e] * xv[e];
-        }
-    } else {
-        for (int i = lane; i < n; i += 32) {
-            const float xv = xs[i];
-#pragma unroll
-            for (int j = 0; j < EV_FEATS; ++j)
-                if (j < rows) acc[j] += to_float(w[(size_t)j * stride + i]) * xv;
-        }
+        for (int j = 0; j < EV_FEATS; ++j)
+            if (j < rows) acc[j] += to_float(w[(size_t)j * stride + i]) * xv;
     }
 #pragma unroll
     for (int j = 0; j < EV_FEATS; ++j) acc[j] = warp_sum(acc[j]);
 }
 
 // mid[pair, f] = act(W_up[e][f, :] . x[t, :]).  grid (pairs, feature blocks); x[t] in shared memory as float.
-template <typename T, bool VEC>
+template <typename T>
 __global__ void __launch_bounds__(EV_WARPS * 32) expert_up_kernel(const ExpertParams p) {
     pdl_launch_dependents();
     pdl_wait();
@@ -108,10 +81,10 @@ __global__ void __launch_bounds__(EV_WARPS * 32) expert_up_kernel(const ExpertPa
     const int f0 = (blockIdx.y * EV_WARPS + warp) * EV_FEATS;
     if (f0 >= p.ff) return;
     float acc[EV_FEATS];
-    warp_dots<T, VEC>(w + (size_t)f0 * p.width, (size_t)p.width, p.ff - f0, p.width, xs, lane, acc);
+    warp_dots<T>(w + (size_t)f0 * p.width, (size_t)p.width, p.ff - f0, p.width, xs, lane, acc);
     if (p.gated) {
         float up[EV_FEATS];
-        warp_dots<T, VEC>(w + (size_t)(p.ff + f0) * p.width, (size_t)p.width, p.ff - f0, p.width, xs, lane, up);
+        warp_dots<T>(w + (size_t)(p.ff + f0) * p.width, (size_t)p.width, p.ff - f0, p.width, xs, lane, up);
 #pragma unroll
         for (int j = 0; j < EV_FEATS; ++j)
             if (lane == 0 && f0 + j < p.ff) mid[f0 + j] = from_float<T>(gated_value<false>(acc[j], up[j], p.act, p.limit));
@@ -122,8 +95,16 @@ __global__ void __launch_bounds__(EV_WARPS * 32) expert_up_kernel(const ExpertPa
         if (lane == 0 && f0 + j < p.ff) mid[f0 + j] = from_float<T>(gate_activation<false>(acc[j], p.act));
 }
 
+// The result of token t, column c: the weighted sum over its experts, the further term, into out.
+__device__ __forceinline__ void expert_put(const ExpertParams& p, int t, int c, float total) {
+    const size_t at = (size_t)t * p.width + c;
+    float y = p.pair_weights ? total : total * p.pair_weight;
+    if (p.base) y += (p.row_scale ? p.row_scale[t] : 1.f) * load_sum(p.base, at, p.base_splits, p.base_stride);
+    p.out[at] = y;
+}
+
 // out[t, c] = pair_weight * sum_k W_down[e_k][c, :] . mid[t * top + k, :].  grid (tokens, column blocks).
-template <typename T, bool VEC>
+template <typename T>
 __global__ void __launch_bounds__(EV_WARPS * 32) expert_down_kernel(const ExpertParams p) {
     pdl_launch_dependents();
     pdl_wait();
@@ -142,19 +123,164 @@ __global__ void __launch_bounds__(EV_WARPS * 32) expert_down_kernel(const Expert
         const int e = expert_of(p, t, k);
         const T* w = (const T*)p.down + (size_t)e * p.width * p.ff;
         float acc[EV_FEATS];
-        warp_dots<T, VEC>(w + (size_t)c0 * p.ff, (size_t)p.ff, p.width - c0, p.ff, ms + k * p.ff, lane, acc);
+        warp_dots<T>(w + (size_t)c0 * p.ff, (size_t)p.ff, p.width - c0, p.ff, ms + k * p.ff, lane, acc);
         const float weight = p.pair_weights ? p.pair_weights[(size_t)t * p.top + k] : 1.f;
 #pragma unroll
         for (int j = 0; j < EV_FEATS; ++j) total[j] += acc[j] * weight;
     }
 #pragma unroll
     for (int j = 0; j < EV_FEATS; ++j)
-        if (lane == 0 && c0 + j < p.width) {
-            const size_t at = (size_t)t * p.width + c0 + j;
-            float y = p.pair_weights ? total[j] : total[j] * p.pair_weight;
-            if (p.base) y += (p.row_scale ? p.row_scale[t] : 1.f) * load_sum(p.base, at, p.base_splits, p.base_stride);
-            p.out[at] = y;
-        }
+        if (lane == 0 && c0 + j < p.width) expert_put(p, t, c0 + j, total[j]);
+}
+
+// The same two passes for rows that lie on 16-byte boundaries (width and ff multiples of 8).  Bound by the experts' bytes, if enough of
+// them are asked for at once: which expert it is is known only when the router is done, so nothing can be fetched ahead, and a
+// warp that walks its rows 16 bytes a lane and turn waits out the memory once per turn.  A warp takes FEATS features (gate and up
+// rows of each together), a lane asks for EV_BYTES of weights before it uses the first, and the rows of x and mid are read where
+// they lie (a block that stages them makes every weight wait for two more trips and a barrier).  FEATS falls from 4 to 1 with the
+// pairs, so that one token's experts still spread over the machine.
+// Both passes, weights not in L2, before / now: one token of 2 experts of 1,024 x 2,048 33 / 15.5 us, of one of 2,048 x 1,024 26 / 13 us,
+// 8 tokens of one of 8 such experts 30 / 23.6 us, 16 tokens of 2 of 16 experts of 1,024 x 2,048 69 / 61 us.
+constexpr int EV_BYTES = 256;
+
+template <typename T> struct Eight { uint4 raw[sizeof(T) / 2]; };
+template <typename T> __device__ __forceinline__ Eight<T> load_weights(const T* p) {        // read once: past L1
+    Eight<T> r;
+#pragma unroll
+    for (int i = 0; i < (int)(sizeof(T) / 2); ++i)
+        asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0, %1, %2, %3}, [%4];"
+                     : "=r"(r.raw[i].x), "=r"(r.raw[i].y), "=r"(r.raw[i].z), "=r"(r.raw[i].w) : "l"(reinterpret_cast<const uint4*>(p) + i));
+    return r;
+}
+template <typename T> __device__ __forceinline__ Eight<T> load_eight(const T* p) {
+    Eight<T> r;
+#pragma unroll
+    for (int i = 0; i < (int)(sizeof(T) / 2); ++i) r.raw[i] = reinterpret_cast<const uint4*>(p)[i];
+    return r;
+}
+__device__ __forceinline__ void floats_of(const Eight<float>& r, float (&v)[8]) {
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+        v[4 * i] = __uint_as_float(r.raw[i].x); v[4 * i + 1] = __uint_as_float(r.raw[i].y);
+        v[4 * i + 2] = __uint_as_float(r.raw[i].z); v[4 * i + 3] = __uint_as_float(r.raw[i].w);
+    }
+}
+__device__ __forceinline__ void floats_of(const Eight<__nv_bfloat16>& r, float (&v)[8]) {
+    const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&r.raw[0]);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) { v[2 * j] = __low2float(h[j]); v[2 * j + 1] = __high2float(h[j]); }
+}
+
+// acc[j] += this lane's part of row[j] . (x times factor), n elements.
+template <typename T, int ROWS>
+__device__ __forceinline__ void lane_dots(const T* const (&row)[ROWS], const T* __restrict__ x, float factor, int n, int lane, float (&acc)[ROWS]) {
+    constexpr int AT_ONCE = EV_BYTES / (ROWS * 8 * (int)sizeof(T)), TURNS = AT_ONCE < 1 ? 1 : AT_ONCE > 8 ? 8 : AT_ONCE;
+    for (int i0 = lane * 8; i0 < n; i0 += 256 * TURNS) {
+        Eight<T> w[TURNS][ROWS], v[TURNS];
+#pragma unroll
+        for (int u = 0; u < TURNS; ++u)
+            if (i0 + 256 * u < n) {
+#pragma unroll
+                for (int j = 0; j < ROWS; ++j) w[u][j] = load_weights(row[j] + i0 + 256 * u);
+                v[u] = load_eight(x + i0 + 256 * u);
+            }
+#pragma unroll
+        for (int u = 0; u < TURNS; ++u)
+            if (i0 + 256 * u < n) {
+                float xv[8];
+                floats_of(v[u], xv);
+#pragma unroll
+                for (int i = 0; i < 8; ++i) xv[i] *= factor;
+#pragma unroll
+                for (int j = 0; j < ROWS; ++j) {
+                    float wv[8];
+                    floats_of(w[u][j], wv);
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) acc[j] += wv[i] * xv[i];
+                }
+            }
+    }
+}
+
+// grid (pairs, feature blocks)
+template <typename T, int FEATS, bool GATED>
+__global__ void __launch_bounds__(EV_WARPS * 32) expert_up_vec_kernel(const ExpertParams p) {
+    constexpr int ROWS = GATED ? 2 * FEATS : FEATS;
+    pdl_launch_dependents();
+    pdl_wait();
+    const int pair = blockIdx.x, t = pair / p.top, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int f0 = (blockIdx.y * EV_WARPS + warp) * FEATS;
+    if (f0 >= p.ff) return;
+    const T* w = (const T*)p.up + (size_t)expert_of(p, t, pair % p.top) * (GATED ? 2 : 1) * p.ff * p.width;
+    const T* row[ROWS];
+#pragma unroll
+    for (int j = 0; j < FEATS; ++j) {
+        const int f = min(f0 + j, p.ff - 1);
+        row[j] = w + (size_t)f * p.width;
+        if (GATED) row[FEATS + j] = w + (size_t)(p.ff + f) * p.width;
+    }
+    float acc[ROWS] = {};
+    lane_dots<T, ROWS>(row, (const T*)p.x + (size_t)t * p.width, p.in_weights ? p.in_weights[pair] : 1.f, p.width, lane, acc);
+#pragma unroll
+    for (int j = 0; j < ROWS; ++j) acc[j] = warp_sum(acc[j]);
+    T* mid = (T*)p.mid + (size_t)pair * p.ff;
+#pragma unroll
+    for (int j = 0; j < FEATS; ++j)
+        if (lane == j && f0 + j < p.ff)
+            mid[f0 + j] = from_float<T>(GATED ? gated_value<false>(acc[j], acc[GATED ? FEATS + j : j], p.act, p.limit) : gate_activation<false>(acc[j], p.act));
+}
+
+// grid (tokens, column blocks)
+template <typename T, int FEATS>
+__global__ void __launch_bounds__(EV_WARPS * 32) expert_down_vec_kernel(const ExpertParams p) {
+    pdl_launch_dependents();
+    pdl_wait();
+    const int t = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int c0 = (blockIdx.y * EV_WARPS + warp) * FEATS;
+    if (c0 >= p.width) return;
+    float total[FEATS] = {};
+    for (int k = 0; k < p.top; ++k) {                      // in the order of the table's row
+        const T* w = (const T*)p.down + (size_t)expert_of(p, t, k) * p.width * p.ff;
+        const T* row[FEATS];
+#pragma unroll
+        for (int j = 0; j < FEATS; ++j) row[j] = w + (size_t)min(c0 + j, p.width - 1) * p.ff;
+        float acc[FEATS] = {};
+        lane_dots<T, FEATS>(row, (const T*)p.mid + ((size_t)t * p.top + k) * p.ff, 1.f, p.ff, lane, acc);
+        const float weight = p.pair_weights ? p.pair_weights[(size_t)t * p.top + k] : 1.f;
+#pragma unroll
+        for (int j = 0; j < FEATS; ++j) total[j] += acc[j] * weight;
+    }
+#pragma unroll
+    for (int j = 0; j < FEATS; ++j) total[j] = warp_sum(total[j]);
+#pragma unroll
+    for (int j = 0; j < FEATS; ++j)
+        if (lane == j && c0 + j < p.width) expert_put(p, t, c0 + j, total[j]);
+}
+
+// Features a warp takes: the most that still give every SM a block.  4 pairs of 2,048 x 1,024 and 4 features in both passes 25.6 us, 2
+// 27.7 us, 1 31.7 us; one token of 2 such experts 19.5, 17.4 and 15.5 us (both with cold caches, two launches).
+static int feats_for(long long rows, int features) {
+    for (int feats = 4; feats > 1; feats /= 2)
+        if (rows * ((features + EV_WARPS * feats - 1) / (EV_WARPS * feats)) >= sm_count()) return feats;
+    return 1;
+}
+
+template <typename T> static int launch_expert_rows(const ExpertParams& p, cudaStream_t s) {
+    const dim3 block(EV_WARPS * 32);
+    const int pairs = p.n_tokens * p.top;
+    const int fu = feats_for(pairs, p.ff), fd = feats_for(p.n_tokens, p.width);
+    const dim3 up(pairs, (p.ff + EV_WARPS * fu - 1) / (EV_WARPS * fu)), down(p.n_tokens, (p.width + EV_WARPS * fd - 1) / (EV_WARPS * fd));
+#define QT_EXPERT_UP(F) (p.gated ? launch_kernel(expert_up_vec_kernel<T, F, true>, up, block, 0, s, p) : launch_kernel(expert_up_vec_kernel<T, F, false>, up, block, 0, s, p))
+    if (fu == 4) QT_EXPERT_UP(4);
+    else if (fu == 2) QT_EXPERT_UP(2);
+    else QT_EXPERT_UP(1);
+#undef QT_EXPERT_UP
+    QT_CHECK_LAUNCH("expert_up");
+    if (fd == 4) launch_kernel(expert_down_vec_kernel<T, 4>, down, block, 0, s, p);
+    else if (fd == 2) launch_kernel(expert_down_vec_kernel<T, 2>, down, block, 0, s, p);
+    else launch_kernel(expert_down_vec_kernel<T, 1>, down, block, 0, s, p);
+    QT_CHECK_LAUNCH("expert_down");
+    return QT_OK;
 }
 
 static int check_experts(const char* name, int n_tokens, int vocab, int top, int experts, int width, int ff, int act) {
@@ -180,21 +306,13 @@ extern "C" int qt_experts_by_pair(const void* x, const int* token_ids, const int
     return QT_DISPATCH_DTYPE(dtype, "experts_by_pair", {
         const size_t smem_up = (size_t)width * sizeof(float), smem_down = (size_t)top * ff * sizeof(float);
         const dim3 grid_up(n_tokens * top, (ff + per_block - 1) / per_block), grid_down(n_tokens, (width + per_block - 1) / per_block);
-        // 16-byte loads: rows of both weights, and the experts' matrices, start on 16-byte boundaries
-        const bool vec = width % 8 == 0 && ff % 8 == 0 && (uintptr_t)up % 16 == 0 && (uintptr_t)down % 16 == 0;
-        if (vec) {
-            if (smem_up > 48 * 1024) cudaFuncSetAttribute(expert_up_kernel<T, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_up);
-            if (smem_down > 48 * 1024) cudaFuncSetAttribute(expert_down_kernel<T, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_down);
-            launch_kernel(expert_up_kernel<T, true>, grid_up, dim3(EV_WARPS * 32), smem_up, s, p);
-            QT_CHECK_LAUNCH("expert_up");
-            launch_kernel(expert_down_kernel<T, true>, grid_down, dim3(EV_WARPS * 32), smem_down, s, p);
-        } else {
-            if (smem_up > 48 * 1024) cudaFuncSetAttribute(expert_up_kernel<T, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_up);
-            if (smem_down > 48 * 1024) cudaFuncSetAttribute(expert_down_kernel<T, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_down);
-            launch_kernel(expert_up_kernel<T, false>, grid_up, dim3(EV_WARPS * 32), smem_up, s, p);
-            QT_CHECK_LAUNCH("expert_up");
-            launch_kernel(expert_down_kernel<T, false>, grid_down, dim3(EV_WARPS * 32), smem_down, s, p);
-        }
+        // 16-byte loads: rows of both weights, of x and of mid start on 16-byte boundaries
+        if (width % 8 == 0 && ff % 8 == 0 && (((uintptr_t)up | (uintptr_t)down | (uintptr_t)x | (uintptr_t)mid) & 15) == 0) return launch_expert_rows<T>(p, s);
+        if (smem_up > 48 * 1024) cudaFuncSetAttribute(expert_up_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_up);
+        if (smem_down > 48 * 1024) cudaFuncSetAttribute(expert_down_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_down);
+        launch_kernel(expert_up_kernel<T>, grid_up, dim3(EV_WARPS * 32), smem_up, s, p);
+        QT_CHECK_LAUNCH("expert_up");
+        launch_kernel(expert_down_kernel<T>, grid_down, dim3(EV_WARPS * 32), smem_down, s, p);
         QT_CHECK_LAUNCH("expert_down");
         return QT_OK;
     });

@@ -307,6 +307,30 @@ def test_attention_prefill_float32_at_the_edges_of_its_tiles(d, dv, nq, nkv, nv,
 
 
 @pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("gated", [True, False])
+@pytest.mark.parametrize("tokens, top, experts, width, ff", [(1, 1, 2, 8, 8), (1, 2, 3, 264, 1000), (3, 1, 2, 2056, 40), (16, 2, 4, 520, 1208), (7, 3, 3, 1000, 136),
+                                                             (2, 2, 2, 36, 44), (40, 1, 3, 4104, 24)])
+def test_experts_by_pair(dtype, gated, tokens, top, experts, width, ff):
+    """Rows of whole 16-byte pieces (one to four features a warp, rows shorter and longer than a lane's turns) and others, with the
+    weight on the expert's input, a weight per pair and a further term; sums within the rounding of their longest chain."""
+    x, up = rand(tokens, width, seed=1, dtype=dtype), rand(experts, (2 if gated else 1) * ff, width, seed=2, scale=width ** -0.5, dtype=dtype)
+    down, base = rand(experts, width, ff, seed=3, scale=ff ** -0.5, dtype=dtype), rand(2, tokens, width, seed=4)
+    table = torch.stack([torch.randperm(experts, generator=gen(t))[:top] for t in range(tokens)]).int()
+    ins, pairs, scale = rand(tokens, top, seed=5).abs(), rand(tokens, top, seed=6), rand(tokens, seed=7)
+    mid, out = torch.full((tokens * top, ff), float("nan"), dtype=dtype, device=DEV), torch.full((tokens, width), float("nan"), device=DEV)
+    kernels.experts_by_pair(x, None, table.to(DEV), up, down, mid, out, "silu", pair_weights=pairs, gated=gated, base=GemmOut(base), row_scale=scale, in_weights=ins)
+    xd, upd, downd = x.double().cpu(), up.double().cpu(), down.double().cpu()
+    want = base.sum(0).double().cpu() * scale.double().cpu()[:, None]
+    for t in range(tokens):
+        for j in range(top):
+            h = upd[table[t, j]] @ (xd[t] * float(ins[t, j]))
+            act = h[:ff] * torch.sigmoid(h[:ff]) * (h[ff:] if gated else 1.0)
+            torch.testing.assert_close(mid[t * top + j].double().cpu(), act, **(dict(atol=1e-5, rtol=1e-5) if dtype == torch.float32 else dict(atol=1e-5, rtol=2.0 ** -8)))
+            want[t] += float(pairs[t, j]) * (downd[table[t, j]] @ mid[t * top + j].double().cpu())
+    torch.testing.assert_close(out.double().cpu(), want, atol=2e-5, rtol=2e-5)
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("nq, nkv, d, window, ring, splits", [
     (6, 2, 80, None, 0, 1), (6, 2, 80, None, 0, 5), (4, 4, 16, 40, 128, 2), (16, 1, 128, None, 0, 3),
     (32, 8, 128, None, 0, 4), (5, 5, 112, 300, 0, 7), (10, 2, 48, None, 0, 64), (40, 2, 64, None, 0, 2), (8, 2, 96, 130, 256, 3)])
