@@ -15,7 +15,7 @@
 //   delta_step_kernel      the recurrence token by token (steps of few tokens per sequence: a state is read and written once
 //                          per step anyway, and the kernel is laid out for those bytes); delta_scan_kernel is an older
 //                          form of it (QT_B200_DELTA_STEP=0), a column's rows over 8 lanes
-//   delta_chunk_prepare_kernel, delta_chunk_scan_kernel
+//   delta_chunk_prepare_kernel, delta_chunk_walk_kernel (the usual sizes), delta_chunk_scan_kernel
 //                          the same recurrence in chunks of 16 tokens for longer steps (see there)
 //   gated_head_norm_kernel o / rms(o) * w * gate per head, into the element type of the output projection's input
 #include "common.cuh"
@@ -370,17 +370,51 @@ struct ChunkParams {
     const float* q; const float* k; const float* log_decay;      // [T, kv_heads, dim] x 2, [T, heads, dim]
     float* kt; float* qt; float* kb; float* gc;                    // [T, heads, dim]: e^{L_t} k_t, e^{L_t} q_t, e^{L_last - L_t} k_t; e^{L_last} in a chunk's first row
     const float* beta;                                             // [T, heads]
-    float* ab;                                                     // [T, heads, AB]: beta_s at [2 CH], and for token s, A[t, s] for every t of its chunk (0 unless s < t), then B[t, s] (0 unless s <= t)
+    // [T, heads, AB], beta at [2 CH] and in front of it, for delta_chunk_scan_kernel, a token s's columns of the triangles: A[t, s] for every
+    // t of its chunk (0 unless s < t), then B[t, s] (0 unless s <= t).  solved, for delta_chunk_walk_kernel: a token t's rows, of
+    // (I + diag(beta) A)^-1 and of B
+    float* ab;
     const int* seq_start;
-    int heads, kv_heads, dim;
+    int heads, kv_heads, dim, solved;
 };
 
-// grid (chunks of the longest sequence, heads, sequences), 128 threads.
+// Sixteen values per lane, summed over the lanes of the warp: lane l gets the sum of value l % 16.
+__device__ __forceinline__ float transpose_sum(float (&part)[CH], int lane) {
+#pragma unroll
+    for (int half = CH / 2; half >= 1; half >>= 1) {
+        const bool upper = (lane & half) != 0;
+#pragma unroll
+        for (int j = 0; j < half; ++j) {
+            const float give = upper ? part[j] : part[j + half], keep = upper ? part[j + half] : part[j];
+            part[j] = keep + __shfl_xor_sync(0xffffffffu, give, half);
+        }
+    }
+    return part[0] + __shfl_xor_sync(0xffffffffu, part[0], 16);
+}
+
+// grid (chunks of the longest sequence, heads, sequences), 128 threads.  The triangles: a warp takes two neighbouring s, its lanes hold
+// k_s decayed so far and multiply it by e^{g_t} as t goes on (an exponential per pair and channel took half of the kernel's time:
+// 2,048 tokens of 16 heads of 128 97 us, 43 us so).
+template <int V> struct Elems { float v[V]; };
+template <int V> __device__ __forceinline__ Elems<V> get(const float* p) {
+    Elems<V> r;
+    if constexpr (V == 4) { const float4 x = *reinterpret_cast<const float4*>(p); r.v[0] = x.x; r.v[1] = x.y; r.v[2] = x.z; r.v[3] = x.w; }
+    else r.v[0] = *p;
+    return r;
+}
+template <int V> __device__ __forceinline__ void put(float* p, const Elems<V>& r) {
+    if constexpr (V == 4) *reinterpret_cast<float4*>(p) = make_float4(r.v[0], r.v[1], r.v[2], r.v[3]);
+    else *p = r.v[0];
+}
+
+// V: neighbouring channels a thread loads at once (4 where every row starts on a 16-byte boundary)
+template <int V>
 __global__ void __launch_bounds__(128) delta_chunk_prepare_kernel(const ChunkParams p) {
     pdl_launch_dependents();
     pdl_wait();
-    extern __shared__ float sm[];
-    const int dim = p.dim, head = blockIdx.y, seq = blockIdx.z;
+    extern __shared__ __align__(16) float sm[];
+    __shared__ float tri_a[CH][CH + 1], tri_b[CH][CH + 1], inverse[CH][CH + 1], betas[CH];      // [t][s]
+    const int dim = p.dim, head = blockIdx.y, seq = blockIdx.z, pieces = dim / V;
     const int kvh = head / (p.heads / p.kv_heads);
     const int row0 = p.seq_start[seq], count = p.seq_start[seq + 1] - row0;
     const int first = blockIdx.x * CH;
@@ -388,50 +422,85 @@ __global__ void __launch_bounds__(128) delta_chunk_prepare_kernel(const ChunkPar
     const int n = min(CH, count - first);
     float* qs = sm;                       // [CH][dim]
     float* ks = qs + CH * dim;            // [CH][dim]
-    float* ls = ks + CH * dim;            // [CH][dim] running sums of the logarithms
-    for (int e = threadIdx.x; e < CH * dim; e += blockDim.x) {
-        const int tt = e / dim, c = e % dim;
+    float* ls = ks + CH * dim;            // [CH][dim] logarithms of the decays
+    float* gs = ls + CH * dim;            // [CH][dim] decays
+#pragma unroll 4
+    for (int e = threadIdx.x; e < CH * pieces; e += 128) {
+        const int tt = e / pieces, c = V * (e - tt * pieces);
         const size_t t = (size_t)(row0 + first + tt);
-        const bool in = tt < n;
-        qs[e] = in ? p.q[(t * p.kv_heads + kvh) * dim + c] : 0.f;
-        ks[e] = in ? p.k[(t * p.kv_heads + kvh) * dim + c] : 0.f;
-        ls[e] = in ? p.log_decay[(t * p.heads + head) * dim + c] : 0.f;
+        Elems<V> q = {}, k = {}, g = {};
+        if (tt < n) {
+            q = get<V>(p.q + (t * p.kv_heads + kvh) * dim + c);
+            k = get<V>(p.k + (t * p.kv_heads + kvh) * dim + c);
+            g = get<V>(p.log_decay + (t * p.heads + head) * dim + c);
+        }
+        put<V>(qs + V * e, q);
+        put<V>(ks + V * e, k);
+        put<V>(ls + V * e, g);
+#pragma unroll
+        for (int i = 0; i < V; ++i) g.v[i] = expf(g.v[i]);
+        put<V>(gs + V * e, g);
     }
+    if (threadIdx.x < CH) betas[threadIdx.x] = threadIdx.x < n ? p.beta[(size_t)(row0 + first + threadIdx.x) * p.heads + head] : 0.f;
     __syncthreads();
-    for (int c = threadIdx.x; c < dim; c += blockDim.x) {
-        float run = 0.f;
-        for (int tt = 0; tt < CH; ++tt) { run += ls[tt * dim + c]; ls[tt * dim + c] = run; }
-    }
-    __syncthreads();
-    for (int e = threadIdx.x; e < n * dim; e += blockDim.x) {
-        const int tt = e / dim, c = e % dim;
-        const size_t at = ((size_t)(row0 + first + tt) * p.heads + head) * dim + c;
-        const float grow = expf(ls[e]), rest = expf(ls[(n - 1) * dim + c] - ls[e]);
-        p.kt[at] = grow * ks[e];
-        p.qt[at] = grow * qs[e];
-        p.kb[at] = rest * ks[e];
-        if (tt == 0) p.gc[at] = expf(ls[(n - 1) * dim + c]);
+    // a channel's running sums, in double: 16 additions and a difference cost nothing here, and every key and query of the walk carries their rounding
+    for (int c = threadIdx.x; c < dim; c += 128) {
+        double upto[CH];
+#pragma unroll
+        for (int tt = 0; tt < CH; ++tt) upto[tt] = (tt ? upto[tt - 1] : 0.0) + (double)ls[tt * dim + c];
+        const size_t at = ((size_t)(row0 + first) * p.heads + head) * dim + c, row = (size_t)p.heads * dim;
+#pragma unroll
+        for (int tt = 0; tt < CH; ++tt) {
+            if (tt >= n) break;
+            const float grow = expf((float)upto[tt]), rest = expf((float)(upto[CH - 1] - upto[tt])), k = ks[tt * dim + c];     // missing tokens add 0
+            p.kt[at + tt * row] = grow * k;
+            p.qt[at + tt * row] = grow * qs[tt * dim + c];
+            p.kb[at + tt * row] = rest * k;
+        }
+        p.gc[at] = expf((float)upto[CH - 1]);
     }
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    for (int pair = warp; pair < CH * CH; pair += 4) {
-        const int s = pair / CH, t = pair % CH;
-        if (s >= n) break;
-        float a = 0.f, b = 0.f;
-        if (s <= t && t < n) {
-            for (int c = lane; c < dim; c += 32) {
-                const float w = ks[s * dim + c] * expf(ls[t * dim + c] - ls[s * dim + c]);
-                a += ks[t * dim + c] * w;
-                b += qs[t * dim + c] * w;
+    for (int s = 2 * warp; s < CH; s += 8) {
+        float a0[CH], a1[CH], b0[CH], b1[CH];
+#pragma unroll
+        for (int t = 0; t < CH; ++t) a0[t] = a1[t] = b0[t] = b1[t] = 0.f;
+        for (int c = lane; c < dim; c += 32) {
+            float w0 = ks[s * dim + c], w1 = ks[(s + 1) * dim + c];
+#pragma unroll
+            for (int t = 0; t < CH; ++t) {
+                if (t < s) continue;
+                const float q = qs[t * dim + c], k = ks[t * dim + c], g = gs[t * dim + c];
+                if (t > s) { w0 *= g; a0[t] = fmaf(k, w0, a0[t]); }
+                b0[t] = fmaf(q, w0, b0[t]);
+                if (t > s + 1) { w1 *= g; a1[t] = fmaf(k, w1, a1[t]); }
+                if (t > s) b1[t] = fmaf(q, w1, b1[t]);
             }
-            a = warp_sum(a);
-            b = warp_sum(b);
         }
-        if (lane == 0) {
-            float* row = p.ab + ((size_t)(row0 + first + s) * p.heads + head) * AB;
-            row[t] = s < t ? a : 0.f;
-            row[CH + t] = b;
-            if (t == 0) row[2 * CH] = p.beta[(size_t)(row0 + first + s) * p.heads + head];
+        const float ra0 = transpose_sum(a0, lane), ra1 = transpose_sum(a1, lane), rb0 = transpose_sum(b0, lane), rb1 = transpose_sum(b1, lane);
+        if (lane < CH) { tri_a[lane][s] = ra0; tri_a[lane][s + 1] = ra1; tri_b[lane][s] = rb0; tri_b[lane][s + 1] = rb1; }
+    }
+    __syncthreads();
+    if (p.solved && warp == 0) {                                            // lane j: column j of the inverse, from the top
+        const int j = lane & (CH - 1);
+        float x[CH];
+#pragma unroll
+        for (int t = 0; t < CH; ++t) {
+            float sum = 0.f;
+#pragma unroll
+            for (int s = 0; s < CH; ++s)
+                if (s < t) sum = fmaf(tri_a[t][s], x[s], sum);
+            x[t] = (t == j ? 1.f : 0.f) - betas[t] * sum;
+            if (lane < CH) inverse[t][j] = x[t];
         }
+    }
+    __syncthreads();
+    for (int e = threadIdx.x; e < n * 2 * CH; e += blockDim.x) {
+        const int tt = e / (2 * CH), c = e % CH;
+        const bool second = e % (2 * CH) >= CH;
+        float* row = p.ab + ((size_t)(row0 + first + tt) * p.heads + head) * AB;
+        if (p.solved) row[e % (2 * CH)] = second ? tri_b[tt][c] : inverse[tt][c];
+        else row[e % (2 * CH)] = second ? tri_b[c][tt] : tri_a[c][tt];
+        if (c == 0 && !second) row[2 * CH] = betas[tt];
     }
 }
 
@@ -567,134 +636,195 @@ __global__ void __launch_bounds__(SCAN_COLS * SCAN_LANES) delta_chunk_scan_kerne
     }
 }
 
-// The same walk for the usual sizes (dim a multiple of 64 up to 256, vdim a multiple of 16), written for few instructions:
-// a column of the state belongs to CH = 16 neighbouring lanes, lane l of them holding the rows 4 (l + 16 q) + e
-// (q < RQ, e < 4: 16-byte pieces that the 16 lanes read side by side) and owning the scalars of the chunk's token l.
-// The per-token sums over the state's rows are reduced so that token l's sum lands in lane l (15 exchanges instead of
-// 64), the triangular solve passes each u_t on by one shuffle, and chunk data arrives by 16-byte copies; a chunk's
-// missing tokens are zeros, which change nothing.  grid (vdim / 16, heads, sequences), 256 threads.
-constexpr int FAST_COLS = 16;
+// The same walk for the usual sizes (dim = 64 P up to 256, vdim a multiple of 16).  A sequence's chunks follow one another, so what counts is
+// the time of one chunk: its instructions, its reads of shared memory and the chain from S0 to the next S.  A warp owns two columns of
+// the state, a lane 2 P rows of each as P pairs of neighbouring rows (fma.rn.f32x2), so every 16 bytes of a key, a query or a decay that a
+// lane reads serve two columns, and everything but the chunk's data stays within the warp.  Per chunk: the sums over the rows, S0^T (e^L
+// k) and S0^T (e^L q), are reduced so that lane (h, l) ends with token l of column h (31 exchanges each); r = beta (v - S0^T (e^L k)) and
+// u = (I + diag(beta) A)^-1 r pass through shared memory, 16 independent products in the place of a solve from token to
+// token; then S.  Chunk data arrives by 16-byte copies under the chunk before; a chunk's missing tokens are zeros, which
+// change nothing.  grid (vdim / 16, heads, sequences), 256 threads.  16 heads of 128 x 128, one prompt of 2,048 tokens: 255 us;
+// 298 us with four columns a warp (one warp a scheduler, which then issues every third cycle); 451 us with one column over 16
+// lanes and the solve passed on by shuffles.
+constexpr int WALK_COLS = 16, WALK_THREADS = 256;
 
 __device__ __forceinline__ void cp_async16(float* dst, const float* src) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
 }
+__device__ __forceinline__ unsigned long long pair_of(float lo, float hi) {
+    unsigned long long r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+    return r;
+}
+__device__ __forceinline__ float2 unpair(unsigned long long v) {
+    float2 r;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+    return r;
+}
+__device__ __forceinline__ unsigned long long fma_pair(unsigned long long a, unsigned long long b, unsigned long long c) {
+    unsigned long long r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
 
-// LPC lanes per column: 16 as described, or 32 (a warp per column, dim a multiple of 128: twice the warps, each with half
-// the rows; lanes l and l + 16 then both carry token l's scalars).
-template <int LPC, int RQ>
-__global__ void __launch_bounds__(FAST_COLS * LPC) delta_chunk_scan_fast_kernel(const ChunkScanParams p) {
+// The first row of a lane's pair m, and a lane's P pairs of neighbouring elements of a row of 64 P.
+template <int P> __device__ __forceinline__ int pair_row(int lane, int m) { return P % 2 ? 2 * (lane + 32 * m) : 4 * (lane + 32 * (m / 2)) + 2 * (m & 1); }
+template <int P> __device__ __forceinline__ void load_pairs(const float* row, int lane, unsigned long long (&v)[P]) {
+    if constexpr (P % 2) {
+#pragma unroll
+        for (int m = 0; m < P; ++m) v[m] = *reinterpret_cast<const unsigned long long*>(row + 2 * (lane + 32 * m));
+    } else {
+#pragma unroll
+        for (int m = 0; m < P; m += 2) {
+            const ulonglong2 x = *reinterpret_cast<const ulonglong2*>(row + 4 * (lane + 32 * (m / 2)));
+            v[m] = x.x; v[m + 1] = x.y;
+        }
+    }
+}
+
+// sum over the state's rows of rows[t][.] s[.][c] for 16 tokens and 2 columns: lane (h, l) gets token l, column h
+template <int P> __device__ __forceinline__ float column_sums(const float* rows, const unsigned long long (&s)[P][2], int lane) {
+    float x[CH][2];
+#pragma unroll
+    for (int t = 0; t < CH; ++t) {
+        unsigned long long k[P];
+        load_pairs<P>(rows + t * 64 * P, lane, k);
+#pragma unroll
+        for (int c = 0; c < 2; ++c) {
+            unsigned long long acc = 0ull;
+#pragma unroll
+            for (int m = 0; m < P; ++m) acc = fma_pair(k[m], s[m][c], acc);
+            const float2 both = unpair(acc);
+            x[t][c] = both.x + both.y;
+        }
+    }
+    const bool right = (lane & 16) != 0;
+    float y[CH];
+#pragma unroll
+    for (int t = 0; t < CH; ++t) {
+        const float give = right ? x[t][0] : x[t][1], keep = right ? x[t][1] : x[t][0];
+        y[t] = keep + __shfl_xor_sync(0xffffffffu, give, 16);
+    }
+#pragma unroll
+    for (int half = CH / 2; half >= 1; half >>= 1) {
+        const bool upper = (lane & half) != 0;
+#pragma unroll
+        for (int t = 0; t < half; ++t) {
+            const float give = upper ? y[t] : y[t + half], keep = upper ? y[t + half] : y[t];
+            y[t] = keep + __shfl_xor_sync(0xffffffffu, give, half);
+        }
+    }
+    return y[0];
+}
+
+// sum over s of row[s] x[s]
+__device__ __forceinline__ float token_sum(const float* row, const float* x) {
+    float sum[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+    for (int s = 0; s < CH; s += 4) {
+        const float4 w = *reinterpret_cast<const float4*>(row + s), v = *reinterpret_cast<const float4*>(x + s);
+        sum[0] = fmaf(w.x, v.x, sum[0]);
+        sum[1] = fmaf(w.y, v.y, sum[1]);
+        sum[2] = fmaf(w.z, v.z, sum[2]);
+        sum[3] = fmaf(w.w, v.w, sum[3]);
+    }
+    return (sum[0] + sum[1]) + (sum[2] + sum[3]);
+}
+
+template <int P>
+__global__ void __launch_bounds__(WALK_THREADS) delta_chunk_walk_kernel(const ChunkScanParams p) {
+    constexpr int DIM = 64 * P, ROWS = CH * DIM;
+    constexpr int PER_CHUNK = 3 * ROWS + CH * AB + CH * WALK_COLS + DIM;     // kt, qt, kb, the tokens' rows of `ab`, v columns, e^{L_last}
     pdl_launch_dependents();
     pdl_wait();
     extern __shared__ __align__(16) float sm[];
-    constexpr int DIM = 4 * LPC * RQ;
-    constexpr int PER_TOKEN = 3 * DIM + AB + FAST_COLS;           // kt, qt, kb rows, the token's row of `ab` (with beta), v columns
-    constexpr int PER_CHUNK = CH * PER_TOKEN + DIM;
-    float* buffers[2] = {sm, sm + PER_CHUNK};
+    __shared__ __align__(16) float wanted[WALK_COLS][CH], found[WALK_COLS][CH];     // r and u of the block's columns
     const int vdim = p.vdim, head = blockIdx.y, seq = blockIdx.z;
-    const int lane = threadIdx.x & 31, row_lane = threadIdx.x & (LPC - 1), l = threadIdx.x & 15, col = threadIdx.x / LPC;
-    const int j = blockIdx.x * FAST_COLS + col;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, h = lane >> 4, l = lane & 15;
+    const int col = 2 * warp + h, j0 = blockIdx.x * WALK_COLS + 2 * warp;
     const int row0 = p.seq_start[seq], count = p.seq_start[seq + 1] - row0;
-    float* state = p.state + ((size_t)p.slots[seq] * p.heads + head) * DIM * vdim;
+    float* state = p.state + ((size_t)p.slots[seq] * p.heads + head) * DIM * vdim + j0;
 
-    float s[RQ][4];
+    unsigned long long s[P][2];
 #pragma unroll
-    for (int q = 0; q < RQ; ++q)
-#pragma unroll
-        for (int e = 0; e < 4; ++e) s[q][e] = state[(size_t)(4 * (row_lane + LPC * q) + e) * vdim + j];
-
-    auto fetch = [&](int chunk, float* buf) {
+    for (int m = 0; m < P; ++m) {
+        const float2 a = *reinterpret_cast<const float2*>(state + (size_t)pair_row<P>(lane, m) * vdim);
+        const float2 b = *reinterpret_cast<const float2*>(state + (size_t)(pair_row<P>(lane, m) + 1) * vdim);
+        s[m][0] = pair_of(a.x, b.x); s[m][1] = pair_of(a.y, b.y);
+    }
+    auto fetch = [&](int chunk) {
+        float* buf = sm + (chunk & 1) * PER_CHUNK;
         const int first = chunk * CH, n = min(CH, count - first);
-        constexpr int PIECES = PER_TOKEN / 4;                      // 16-byte pieces of a token's data
-        for (int e = threadIdx.x; e < CH * PIECES; e += blockDim.x) {
-            const int tt = e / PIECES, c = 4 * (e % PIECES);
-            float* dst = buf + tt * PER_TOKEN + c;
-            if (tt >= n) { *reinterpret_cast<float4*>(dst) = make_float4(0.f, 0.f, 0.f, 0.f); continue; }
-            const size_t at = (size_t)(row0 + first + tt) * p.heads + head;
-            if (c < DIM) cp_async16(dst, p.kt + at * DIM + c);
-            else if (c < 2 * DIM) cp_async16(dst, p.qt + at * DIM + (c - DIM));
-            else if (c < 3 * DIM) cp_async16(dst, p.kb + at * DIM + (c - 2 * DIM));
-            else if (c < 3 * DIM + AB) cp_async16(dst, p.ab + at * AB + (c - 3 * DIM));
-            else cp_async16(dst, p.v + at * vdim + blockIdx.x * FAST_COLS + (c - 3 * DIM - AB));
+        const size_t at0 = (size_t)(row0 + first) * p.heads + head;
+        auto piece = [&](float* dst, const float* src, int tt) {
+            if (tt < n) cp_async16(dst, src);
+            else *reinterpret_cast<float4*>(dst) = make_float4(0.f, 0.f, 0.f, 0.f);
+        };
+#pragma unroll
+        for (int i = 0; i < ROWS / 4 / WALK_THREADS; ++i) {
+            const int e = threadIdx.x + i * WALK_THREADS, tt = e / (DIM / 4), c = 4 * (e % (DIM / 4));
+            const size_t at = (at0 + (size_t)tt * p.heads) * DIM + c;
+            piece(buf + 4 * e, p.kt + at, tt);
+            piece(buf + ROWS + 4 * e, p.qt + at, tt);
+            piece(buf + 2 * ROWS + 4 * e, p.kb + at, tt);
         }
-        for (int e = threadIdx.x; e < DIM / 4; e += blockDim.x)
-            cp_async16(buf + CH * PER_TOKEN + 4 * e, p.gc + ((size_t)(row0 + first) * p.heads + head) * DIM + 4 * e);
+        static_assert(CH * AB / 4 <= WALK_THREADS && CH * WALK_COLS / 4 <= WALK_THREADS && DIM / 4 <= WALK_THREADS, "a piece a thread");
+        if (threadIdx.x < CH * AB / 4) {
+            const int tt = threadIdx.x / (AB / 4);
+            piece(buf + 3 * ROWS + 4 * threadIdx.x, p.ab + (at0 + (size_t)tt * p.heads) * AB + 4 * (threadIdx.x % (AB / 4)), tt);
+        }
+        if (threadIdx.x < CH * WALK_COLS / 4) {
+            const int tt = threadIdx.x / (WALK_COLS / 4);
+            piece(buf + 3 * ROWS + CH * AB + 4 * threadIdx.x, p.v + (at0 + (size_t)tt * p.heads) * vdim + blockIdx.x * WALK_COLS + 4 * (threadIdx.x % (WALK_COLS / 4)), tt);
+        }
+        if (threadIdx.x < DIM / 4) cp_async16(buf + PER_CHUNK - DIM + 4 * threadIdx.x, p.gc + at0 * DIM + 4 * threadIdx.x);
         cp_async_commit();
     };
     const int chunks = (count + CH - 1) / CH;
-    if (chunks > 0) fetch(0, buffers[0]);
+    if (chunks > 0) fetch(0);
     for (int chunk = 0; chunk < chunks; ++chunk) {
         cp_async_wait_all();
-        __syncthreads();
-        if (chunk + 1 < chunks) fetch(chunk + 1, buffers[(chunk + 1) & 1]);
-        const float* buf = buffers[chunk & 1];
-        const int n = min(CH, count - chunk * CH);
-        // this lane's share of S0^T (e^L k_t) and S0^T (e^L q_t) for every token of the chunk
-        float pred[CH], read[CH];
+        __syncthreads();                                                    // this chunk has landed; everyone is done with the other buffer
+        if (chunk + 1 < chunks) fetch(chunk + 1);
+        const float* buf = sm + (chunk & 1) * PER_CHUNK;
+        const float* ab = buf + 3 * ROWS + l * AB;                          // token l's rows of the inverse and of B, its beta
+        const float pred = column_sums<P>(buf, s, lane);
+        wanted[col][l] = ab[2 * CH] * (buf[3 * ROWS + CH * AB + l * WALK_COLS + col] - pred);
+        __syncwarp();
+        found[col][l] = token_sum(ab, wanted[col]);
+        const float o = column_sums<P>(buf + ROWS, s, lane);                // reads the old state
+        __syncwarp();
+        unsigned long long g[P];
+        load_pairs<P>(buf + PER_CHUNK - DIM, lane, g);
 #pragma unroll
-        for (int tt = 0; tt < CH; ++tt) {
-            float a = 0.f, b = 0.f;
+        for (int m = 0; m < P; ++m)
 #pragma unroll
-            for (int q = 0; q < RQ; ++q) {
-                const float4 kt = *reinterpret_cast<const float4*>(buf + tt * PER_TOKEN + 4 * (row_lane + LPC * q));
-                const float4 qt = *reinterpret_cast<const float4*>(buf + tt * PER_TOKEN + DIM + 4 * (row_lane + LPC * q));
-                a += kt.x * s[q][0] + kt.y * s[q][1] + kt.z * s[q][2] + kt.w * s[q][3];
-                b += qt.x * s[q][0] + qt.y * s[q][1] + qt.z * s[q][2] + qt.w * s[q][3];
-            }
-            pred[tt] = a;
-            read[tt] = b;
-        }
-        // sums over the lanes of the column, token l's landing in lane l: halve the tokens a lane carries four times
-        if (LPC == 32) {
+            for (int c = 0; c < 2; ++c) s[m][c] = fma_pair(s[m][c], g[m], 0ull);
 #pragma unroll
-            for (int tt = 0; tt < CH; ++tt) {
-                pred[tt] += __shfl_xor_sync(0xffffffffu, pred[tt], 16);
-                read[tt] += __shfl_xor_sync(0xffffffffu, read[tt], 16);
-            }
-        }
+        for (int t0 = 0; t0 < CH; t0 += 4) {
+            const float4 u[2] = {*reinterpret_cast<const float4*>(&found[2 * warp][t0]), *reinterpret_cast<const float4*>(&found[2 * warp + 1][t0])};
+            const float us[2][4] = {{u[0].x, u[0].y, u[0].z, u[0].w}, {u[1].x, u[1].y, u[1].z, u[1].w}};
 #pragma unroll
-        for (int step = 8; step >= 1; step >>= 1) {
-            const bool upper = (l & step) != 0;
+            for (int i = 0; i < 4; ++i) {
+                unsigned long long kb[P];
+                load_pairs<P>(buf + 2 * ROWS + (t0 + i) * DIM, lane, kb);
 #pragma unroll
-            for (int i = 0; i < step; ++i) {
-                const float give_p = upper ? pred[i] : pred[i + step], keep_p = upper ? pred[i + step] : pred[i];
-                const float give_r = upper ? read[i] : read[i + step], keep_r = upper ? read[i + step] : read[i];
-                pred[i] = keep_p + __shfl_xor_sync(0xffffffffu, give_p, step);
-                read[i] = keep_r + __shfl_xor_sync(0xffffffffu, give_r, step);
+                for (int c = 0; c < 2; ++c) {
+                    const unsigned long long uu = pair_of(us[c][i], us[c][i]);
+#pragma unroll
+                    for (int m = 0; m < P; ++m) s[m][c] = fma_pair(kb[m], uu, s[m][c]);
+                }
             }
         }
-        // lane l now holds token l's sums in pred[0] and read[0]
-        float mine_p = pred[0], mine_r = read[0];
-        const float beta = buf[l * PER_TOKEN + 3 * DIM + 2 * CH];
-        const float vj = buf[l * PER_TOKEN + 3 * DIM + AB + col];
-        float u[CH];
-#pragma unroll
-        for (int tt = 0; tt < CH; ++tt) {
-            const float candidate = beta * (vj - mine_p);                       // u of this lane's token, final once tt reaches it
-            u[tt] = __shfl_sync(0xffffffffu, candidate, LPC == 32 ? tt : (lane & 16) + tt);
-            const float* column = buf + tt * PER_TOKEN + 3 * DIM;              // what u_tt adds to the later tokens
-            mine_p += column[l] * u[tt];                                        // zero unless l > tt
-            mine_r += column[CH + l] * u[tt];                                   // zero unless l >= tt
-        }
-        if (row_lane < n) p.out[((size_t)(row0 + chunk * CH + l) * p.heads + head) * vdim + j] = mine_r;
-        // the state behind the chunk
-        const float* gc = buf + CH * PER_TOKEN;
-#pragma unroll
-        for (int q = 0; q < RQ; ++q) {
-            const float4 g = *reinterpret_cast<const float4*>(gc + 4 * (row_lane + LPC * q));
-            float acc[4] = {g.x * s[q][0], g.y * s[q][1], g.z * s[q][2], g.w * s[q][3]};
-#pragma unroll
-            for (int tt = 0; tt < CH; ++tt) {
-                const float4 kb = *reinterpret_cast<const float4*>(buf + tt * PER_TOKEN + 2 * DIM + 4 * (row_lane + LPC * q));
-                acc[0] += kb.x * u[tt]; acc[1] += kb.y * u[tt]; acc[2] += kb.z * u[tt]; acc[3] += kb.w * u[tt];
-            }
-#pragma unroll
-            for (int e = 0; e < 4; ++e) s[q][e] = acc[e];
-        }
+        const float more = token_sum(ab + CH, found[col]);
+        if (chunk * CH + l < count) p.out[((size_t)(row0 + chunk * CH + l) * p.heads + head) * vdim + blockIdx.x * WALK_COLS + col] = o + more;
     }
 #pragma unroll
-    for (int q = 0; q < RQ; ++q)
-#pragma unroll
-        for (int e = 0; e < 4; ++e) state[(size_t)(4 * (row_lane + LPC * q) + e) * vdim + j] = s[q][e];
+    for (int m = 0; m < P; ++m) {
+        const float2 x = unpair(s[m][0]), y = unpair(s[m][1]);
+        *reinterpret_cast<float2*>(state + (size_t)pair_row<P>(lane, m) * vdim) = make_float2(x.x, y.x);
+        *reinterpret_cast<float2*>(state + (size_t)(pair_row<P>(lane, m) + 1) * vdim) = make_float2(x.y, y.y);
+    }
 }
 
 // out[t, h, :] = o / sqrt(mean(o^2) + eps) * w * gate[t, h, :].  One warp per (token, head).
@@ -905,17 +1035,22 @@ static int launch_chunk_scan(const ChunkScanParams& p, int n_seqs, cudaStream_t 
     return QT_OK;
 }
 
-template <int LPC, int RQ>
-static int launch_chunk_scan_fast(const ChunkScanParams& p, int n_seqs, cudaStream_t s) {
-    const size_t smem = 2 * ((size_t)CH * (3 * 4 * LPC * RQ + AB + FAST_COLS) + 4 * LPC * RQ) * sizeof(float);
+template <int P>
+static int launch_chunk_walk(const ChunkScanParams& p, int n_seqs, cudaStream_t s) {
+    const size_t smem = 2 * ((size_t)CH * (3 * 64 * P + AB + WALK_COLS) + 64 * P) * sizeof(float);
     static bool configured = false;
     if (!configured) {
-        cudaError_t err = cudaFuncSetAttribute(delta_chunk_scan_fast_kernel<LPC, RQ>, cudaFuncAttributeMaxDynamicSharedMemorySize, 120 * 1024);
-        if (err != cudaSuccess) QT_FAIL(QT_ERR_LAUNCH, "delta_chunk_scan: cannot raise shared memory: %s", cudaGetErrorString(err));
+        cudaError_t err = cudaFuncSetAttribute(delta_chunk_walk_kernel<P>, cudaFuncAttributeMaxDynamicSharedMemorySize, 120 * 1024);
+        if (err != cudaSuccess) QT_FAIL(QT_ERR_LAUNCH, "delta_chunk_walk: cannot raise shared memory: %s", cudaGetErrorString(err));
         configured = true;
     }
-    launch_kernel(delta_chunk_scan_fast_kernel<LPC, RQ>, dim3(p.vdim / FAST_COLS, p.heads, n_seqs), dim3(FAST_COLS * LPC), smem, s, p);
-    QT_CHECK_LAUNCH("delta_chunk_scan");
+    // Blocks start while the kernel before still runs on most SMs; as much shared memory as it takes to keep them from piling up on
+    // the first SMs that fall free (646 us in place of 255 us where two or three share an SM and others stand idle).
+    const long long blocks = (long long)(p.vdim / WALK_COLS) * p.heads * n_seqs, per_sm = (blocks + sm_count() - 1) / sm_count();
+    const size_t spread = (size_t)(228 * 1024) / (size_t)(per_sm + 1);
+    const size_t asked = spread > smem && spread <= 120 * 1024 ? spread : smem;
+    launch_kernel(delta_chunk_walk_kernel<P>, dim3(p.vdim / WALK_COLS, p.heads, n_seqs), dim3(WALK_THREADS), asked, s, p);
+    QT_CHECK_LAUNCH("delta_chunk_walk");
     return QT_OK;
 }
 
@@ -930,27 +1065,29 @@ extern "C" int qt_delta_scan_chunked(const float* q, const float* k, const float
     QT_REQUIRE(n_seqs <= 65535 && heads <= 65535, "delta_scan_chunked: too many sequences or heads for one launch");
     if (n_seqs == 0 || max_tokens == 0) return QT_OK;
     cudaStream_t s = (cudaStream_t)stream;
-    ChunkParams cp{q, k, log_decay, kt, qt, kb, gc, beta, ab, seq_start, heads, kv_heads, dim};
-    const size_t smem = 3 * (size_t)CH * dim * sizeof(float);
+    static const bool plain_only = [] { const char* env = getenv("QT_B200_DELTA_FAST"); return env && env[0] == '0'; }();
+    const bool aligned = (((uintptr_t)kt | (uintptr_t)qt | (uintptr_t)kb | (uintptr_t)gc | (uintptr_t)ab | (uintptr_t)v | (uintptr_t)state | (uintptr_t)out) & 15) == 0;
+    const bool walk = !plain_only && aligned && dim % 64 == 0 && dim <= 256 && vdim % WALK_COLS == 0;
+    ChunkParams cp{q, k, log_decay, kt, qt, kb, gc, beta, ab, seq_start, heads, kv_heads, dim, walk ? 1 : 0};
+    const size_t smem = 4 * (size_t)CH * dim * sizeof(float);
     static bool configured = false;
     if (!configured) {
-        cudaError_t err = cudaFuncSetAttribute(delta_chunk_prepare_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * 1024);
+        cudaError_t err = cudaFuncSetAttribute(delta_chunk_prepare_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * 1024);
+        if (err == cudaSuccess) err = cudaFuncSetAttribute(delta_chunk_prepare_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * 1024);
         if (err != cudaSuccess) QT_FAIL(QT_ERR_LAUNCH, "delta_chunk_prepare: cannot raise shared memory: %s", cudaGetErrorString(err));
         configured = true;
     }
-    launch_kernel(delta_chunk_prepare_kernel, dim3((max_tokens + CH - 1) / CH, heads, n_seqs), dim3(128), smem, s, cp);
+    const bool fours = dim % 4 == 0 && (((uintptr_t)q | (uintptr_t)k | (uintptr_t)log_decay) & 15) == 0;
+    const dim3 chunk_grid((max_tokens + CH - 1) / CH, heads, n_seqs);
+    if (fours) launch_kernel(delta_chunk_prepare_kernel<4>, chunk_grid, dim3(128), smem, s, cp);
+    else launch_kernel(delta_chunk_prepare_kernel<1>, chunk_grid, dim3(128), smem, s, cp);
     QT_CHECK_LAUNCH("delta_chunk_prepare");
     ChunkScanParams sp{kt, qt, kb, gc, ab, v, beta, state, out, seq_start, slots, heads, dim, vdim};
-    static const bool plain_only = [] { const char* env = getenv("QT_B200_DELTA_FAST"); return env && env[0] == '0'; }();
-    const bool aligned = ((uintptr_t)kt % 16 == 0) && ((uintptr_t)qt % 16 == 0) && ((uintptr_t)kb % 16 == 0) && ((uintptr_t)gc % 16 == 0) &&
-                         ((uintptr_t)ab % 16 == 0) && ((uintptr_t)v % 16 == 0);
-    if (!plain_only && aligned && dim % 64 == 0 && dim <= 256 && vdim % FAST_COLS == 0) {
-        // 16 lanes per column unless QT_B200_DELTA_LANES=32: a warp per column measured 3 to 7 % slower in a prefill of 2,048 tokens
-        static const bool half_warps = [] { const char* env = getenv("QT_B200_DELTA_LANES"); return !(env && env[0] == '3' && env[1] == '2'); }();
-        if (dim == 64) return launch_chunk_scan_fast<16, 1>(sp, n_seqs, s);
-        if (dim == 128) return half_warps ? launch_chunk_scan_fast<16, 2>(sp, n_seqs, s) : launch_chunk_scan_fast<32, 1>(sp, n_seqs, s);
-        if (dim == 192) return launch_chunk_scan_fast<16, 3>(sp, n_seqs, s);
-        return half_warps ? launch_chunk_scan_fast<16, 4>(sp, n_seqs, s) : launch_chunk_scan_fast<32, 2>(sp, n_seqs, s);
+    if (walk) {
+        if (dim == 64) return launch_chunk_walk<1>(sp, n_seqs, s);
+        if (dim == 128) return launch_chunk_walk<2>(sp, n_seqs, s);
+        if (dim == 192) return launch_chunk_walk<3>(sp, n_seqs, s);
+        return launch_chunk_walk<4>(sp, n_seqs, s);
     }
     if (dim <= 32) return launch_chunk_scan<4>(sp, n_seqs, s);
     if (dim <= 64) return launch_chunk_scan<8>(sp, n_seqs, s);

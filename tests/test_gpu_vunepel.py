@@ -406,6 +406,35 @@ def test_delta_rule_state_keeps_a_far_write(chunked):
     torch.testing.assert_close(state[0, 0].cpu(), s.float(), atol=1e-4, rtol=1e-4)
 
 
+@pytest.mark.parametrize("heads, kv_heads, dim, vdim", [(3, 1, 64, 16), (2, 2, 128, 48), (4, 2, 192, 32), (1, 1, 256, 16), (2, 1, 128, 20), (2, 2, 66, 16)])
+@pytest.mark.parametrize("lengths", [(1, 15, 16, 17, 33), (64,), (2, 31) * 60])
+def test_chunked_recurrence_at_the_edges_of_its_chunks(heads, kv_heads, dim, vdim, lengths):
+    """The walk (dim a multiple of 64, vdim of 16) and the general form, one sequence and more blocks than SMs, from states that are
+    not zero; 64-bit walk token by token.  Sums of up to 256 products and chains of 64 tokens round to a few 1e-7 of the largest value."""
+    torch.manual_seed(dim + len(lengths))
+    total, count = sum(lengths), len(lengths)
+    q = torch.nn.functional.normalize(torch.randn(total, kv_heads, dim), dim=-1) * dim ** -0.5
+    k = torch.nn.functional.normalize(torch.randn(total, kv_heads, dim), dim=-1)
+    v, beta = torch.randn(total, heads, vdim), torch.rand(total, heads)
+    decay = -torch.exp(torch.randn(total, heads, dim) - 2.0)
+    states = torch.randn(count + 2, heads, dim, vdim)
+    slots = torch.randperm(count + 1)[:count].tolist()
+    got_states, read = states.to(DEV), torch.full((total, heads, vdim), float("nan"), device=DEV)
+    scan(True, q.to(DEV), k.to(DEV), v.to(DEV), beta.to(DEV), decay.to(DEV), got_states, read, _Step(list(lengths), [0] * count, slots))
+    want, wanted, at = torch.zeros(total, heads, vdim, dtype=torch.float64), states.double(), 0
+    for n, slot in zip(lengths, slots):
+        s = wanted[slot]
+        for t in range(at, at + n):
+            keys, queries = (x[t].double().repeat_interleave(heads // kv_heads, 0) for x in (k, q))
+            s = s * decay[t].double().exp()[:, :, None]
+            u = beta[t].double()[:, None] * (v[t].double() - torch.einsum("hdv,hd->hv", s, keys))
+            s = s + keys[:, :, None] * u[:, None, :]
+            want[t] = torch.einsum("hdv,hd->hv", s, queries)
+        wanted[slot], at = s, at + n
+    assert float((read.cpu().double() - want).abs().max()) < 3e-6 * float(want.abs().max())
+    assert float((got_states.cpu().double() - wanted).abs().max()) < 3e-6 * float(wanted.abs().max())
+
+
 def test_chunked_recurrence_with_decays_that_underflow():
     """Decays down to e^-30 a token: over a chunk their product is far below what a float holds, and the chunked form,
     which only ever multiplies by products of decays over ranges, still agrees with the token-by-token form."""
