@@ -36,11 +36,17 @@
 // used.  `sinks` (or `sink` alone: 0): the softmax's denominator has one more term, exp of the head's number, which is neither
 // scaled nor capped and has no value; it joins a row's sum once, at the end.
 //
+// DENSE (qt_attention_prefill_rows): prompts whose heads have keys and values of their own, formed for the step, in halves; keys of 128 or 192
+// elements, values of 64 or 128, a gate on the result ahead of its rounding.  Bound like the cached form by the softmax beside the MMAs: 2,048
+// tokens of 16 heads of 192 and 128 in 43 us (62 us with the gate's sums), 505 TFLOP/s; the same attention over cached rows of 576
+// and 512 elements (attention_latent.cu) 363 us.
+//
 // Counterpart in luozoupi/Qwen-Triton: kernels/flash_attention.py:54-152 (32 x 32 tl.dot tiles) and the masked
 // SDPA branch of modules/attention.py:110-123.
 #include "tc_common.cuh"
 #include "score_cap.cuh"
 
+#include <cuda_fp16.h>
 #include <math.h>
 
 using namespace qt;
@@ -51,8 +57,9 @@ namespace {
 constexpr int PAGE = 64;
 constexpr int BQ = 128;            // query rows per block = MMA M
 constexpr int THREADS = 224;        // warp 0: TMA of Q and K, warp 1: MMA + tensor-memory allocation, warps 2..5: softmax, warp 6: TMA of V
-constexpr uint32_t ALIGN_SLACK = 1024;  // shared memory asked for beyond the tiles, to round their base up to 1,024 bytes (the
-                                        // kernel refuses to run if the base ever needs more)
+// shared memory asked for beyond the tiles, to round their base up to 1,024 bytes (the kernel refuses to run if the base ever needs
+// more; without static shared memory it needs none): what is left of an SM's half beside keys of 192 elements
+template <int HD> constexpr uint32_t ALIGN_SLACK = HD > 128 ? 768 : 1024;
 constexpr float RESCALE_STEP = 8.f; // a row's scaling maximum moves only when the true one is more than 2^8 above it
 constexpr float LOG2E = 1.4426950408889634f;
 constexpr uint32_t HALF_BYTES = 128 * 64 * 2;   // a [128 rows][64 columns] bfloat16 half tile: 16 KB
@@ -71,6 +78,9 @@ struct TcAttnParams {
     int sink;                      // 1: the softmax has one more term without a value, of score sinks[head] (null: 0)
     const float* sinks;
     float softcap;                 // of the score cap (CAP)
+    int v_col;                     // DENSE: first value column of a row (key columns are in front: head * HD)
+    // DENSE: the result times sigmoid(gate[t, gate_offset + head * dv + c]), or with gate_per_head of column gate_offset + head; or null
+    const float* gate; int gate_splits; size_t gate_split_stride; int gate_cols, gate_offset, gate_per_head;
 };
 
 __device__ __forceinline__ float fast_log2(float x) {
@@ -131,6 +141,11 @@ __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
     return *reinterpret_cast<uint32_t*>(&v);
 }
 
+__device__ __forceinline__ uint32_t pack_half(float lo, float hi) {
+    __half2 v = __floats2half2_rn(lo, hi);
+    return *reinterpret_cast<uint32_t*>(&v);
+}
+
 // Operand descriptor of an MN-major tile stored as [64-element MN blocks][K rows][64 elements], 128-byte swizzle:
 // groups of 8 K rows lie 1024 bytes apart (stride byte offset), MN blocks `mn_block_bytes` apart (leading byte offset).
 __device__ __forceinline__ uint64_t operand_desc_mn(uint32_t saddr, uint32_t mn_block_bytes) {
@@ -151,7 +166,10 @@ __device__ __forceinline__ int cache_page(const int* table, int max_blocks, int 
 
 // BKEY: keys per tile, one page or two.  One page: half the shared memory and tensor memory, so that two blocks share
 // an SM and one's softmax runs under the other's MMAs.
-template <int HD, int BKEY, bool PEN, int CAP>
+// HD: elements of queries and keys, HDV of values.  DENSE: keys and values are not in a cache but columns of one matrix with a row per
+// token of this step (kv_row, below), and no token comes from before; queries, keys, values and P are then halves (11 bits of a number in
+// the place of bfloat16's 8: keys and values are rounded once more than the rows they are made from; P is at most 2^8).
+template <int HD, int HDV, int BKEY, bool PEN, int CAP, bool DENSE>
 __global__ void __launch_bounds__(THREADS, BKEY == 64 ? 2 : 1) attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q,
                                                                        const __grid_constant__ CUtensorMap map_k,
                                                                        const __grid_constant__ CUtensorMap map_v,
@@ -160,12 +178,18 @@ __global__ void __launch_bounds__(THREADS, BKEY == 64 ? 2 : 1) attention_prefill
     constexpr uint32_t Q_BYTES = HALVES * HALF_BYTES;     // [128 rows][HD]
     constexpr int PAGES = BKEY / PAGE;                    // pages per key tile
     constexpr uint32_t KEY_HALF_BYTES = BKEY * 64 * 2;    // a [BKEY keys][64 columns] half of a key or value tile
-    constexpr uint32_t KV_BYTES = HALVES * KEY_HALF_BYTES;   // [BKEY keys][HD]
+    constexpr uint32_t K_BYTES = HALVES * KEY_HALF_BYTES;    // [BKEY keys][HD]
+    constexpr int V_HALVES = HDV / 64;
+    constexpr uint32_t V_BYTES = V_HALVES * KEY_HALF_BYTES;  // [BKEY keys][HDV]
+    // Keys of 192 elements leave room for one value tile if two blocks are to share an SM.  The next values then wait for P V, the next
+    // keys (which Q K^T needs while this tile's softmax runs) do not.
+    constexpr int V_STAGES = HD > 128 ? 1 : 2;
     constexpr uint32_t TMEM_COLS = BKEY == 64 ? 256 : 512;
     constexpr uint32_t S_COL0 = 0, S_COL1 = BKEY, O_COL = 2 * BKEY;
     // S = Q K^T: M 128, N 128 keys, both operands K-major.  O = P V: M 128, N HD, A K-major, B MN-major.
-    constexpr uint32_t IDESC_QK = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BKEY >> 3) << 17) | ((uint32_t)(BQ >> 4) << 24);
-    constexpr uint32_t IDESC_PV = (1u << 4) | (1u << 7) | (1u << 10) | (1u << 16) | ((uint32_t)(HD >> 3) << 17) | ((uint32_t)(BQ >> 4) << 24);
+    constexpr uint32_t OPERANDS = DENSE ? 0u : (1u << 7) | (1u << 10);        // half or bfloat16, both operands alike
+    constexpr uint32_t IDESC_QK = (1u << 4) | OPERANDS | ((uint32_t)(BKEY >> 3) << 17) | ((uint32_t)(BQ >> 4) << 24);
+    constexpr uint32_t IDESC_PV = (1u << 4) | OPERANDS | (1u << 16) | ((uint32_t)(HDV >> 3) << 17) | ((uint32_t)(BQ >> 4) << 24);
 
     pdl_launch_dependents();
     const int seq = blockIdx.z, head = blockIdx.x;
@@ -176,9 +200,10 @@ __global__ void __launch_bounds__(THREADS, BKEY == 64 ? 2 : 1) attention_prefill
     const int q0 = ((int)gridDim.y - 1 - (int)blockIdx.y) * BQ;
     if (q0 >= q_len) return;                              // uniform for the block, before any barrier or allocation
     const int rows = min(BQ, q_len - q0);
-    const int past = p.seq_past[seq];
+    const int past = DENSE ? 0 : p.seq_past[seq];
     const int kvh = head / (p.nq / p.nkv);
-    const int* table = p.block_table + (size_t)seq * p.max_blocks;
+    const int* table = DENSE ? nullptr : p.block_table + (size_t)seq * p.max_blocks;
+    const int kv_row = (q_begin / PAGE + seq) * PAGE;     // DENSE: the sequence's first row; runs of whole pages, apart for distinct sequences
     const int p_first = past + q0, p_last = past + q0 + rows - 1;
     const int lo = max(p.window > 0 ? max(0, p_first - p.window + 1) : 0, p.chunk > 0 ? p_first / p.chunk * p.chunk : 0);
     const int vh = kvh % p.nv;
@@ -188,13 +213,13 @@ __global__ void __launch_bounds__(THREADS, BKEY == 64 ? 2 : 1) attention_prefill
     extern __shared__ uint8_t smem_raw[];
     const uint32_t raw = smem_u32(smem_raw);
     const uint32_t base = (raw + 1023u) & ~1023u;
-    if (base - raw > ALIGN_SLACK) {                       // the launch asked for less slack than this base needs: refuse, uniformly
+    if (base - raw > ALIGN_SLACK<HD>) {                       // the launch asked for less slack than this base needs: refuse, uniformly
         if (threadIdx.x == 0) atomicCAS(p.status, 0, 5);
         return;
     }
     uint8_t* smem = smem_raw + (base - raw);
-    const uint32_t q_s = base, k_s = q_s + Q_BYTES, v_s = k_s + 2 * KV_BYTES;
-    const uint32_t bars = v_s + 2 * KV_BYTES;
+    const uint32_t q_s = base, k_s = q_s + Q_BYTES, v_s = k_s + 2 * K_BYTES;
+    const uint32_t bars = v_s + V_STAGES * V_BYTES;
     // barriers: q_full, k_full[2], k_empty[2], v_full[2], v_empty[2], s_full[2], p_full[2], pv_full[2]
     const uint32_t q_full = bars, k_full = bars + 8, k_empty = bars + 24, v_full = bars + 40, v_empty = bars + 56;
     const uint32_t s_full = bars + 72, p_full = bars + 88, pv_full = bars + 104;
@@ -232,11 +257,12 @@ __global__ void __launch_bounds__(THREADS, BKEY == 64 ? 2 : 1) attention_prefill
                 const int s = j & 1;
                 const uint32_t phase = (uint32_t)(j >> 1) & 1u;
                 if (!mbar_wait(k_empty + 8 * s, phase ^ 1u, status, 1)) break;
-                mbar_expect_tx(k_full + 8 * s, KV_BYTES);
+                mbar_expect_tx(k_full + 8 * s, K_BYTES);
                 for (int pg = 0; pg < PAGES; ++pg) {
-                    const int row0 = (cache_page(table, p.max_blocks, (tile_begin + j) * PAGES + pg, p.ring_tokens) * p.nkv + kvh) * PAGE;
+                    const int page = (tile_begin + j) * PAGES + pg;
+                    const int row0 = DENSE ? kv_row + page * PAGE : (cache_page(table, p.max_blocks, page, p.ring_tokens) * p.nkv + kvh) * PAGE;
                     for (int h = 0; h < HALVES; ++h)
-                        tma_load_2d(k_s + s * KV_BYTES + h * KEY_HALF_BYTES + pg * (PAGE * 128), &map_k, k_full + 8 * s, h * 64, row0);
+                        tma_load_2d(k_s + s * K_BYTES + h * KEY_HALF_BYTES + pg * (PAGE * 128), &map_k, k_full + 8 * s, (DENSE ? head * HD : 0) + h * 64, row0);
                 }
             }
         }
@@ -244,14 +270,15 @@ __global__ void __launch_bounds__(THREADS, BKEY == 64 ? 2 : 1) attention_prefill
         if (lane == 0) {
             pdl_wait();
             for (int j = 0; j < n_tiles; ++j) {
-                const int s = j & 1;
-                const uint32_t phase = (uint32_t)(j >> 1) & 1u;
+                const int s = j % V_STAGES;
+                const uint32_t phase = (uint32_t)(j / V_STAGES) & 1u;
                 if (!mbar_wait(v_empty + 8 * s, phase ^ 1u, status, 1)) break;
-                mbar_expect_tx(v_full + 8 * s, KV_BYTES);
+                mbar_expect_tx(v_full + 8 * s, V_BYTES);
                 for (int pg = 0; pg < PAGES; ++pg) {
-                    const int row0 = (cache_page(table, p.max_blocks, (tile_begin + j) * PAGES + pg, p.ring_tokens) * p.nv + vh) * PAGE;
-                    for (int h = 0; h < HALVES; ++h)
-                        tma_load_2d(v_s + s * KV_BYTES + h * KEY_HALF_BYTES + pg * (PAGE * 128), &map_v, v_full + 8 * s, h * 64, row0);
+                    const int page = (tile_begin + j) * PAGES + pg;
+                    const int row0 = DENSE ? kv_row + page * PAGE : (cache_page(table, p.max_blocks, page, p.ring_tokens) * p.nv + vh) * PAGE;
+                    for (int h = 0; h < V_HALVES; ++h)
+                        tma_load_2d(v_s + s * V_BYTES + h * KEY_HALF_BYTES + pg * (PAGE * 128), &map_v, v_full + 8 * s, (DENSE ? p.v_col + head * HDV : 0) + h * 64, row0);
                 }
             }
         }
@@ -270,7 +297,7 @@ __global__ void __launch_bounds__(THREADS, BKEY == 64 ? 2 : 1) attention_prefill
                 // pipe runs its instructions in order
                 tc_fence_after();
                 const uint32_t acc = tmem_base + (s ? S_COL1 : S_COL0);
-                const uint64_t k_desc = k_desc0 + (uint64_t)(s * (KV_BYTES >> 4));
+                const uint64_t k_desc = k_desc0 + (uint64_t)(s * (K_BYTES >> 4));
 #pragma unroll
                 for (int ks = 0; ks < HD / 16; ++ks) {    // 16 dims per MMA; 4 MMAs per 64-column half
                     const uint32_t in_half = (uint32_t)(ks & 3) * 32u;
@@ -286,9 +313,10 @@ __global__ void __launch_bounds__(THREADS, BKEY == 64 ? 2 : 1) attention_prefill
                 if (j + 1 < n_tiles) { ok = issue_qk(j + 1); if (!ok) break; }
                 const int s = j & 1;
                 if (!mbar_wait(p_full + 8 * s, (uint32_t)(j >> 1) & 1u, status, 2)) break;
-                if (!mbar_wait(v_full + 8 * s, (uint32_t)(j >> 1) & 1u, status, 2)) break;
+                const int vs = j % V_STAGES;
+                if (!mbar_wait(v_full + 8 * vs, (uint32_t)(j / V_STAGES) & 1u, status, 2)) break;
                 tc_fence_after();
-                const uint64_t v_desc = v_desc0 + (uint64_t)(s * (KV_BYTES >> 4));
+                const uint64_t v_desc = v_desc0 + (uint64_t)(vs * (V_BYTES >> 4));
                 const uint32_t p_tmem = tmem_base + (s ? S_COL1 : S_COL0);     // P lies over the scores it came from
 #pragma unroll
                 for (int ks = 0; ks < BKEY / 16; ++ks) {  // 16 keys per MMA = 8 columns of packed pairs
@@ -296,7 +324,7 @@ __global__ void __launch_bounds__(THREADS, BKEY == 64 ? 2 : 1) attention_prefill
                     umma_bf16_a_tmem(tmem_base + O_COL, p_tmem + (uint32_t)(ks * 8), b_desc, IDESC_PV, (j > 0 || ks > 0) ? 1u : 0u);    // O accumulates over the tiles
                 }
                 umma_commit(pv_full + 8 * s);
-                umma_commit(v_empty + 8 * s);
+                umma_commit(v_empty + 8 * vs);
             }
         }
     } else if (warp < 6) {
@@ -378,7 +406,7 @@ __global__ void __launch_bounds__(THREADS, BKEY == 64 ? 2 : 1) attention_prefill
                 tc_fence_after();
                 {
 #pragma unroll 1
-                    for (int c0 = 0; c0 < HD; c0 += 32) {
+                    for (int c0 = 0; c0 < HDV; c0 += 32) {
                         uint32_t o[32];
                         tmem_load32(lane_addr + O_COL + (uint32_t)c0, o);
 #pragma unroll
@@ -403,7 +431,7 @@ __global__ void __launch_bounds__(THREADS, BKEY == 64 ? 2 : 1) attention_prefill
                         unpair_f32(fma2(pair_u32(v[2 * h + q][c], v[2 * h + q][c + 1]), scale22, neg_m2), x0, x1);
                         const float e0 = fast_exp2(x0), e1 = fast_exp2(x1);
                         sum2[(c >> 1) & 1] = add2(sum2[(c >> 1) & 1], pair_f32(e0, e1));
-                        packed[q * 16 + (c >> 1)] = pack_bf16(e0, e1);
+                        packed[q * 16 + (c >> 1)] = DENSE ? pack_half(e0, e1) : pack_bf16(e0, e1);
                     }
                 tmem_store32(s_addr + (uint32_t)(h * 32), packed);
             }
@@ -427,12 +455,35 @@ __global__ void __launch_bounds__(THREADS, BKEY == 64 ? 2 : 1) attention_prefill
                 l_run = l_run * factor + fast_exp2(s2 - top);
             }
             const float inv = factor / l_run;
-            __nv_bfloat16* dst = p.out + ((size_t)(q_begin + q0 + r) * p.nq + head) * HD;
+            __nv_bfloat16* dst = p.out + ((size_t)(q_begin + q0 + r) * p.nq + head) * HDV;
 #pragma unroll 1
-            for (int c0 = 0; c0 < HD; c0 += 32) {
+            for (int c0 = 0; c0 < HDV; c0 += 32) {
                 uint32_t o[32];
                 tmem_load32(lane_addr + O_COL + (uint32_t)c0, o);
                 if (r < rows) {
+                    if (DENSE && p.gate) {                // ahead of the one rounding of the result
+                        const float* gate = p.gate + (size_t)(q_begin + q0 + r) * p.gate_cols + p.gate_offset + (p.gate_per_head ? head : head * HDV + c0);
+                        if (p.gate_per_head) {
+                            float g = __ldg(gate);
+                            for (int sp = 1; sp < p.gate_splits; ++sp) g += __ldg(gate + sp * p.gate_split_stride);
+                            const float f = 1.f / (1.f + expf(-g));
+#pragma unroll
+                            for (int c = 0; c < 32; ++c) o[c] = __float_as_uint(__uint_as_float(o[c]) * f);
+                        } else {
+#pragma unroll
+                            for (int c = 0; c < 32; c += 4) {
+                                float4 g = __ldg(reinterpret_cast<const float4*>(gate + c));
+                                for (int sp = 1; sp < p.gate_splits; ++sp) {
+                                    const float4 more = __ldg(reinterpret_cast<const float4*>(gate + sp * p.gate_split_stride + c));
+                                    g.x += more.x; g.y += more.y; g.z += more.z; g.w += more.w;
+                                }
+                                o[c] = __float_as_uint(__uint_as_float(o[c]) / (1.f + expf(-g.x)));
+                                o[c + 1] = __float_as_uint(__uint_as_float(o[c + 1]) / (1.f + expf(-g.y)));
+                                o[c + 2] = __float_as_uint(__uint_as_float(o[c + 2]) / (1.f + expf(-g.z)));
+                                o[c + 3] = __float_as_uint(__uint_as_float(o[c + 3]) / (1.f + expf(-g.w)));
+                            }
+                        }
+                    }
 #pragma unroll
                     for (int c = 0; c < 32; c += 8) {
                         uint4 w;
@@ -457,20 +508,20 @@ __global__ void __launch_bounds__(THREADS, BKEY == 64 ? 2 : 1) attention_prefill
     }
 }
 
-template <int HD, int BKEY, bool PEN, int CAP>
+template <int HD, int HDV, int BKEY, bool PEN, int CAP, bool DENSE>
 int launch(const CUtensorMap& map_q, const CUtensorMap& map_k, const CUtensorMap& map_v, const TcAttnParams& p, int n_seqs,
            int max_q_len, cudaStream_t stream) {
-    constexpr uint32_t HALVES = HD / 64;
-    // Q, two key and two value tiles, alignment slack, barriers
-    const size_t smem = (size_t)HALVES * HALF_BYTES + 4 * (size_t)HALVES * BKEY * 128 + ALIGN_SLACK + 128 + 64;
+    // Q, two key tiles, the value tiles, alignment slack, barriers
+    const size_t smem = (size_t)(HD / 64) * HALF_BYTES + 2 * (size_t)(HD / 64) * BKEY * 128 + (HD > 128 ? 1 : 2) * (size_t)(HDV / 64) * BKEY * 128 + ALIGN_SLACK<HD> +
+                        128 + 64;
     static bool configured = false;
     if (!configured) {
-        cudaError_t err = cudaFuncSetAttribute(attention_prefill_tc_kernel<HD, BKEY, PEN, CAP>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+        cudaError_t err = cudaFuncSetAttribute(attention_prefill_tc_kernel<HD, HDV, BKEY, PEN, CAP, DENSE>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
         if (err != cudaSuccess) QT_FAIL(QT_ERR_LAUNCH, "attention_prefill_tc: cannot raise shared memory: %s", cudaGetErrorString(err));
         configured = true;
     }
     dim3 grid(p.nq, (max_q_len + BQ - 1) / BQ, n_seqs);
-    launch_kernel(attention_prefill_tc_kernel<HD, BKEY, PEN, CAP>, grid, dim3(THREADS), smem, stream, map_q, map_k, map_v, p);
+    launch_kernel(attention_prefill_tc_kernel<HD, HDV, BKEY, PEN, CAP, DENSE>, grid, dim3(THREADS), smem, stream, map_q, map_k, map_v, p);
     QT_CHECK_LAUNCH("attention_prefill_tc");
     return QT_OK;
 }
@@ -509,19 +560,50 @@ extern "C" int qt_attention_prefill_tc(const void* q, const void* k_cache, const
     rc = tensor_map(&map_v, v_cache, (uint64_t)n_pages * nv * PAGE, (uint64_t)d, PAGE);
     if (rc) return rc;
     TcAttnParams p{(__nv_bfloat16*)out, block_table, max_blocks, seq_start, seq_past, nq, nkv, ring_tokens, window, chunk, nv, scale, status, r1, r2,
-                   sink, sinks, softcap};
+                   sink, sinks, softcap, 0, nullptr, 1, 0, 0, 0, 0};
     cudaStream_t s = (cudaStream_t)stream;
     // key tiles of one page, two blocks per SM: measured 12-22 % faster than tiles of two pages with one block per SM
 #define QT_LAUNCH_TC(PEN, CAP)                                                                      \
     do {                                                                                            \
-        if (d == 64) return launch<64, 64, PEN, CAP>(map_q, map_k, map_v, p, n_seqs, max_q_len, s); \
-        return launch<128, 64, PEN, CAP>(map_q, map_k, map_v, p, n_seqs, max_q_len, s);             \
+        if (d == 64) return launch<64, 64, 64, PEN, CAP, false>(map_q, map_k, map_v, p, n_seqs, max_q_len, s); \
+        return launch<128, 128, 64, PEN, CAP, false>(map_q, map_k, map_v, p, n_seqs, max_q_len, s);             \
     } while (0)
     if (r1) QT_LAUNCH_TC(true, CAP_NONE);
     if (softcap > 0.f && cap_small) QT_LAUNCH_TC(false, CAP_SMALL);
     if (softcap > 0.f) QT_LAUNCH_TC(false, CAP_ANY);
     QT_LAUNCH_TC(false, CAP_NONE);
 #undef QT_LAUNCH_TC
+}
+
+// Causal attention of packed sequences that start at position 0, every head with keys and values of its own: q [n_tokens, heads, dk], kv
+// [kv_rows, heads * dk + heads * dv] (a row's keys by head, then its values by head) in halves, out [n_tokens, heads, dv] bfloat16.  The tokens of
+// sequence i are the rows from 64 (seq_start[i] / 64 + i) on; its last run of 64 rows is filled up with finite numbers.  gate [gate_splits, n_tokens,
+// gate_cols] float or null: the result is multiplied by the sigmoid of the sums of the columns from gate_offset on (one a head or one an element).
+extern "C" int qt_attention_prefill_rows(const void* q, const void* kv, void* out, int n_tokens, int kv_rows, const int* seq_start, int n_seqs, int max_q_len,
+                                         int heads, int dk, int dv, int window, float scale, const float* gate, int gate_splits, long long gate_split_stride,
+                                         int gate_cols, int gate_offset, int gate_per_head, int* status, void* stream) {
+    if (n_seqs == 0 || max_q_len == 0) return QT_OK;
+    QT_REQUIRE(n_seqs > 0 && heads > 0 && n_tokens > 0 && (dk == 128 || dk == 192) && (dv == 64 || dv == 128),
+               "attention_prefill_rows: %d heads of %d and %d (this kernel takes 128 or 192 and 64 or 128)", heads, dk, dv);
+    QT_REQUIRE(n_seqs <= 65535 && (max_q_len + BQ - 1) / BQ <= 65535 && kv_rows >= (n_tokens / PAGE + n_seqs) * PAGE, "attention_prefill_rows: %d rows for %d tokens of %d sequences",
+               kv_rows, n_tokens, n_seqs);
+    QT_REQUIRE(status != nullptr && window >= 0 && scale > 0.f, "attention_prefill_rows: a status word and a positive scale are required");
+    QT_REQUIRE((((uintptr_t)q | (uintptr_t)kv | (uintptr_t)out) & 15) == 0, "attention_prefill_rows: operands must be 16-byte aligned");
+    QT_REQUIRE(!gate || (gate_splits >= 1 && gate_offset >= 0 && gate_offset + heads * (gate_per_head ? 1 : dv) <= gate_cols &&
+                         (gate_per_head || (((uintptr_t)gate & 15) == 0 && gate_offset % 4 == 0 && gate_cols % 4 == 0 && gate_split_stride % 4 == 0))),
+               "attention_prefill_rows: a gate at column %d of %d", gate_offset, gate_cols);
+    CUtensorMap map_q, map_kv;
+    int rc = tensor_map(&map_q, q, (uint64_t)n_tokens, (uint64_t)heads * dk, BQ);
+    if (rc) return rc;
+    rc = tensor_map(&map_kv, kv, (uint64_t)kv_rows, (uint64_t)heads * (dk + dv), PAGE);
+    if (rc) return rc;
+    TcAttnParams p{(__nv_bfloat16*)out, nullptr, 0, seq_start, nullptr, heads, heads, 0, window, 0, heads, scale, status, nullptr, nullptr, 0, nullptr, 0.f, heads * dk, gate,
+                   gate_splits, (size_t)gate_split_stride, gate_cols, gate_offset, gate_per_head};
+    cudaStream_t s = (cudaStream_t)stream;
+    if (dk == 128 && dv == 64) return launch<128, 64, 64, false, CAP_NONE, true>(map_q, map_kv, map_kv, p, n_seqs, max_q_len, s);
+    if (dk == 128) return launch<128, 128, 64, false, CAP_NONE, true>(map_q, map_kv, map_kv, p, n_seqs, max_q_len, s);
+    if (dv == 64) return launch<192, 64, 64, false, CAP_NONE, true>(map_q, map_kv, map_kv, p, n_seqs, max_q_len, s);
+    return launch<192, 128, 64, false, CAP_NONE, true>(map_q, map_kv, map_kv, p, n_seqs, max_q_len, s);
 }
 
 QT_DEFINE_LAST_ERROR(attention_tc)

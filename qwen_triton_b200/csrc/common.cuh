@@ -7,6 +7,7 @@
 #pragma once
 
 #include <cuda_bf16.h>
+#include <cuda_fp16.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
 #include <stdio.h>
@@ -22,6 +23,7 @@
 // element types of activations, weights and caches
 #define QT_F32 0
 #define QT_BF16 1
+#define QT_F16 2      // only where a kernel says so
 
 namespace qt {
 
@@ -140,6 +142,11 @@ __device__ __forceinline__ float to_float(__nv_bfloat16 v) { return __bfloat162f
 template <typename T> __device__ __forceinline__ T from_float(float v);
 template <> __device__ __forceinline__ float from_float<float>(float v) { return v; }
 template <> __device__ __forceinline__ __nv_bfloat16 from_float<__nv_bfloat16>(float v) { return __float2bfloat16_rn(v); }
+// Halves end at 65,504: finite numbers beyond become that, so that no infinity arises that bfloat16 would not have.
+template <> __device__ __forceinline__ __half from_float<__half>(float v) {
+    const float size = fabsf(v);
+    return __float2half_rn(size > 65504.f && size < INFINITY ? copysignf(65504.f, v) : v);
+}
 
 // Gate activations of a gated feed-forward, out = act(gate) * up (a parameter of the part, a code here).
 #define QT_ACT_SILU 0

@@ -314,6 +314,12 @@ template <> __device__ __forceinline__ void store8<float>(float* dst, const floa
     reinterpret_cast<float4*>(dst)[0] = make_float4(f[0], f[1], f[2], f[3]);
     reinterpret_cast<float4*>(dst)[1] = make_float4(f[4], f[5], f[6], f[7]);
 }
+template <> __device__ __forceinline__ void store8<__half>(__half* dst, const float (&f)[8]) {
+    __half h[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) h[i] = from_float<__half>(f[i]);
+    *reinterpret_cast<uint4*>(dst) = *reinterpret_cast<const uint4*>(h);
+}
 template <> __device__ __forceinline__ void store8<__nv_bfloat16>(__nv_bfloat16* dst, const float (&f)[8]) {
     uint4 packed;
     __nv_bfloat162 h;
@@ -758,7 +764,7 @@ extern "C" int qt_gemm_tc(const void* x, const void* w, void* out, int out_dtype
     QT_FAIL(QT_ERR_ARG, "gemm_tc: unknown output type %d", out_dtype);
 }
 
-// The same product by pairs of blocks (see gemm_tc_pair_kernel): bfloat16 or float output, meant for many tokens (a
+// The same product by pairs of blocks (see gemm_tc_pair_kernel): bfloat16 or float output (without `swiglu` and splits also halves), meant for many tokens (a
 // pair covers 256 weight rows x 256 tokens); out[splits, M, N] in float when `splits` > 1, under the rule above.  With `swiglu` the weight's rows alternate 16 of a gate and
 // 16 of an up projection and `out` is [M, N / 2] = act(gate) * up (`act`: one of QT_ACT_*); `swiglu` 2: `out` [M, N] = act(product).  Codes in `status`: as above, 4 = the MMA issuer
 // waiting for the epilogues to free an accumulator.
@@ -791,6 +797,7 @@ extern "C" int qt_gemm_tc_pair(const void* x, const void* w, void* out, int out_
     if (out_dtype == QT_BF16 && swiglu == ACTIVATED)
         return launch_pair<__nv_bfloat16, ACTIVATED>(map_w, map_x, (__nv_bfloat16*)out, M, N, kb_total, 1, 0, act, 0.f, tail, tail_scratch, tail_flags, tail_pairs, bias, status, s);
     if (out_dtype == QT_BF16 && swiglu) return launch_pair<__nv_bfloat16, GATED>(map_w, map_x, (__nv_bfloat16*)out, M, N, kb_total, 1, 0, act, limit, tail, tail_scratch, tail_flags, tail_pairs, bias, status, s);
+    if (out_dtype == QT_F16 && !swiglu) return launch_pair<__half, PLAIN>(map_w, map_x, (__half*)out, M, N, kb_total, 1, 0, 0, 0.f, tail, tail_scratch, tail_flags, tail_pairs, bias, status, s);
     if (out_dtype == QT_BF16) return launch_pair<__nv_bfloat16, PLAIN>(map_w, map_x, (__nv_bfloat16*)out, M, N, kb_total, 1, 0, 0, 0.f, tail, tail_scratch, tail_flags, tail_pairs, bias, status, s);
     if (out_dtype == QT_F32 && !swiglu) return launch_pair<float, PLAIN>(map_w, map_x, (float*)out, M, N, kb_total, splits, (size_t)split_stride, 0, 0.f, tail, tail_scratch, tail_flags, tail_pairs, bias, status, s);
     QT_FAIL(QT_ERR_ARG, "gemm_tc_pair: output type %d%s is not offered", out_dtype, swiglu ? " with the SiLU-gated epilogue" : "");

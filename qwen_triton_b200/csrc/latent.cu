@@ -11,6 +11,7 @@
 //                         query latent -> cq_out; RMS norm of the key/value latent and rotation of the shared key part
 //                         by the token's position -> the cache row.
 // latent_query_rot_kernel the rotated part of every head's query: rotation by position into the query rows.
+// latent_rows_kernel, latent_queries_kernel   the operands of a prompt whose keys and values are formed per head (attention_tc.cu)
 // head_product_kernel     Y[t, h, n] = sum_k X[t, h, k] W[h, n, k] for every head with its own matrix (float sums), with
 //                         strides for X and Y and optionally times sigmoid(gate[t, h * N + n]) or sigmoid(gate[t, h]).
 // head_product_mma_kernel the same on the tensor cores (mma.sync m16n8k16) for bfloat16 matrices and results.
@@ -156,6 +157,103 @@ extern "C" int qt_latent_query_rot(const void* q, int in_dtype, int n_splits, lo
     else QT_FAIL(QT_ERR_ARG, "latent_query_rot: element types %d/%d", in_dtype, out_dtype);
 #undef QT_LAUNCH_ROT
     QT_CHECK_LAUNCH("latent_query_rot");
+    return QT_OK;
+}
+
+// ----------------------------------------------------------------------------- prompts with keys and values per head
+// The cached rows of a step's sequences, all from position 0 on, side by side: rows [64 (seq_start[i] / 64 + i) + position, row], the last run
+// of 64 of a sequence filled up with zeros.  A run is a page of the cache.  grid (runs of the longest sequence, sequences).
+__global__ void __launch_bounds__(256) latent_rows_kernel(const uint4* __restrict__ cache, uint4* __restrict__ rows, const int* __restrict__ block_table,
+                                                          int max_blocks, const int* __restrict__ seq_start, int pieces, int ring_pages) {
+    pdl_launch_dependents();
+    pdl_wait();
+    const int seq = blockIdx.y, run = blockIdx.x, begin = seq_start[seq], count = seq_start[seq + 1] - begin;
+    const int live = min(64, count - run * 64);
+    if (live <= 0) return;
+    const int page = block_table[(size_t)seq * max_blocks + (ring_pages ? run % ring_pages : run)];
+    const uint4* from = cache + (size_t)page * 64 * pieces;
+    uint4* to = rows + (size_t)(begin / 64 + seq + run) * 64 * pieces;
+#pragma unroll 4
+    for (int i = threadIdx.x; i < 64 * pieces; i += 256) to[i] = i < live * pieces ? from[i] : make_uint4(0u, 0u, 0u, 0u);
+}
+
+extern "C" int qt_latent_rows(const void* cache, void* rows, const int* block_table, int max_blocks, const int* seq_start, int n_seqs, int max_tokens, int row,
+                              int page_tokens, int ring_tokens, void* stream) {
+    QT_REQUIRE(n_seqs >= 0 && n_seqs <= 65535 && max_tokens >= 0 && row > 0 && row % 8 == 0 && page_tokens == 64 && ring_tokens % 64 == 0, "latent_rows: bad sizes");
+    QT_REQUIRE((((uintptr_t)cache | (uintptr_t)rows) & 15) == 0 && (max_tokens + 63) / 64 <= (ring_tokens ? ring_tokens / 64 : max_blocks),
+               "latent_rows: %d tokens in %d pages", max_tokens, ring_tokens ? ring_tokens / 64 : max_blocks);
+    if (n_seqs == 0 || max_tokens == 0) return QT_OK;
+    launch_kernel(latent_rows_kernel, dim3((max_tokens + 63) / 64, n_seqs), dim3(256), 0, (cudaStream_t)stream, (const uint4*)cache, (uint4*)rows, block_table,
+                  max_blocks, seq_start, row / 8, ring_tokens / 64);
+    QT_CHECK_LAUNCH("latent_rows");
+    return QT_OK;
+}
+
+// q [splits, T, q_cols >= heads * (dim + rot)] -> out [T, heads, out_row] halves: a head's dim elements, its rot elements turned by the
+// token's position, zeros up to out_row.  A thread takes eight neighbouring elements of a head (all of dim, rot, rotary_dim / 2 and
+// out_row are multiples of 8).
+__device__ __forceinline__ void sum_eight(const float* p, int n_splits, size_t stride, float (&v)[8]) {
+#pragma unroll
+    for (int i = 0; i < 8; ++i) v[i] = 0.f;
+    for (int s = 0; s < n_splits; ++s) {
+        const float4 a = __ldg(reinterpret_cast<const float4*>(p + (size_t)s * stride)), b = __ldg(reinterpret_cast<const float4*>(p + (size_t)s * stride) + 1);
+        v[0] += a.x; v[1] += a.y; v[2] += a.z; v[3] += a.w; v[4] += b.x; v[5] += b.y; v[6] += b.z; v[7] += b.w;
+    }
+}
+__device__ __forceinline__ void sum_eight(const __nv_bfloat16* p, int, size_t, float (&v)[8]) {
+    const uint4 raw = __ldg(reinterpret_cast<const uint4*>(p));
+    const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&raw);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) { v[2 * i] = __low2float(h[i]); v[2 * i + 1] = __high2float(h[i]); }
+}
+
+template <typename TI>
+__global__ void __launch_bounds__(256) latent_queries_kernel(const TI* __restrict__ q, int n_splits, size_t split_stride, int q_cols, const float* __restrict__ cos_sin,
+                                                             int rotary_dim, const int* __restrict__ token_pos, uint4* __restrict__ out, long long pieces,
+                                                             int heads, int dim, int rot, int out_row) {
+    pdl_launch_dependents();
+    pdl_wait();
+    const long long at = (long long)blockIdx.x * 256 + threadIdx.x;
+    if (at >= pieces) return;
+    const int per_head = out_row / 8, c = (int)(at % per_head) * 8, half = rotary_dim / 2;
+    const long long th = at / per_head;
+    const int h = (int)(th % heads);
+    const long long t = th / heads;
+    const TI* head = q + (size_t)t * q_cols + (size_t)h * (dim + rot);
+    float v[8] = {};
+    if (c < dim + rot) sum_eight(head + c, n_splits, split_stride, v);
+    const int i = c - dim;
+    if (i >= 0 && i < rotary_dim) {
+        const bool low = i < half;
+        const int pair = low ? i : i - half;
+        float other[8], cs[8], sn[8];
+        sum_eight(head + (low ? c + half : c - half), n_splits, split_stride, other);
+        const float* table = cos_sin + (size_t)token_pos[t] * rotary_dim + pair;
+        sum_eight(table, 1, 0, cs);
+        sum_eight(table + half, 1, 0, sn);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) v[j] = low ? v[j] * cs[j] - other[j] * sn[j] : v[j] * cs[j] + other[j] * sn[j];
+    }
+    __align__(16) __half rounded[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) rounded[j] = from_float<__half>(v[j]);
+    out[at] = *reinterpret_cast<const uint4*>(rounded);
+}
+
+extern "C" int qt_latent_queries(const void* q, int in_dtype, int n_splits, long long split_stride, int q_cols, const float* cos_sin, int rotary_dim,
+                                 const int* token_pos, void* out, int n_tokens, int heads, int dim, int rot, int out_row, void* stream) {
+    QT_REQUIRE(n_tokens >= 0 && heads > 0 && dim > 0 && rot >= 0 && dim + rot <= out_row && q_cols >= heads * (dim + rot), "latent_queries: bad sizes");
+    QT_REQUIRE(dim % 8 == 0 && rot % 8 == 0 && out_row % 8 == 0 && q_cols % 8 == 0 && rotary_dim % 16 == 0 && rotary_dim <= rot && split_stride % 4 == 0 &&
+               (((uintptr_t)q | (uintptr_t)out | (uintptr_t)cos_sin) & 15) == 0, "latent_queries: heads of %d + %d (%d turn) are not whole 16-byte pieces", dim, rot, rotary_dim);
+    if (n_tokens == 0) return QT_OK;
+    const long long pieces = (long long)n_tokens * heads * (out_row / 8);
+    const dim3 grid((unsigned)((pieces + 255) / 256));
+    cudaStream_t s = (cudaStream_t)stream;
+    if (in_dtype == QT_F32) launch_kernel(latent_queries_kernel<float>, grid, dim3(256), 0, s, (const float*)q, n_splits, (size_t)split_stride, q_cols, cos_sin, rotary_dim,
+                                          token_pos, (uint4*)out, pieces, heads, dim, rot, out_row);
+    else launch_kernel(latent_queries_kernel<__nv_bfloat16>, grid, dim3(256), 0, s, (const __nv_bfloat16*)q, n_splits, (size_t)split_stride, q_cols, cos_sin, rotary_dim,
+                       token_pos, (uint4*)out, pieces, heads, dim, rot, out_row);
+    QT_CHECK_LAUNCH("latent_queries");
     return QT_OK;
 }
 

@@ -58,6 +58,7 @@ class StepContext:
         self.n_tokens = self.n_seqs = self.n_want = 0
         self.max_q_len = 0
         self.max_context = 0       # longest sequence after this pass
+        self.from_start = False    # every sequence of the pass starts at position 0
         self.is_decode = False
         self.token_ids = self.token_seq = self.token_pos = None
         self.seq_start = self.seq_past = self.seq_len = self.slots = self.want_rows = None
@@ -110,6 +111,7 @@ class StepContext:
         self.max_q_len = max(q_lens) if q_lens else 0
         self.max_context = max_context if max_context is not None else (int(seq_len.max()) if n_seqs else 0)
         self.is_decode = bool(q_lens) and all(q == 1 for q in q_lens)
+        self.from_start = not past_arr.any()
 
     # ------------------------------------------------------------------ one token per sequence
     def prepare_decode(self, slots: list[int], past: list[int], tables: list[np.ndarray]):
@@ -151,7 +153,7 @@ class StepContext:
         self.n_tokens = self.n_seqs = self.n_want = n
         self.max_q_len = 1
         self.max_context = max_context
-        self.is_decode = True
+        self.is_decode, self.from_start = True, False
 
 
 class _DecodePlan:

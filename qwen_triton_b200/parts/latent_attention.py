@@ -22,7 +22,8 @@ A rotation of neighbouring pairs (2i, 2i + 1) becomes one of (i, i + dims / 2) w
 query's and of the shared key part's matrices are put in that order, which changes no score.
 
 Norms, rotation (float cos/sin table), scores, softmax and the gate are float; the query latent, the queries, the cache
-rows and the heads' outputs are rounded to the activation type between the products.
+rows and the heads' outputs are rounded to the activation type between the products (in a prompt that forms keys and values per head, queries,
+keys and values to halves).
 
 Parameters: ``hidden_size``, ``num_heads``, ``head_dim``, ``rot_dim``, ``v_head_dim``, ``q_rank``, ``kv_rank``, ``scale``, ``eps``,
 ``position`` (a position part over ``rot_dim``; either pairing), ``window``, ``own_kv``, ``gate``, ``float_out``, and the tensor-name pieces ``dq``, ``uq``
@@ -39,6 +40,7 @@ from .base import DeferredProduct, KVRequest, Runtime, part_class, register_mixe
 from .linear import Linear
 
 
+_EXPAND_TOKENS = 64      # longest portion from which a prompt forms keys and values per head
 _MANY_TOKENS = 256       # steps of more tokens form the queries and the cache rows in products of their own (without a query latent)
 
 
@@ -90,7 +92,17 @@ class LatentAttention:
         ws.declare("latent.heads", tokens * self.heads * self.dv, runtime.dtype)
         ws.declare("attn.part_acc", _MAX_SPLIT_PAIRS * self.heads * self.rank, torch.float32)
         ws.declare("attn.part_ml", _MAX_SPLIT_PAIRS * self.heads * 2, torch.float32)
-        self.q_norm = self.kv_norm = self.uk_t = self.uv = None
+        # Prompts from position 0 on form every head's keys and values from the cached rows in one product and run over those (forward)
+        turning = getattr(self.position, "rotary_dim", 0)
+        self.key = 128 if self.d + self.rot <= 128 else 192                     # a head's query and key there, filled up with zeros
+        self.expands = (runtime.dtype == torch.bfloat16 and runtime.page_tokens == 64 and self.d + self.rot <= 192 and self.dv in (64, 128) and self.scale > 0
+                        and self.d % 8 == 0 and self.rot % 8 == 0 and turning % 16 == 0 and self.row % 8 == 0 and self.at_kv % 8 == 0)
+        self.most_runs = tokens // 64 + 64
+        if self.expands:
+            ws.declare("latent.rows", 64 * self.most_runs * self.row, runtime.dtype)
+            ws.declare("latent.keys_values", 64 * self.most_runs * self.heads * (self.key + self.dv), torch.float16)
+            ws.declare("latent.queries", tokens * self.heads * self.key, torch.float16)
+        self.q_norm = self.kv_norm = self.uk_t = self.uv = self.expand = None
 
     # ------------------------------------------------------------------ weights
     @staticmethod
@@ -154,6 +166,14 @@ class LatentAttention:
         # query part into the latent's space; W_uv is stored as that product's matrix already: [heads, v_head_dim, kv_rank]
         self.uk_t = to_device(source(n["uk"]).view(self.heads, self.d, self.rank).transpose(1, 2), dtype, device)
         self.uv = to_device(source(n["uv"]).view(self.heads, self.dv, self.rank), dtype, device)
+        if self.expands:
+            # [heads * key | heads * dv, row]: W_uk of a head on the latent, ones that hand its shared rotated part on, zero rows; then W_uv
+            expand = torch.zeros(self.heads * (self.key + self.dv), self.row, dtype=dtype, device=device)
+            keys = expand[:self.heads * self.key].view(self.heads, self.key, self.row)
+            keys[:, :self.d, :self.rank] = self.uk_t.transpose(1, 2)
+            keys[:, self.d:self.d + self.rot, self.rank:] = torch.eye(self.rot, dtype=dtype, device=device)
+            expand[self.heads * self.key:].view(self.heads, self.dv, self.row)[:, :, :self.rank] = self.uv
+            self.expand = expand
         tables = self.runtime.options.setdefault("position_tables", {})
         key = self.position.key() + (self.runtime.max_positions,)
         if key not in tables:
@@ -182,6 +202,32 @@ class LatentAttention:
         return max(1, min(most, (2 * self.runtime.sm_count) // max(blocks, 1)))
 
     # ------------------------------------------------------------------ run
+    def _expands_for(self, ctx, tokens: int) -> bool:
+        """Whether a step forms keys and values per head: where all its sequences start at position 0, one of them is long enough and the
+        scratch holds their runs.  Over latent rows a query and key cost rank + rot and rank multiplications, over keys and values
+        of its own d + rot and dv (a third), at the price of one product over the step's tokens.  16 heads of
+        128 + 64 over rows of 512 + 64, two layers with their own products, over rows / over keys and values of its own: 2,000 tokens
+        1,001 / 294 us, 2 x 600 tokens 374 / 200, 32 x 100 tokens 617 / 395, one of 64 tokens 159 / 145; 32 x 32 tokens 238 / 238, 32 x 17 tokens
+        168 / 204.  8 heads of 64 + 32 over 256 + 32: 2,000 tokens 124 / 64 us, 32 x 100 tokens 90 / 60, 32 x 17 tokens 44 / 44."""
+        return (self.expands and getattr(ctx, "from_start", False) and not ctx.is_decode and ctx.max_q_len >= _EXPAND_TOKENS
+                and tokens // 64 + ctx.n_seqs <= self.most_runs)
+
+    def _over_own_keys(self, q_full, gate, gate_offset: int, ctx, cache, table):
+        """[T, heads, dv]: attention over every head's own keys and values, made from the cached rows.  They and the queries are halves:
+        in bfloat16 the one rounding that keys and values have more than latent rows puts the result 3 % further off."""
+        ws, tokens = self.runtime.workspace, q_full.rows
+        count = kernels.rows_of_runs(tokens, ctx.n_seqs)
+        rows = ws.view("latent.rows", count, self.row)
+        kernels.latent_rows(cache.k, rows, table, ctx.seq_start, ctx.n_seqs, ctx.max_q_len, cache.page_tokens, cache.ring_tokens)
+        keys_values = ws.view("latent.keys_values", 1, count, self.heads * (self.key + self.dv))
+        kernels.gemm_tc_pair(rows, self.expand, kernels.GemmOut(keys_values))
+        q = ws.view("latent.queries", tokens, self.heads, self.key)
+        kernels.latent_queries(q_full, self.cos_sin, ctx.token_pos, q, self.d, self.rot)
+        out = ws.view("latent.heads", tokens, self.heads, self.dv)
+        kernels.attention_prefill_rows(q, keys_values[0], out, ctx.seq_start, ctx.n_seqs, ctx.max_q_len, self.window, self.scale,
+                                       gate=gate, gate_offset=gate_offset, gate_per_head=self.head_gate)
+        return out
+
     def forward(self, x, ctx, cache):
         tokens = x.shape[0]
         ws = self.runtime.workspace
@@ -199,6 +245,9 @@ class LatentAttention:
                                    at_kv=self.at_kv - skipped)
         # [*, T, heads * (d + rot)], or with the first projection's other columns behind
         q_full = self.uq(cq) if cq is not None else self.many[0](x) if own_queries else proj
+        if self._expands_for(ctx, tokens):
+            heads = self._over_own_keys(q_full, proj if self.gated else None, self.at_gate - skipped, ctx, cache, table).view(tokens, self.heads * self.dv)
+            return DeferredProduct(self.o, heads) if self.o.fusable(tokens) else self.o(heads)
         q = ws.view("latent.q", tokens, self.heads, self.row)
         kernels.head_product(q_full, self.uk_t, q, x_row=q_full.cols, x_head=self.d + self.rot)
         kernels.latent_query_rot(q_full, self.cos_sin, ctx.token_pos, q, self.heads, self.d, self.rot, self.rank)

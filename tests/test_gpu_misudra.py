@@ -202,6 +202,90 @@ def ring_pool(rows, upto, ring_pages, order, store):
     return pool
 
 
+class _Prompts:
+    """The fields of a step that the latent mixer reads; every sequence starts at position 0 unless ``past`` says otherwise."""
+
+    def __init__(self, lengths, width, order, past=0):
+        self.n_seqs, self.max_q_len, self.is_decode, self.from_start = len(lengths), max(lengths), False, past == 0
+        self.seq_start, self.seq_past = as_int([sum(lengths[:i]) for i in range(len(lengths) + 1)]), as_int([past] * len(lengths))
+        self.token_seq = as_int([i for i, n in enumerate(lengths) for _ in range(n)])
+        self.token_pos = as_int([past + t for n in lengths for t in range(n)])
+        self.table = as_int(torch.tensor(order).view(len(lengths), width).tolist())
+
+    def block_table(self, group):
+        return self.table
+
+
+@pytest.mark.parametrize("d, rot, turning, dv, rank, q_rank, gate, window, interleaved", [
+    (128, 64, 64, 128, 512, 96, False, None, False), (64, 32, 32, 64, 256, 0, "head", 70, False), (120, 16, 16, 64, 40, 40, True, None, True),
+    (136, 8, 0, 128, 64, 0, True, 33, False), (8, 64, 32, 64, 512, 0, False, 1, False), (128, 0, 0, 128, 256, 0, True, None, False)])
+@pytest.mark.parametrize("lengths", [(17, 1, 64, 65, 127), (128, 129), (300,)])
+def test_prompts_over_keys_and_values_per_head(d, rot, turning, dv, rank, q_rank, gate, window, interleaved, lengths):
+    """A prompt's keys and values formed per head against the attention over latent rows and against 64 bits, around the edges of its
+    runs (64) and tiles (128), with unused pages full of large numbers: no further off than the form over latent rows (by more than a
+    tenth, for single draws), and within what five roundings to 8 bits on the way (2^-9 each, at most, twice that through sharp scores) leave."""
+    from qwen_triton_b200.config.spec import PartSpec
+    from qwen_triton_b200.parts import latent_attention as module
+    from qwen_triton_b200.parts.base import Runtime, Workspace
+    torch.manual_seed(d + rank)
+    device, hidden, heads, scale = torch.device(DEV), 64, 3, (d + rot) ** -0.5
+    runtime = Runtime(device=device, dtype=torch.bfloat16, max_step_tokens=512, max_positions=512, workspace=Workspace(device), page_tokens=64)
+    position = PartSpec("rope", {"theta": 1e4, "rotary_dim": turning, "head_dim": rot, "pairing": "interleaved" if interleaved else "half"}) if turning else PartSpec("none", {})
+    params = {"hidden_size": hidden, "num_heads": heads, "head_dim": d, "rot_dim": rot, "v_head_dim": dv, "q_rank": q_rank, "kv_rank": rank, "scale": scale,
+              "position": position, "window": window, "gate": gate, "float_out": True}
+    mixer = module.LatentAttention(params, "m", runtime)
+    tensors = {}
+    for name, spec in module.LatentAttention.expected_tensors(params, "m").items():
+        std = 1.0 if spec.role == "vector" else spec.shape[1] ** -0.5 * (3.0 if name in ("m.uq.weight", "m.q.weight", "m.uk.weight") else 1.0)
+        tensors[name] = torch.randn(*spec.shape) * std
+        tensors[name] = tensors[name] if spec.role == "vector" else tensors[name].bfloat16().float()
+    mixer.load(lambda name: tensors[name])
+    runtime.workspace.allocate()
+    assert mixer.expands
+    width = 5
+    order = torch.randperm(width * len(lengths)).tolist()
+    x = torch.randn(sum(lengths), hidden).bfloat16()
+    got = {}
+    for form in ("rows", "expanded"):
+        step = _Prompts(lengths, width, order)
+        step.from_start = form == "expanded"
+        cache = type("View", (), {"k": torch.full((width * len(lengths), 1, 64, rank + rot), 1e4, dtype=torch.bfloat16, device=DEV), "page_tokens": 64, "ring_tokens": 0,
+                                  "writable": True, "group": 0})()
+        cache.v = cache.k
+        out = mixer.forward(x.to(DEV), step, cache)
+        got[form] = out.value().cpu().double()
+        kernels.check_status(device)
+    t = {name.removeprefix("m."): value.double() for name, value in tensors.items()}
+    want = []
+    for sequence in x.double().split(list(lengths)):
+        n = len(sequence)
+        norm = lambda v, w: v / torch.sqrt((v * v).mean(-1, keepdim=True) + mixer.eps) * w
+        q = norm(sequence @ t["dq.weight"].T, t["dq.norm"]) @ t["uq.weight"].T if q_rank else sequence @ t["q.weight"].T
+        down = sequence @ t["dkv.weight"].T
+        c, shared, q = norm(down[:, :rank], t["dkv.norm"]), down[:, None, rank:], q.view(n, heads, d + rot)
+        angle = torch.arange(n).double()[:, None] * (1e4 ** (-torch.arange(0, max(turning, 2), 2).double() / max(turning, 1)))[None]
+        cos, sin = angle.cos()[:, None], angle.sin()[:, None]
+
+        def turn(v):
+            if not turning:
+                return v
+            a, b = (v[..., 0:turning:2], v[..., 1:turning:2]) if interleaved else (v[..., :turning // 2], v[..., turning // 2:turning])
+            both = torch.stack((a * cos - b * sin, b * cos + a * sin), -1).flatten(-2) if interleaved else torch.cat((a * cos - b * sin, b * cos + a * sin), -1)
+            return torch.cat((both, v[..., turning:]), -1)
+
+        k = torch.cat(((c @ t["uk.weight"].T).view(n, heads, d), turn(shared).expand(n, heads, rot)), -1)
+        score = torch.einsum("qhd,khd->hqk", torch.cat((q[..., :d], turn(q[..., d:])), -1), k) * scale
+        age = torch.arange(n)[:, None] - torch.arange(n)[None]
+        seen = (age >= 0) & (age < (window or n))
+        o = torch.einsum("hqk,khd->qhd", score.masked_fill(~seen, float("-inf")).softmax(-1), (c @ t["uv.weight"].T).view(n, heads, dv))
+        if gate:
+            o = o * torch.sigmoid(sequence @ t["g.weight"].T).view(n, heads, -1)
+        want.append(o.reshape(n, heads * dv) @ t["o.weight"].T)
+    want = torch.cat(want)
+    off = {form: float((value - want).norm() / want.norm()) for form, value in got.items()}
+    assert off["expanded"] < 5 * 2.0 ** -9 * 2 and off["expanded"] < 1.1 * off["rows"], off
+
+
 @pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("heads, rank, rot, window", [(3, 40, 16, 37), (20, 64, 32, 64), (40, 72, 24, 65), (1, 11, 6, 1), (70, 16, 8, 130), (5, 264, 8, 100),
                                                       (8, 32, 8, None)])
