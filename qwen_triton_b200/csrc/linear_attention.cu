@@ -11,7 +11,7 @@
 //   transposed, [slots, heads, vdim, dim], so that the 8 lanes of a column read and write 8 RPL consecutive floats.
 //   A sequence's tokens are walked in order, 16 at a time through shared memory; a one-token step is the same kernel
 //   with one token, whose cost is the state's bytes.
-// linear_attention_step_kernel   few tokens a sequence; it also takes decays that depend on the token, per head or per key
+// linear_attention_step_rows_kernel, linear_attention_step_kernel   few tokens a sequence (the usual sizes; any); they also take decays that depend on the token, per head or per key
 //   channel, a factor on v and q/k heads shared by several heads (qt_decayed_attention_steps).
 // group_gate_norm_kernel   out = o / sqrt(mean(o^2) + eps) * weight * gate, the mean over the whole row or over equal parts of it,
 //   the gate (sigmoid or SiLU of projection columns) behind the norm or ahead of it, with an optional skip term; rounded
@@ -477,6 +477,95 @@ __global__ void __launch_bounds__(LW_THREADS) linear_attention_scan_warp_kernel(
     }
 }
 
+// The same steps for rows of whole 16-byte pieces (dim 64, 128 or 256, one finished plane of projections).  Bound by the state's bytes, read
+// and written once a step, if enough of them are asked for at once: a column lies over LANES neighbouring lanes, four (LANES x Q: dim / 4)
+// consecutive floats each, so that a lane's share of q, k and the decays is Q 16-byte pieces for all COLS columns of its group
+// and the columns' own pieces are all that it asks for beside them (about 50 registers; with a column over 8 lanes it was 100, two blocks an SM).
+// grid (vdim / 32, heads, sequences).  32 sequences of one token, 16 heads of 128 x 128, decays per channel 13.5 us (29.8 us), 32
+// heads of 128 x 64, decays per head 14.0 us (26.5 us): 67 MB.
+template <int LANES, int Q, int MODE>
+__global__ void __launch_bounds__(256) linear_attention_step_rows_kernel(const LinAttnParams p) {
+    constexpr int DIM = 4 * LANES * Q, GROUPS = 256 / LANES, COLS = 32 / GROUPS;
+    pdl_launch_dependents();
+    pdl_wait();
+    const int head = blockIdx.y, seq = blockIdx.z, lane = threadIdx.x % LANES, group = threadIdx.x / LANES;
+    const int begin = p.seq_start[seq], end = p.seq_start[seq + 1];
+    if (begin >= end) return;
+    const int key_head = MODE == LA_CONSTANT ? head : head / p.heads_per_key;
+    const int col0 = blockIdx.x * 32 + group;                    // this group's columns: col0 + GROUPS c
+    float* state = p.state + ((size_t)p.slots[seq] * p.heads + head) * p.vdim * DIM + 4 * lane;
+    float4 S[COLS][Q];
+#pragma unroll
+    for (int c = 0; c < COLS; ++c)
+#pragma unroll
+        for (int j = 0; j < Q; ++j)
+            S[c][j] = col0 + GROUPS * c < p.vdim ? *reinterpret_cast<const float4*>(state + (size_t)(col0 + GROUPS * c) * DIM + 4 * LANES * j) : make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int t = begin; t < end; ++t) {
+        const float* row = p.proj + (size_t)t * p.proj_cols;
+        const size_t th = (size_t)t * p.heads + head;
+        float4 q[Q], k[Q], d[Q];
+        float v[COLS];
+#pragma unroll
+        for (int j = 0; j < Q; ++j) {
+            q[j] = __ldg(reinterpret_cast<const float4*>(row + p.at_q + key_head * DIM + 4 * (lane + LANES * j)));
+            k[j] = __ldg(reinterpret_cast<const float4*>(row + p.at_k + key_head * DIM + 4 * (lane + LANES * j)));
+            if (MODE == LA_PER_CHANNEL) d[j] = __ldg(reinterpret_cast<const float4*>(p.log_decay + th * DIM + 4 * (lane + LANES * j)));
+        }
+#pragma unroll
+        for (int c = 0; c < COLS; ++c) v[c] = col0 + GROUPS * c < p.vdim ? __ldg(row + p.at_v + (size_t)head * p.vdim + col0 + GROUPS * c) : 0.f;
+        const float whole = MODE == LA_CONSTANT ? p.decay[head] : MODE == LA_PER_HEAD ? expf(__ldg(p.log_decay + th)) : 0.f;
+        const float factor = MODE != LA_CONSTANT && p.v_scale ? __ldg(p.v_scale + th) : 1.f;
+#pragma unroll
+        for (int j = 0; j < Q; ++j) {
+            if (MODE == LA_PER_CHANNEL) d[j] = make_float4(expf(d[j].x), expf(d[j].y), expf(d[j].z), expf(d[j].w));
+            else d[j] = make_float4(whole, whole, whole, whole);
+            if (p.act) {
+                q[j] = make_float4(la_act(p, q[j].x), la_act(p, q[j].y), la_act(p, q[j].z), la_act(p, q[j].w));
+                k[j] = make_float4(la_act(p, k[j].x), la_act(p, k[j].y), la_act(p, k[j].z), la_act(p, k[j].w));
+            }
+        }
+        float sum[COLS];
+#pragma unroll
+        for (int c = 0; c < COLS; ++c) {
+            const float x = la_act(p, v[c]) * factor;
+            sum[c] = 0.f;
+#pragma unroll
+            for (int j = 0; j < Q; ++j) {
+                float4& s = S[c][j];
+                s = make_float4(fmaf(d[j].x, s.x, k[j].x * x), fmaf(d[j].y, s.y, k[j].y * x), fmaf(d[j].z, s.z, k[j].z * x), fmaf(d[j].w, s.w, k[j].w * x));
+                sum[c] = fmaf(s.x, q[j].x, fmaf(s.y, q[j].y, fmaf(s.z, q[j].z, fmaf(s.w, q[j].w, sum[c]))));
+            }
+        }
+#pragma unroll
+        for (int off = LANES / 2; off > 0; off >>= 1)
+#pragma unroll
+            for (int c = 0; c < COLS; ++c) sum[c] += __shfl_xor_sync(0xffffffffu, sum[c], off);
+#pragma unroll
+        for (int c = 0; c < COLS; ++c)
+            if (lane == c && col0 + GROUPS * c < p.vdim) p.out[th * p.vdim + col0 + GROUPS * c] = MODE == LA_CONSTANT ? sum[c] : sum[c] * p.out_scale;
+    }
+#pragma unroll
+    for (int c = 0; c < COLS; ++c)
+#pragma unroll
+        for (int j = 0; j < Q; ++j)
+            if (col0 + GROUPS * c < p.vdim) *reinterpret_cast<float4*>(state + (size_t)(col0 + GROUPS * c) * DIM + 4 * LANES * j) = S[c][j];
+}
+
+template <int MODE>
+static int launch_steps(const LinAttnParams& p, int n_seqs, cudaStream_t s) {
+    const dim3 grid((p.vdim + 31) / 32, p.heads, n_seqs), block(256);
+    const bool rows = (p.dim == 64 || p.dim == 128 || p.dim == 256) && p.n_splits == 1 && p.at_q % 4 == 0 && p.at_k % 4 == 0 && p.proj_cols % 4 == 0 &&
+                      (((uintptr_t)p.proj | (uintptr_t)p.state | (MODE == LA_PER_CHANNEL ? (uintptr_t)p.log_decay : 0)) & 15) == 0;
+    if (rows && p.dim == 64) launch_kernel(linear_attention_step_rows_kernel<16, 1, MODE>, grid, block, 0, s, p);
+    else if (rows && p.dim == 128) launch_kernel(linear_attention_step_rows_kernel<32, 1, MODE>, grid, block, 0, s, p);
+    else if (rows) launch_kernel(linear_attention_step_rows_kernel<32, 2, MODE>, grid, block, 0, s, p);
+    else if (p.dim <= LA_LANES * 8) launch_kernel(linear_attention_step_kernel<8, MODE>, grid, block, 0, s, p);
+    else if (p.dim <= LA_LANES * 16) launch_kernel(linear_attention_step_kernel<16, MODE>, grid, block, 0, s, p);
+    else launch_kernel(linear_attention_step_kernel<32, MODE>, grid, block, 0, s, p);
+    QT_CHECK_LAUNCH("linear_attention_steps");
+    return QT_OK;
+}
+
 extern "C" int qt_linear_attention_scan(const float* proj, int n_splits, long long split_stride, int proj_cols, int at_q, int at_k, int at_v,
                                         const float* decay, float* state, float* out, const int* seq_start, const int* slots, int n_seqs,
                                         int heads, int dim, int vdim, int act, int max_q_len, void* stream) {
@@ -491,14 +580,7 @@ extern "C" int qt_linear_attention_scan(const float* proj, int n_splits, long lo
     // blocks of 32 columns where they fill the machine twice over (many sequences: every block stages its head's q and k
     // itself), else of 16, so that one prompt still gives most SMs a block
     const bool wide = (long long)((vdim + 31) / 32) * heads * n_seqs >= 2LL * sm_count();
-    if (max_q_len <= 4) {                                  // few tokens a sequence: the short kernel
-        const dim3 grid((vdim + 31) / 32, heads, n_seqs), block(32 * LA_LANES);
-        if (dim <= LA_LANES * 8) launch_kernel(linear_attention_step_kernel<8, LA_CONSTANT>, grid, block, 0, s, p);
-        else if (dim <= LA_LANES * 16) launch_kernel(linear_attention_step_kernel<16, LA_CONSTANT>, grid, block, 0, s, p);
-        else launch_kernel(linear_attention_step_kernel<32, LA_CONSTANT>, grid, block, 0, s, p);
-        QT_CHECK_LAUNCH("linear_attention_scan");
-        return QT_OK;
-    }
+    if (max_q_len <= 4) return launch_steps<LA_CONSTANT>(p, n_seqs, s);      // few tokens a sequence: the short kernels
     // long portions of few sequences, with a head's rows within what 32 lanes hold four at a time: a warp per column
     static const bool warp_form = [] { const char* env = getenv("QT_B200_LINEAR_WARP"); return !(env && env[0] == '0'); }();
     if (warp_form && max_q_len >= 64 && dim > 64 && (long long)((vdim + 15) / 16) * heads * n_seqs < 2LL * sm_count()) {
@@ -538,18 +620,7 @@ extern "C" int qt_decayed_attention_steps(const float* proj, int n_splits, long 
     LinAttnParams p{proj, n_splits, (size_t)split_stride, proj_cols, at_q, at_k, at_v, nullptr, state, out, seq_start, slots, heads, dim, vdim, 0,
                     log_decay, v_scale, heads_per_key, out_scale};
     cudaStream_t s = (cudaStream_t)stream;
-    const dim3 grid((vdim + 31) / 32, heads, n_seqs), block(32 * LA_LANES);
-#define QT_LAUNCH_STEPS(RPL)                                                                             \
-    do {                                                                                                 \
-        if (per_channel) launch_kernel(linear_attention_step_kernel<RPL, LA_PER_CHANNEL>, grid, block, 0, s, p); \
-        else launch_kernel(linear_attention_step_kernel<RPL, LA_PER_HEAD>, grid, block, 0, s, p);         \
-    } while (0)
-    if (dim <= LA_LANES * 8) QT_LAUNCH_STEPS(8);
-    else if (dim <= LA_LANES * 16) QT_LAUNCH_STEPS(16);
-    else QT_LAUNCH_STEPS(32);
-#undef QT_LAUNCH_STEPS
-    QT_CHECK_LAUNCH("decayed_attention_steps");
-    return QT_OK;
+    return per_channel ? launch_steps<LA_PER_CHANNEL>(p, n_seqs, s) : launch_steps<LA_PER_HEAD>(p, n_seqs, s);
 }
 
 // ----------------------------------------------------------------------------- skip, gate and norm behind a recurrence

@@ -752,3 +752,30 @@ def test_gemm_dispatch_is_static():
         kernels.gemm_tc(a, w, GemmOut(out))
     assert kernels.tc_normalise_splits(320, 4) == 3 and kernels.tc_normalise_splits(4096, 3) == 3
     assert kernels.tc_normalise_splits(64, 8) == 1
+
+
+@pytest.mark.parametrize("heads, kv, dim, vdim", [(3, 3, 64, 40), (4, 2, 128, 33), (2, 1, 256, 64), (2, 2, 100, 16)])
+@pytest.mark.parametrize("channel", [False, True])
+def test_recurrence_steps_of_few_tokens(heads, kv, dim, vdim, channel):
+    """Rows of whole 16-byte pieces (64, 128, 256 key channels, value columns that fill no block) and others; sequences of 1 to 16 tokens
+    in slots out of order; chains of 16 tokens and sums of 256 products round to less than 2e-6 of the largest value."""
+    counts, slots = [1, 16, 2, 7], [3, 0, 4, 1]
+    total, cols = sum(counts), 2 * kv * dim + heads * vdim
+    rows, states = rand(total, cols, seed=1), rand(6, heads, vdim, dim, seed=2)
+    logs = -rand(total, heads, dim, seed=3).abs() if channel else -rand(total, heads, seed=3).abs()
+    scale, out, got = rand(total, heads, seed=4), torch.full((total, heads, vdim), float("nan"), device=DEV), states.clone()
+    ctx = type("Step", (), {"n_seqs": 4, "max_q_len": 16, "seq_start": torch.tensor([0, 1, 17, 19, 26], dtype=torch.int32, device=DEV),
+                            "slots": torch.tensor(slots, dtype=torch.int32, device=DEV)})()
+    kernels.decayed_attention(GemmOut(rows[None]), 0, kv * dim, 2 * kv * dim, logs, got, out, ctx, dim, None, heads_per_key=heads // kv, v_scale=scale, out_scale=0.5)
+    want, wanted, at = torch.zeros(total, heads, vdim, dtype=torch.float64), states.double().cpu(), 0
+    r, g, sc = rows.double().cpu(), logs.double().cpu().view(total, heads, -1), scale.double().cpu()
+    for n, slot in zip(counts, slots):
+        s = wanted[slot]
+        for t in range(at, at + n):
+            q, k = (r[t, i * kv * dim:(i + 1) * kv * dim].view(kv, dim).repeat_interleave(heads // kv, 0) for i in (0, 1))
+            v = r[t, 2 * kv * dim:].view(heads, vdim) * sc[t][:, None]
+            s = g[t].exp()[:, None] * s + v[:, :, None] * k[:, None]
+            want[t] = 0.5 * torch.einsum("hvd,hd->hv", s, q)
+        wanted[slot], at = s, at + n
+    assert float((out.cpu().double() - want).abs().max()) < 2e-6 * float(want.abs().max())
+    assert float((got.cpu().double() - wanted).abs().max()) < 2e-6 * float(wanted.abs().max())
