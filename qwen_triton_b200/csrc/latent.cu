@@ -464,6 +464,115 @@ __global__ void __launch_bounds__(128) head_product_mma_kernel(const HeadProduct
     }
 }
 
+// The same for up to 64 tokens (one-token steps).  Bound by latency: a block's operands are a few ten KB, so all of K is asked for at once, the
+// weights ahead of the dependency wait (no kernel of a step writes them), the gates with the rows.  A block forms 16 MT tokens x 8 NT outputs; NT
+// is small so that the heads' matrices spread over the machine.  32 tokens of 16 heads, 128 x 512 10.3 us (21.7 us through the
+// two-stage ring), 512 x 128 from float sums 6.4 us (8.0 us), in a step.
+template <typename TI, int MT, int NT>
+__global__ void __launch_bounds__(128) head_product_few_kernel(const HeadProductParams p, int k_padded) {
+    using namespace qt_mma;
+    extern __shared__ __align__(16) __nv_bfloat16 operands[];
+    const int ld = k_padded + 8, pieces = k_padded / 8;
+    __nv_bfloat16* ws = operands;                        // [8 NT][ld]
+    __nv_bfloat16* xs = ws + 8 * NT * ld;                // [16 MT][ld]
+    const int h = blockIdx.y, n0 = blockIdx.x * 8 * NT, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
+    const __nv_bfloat16* w = (const __nv_bfloat16*)p.w + (size_t)h * p.n * p.k;
+    pdl_launch_dependents();
+    for (int i = tid; i < 8 * NT * pieces; i += 128) {
+        const int r = i / pieces, c = (i - r * pieces) * 8;
+        __nv_bfloat16* dst = ws + r * ld + c;
+        if (n0 + r < p.n && c < p.k) cp_async16(smem_u32(dst), w + (size_t)(n0 + r) * p.k + c);
+        else *reinterpret_cast<uint4*>(dst) = make_uint4(0, 0, 0, 0);
+    }
+    pdl_wait();
+#pragma unroll 4
+    for (int i = tid; i < 16 * MT * pieces; i += 128) {
+        const int r = i / pieces, c = (i - r * pieces) * 8;
+        __nv_bfloat16* dst = xs + r * ld + c;
+        const bool there = r < p.n_tokens && c < p.k;
+        const TI* at = (const TI*)p.x + (there ? (long long)r * p.x_row + (long long)h * p.x_head + p.x_offset + c : 0);
+        if constexpr (sizeof(TI) == 2) {
+            if (there) cp_async16(smem_u32(dst), at);
+            else *reinterpret_cast<uint4*>(dst) = make_uint4(0, 0, 0, 0);
+        } else {
+            float4 lo = make_float4(0.f, 0.f, 0.f, 0.f), hi = lo;
+            if (there)
+                for (int sp = 0; sp < p.x_splits; ++sp) {
+                    const float4 a = __ldg(reinterpret_cast<const float4*>(at + (size_t)sp * p.x_split_stride)), b = __ldg(reinterpret_cast<const float4*>(at + (size_t)sp * p.x_split_stride) + 1);
+                    lo.x += a.x; lo.y += a.y; lo.z += a.z; lo.w += a.w;
+                    hi.x += b.x; hi.y += b.y; hi.z += b.z; hi.w += b.w;
+                }
+            *reinterpret_cast<uint4*>(dst) = make_uint4(pack_bf16(lo.x, lo.y), pack_bf16(lo.z, lo.w), pack_bf16(hi.x, hi.y), pack_bf16(hi.z, hi.w));
+        }
+    }
+    cp_async_commit();
+    float gates[NT][4];
+    if (p.gate && warp < MT) {
+#pragma unroll
+        for (int nt = 0; nt < NT; ++nt) gates[nt][0] = gates[nt][1] = gates[nt][2] = gates[nt][3] = 0.f;
+        for (int sp = 0; sp < p.gate_splits; ++sp)
+#pragma unroll
+            for (int e = 0; e < 4 * NT; ++e) {
+                const int tok = warp * 16 + g + 8 * ((e >> 1) & 1), n = n0 + (e >> 2) * 8 + 2 * t + (e & 1);
+                if (tok < p.n_tokens && n < p.n)
+                    gates[e >> 2][e & 3] += __ldg(p.gate + (size_t)sp * p.gate_split_stride + (size_t)tok * p.gate_cols + p.gate_offset + (size_t)h * p.gate_head + (size_t)n * p.gate_elem);
+            }
+    }
+    cp_async_wait<0>();
+    __syncthreads();
+    if (warp >= MT) return;
+    float acc[NT][4] = {};
+    const uint32_t a_at = smem_u32(xs) + (uint32_t)((warp * 16 + (lane & 7) + ((lane >> 3) & 1) * 8) * ld + (lane >> 4) * 8) * 2u;
+    const uint32_t b_at = smem_u32(ws) + (uint32_t)(((lane >> 4) * 8 + (lane & 7)) * ld + ((lane >> 3) & 1) * 8) * 2u;
+#pragma unroll 4
+    for (int k0 = 0; k0 < k_padded; k0 += 16) {
+        uint32_t a[4];
+        ldmatrix_x4(a, a_at + (uint32_t)k0 * 2u);
+#pragma unroll
+        for (int np = 0; np < NT / 2; ++np) {
+            uint32_t b[4];
+            ldmatrix_x4(b, b_at + (uint32_t)(np * 16 * ld + k0) * 2u);
+            mma_bf16(acc[2 * np], a, b[0], b[1]);
+            mma_bf16(acc[2 * np + 1], a, b[2], b[3]);
+        }
+    }
+    __nv_bfloat16* y = (__nv_bfloat16*)p.y;
+#pragma unroll
+    for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            const int tok = warp * 16 + g + 8 * (e >> 1), n = n0 + nt * 8 + 2 * t + (e & 1);
+            const float v = p.gate ? acc[nt][e] / (1.f + expf(-gates[nt][e])) : acc[nt][e];
+            if (tok < p.n_tokens && n < p.n) y[(size_t)((long long)tok * p.y_row + (long long)h * p.y_head + p.y_offset + n)] = __float2bfloat16_rn(v);
+        }
+}
+
+constexpr int HF_MOST_TOKENS = 64, HF_MOST_K = 512;
+
+template <typename TI, int MT, int NT>
+static int launch_head_few(const HeadProductParams& p, cudaStream_t s) {
+    const int k_padded = (p.k + 15) / 16 * 16;
+    static bool configured = false;
+    if (!configured) {
+        cudaError_t err = cudaFuncSetAttribute(head_product_few_kernel<TI, MT, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (16 * MT + 8 * NT) * (HF_MOST_K + 8) * 2);
+        if (err != cudaSuccess) QT_FAIL(QT_ERR_LAUNCH, "head_product: cannot raise shared memory: %s", cudaGetErrorString(err));
+        configured = true;
+    }
+    launch_kernel(head_product_few_kernel<TI, MT, NT>, dim3((p.n + 8 * NT - 1) / (8 * NT), p.heads), dim3(128), (size_t)(16 * MT + 8 * NT) * (k_padded + 8) * 2, s, p, k_padded);
+    QT_CHECK_LAUNCH("head_product_few");
+    return QT_OK;
+}
+template <typename TI>
+static int head_few(const HeadProductParams& p, cudaStream_t s) {
+    // 32 outputs a block where that leaves every SM one, else 16
+    const bool wide = (long long)((p.n + 31) / 32) * p.heads >= sm_count();
+#define QT_HEAD_FEW(MT) return wide ? launch_head_few<TI, MT, 4>(p, s) : launch_head_few<TI, MT, 2>(p, s)
+    if (p.n_tokens <= 16) QT_HEAD_FEW(1);
+    if (p.n_tokens <= 32) QT_HEAD_FEW(2);
+    QT_HEAD_FEW(4);
+#undef QT_HEAD_FEW
+}
+
 extern "C" int qt_head_product(const void* x, int x_dtype, int x_splits, long long x_split_stride, long long x_row, long long x_head, int x_offset,
                                const void* w, int w_dtype, void* y, int y_dtype, long long y_row, long long y_head, int y_offset,
                                const float* gate, int gate_splits, long long gate_split_stride, int gate_cols, int gate_offset,
@@ -484,6 +593,7 @@ extern "C" int qt_head_product(const void* x, int x_dtype, int x_splits, long lo
         ((x_dtype == QT_F32 && x_row % 4 == 0 && x_head % 4 == 0 && x_offset % 4 == 0 && x_split_stride % 4 == 0 && ((uintptr_t)x & 15) == 0) ||
          (x_dtype == QT_BF16 && x_splits == 1 && x_row % 8 == 0 && x_head % 8 == 0 && x_offset % 8 == 0 && ((uintptr_t)x & 15) == 0)) &&
         ((uintptr_t)w & 15) == 0) {
+        if (n_tokens <= HF_MOST_TOKENS && k <= HF_MOST_K) return x_dtype == QT_F32 ? head_few<float>(p, s) : head_few<__nv_bfloat16>(p, s);
         dim3 tiles((n + HM_N - 1) / HM_N, (n_tokens + HM_T - 1) / HM_T, heads);
         if (x_dtype == QT_F32) launch_kernel(head_product_mma_kernel<float>, tiles, dim3(128), 0, s, p);
         else launch_kernel(head_product_mma_kernel<__nv_bfloat16>, tiles, dim3(128), 0, s, p);

@@ -754,6 +754,27 @@ def test_gemm_dispatch_is_static():
     assert kernels.tc_normalise_splits(64, 8) == 1
 
 
+@pytest.mark.parametrize("splits, x_dtype", [(1, torch.bfloat16), (1, torch.float32), (3, torch.float32)])
+@pytest.mark.parametrize("heads, n, k, gate", [(3, 24, 8, None), (16, 130, 128, "each"), (5, 128, 512, "each"), (40, 512, 40, "head"), (2, 65, 520, None)])
+@pytest.mark.parametrize("tokens", [1, 16, 17, 32, 33, 64, 65])
+def test_head_product_of_few_tokens(splits, x_dtype, heads, n, k, gate, tokens):
+    """All of K at once (up to 64 tokens and K = 512) and the ring behind it: edges of the token tiles, outputs and K that fill no tile,
+    results and gates beside columns that stay as they are.  Products of bfloat16 in float, one rounding."""
+    x = rand(splits, tokens, heads * (k + 8), seed=1, dtype=x_dtype)
+    w, gates = rand(heads, n, k, seed=2, scale=k ** -0.5, dtype=torch.bfloat16), rand(2, tokens, 8 + heads * (n if gate == "each" else 1), seed=3)
+    y = torch.full((tokens, heads, n + 6), 7.0, dtype=torch.bfloat16, device=DEV)
+    kernels.head_product(GemmOut(x) if x_dtype == torch.float32 else x[0], w, y, x_row=heads * (k + 8), x_head=k + 8, x_offset=8, out_offset=6,
+                         gate=GemmOut(gates) if gate else None, gate_offset=8, gate_per_head=gate == "head")
+    rows = x.double().sum(0).view(tokens, heads, k + 8)[:, :, 8:].float().bfloat16().double()
+    want = torch.einsum("thk,hnk->thn", rows, w.double())
+    if gate:
+        want = want * torch.sigmoid(gates.double().sum(0)[:, 8:].view(tokens, heads, -1))
+    # the operand's rounding may fall the other way where partial sums are added in float; then one rounding of the result
+    size = torch.einsum("thk,hnk->thn", rows.abs(), w.double().abs())
+    assert bool(((y[:, :, 6:].double() - want).abs() <= want.abs() * 2.0 ** -8 + size * (2.0 ** -9 if splits > 1 else 2.0 ** -20)).all())
+    assert bool((y[:, :, :6] == 7.0).all())
+
+
 @pytest.mark.parametrize("heads, kv, dim, vdim", [(3, 3, 64, 40), (4, 2, 128, 33), (2, 1, 256, 64), (2, 2, 100, 16)])
 @pytest.mark.parametrize("channel", [False, True])
 def test_recurrence_steps_of_few_tokens(heads, kv, dim, vdim, channel):
