@@ -14,6 +14,7 @@ from dataclasses import dataclass
 
 import torch
 
+from ..ops import kernels
 from ..parts.base import KVRequest, StateRequest
 from .book import CacheBook, GroupGeometry
 
@@ -111,6 +112,12 @@ class SequenceCache:
                                        request.v_head_dim or request.head_dim), dtype=dtype, device=device)
             for key, request in self._state_requests.items():
                 self._state_of[key] = torch.zeros((self.num_slots + 1, *request.shape), dtype=request.dtype, device=device)
+        # a new sequence's states are zeroed in one launch; those whose rows are not whole 16-byte pieces one by one
+        def whole(state):
+            return state.is_cuda and state[0].numel() * state.element_size() % 16 == 0
+        together = [state for state in self._state_of.values() if whole(state)]
+        self._apart = [state for state in self._state_of.values() if not whole(state)]
+        self._row_table = kernels.row_table(together) if together else None
 
     # ------------------------------------------------------------------ views
     def view(self, position: int):
@@ -136,7 +143,10 @@ class SequenceCache:
     # ------------------------------------------------------------------ slots
     def alloc(self) -> int:
         slot = self.book.alloc()
-        for state in self._state_of.values():
+        if self._row_table is not None:
+            with torch.cuda.device(self.device):
+                kernels.zero_rows(*self._row_table, slot)
+        for state in self._apart:
             state[slot].zero_()
         return slot
 

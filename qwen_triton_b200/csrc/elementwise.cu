@@ -1140,4 +1140,25 @@ extern "C" int qt_swiglu(const void* gate_up, int in_dtype, int n_splits, long l
     return QT_OK;
 }
 
+// ----------------------------------------------------------------------------- a new sequence's states
+// Zeros row `slot` of every tensor of a table: table[i] = {address, bytes of a row}, rows of whole 16-byte pieces.  One launch in the place of
+// one per layer: 32 sequences of four states each spent 1.3 ms of a 12.5 ms job in 128 fills.  grid (blocks, tensors).
+__global__ void __launch_bounds__(256) zero_rows_kernel(const long long* __restrict__ table, int slot) {
+    pdl_launch_dependents();
+    pdl_wait();                                          // a kernel before may still read what the slot held for its last sequence
+    const long long bytes = table[2 * blockIdx.y + 1];
+    uint4* row = reinterpret_cast<uint4*>(table[2 * blockIdx.y] + bytes * slot);
+    for (long long i = (long long)blockIdx.x * 256 + threadIdx.x; i < bytes / 16; i += (long long)gridDim.x * 256) row[i] = make_uint4(0u, 0u, 0u, 0u);
+}
+
+extern "C" int qt_zero_rows(const long long* table, int tensors, long long most_bytes, int slot, void* stream) {
+    QT_REQUIRE(tensors >= 0 && tensors <= 65535 && slot >= 0 && most_bytes >= 0 && most_bytes % 16 == 0, "zero_rows: bad sizes");
+    if (tensors == 0 || most_bytes == 0) return QT_OK;
+    long long blocks = (most_bytes / 16 + 1023) / 1024;   // four pieces a thread
+    if (blocks > sm_count()) blocks = sm_count();
+    launch_kernel(zero_rows_kernel, dim3((unsigned)blocks, tensors), dim3(256), 0, (cudaStream_t)stream, table, slot);
+    QT_CHECK_LAUNCH("zero_rows");
+    return QT_OK;
+}
+
 QT_DEFINE_LAST_ERROR(elementwise)

@@ -22,6 +22,7 @@ _c_int, _c_ll, _c_float, _c_ptr = ctypes.c_int, ctypes.c_longlong, ctypes.c_floa
 
 _SIGNATURES = {
     "elementwise": {
+        "qt_zero_rows": [_c_ptr, _c_int, _c_ll, _c_int, _c_ptr],
         "qt_embedding": [_c_ptr, _c_ptr, _c_ptr, _c_int, _c_int, _c_int, _c_int, _c_float, _c_ptr, _c_float, _c_ptr, _c_int, _c_ptr],
         "qt_stream_concat": [_c_ptr, _c_ptr, _c_int, _c_int, _c_ll, _c_ptr, _c_ptr, _c_int, _c_int, _c_int, _c_ptr],
         "qt_add_bias": [_c_ptr, _c_ptr, _c_int, _c_int, _c_ptr],
@@ -273,6 +274,23 @@ class GemmOut:
 
 
 # ----------------------------------------------------------------------------- elementwise
+def row_table(tensors: list[torch.Tensor]) -> tuple[torch.Tensor, int]:
+    """What ``zero_rows`` takes for contiguous tensors [rows, ...] on one device whose rows are whole 16-byte pieces: their addresses and the
+    bytes of a row, int64 [n, 2] on that device, and the most bytes of a row.  The tensors must outlive it."""
+    entries = []
+    for tensor in tensors:
+        if not tensor.is_cuda or not tensor.is_contiguous() or tensor.data_ptr() % 16 or tensor[0].numel() * tensor.element_size() % 16:
+            raise KernelError(f"row_table: a tensor {tuple(tensor.shape)} whose rows are not whole 16-byte pieces")
+        entries.append([tensor.data_ptr(), tensor[0].numel() * tensor.element_size()])
+    return torch.tensor(entries, dtype=torch.int64, device=tensors[0].device), max(size for _, size in entries)
+
+
+def zero_rows(table: torch.Tensor, most_bytes: int, row: int) -> None:
+    """Zeros in row ``row`` of every tensor of ``table`` (``row_table``)."""
+    _need(table, "table", torch.int64)
+    _call("elementwise", "qt_zero_rows", _ptr(table), table.shape[0], int(most_bytes), int(row), _stream())
+
+
 def embedding(residual: torch.Tensor, table: torch.Tensor, ids: torch.Tensor, scale: float = 1.0, norm_weight: torch.Tensor | None = None,
               eps: float = 0.0, start: torch.Tensor | None = None) -> None:
     """residual[t] = table[ids[t]] * scale in float, RMS-normed with ``norm_weight`` [H] where given.  ids: int32 [T].

@@ -800,3 +800,13 @@ def test_recurrence_steps_of_few_tokens(heads, kv, dim, vdim, channel):
         wanted[slot], at = s, at + n
     assert float((out.cpu().double() - want).abs().max()) < 2e-6 * float(want.abs().max())
     assert float((got.cpu().double() - wanted).abs().max()) < 2e-6 * float(wanted.abs().max())
+
+
+def test_zero_rows_of_several_tensors():
+    tensors = [torch.ones(5, 3, 4, device=DEV), torch.ones(5, 1024, 33, 8, device=DEV), torch.ones(5, 8, dtype=torch.bfloat16, device=DEV)]
+    table = kernels.row_table(tensors)
+    kernels.zero_rows(*table, 3)
+    for tensor in tensors:
+        assert float(tensor[3].abs().max()) == 0.0 and float(tensor[[0, 1, 2, 4]].float().min()) == 1.0
+    with pytest.raises(kernels.KernelError):
+        kernels.row_table([torch.ones(5, 3, device=DEV)])
