@@ -27,10 +27,14 @@
 // absolute position p iff j <= p and, in a windowed group, j > p - window.  Every mbarrier wait is bounded and
 // reports through a status word.
 //
-// PEN: a distance penalty, the score of key j for the query at position i loses r1_h ln(1 + r2_h (i - j)).  The softmax
+// PEN_LOG: a distance penalty, the score of key j for the query at position i loses r1_h ln(1 + r2_h (i - j)).  The softmax
 // thread takes it off the row it holds in registers before the maximum, in the base-2 domain the row is scaled into:
 // s - (r1 / (scale log2 e)) log2(1 + r2 (i - j)), one FMA for the argument (the key's place in the tile is a constant
 // of the unrolled loop), lg2.approx, one FMA; keys ahead of the query give arguments that the mask then overwrites.
+//
+// PEN_LINEAR: the score loses r1_h (i - j): one addition and one FMA on the unscaled score.  KEEP: a windowed query also sees the first
+// keys; 2,048 tokens of 16 heads of 128, a window of 1,024 beside 64 kept keys 34 us, with the linear penalty and a sink
+// 41 us (108 and 119 us on mma.sync).
 //
 // CAP: scores pass softcap tanh(s / softcap) before the maximum (score_cap.cuh), in the same place; no score of a masked key is
 // used.  `sinks` (or `sink` alone: 0): the softmax's denominator has one more term, exp of the head's number, which is neither
@@ -55,6 +59,7 @@ using namespace qt_tc;
 namespace {
 
 constexpr int PAGE = 64;
+constexpr int PEN_NONE = 0, PEN_LOG = 1, PEN_LINEAR = 2;     // distance penalty: none, r1 ln(1 + r2 distance), r1 distance
 constexpr int BQ = 128;            // query rows per block = MMA M
 constexpr int THREADS = 224;        // warp 0: TMA of Q and K, warp 1: MMA + tensor-memory allocation, warps 2..5: softmax, warp 6: TMA of V
 // shared memory asked for beyond the tiles, to round their base up to 1,024 bytes (the kernel refuses to run if the base ever needs
@@ -78,6 +83,7 @@ struct TcAttnParams {
     int sink;                      // 1: the softmax has one more term without a value, of score sinks[head] (null: 0)
     const float* sinks;
     float softcap;                 // of the score cap (CAP)
+    int keep_first;                // KEEP: keys at positions below this stay visible under the window
     int v_col;                     // DENSE: first value column of a row (key columns are in front: head * HD)
     // DENSE: the result times sigmoid(gate[t, gate_offset + head * dv + c]), or with gate_per_head of column gate_offset + head; or null
     const float* gate; int gate_splits; size_t gate_split_stride; int gate_cols, gate_offset, gate_per_head;
@@ -169,7 +175,8 @@ __device__ __forceinline__ int cache_page(const int* table, int max_blocks, int 
 // HD: elements of queries and keys, HDV of values.  DENSE: keys and values are not in a cache but columns of one matrix with a row per
 // token of this step (kv_row, below), and no token comes from before; queries, keys, values and P are then halves (11 bits of a number in
 // the place of bfloat16's 8: keys and values are rounded once more than the rows they are made from; P is at most 2^8).
-template <int HD, int HDV, int BKEY, bool PEN, int CAP, bool DENSE>
+// KEEP: a windowed query also sees the keys at positions below keep_first: their tiles come first, then the window's.
+template <int HD, int HDV, int BKEY, int PEN, int CAP, bool DENSE, bool KEEP>
 __global__ void __launch_bounds__(THREADS, BKEY == 64 ? 2 : 1) attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q,
                                                                        const __grid_constant__ CUtensorMap map_k,
                                                                        const __grid_constant__ CUtensorMap map_v,
@@ -208,7 +215,10 @@ __global__ void __launch_bounds__(THREADS, BKEY == 64 ? 2 : 1) attention_prefill
     const int lo = max(p.window > 0 ? max(0, p_first - p.window + 1) : 0, p.chunk > 0 ? p_first / p.chunk * p.chunk : 0);
     const int vh = kvh % p.nv;
     const int tile_begin = lo / BKEY;
-    const int n_tiles = p_last / BKEY - tile_begin + 1;
+    // KEEP: tiles of kept keys in front of the window's first tile, which the masks then treat like any other
+    const int kept_tiles = KEEP && p.window > 0 ? (min(p.keep_first, tile_begin * BKEY) + BKEY - 1) / BKEY : 0;
+    const int n_tiles = kept_tiles + p_last / BKEY - tile_begin + 1;
+    auto tile_at = [&](int j) { return KEEP && j < kept_tiles ? j : tile_begin + j - kept_tiles; };
 
     extern __shared__ uint8_t smem_raw[];
     const uint32_t raw = smem_u32(smem_raw);
@@ -259,7 +269,7 @@ __global__ void __launch_bounds__(THREADS, BKEY == 64 ? 2 : 1) attention_prefill
                 if (!mbar_wait(k_empty + 8 * s, phase ^ 1u, status, 1)) break;
                 mbar_expect_tx(k_full + 8 * s, K_BYTES);
                 for (int pg = 0; pg < PAGES; ++pg) {
-                    const int page = (tile_begin + j) * PAGES + pg;
+                    const int page = tile_at(j) * PAGES + pg;
                     const int row0 = DENSE ? kv_row + page * PAGE : (cache_page(table, p.max_blocks, page, p.ring_tokens) * p.nkv + kvh) * PAGE;
                     for (int h = 0; h < HALVES; ++h)
                         tma_load_2d(k_s + s * K_BYTES + h * KEY_HALF_BYTES + pg * (PAGE * 128), &map_k, k_full + 8 * s, (DENSE ? head * HD : 0) + h * 64, row0);
@@ -275,7 +285,7 @@ __global__ void __launch_bounds__(THREADS, BKEY == 64 ? 2 : 1) attention_prefill
                 if (!mbar_wait(v_empty + 8 * s, phase ^ 1u, status, 1)) break;
                 mbar_expect_tx(v_full + 8 * s, V_BYTES);
                 for (int pg = 0; pg < PAGES; ++pg) {
-                    const int page = (tile_begin + j) * PAGES + pg;
+                    const int page = tile_at(j) * PAGES + pg;
                     const int row0 = DENSE ? kv_row + page * PAGE : (cache_page(table, p.max_blocks, page, p.ring_tokens) * p.nv + vh) * PAGE;
                     for (int h = 0; h < V_HALVES; ++h)
                         tma_load_2d(v_s + s * V_BYTES + h * KEY_HALF_BYTES + pg * (PAGE * 128), &map_v, v_full + 8 * s, (DENSE ? p.v_col + head * HDV : 0) + h * 64, row0);
@@ -335,7 +345,8 @@ __global__ void __launch_bounds__(THREADS, BKEY == 64 ? 2 : 1) attention_prefill
         const int qlo = p.chunk > 0 ? qpos / p.chunk * p.chunk : 0;          // first key of the row's chunk
         const int last_lo = p.chunk > 0 ? p_last / p.chunk * p.chunk : 0;
         const float scale2 = p.scale * LOG2E;
-        const float pen_c = PEN ? -p.r1[head] / scale2 : 0.f, pen_r2 = PEN ? -p.r2[head] : 0.f;     // negated once, for the FMAs
+        // negated once, for the FMAs; the linear form works on the unscaled score
+        const float pen_c = PEN ? -p.r1[head] / (PEN == PEN_LINEAR ? p.scale : scale2) : 0.f, pen_r2 = PEN == PEN_LOG ? -p.r2[head] : 0.f;
         const ScoreCap cap = CAP != CAP_NONE ? ScoreCap::make<CAP>(p.softcap, p.scale) : ScoreCap{};
         float m_run = -INFINITY, l_run = 0.f;              // the maximum this row scales by (scaled base-2 domain) and its sum
         pdl_wait();                                        // the output may still be read by an earlier kernel
@@ -345,14 +356,20 @@ __global__ void __launch_bounds__(THREADS, BKEY == 64 ? 2 : 1) attention_prefill
             if (!mbar_wait(s_full + 8 * s, (uint32_t)(j >> 1) & 1u, status, 3)) { ok = false; break; }
             tc_fence_after();
             const uint32_t s_addr = lane_addr + (s ? S_COL1 : S_COL0);
-            const int pos0 = (tile_begin + j) * BKEY;
+            const int pos0 = tile_at(j) * BKEY;
             // the whole row of scores, once
             constexpr int QUARTERS = BKEY / 32;            // 32-key pieces of the row
             uint32_t v[QUARTERS][32];
 #pragma unroll
             for (int q = 0; q < QUARTERS; ++q) tmem_load32_start(s_addr + (uint32_t)(q * 32), v[q]);
             tmem_wait_ld();
-            if (PEN) {
+            if (PEN == PEN_LINEAR) {
+                const float first = (float)(qpos - pos0);                         // distance to the tile's first key
+#pragma unroll
+                for (int q = 0; q < QUARTERS; ++q)
+#pragma unroll
+                    for (int c = 0; c < 32; ++c) v[q][c] = __float_as_uint(fmaf(pen_c, first - (float)(q * 32 + c), __uint_as_float(v[q][c])));
+            } else if (PEN == PEN_LOG) {
                 const float first = fmaf(-pen_r2, (float)(qpos - pos0), 1.f);      // 1 + r2 * distance to the tile's first key
 #pragma unroll
                 for (int q = 0; q < QUARTERS; ++q)
@@ -377,14 +394,14 @@ __global__ void __launch_bounds__(THREADS, BKEY == 64 ? 2 : 1) attention_prefill
                     for (int c = 0; c < 32; ++c) v[q][c] = __float_as_uint(capped<CAP>(__uint_as_float(v[q][c]), cap));
             }
             // mask only where some row of the block cannot see the whole tile
-            const bool masked = pos0 + BKEY - 1 > p_first || (p.window > 0 && pos0 <= p_last - p.window) || pos0 < last_lo;
+            const bool masked = pos0 + BKEY - 1 > p_first || (p.window > 0 && pos0 <= p_last - p.window && !(KEEP && pos0 + BKEY <= p.keep_first)) || pos0 < last_lo;
             if (masked) {
 #pragma unroll
                 for (int q = 0; q < QUARTERS; ++q)
 #pragma unroll
                     for (int c = 0; c < 32; ++c) {
                         const int pos = pos0 + q * 32 + c;
-                        if (!(pos <= qpos && (p.window <= 0 || pos > qpos - p.window) && pos >= qlo)) v[q][c] = 0xff800000u;   // -inf
+                        if (!(pos <= qpos && (p.window <= 0 || pos > qpos - p.window || (KEEP && pos < p.keep_first)) && pos >= qlo)) v[q][c] = 0xff800000u;   // -inf
                     }
             }
             float mx[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
@@ -508,7 +525,7 @@ __global__ void __launch_bounds__(THREADS, BKEY == 64 ? 2 : 1) attention_prefill
     }
 }
 
-template <int HD, int HDV, int BKEY, bool PEN, int CAP, bool DENSE>
+template <int HD, int HDV, int BKEY, int PEN, int CAP, bool DENSE = false, bool KEEP = false>
 int launch(const CUtensorMap& map_q, const CUtensorMap& map_k, const CUtensorMap& map_v, const TcAttnParams& p, int n_seqs,
            int max_q_len, cudaStream_t stream) {
     // Q, two key tiles, the value tiles, alignment slack, barriers
@@ -516,12 +533,12 @@ int launch(const CUtensorMap& map_q, const CUtensorMap& map_k, const CUtensorMap
                         128 + 64;
     static bool configured = false;
     if (!configured) {
-        cudaError_t err = cudaFuncSetAttribute(attention_prefill_tc_kernel<HD, HDV, BKEY, PEN, CAP, DENSE>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+        cudaError_t err = cudaFuncSetAttribute(attention_prefill_tc_kernel<HD, HDV, BKEY, PEN, CAP, DENSE, KEEP>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
         if (err != cudaSuccess) QT_FAIL(QT_ERR_LAUNCH, "attention_prefill_tc: cannot raise shared memory: %s", cudaGetErrorString(err));
         configured = true;
     }
     dim3 grid(p.nq, (max_q_len + BQ - 1) / BQ, n_seqs);
-    launch_kernel(attention_prefill_tc_kernel<HD, HDV, BKEY, PEN, CAP, DENSE>, grid, dim3(THREADS), smem, stream, map_q, map_k, map_v, p);
+    launch_kernel(attention_prefill_tc_kernel<HD, HDV, BKEY, PEN, CAP, DENSE, KEEP>, grid, dim3(THREADS), smem, stream, map_q, map_k, map_v, p);
     QT_CHECK_LAUNCH("attention_prefill_tc");
     return QT_OK;
 }
@@ -534,7 +551,7 @@ extern "C" int qt_attention_prefill_tc(const void* q, const void* k_cache, const
                                        int n_pages, const int* block_table, int max_blocks, const int* seq_start,
                                        const int* seq_past, int n_seqs, int max_q_len, int nq, int nkv, int d,
                                        int page_tokens, int ring_tokens, int window, float scale, const float* r1, const float* r2,
-                                       int chunk, int nv, int sink, const float* sinks, float softcap, int cap_small,
+                                       int chunk, int nv, int keep_first, int sink, const float* sinks, float softcap, int cap_small,
                                        int* status, void* stream) {
     if (n_seqs == 0 || max_q_len == 0) return QT_OK;
     QT_REQUIRE(n_seqs > 0 && nq > 0 && nkv > 0 && nq % nkv == 0, "attention_prefill_tc: bad head counts nq=%d nkv=%d (B=%d)", nq, nkv, n_seqs);
@@ -544,8 +561,10 @@ extern "C" int qt_attention_prefill_tc(const void* q, const void* k_cache, const
     QT_REQUIRE(ring_tokens == 0 || (window > 0 && ring_tokens >= window), "attention_prefill_tc: a ring of %d tokens cannot hold a window of %d", ring_tokens, window);
     QT_REQUIRE(n_seqs <= 65535 && (max_q_len + BQ - 1) / BQ <= 65535 && max_blocks > 0 && n_pages > 0 && n_tokens > 0, "attention_prefill_tc: bad sizes");
     QT_REQUIRE(status != nullptr, "attention_prefill_tc: a status word is required");
-    QT_REQUIRE((r1 == nullptr) == (r2 == nullptr) && (r1 == nullptr || scale > 0.f),
-               "attention_prefill_tc: the distance penalty needs both of its factors and a positive score scale");
+    QT_REQUIRE((r1 != nullptr || r2 == nullptr) && (r1 == nullptr || scale > 0.f),
+               "attention_prefill_tc: the distance penalty needs its first factor and a positive score scale");
+    QT_REQUIRE(keep_first >= 0 && (keep_first == 0 || (ring_tokens == 0 && chunk == 0 && !r2 && softcap == 0.f)),
+               "attention_prefill_tc: kept first keys (%d) go with no ring, no chunks of positions, no logarithmic penalty and no score cap", keep_first);
     QT_REQUIRE(softcap >= 0.f && (softcap == 0.f || (!r1 && scale > 0.f)), "attention_prefill_tc: a score cap of %g goes with a positive scale and no distance penalty",
                (double)softcap);
     QT_REQUIRE(((uintptr_t)q % 16 == 0) && ((uintptr_t)k_cache % 16 == 0) && ((uintptr_t)v_cache % 16 == 0) && ((uintptr_t)out % 16 == 0),
@@ -560,18 +579,24 @@ extern "C" int qt_attention_prefill_tc(const void* q, const void* k_cache, const
     rc = tensor_map(&map_v, v_cache, (uint64_t)n_pages * nv * PAGE, (uint64_t)d, PAGE);
     if (rc) return rc;
     TcAttnParams p{(__nv_bfloat16*)out, block_table, max_blocks, seq_start, seq_past, nq, nkv, ring_tokens, window, chunk, nv, scale, status, r1, r2,
-                   sink, sinks, softcap, 0, nullptr, 1, 0, 0, 0, 0};
+                   sink, sinks, softcap, keep_first, 0, nullptr, 1, 0, 0, 0, 0};
     cudaStream_t s = (cudaStream_t)stream;
     // key tiles of one page, two blocks per SM: measured 12-22 % faster than tiles of two pages with one block per SM
 #define QT_LAUNCH_TC(PEN, CAP)                                                                      \
     do {                                                                                            \
-        if (d == 64) return launch<64, 64, 64, PEN, CAP, false>(map_q, map_k, map_v, p, n_seqs, max_q_len, s); \
-        return launch<128, 128, 64, PEN, CAP, false>(map_q, map_k, map_v, p, n_seqs, max_q_len, s);             \
+        if (d == 64) return launch<64, 64, 64, PEN, CAP>(map_q, map_k, map_v, p, n_seqs, max_q_len, s); \
+        return launch<128, 128, 64, PEN, CAP>(map_q, map_k, map_v, p, n_seqs, max_q_len, s);             \
     } while (0)
-    if (r1) QT_LAUNCH_TC(true, CAP_NONE);
-    if (softcap > 0.f && cap_small) QT_LAUNCH_TC(false, CAP_SMALL);
-    if (softcap > 0.f) QT_LAUNCH_TC(false, CAP_ANY);
-    QT_LAUNCH_TC(false, CAP_NONE);
+    if ((r1 && !r2) || keep_first > 0) {                   // a linear penalty takes kept keys too, of which there may be none
+        if (d == 64 && r1) return launch<64, 64, 64, PEN_LINEAR, CAP_NONE, false, true>(map_q, map_k, map_v, p, n_seqs, max_q_len, s);
+        if (d == 64) return launch<64, 64, 64, PEN_NONE, CAP_NONE, false, true>(map_q, map_k, map_v, p, n_seqs, max_q_len, s);
+        if (r1) return launch<128, 128, 64, PEN_LINEAR, CAP_NONE, false, true>(map_q, map_k, map_v, p, n_seqs, max_q_len, s);
+        return launch<128, 128, 64, PEN_NONE, CAP_NONE, false, true>(map_q, map_k, map_v, p, n_seqs, max_q_len, s);
+    }
+    if (r1) QT_LAUNCH_TC(PEN_LOG, CAP_NONE);
+    if (softcap > 0.f && cap_small) QT_LAUNCH_TC(PEN_NONE, CAP_SMALL);
+    if (softcap > 0.f) QT_LAUNCH_TC(PEN_NONE, CAP_ANY);
+    QT_LAUNCH_TC(PEN_NONE, CAP_NONE);
 #undef QT_LAUNCH_TC
 }
 
@@ -597,13 +622,13 @@ extern "C" int qt_attention_prefill_rows(const void* q, const void* kv, void* ou
     if (rc) return rc;
     rc = tensor_map(&map_kv, kv, (uint64_t)kv_rows, (uint64_t)heads * (dk + dv), PAGE);
     if (rc) return rc;
-    TcAttnParams p{(__nv_bfloat16*)out, nullptr, 0, seq_start, nullptr, heads, heads, 0, window, 0, heads, scale, status, nullptr, nullptr, 0, nullptr, 0.f, heads * dk, gate,
+    TcAttnParams p{(__nv_bfloat16*)out, nullptr, 0, seq_start, nullptr, heads, heads, 0, window, 0, heads, scale, status, nullptr, nullptr, 0, nullptr, 0.f, 0, heads * dk, gate,
                    gate_splits, (size_t)gate_split_stride, gate_cols, gate_offset, gate_per_head};
     cudaStream_t s = (cudaStream_t)stream;
-    if (dk == 128 && dv == 64) return launch<128, 64, 64, false, CAP_NONE, true>(map_q, map_kv, map_kv, p, n_seqs, max_q_len, s);
-    if (dk == 128) return launch<128, 128, 64, false, CAP_NONE, true>(map_q, map_kv, map_kv, p, n_seqs, max_q_len, s);
-    if (dv == 64) return launch<192, 64, 64, false, CAP_NONE, true>(map_q, map_kv, map_kv, p, n_seqs, max_q_len, s);
-    return launch<192, 128, 64, false, CAP_NONE, true>(map_q, map_kv, map_kv, p, n_seqs, max_q_len, s);
+    if (dk == 128 && dv == 64) return launch<128, 64, 64, PEN_NONE, CAP_NONE, true>(map_q, map_kv, map_kv, p, n_seqs, max_q_len, s);
+    if (dk == 128) return launch<128, 128, 64, PEN_NONE, CAP_NONE, true>(map_q, map_kv, map_kv, p, n_seqs, max_q_len, s);
+    if (dv == 64) return launch<192, 64, 64, PEN_NONE, CAP_NONE, true>(map_q, map_kv, map_kv, p, n_seqs, max_q_len, s);
+    return launch<192, 128, 64, PEN_NONE, CAP_NONE, true>(map_q, map_kv, map_kv, p, n_seqs, max_q_len, s);
 }
 
 QT_DEFINE_LAST_ERROR(attention_tc)

@@ -130,7 +130,7 @@ _SIGNATURES = {
     },
     "attention_tc": {
         "qt_attention_prefill_tc": [_c_ptr, _c_ptr, _c_ptr, _c_ptr, _c_int, _c_int, _c_ptr, _c_int, _c_ptr, _c_ptr, _c_int,
-                                    _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_float, _c_ptr, _c_ptr, _c_int, _c_int, _c_int, _c_ptr, _c_float, _c_int, _c_ptr, _c_ptr],
+                                    _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_float, _c_ptr, _c_ptr, _c_int, _c_int, _c_int, _c_int, _c_ptr, _c_float, _c_int, _c_ptr, _c_ptr],
         "qt_attention_prefill_rows": [_c_ptr, _c_ptr, _c_ptr, _c_int, _c_int, _c_ptr, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_float, _c_ptr,
                                       _c_int, _c_ll, _c_int, _c_int, _c_int, _c_ptr, _c_ptr],
     },
@@ -1073,12 +1073,15 @@ def _extended_choice(q, k_cache, v_cache, page_tokens: int, ring_tokens: int, sc
     """The kernel for a call that asks for a linear distance penalty (``penalty`` = (slopes, None)), kept first keys, a
     softmax sink, a cap on the scores, or values that are the head of the cached key rows; None for a call that asks for none of
     these.  The mma.sync kernels (``mma`` names the caller's) compute the first four for values as wide as the keys (a cap goes
-    with no penalty), the tcgen05 prefill kernel a sink and a cap; the generic kernels compute everything."""
+    with no penalty), the tcgen05 prefill kernel each of them, kept keys and the linear penalty without a cap; the generic kernels compute
+    everything."""
     if not ((penalty is not None and penalty[1] is None) or keep_first > 0 or sink or v_dim is not None or softcap is not None):
         return None
     fits = (v_dim is None and v_cache.shape[-1] == q.shape[2] and attention_mma_supported(q, page_tokens) and scale > 0
             and not (keep_first > 0 and (ring_tokens or chunk)) and not (softcap is not None and penalty is not None))
-    if mma == "mma" and impl in (None, "tc") and fits and penalty is None and not keep_first and attention_tc_supported(q, page_tokens):
+    plain = penalty is None and not keep_first
+    kept = softcap is None and chunk is None and (penalty is None or penalty[1] is None)
+    if mma == "mma" and impl in (None, "tc") and fits and (plain or kept) and attention_tc_supported(q, page_tokens):
         return "tc"
     if impl in (None, mma) and fits:
         return mma
@@ -1222,7 +1225,7 @@ def attention_prefill(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Ten
               k_cache.shape[0], _ptr(block_table), block_table.shape[1], _ptr(seq_start), _ptr(seq_past), n_seqs,
               int(max_q_len), num_heads, num_kv_heads, head_dim, page_tokens, ring_tokens, int(window or 0), float(scale),
               _ptr(penalty[0]) if penalty else None, _ptr(penalty[1]) if penalty else None, int(chunk or 0), v_cache.shape[1],
-              1 if sink else 0, _ptr(sinks), cap, cap_small, _ptr(_status_word(q.device)), _stream())
+              int(keep_first), 1 if sink else 0, _ptr(sinks), cap, cap_small, _ptr(_status_word(q.device)), _stream())
         return
     if choice == "mma":
         _call("attention_mma", "qt_attention_prefill_mma", _ptr(q), _ptr(k_cache), _ptr(v_cache), _ptr(out),

@@ -810,3 +810,37 @@ def test_zero_rows_of_several_tensors():
         assert float(tensor[3].abs().max()) == 0.0 and float(tensor[[0, 1, 2, 4]].float().min()) == 1.0
     with pytest.raises(kernels.KernelError):
         kernels.row_table([torch.ones(5, 3, device=DEV)])
+
+
+@pytest.mark.parametrize("d, nq, nkv", [(64, 4, 2), (128, 3, 1)])
+@pytest.mark.parametrize("window, keep_first, linear, sink", [(33, 1, False, False), (64, 63, True, True), (65, 64, False, True), (130, 65, True, False), (1, 200, True, True),
+                                                              (300, 128, False, False), (40, 0, True, False), (None, 0, True, True)])
+def test_tensor_core_prefill_with_kept_keys_and_linear_penalty(d, nq, nkv, window, keep_first, linear, sink):
+    """The tcgen05 kernel's kept tiles in front of the window's: windows and kept keys on, before and behind a tile's edge, more kept keys
+    than lie before the window, portions behind a past; 64 bits.  Bound: weights and operands of 8 bits, 2e-2 as for the other forms."""
+    q_lens, past = [150, 1, 129, 64, 300], [100, 400, 0, 191, 33]
+    totals = [p + n for p, n in zip(past, q_lens)]
+    dtype = torch.bfloat16
+    k = [rand(t, nkv, d, seed=220 + i, dtype=dtype).float().cpu() for i, t in enumerate(totals)]
+    v = [rand(t, nkv, d, seed=230 + i, dtype=dtype).float().cpu() for i, t in enumerate(totals)]
+    k_cache, v_cache, table = paged(k, v, totals, dtype, seed=4)
+    q = rand(sum(q_lens), nq, d, seed=240, dtype=dtype)
+    slope = rand(nq, seed=241).abs() * 0.05
+    out = torch.full_like(q, float("nan"))
+    as_int = lambda values: torch.tensor(values, dtype=torch.int32, device=DEV)
+    kernels.attention_prefill(q, k_cache, v_cache, out, table, as_int([sum(q_lens[:i]) for i in range(len(q_lens) + 1)]), as_int(past), max(q_lens), nkv, PAGE, 0,
+                              window, d ** -0.5, impl="tc", keep_first=keep_first, sink=sink, penalty=(slope, None) if linear else None)
+    kernels.check_status(DEV)
+    start = 0
+    for i, n in enumerate(q_lens):
+        pos, key = torch.arange(past[i], totals[i])[:, None], torch.arange(totals[i])[None]
+        seen = (key <= pos) & ((key > pos - (window or totals[i])) | (key < keep_first))
+        score = torch.einsum("qhd,khd->hqk", q[start:start + n].cpu().double(), k[i].double().repeat_interleave(nq // nkv, 1)) * d ** -0.5
+        if linear:
+            score = score - slope.cpu().double()[:, None, None] * (pos - key)
+        score = score.masked_fill(~seen, float("-inf"))
+        if sink:
+            score = torch.cat((score, torch.zeros(nq, n, 1, dtype=torch.float64)), dim=-1)
+        want = torch.einsum("hqk,khd->qhd", score.softmax(-1)[..., :totals[i]], v[i].double().repeat_interleave(nq // nkv, 1))
+        close(out[start:start + n], want, dtype, f"sequence {i}")
+        start += n
