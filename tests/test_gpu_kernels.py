@@ -844,3 +844,36 @@ def test_tensor_core_prefill_with_kept_keys_and_linear_penalty(d, nq, nkv, windo
         want = torch.einsum("hqk,khd->qhd", score.softmax(-1)[..., :totals[i]], v[i].double().repeat_interleave(nq // nkv, 1))
         close(out[start:start + n], want, dtype, f"sequence {i}")
         start += n
+
+
+@pytest.mark.parametrize("in_dtype, out_dtype, splits", [(torch.float32, torch.float32, 2), (torch.float32, torch.bfloat16, 1), (torch.bfloat16, torch.bfloat16, 1)])
+@pytest.mark.parametrize("nq, nkv, nv, d, rotary, interleaved, norm, extra, ring, kv", [
+    (5, 3, 3, 128, 64, False, "weights", 8, 0, True), (9, 1, 1, 64, 8, False, "unit", 0, 320, True), (17, 4, 2, 128, 128, False, "row", 4, 0, True),
+    (33, 2, 2, 64, 64, False, "none", 0, 0, True), (4, 4, 4, 128, 0, True, "weights", 0, 0, True), (6, 2, 2, 64, 48, False, "weights", 12, 0, False)])
+def test_qk_heads_of_many_tokens_follow_the_few_token_form(in_dtype, out_dtype, splits, nq, nkv, nv, d, rotary, interleaved, norm, extra, ring, kv):
+    """256 tokens and more (a head over 16 or 32 lanes) against the same tokens in calls of 100: any rotated part, norms with and without
+    weights and over the whole row, columns behind, value heads of their own count, a ring, queries alone.  Sums of d squares in another
+    order: a few 2^-24 of a value, and in bfloat16 the rounding that may fall the other way."""
+    tokens, heads = 300, nq + (nkv + nv if kv else 0)
+    qkv = rand(splits, tokens, heads * d + extra, seed=5, dtype=in_dtype)
+    wide = norm == "row"
+    qw, kw = (1.0 + rand(d * (n if wide else 1), seed=6 + n, scale=0.2) for n in (nq, nkv)) if norm in ("weights", "row") else (None, None)
+    cos_sin = rand(512, rotary, seed=8) if rotary else None
+    pos = torch.randperm(300 if ring else 512, generator=gen(3))[:tokens].int().to(DEV)
+    seq = torch.zeros(tokens, dtype=torch.int32, device=DEV)
+    table = torch.randperm(8, generator=gen(4)).int()[None].to(DEV)
+    got = []
+    for step in (tokens, 100):
+        q_out = torch.full((tokens, nq, d), 7.0, dtype=out_dtype, device=DEV)
+        k_cache, v_cache = torch.full((8, nkv, PAGE, d), 7.0, dtype=out_dtype, device=DEV), torch.full((8, nv, PAGE, d), 7.0, dtype=out_dtype, device=DEV)
+        for at in range(0, tokens, step):
+            part = slice(at, at + step)
+            kernels.qk_norm_rope_write(GemmOut(qkv[:, part].contiguous()), q_out[part], k_cache if kv else None, v_cache if kv else None, seq[part], pos[part], table if kv else None,
+                                       qw, kw if kv or wide else None, 1e-5, cos_sin, nq, nkv, d, PAGE, ring, write_kv=kv, kv_in_proj=kv, interleaved=interleaved,
+                                       v_heads=nv, v_head_dim=d, unit_norm=norm == "unit", row_inv=torch.empty(tokens, 2, device=DEV)[:step] if wide else None, extra_cols=extra)
+        got.append((q_out, k_cache, v_cache))
+    for new, old in zip(*got):
+        off, size = (new.double() - old.double()).abs(), old.double().abs()
+        assert float((off - size * (2.0 ** -7 if out_dtype == torch.bfloat16 else 0.0)).max()) < 2e-6
+        if out_dtype == torch.bfloat16:
+            assert float((off > 0).double().mean()) < 0.02
