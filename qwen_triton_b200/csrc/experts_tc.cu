@@ -1,7 +1,7 @@
 // The two products of table-chosen experts for many tokens, on the fifth-generation tensor cores.
 //
-// The rows (token, expert pairs) arrive ordered by expert, every expert's run padded to whole tiles of 128 rows
-// (experts.cu), so a tile's rows all take one expert's weight: Y[rows of the tile, :] = X[rows, :] * W[e]^T with e read
+// The rows (token, expert pairs) arrive ordered by expert, every expert's run padded to whole tiles of 128 rows (or, of few rows an expert, of
+// 32: expert_gemm_few_kernel) (experts.cu), so a tile's rows all take one expert's weight: Y[rows of the tile, :] = X[rows, :] * W[e]^T with e read
 // from `tile_expert`.  A tile beyond the last run (-1) leaves at once.  The weights of all experts are one matrix
 // [E * N, K]; a weight tile of 128 rows that reaches past its expert's N rows reads the next expert's (or zeros past
 // the end), and the epilogue drops those columns.
@@ -312,6 +312,130 @@ int launch_persistent(const void* x, const void* w, TO* out, const int* tile_exp
     return QT_OK;
 }
 
+// Few rows an expert (a decode step of many sequences, a short prompt): runs padded to tiles of FEW_ROWS = 32 rows, and the roles exchanged:
+// 128 weight rows are the MMA's M, the tile's rows its N.  Such a product is bound by the weights' bytes; tiles of 128 rows
+// brought as many bytes of padding through L2.  A five-stage ring of 20 KB, two blocks an SM.  A thread of the epilogue holds one feature of 32 rows, a
+// warp stores 64 bytes of a row at a time.  Route, both products, gate and sum of 64 pairs, weights not in L2, in tiles of
+// 32 / 128 rows: 16 experts of 2,048 x 1,024 65 / 74 us, 8 of 1,024 x 2,048 49 / 57 us (30.8 and 15.4 us of weights at the measured copy rate).
+constexpr int FEW_ROWS = 32, FEW_STAGES = 5;
+constexpr uint32_t FEW_STAGE_BYTES = A_BYTES + FEW_ROWS * BK * 2;
+
+template <bool ACT>
+__global__ void __launch_bounds__(THREADS) expert_gemm_few_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_w,
+                                                                  __nv_bfloat16* __restrict__ out, const int* __restrict__ tile_expert, int n_out, int kb_total,
+                                                                  int w_tiles, int act, int* status) {
+    // instruction descriptor: float accumulator, bfloat16 A (weights) and B (rows), both K-major, N = FEW_ROWS, M = 128
+    constexpr uint32_t IDESC = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(FEW_ROWS >> 3) << 17) | ((uint32_t)(BM >> 4) << 24);
+    extern __shared__ uint8_t smem_raw[];
+    pdl_launch_dependents();
+    pdl_wait();                                                    // the routing and the rows come from the kernels before
+    const int x_tile = blockIdx.x / w_tiles, w_tile = blockIdx.x % w_tiles, expert = tile_expert[x_tile];
+    if (expert < 0) return;                                        // the whole block: nothing is set up yet
+
+    const uint32_t raw = smem_u32(smem_raw), base = (raw + 1023u) & ~1023u;      // swizzled tiles need 1024-byte alignment
+    uint8_t* smem = smem_raw + (base - raw);
+    uint64_t* bars = reinterpret_cast<uint64_t*>(smem + (size_t)FEW_STAGES * FEW_STAGE_BYTES);
+    const uint32_t full0 = base + FEW_STAGES * FEW_STAGE_BYTES, empty0 = full0 + 8 * FEW_STAGES, tmem_full = empty0 + 8 * FEW_STAGES;
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * FEW_STAGES + 1);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, x0 = x_tile * FEW_ROWS, w0 = expert * n_out + w_tile * BM;
+
+    if (threadIdx.x == 0) {
+        prefetch_tensor_map(&map_w);
+        prefetch_tensor_map(&map_x);
+        for (int s = 0; s < FEW_STAGES; ++s) { mbar_init(full0 + 8 * s, 1); mbar_init(empty0 + 8 * s, 1); }
+        mbar_init(tmem_full, 1);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == 1) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"((uint32_t)FEW_ROWS) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem_base = *tmem_slot;
+
+    if (warp == 0) {
+        if (lane == 0) {
+            int s = 0;
+            uint32_t phase = 0;
+            for (int i = 0; i < kb_total; ++i) {
+                if (i >= FEW_STAGES && !mbar_wait(empty0 + 8 * s, phase ^ 1u, status, 1)) break;
+                mbar_expect_tx(full0 + 8 * s, FEW_STAGE_BYTES);
+                const uint32_t dst = base + s * FEW_STAGE_BYTES;
+                tma_load_2d(dst, &map_w, full0 + 8 * s, i * BK, w0);
+                tma_load_2d(dst + A_BYTES, &map_x, full0 + 8 * s, i * BK, x0);
+                if (++s == FEW_STAGES) { s = 0; phase ^= 1u; }
+            }
+        }
+    } else if (warp == 1) {
+        if (lane == 0) {
+            const uint64_t a_desc0 = operand_desc(base), b_desc0 = operand_desc(base + A_BYTES);
+            int s = 0;
+            uint32_t phase = 0;
+            for (int i = 0; i < kb_total; ++i) {
+                if (!mbar_wait(full0 + 8 * s, phase, status, 2)) break;
+                tc_fence_after();
+                const uint64_t a_desc = a_desc0 + (uint64_t)(s * (FEW_STAGE_BYTES >> 4)), b_desc = b_desc0 + (uint64_t)(s * (FEW_STAGE_BYTES >> 4));
+#pragma unroll
+                for (int k = 0; k < BK / UMMA_K; ++k)      // 32 bytes further along K inside the swizzled row
+                    umma_bf16(tmem_base, a_desc + 2 * k, b_desc + 2 * k, IDESC, (i > 0 || k > 0) ? 1u : 0u);
+                umma_commit(empty0 + 8 * s);
+                if (++s == FEW_STAGES) { s = 0; phase ^= 1u; }
+            }
+            umma_commit(tmem_full);
+        }
+    } else {
+        const int quarter = warp & 3, n = w_tile * BM + quarter * 32 + lane;      // the accumulator lanes this warp may read
+        const bool ready = mbar_wait(tmem_full, 0, status, 3);
+        tc_fence_after();
+        if (ready) {
+            uint32_t v[32];
+            tmem_load32(tmem_base + ((uint32_t)(quarter * 32) << 16), v);
+            if (n < n_out) {
+                __nv_bfloat16* dst = out + (size_t)x0 * n_out + n;
+#pragma unroll
+                for (int r = 0; r < FEW_ROWS; ++r) {
+                    const float y = __uint_as_float(v[r]);
+                    dst[(size_t)r * n_out] = __float2bfloat16_rn(ACT ? gate_activation<true>(y, act) : y);
+                }
+            }
+        }
+    }
+    tc_fence_before();
+    __syncthreads();
+    if (*(volatile int*)status != 0) {                     // a wait gave up: let copies in flight land before the block leaves
+        const unsigned long long t0 = global_timer();
+        while (global_timer() - t0 < 2000000ull) __nanosleep(1000);
+    }
+    if (warp == 1) {
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"((uint32_t)FEW_ROWS) : "memory");
+    }
+}
+
+template <bool ACT>
+int launch_few(const void* x, const void* w, __nv_bfloat16* out, const int* tile_expert, int max_tiles, int experts, int n_out, int K, int act, int* status,
+               cudaStream_t stream) {
+    CUtensorMap map_x, map_w;
+    int rc = tensor_map(&map_x, x, (uint64_t)max_tiles * FEW_ROWS, (uint64_t)K, FEW_ROWS);
+    if (rc) return rc;
+    rc = tensor_map(&map_w, w, (uint64_t)experts * n_out, (uint64_t)K, BM);
+    if (rc) return rc;
+    const size_t smem = (size_t)FEW_STAGES * FEW_STAGE_BYTES + 1024 + (2 * FEW_STAGES + 1) * 8 + 16;
+    static bool configured = false;
+    if (!configured) {
+        cudaError_t err = cudaFuncSetAttribute(expert_gemm_few_kernel<ACT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (err != cudaSuccess) QT_FAIL(QT_ERR_LAUNCH, "expert_gemm: cannot raise shared memory: %s", cudaGetErrorString(err));
+        configured = true;
+    }
+    const int w_tiles = (n_out + BM - 1) / BM, kb_total = (K + BK - 1) / BK;
+    QT_REQUIRE((long long)max_tiles * w_tiles < (1ll << 31), "expert_gemm: too many tiles for one launch");
+    launch_kernel(expert_gemm_few_kernel<ACT>, dim3((unsigned)(max_tiles * w_tiles)), dim3(THREADS), smem, stream, map_x, map_w, out, tile_expert, n_out, kb_total,
+                  w_tiles, act, status);
+    QT_CHECK_LAUNCH("expert_gemm_few");
+    return QT_OK;
+}
+
 template <typename TO, bool ACT, int BN, int STAGES>
 int launch_tile(const void* x, const void* w, TO* out, const int* tile_expert, int max_tiles, int experts, int n_out, int K, int act, int* status,
                 cudaStream_t stream) {
@@ -369,6 +493,19 @@ extern "C" int qt_expert_gemm(const void* x, const void* w, void* out, int out_d
     if (out_dtype == QT_BF16) return launch<__nv_bfloat16, false>(x, w, (__nv_bfloat16*)out, tile_expert, max_tiles, experts, n_out, K, 0, status, s);
     if (out_dtype == QT_F32 && act < 0) return launch<float, false>(x, w, (float*)out, tile_expert, max_tiles, experts, n_out, K, 0, status, s);
     QT_FAIL(QT_ERR_ARG, "expert_gemm: output type %d%s is not offered", out_dtype, act >= 0 ? " with an activation" : "");
+}
+
+// The same for tiles of 32 rows: out [max_tiles * 32, n_out] bfloat16 = act?(x [max_tiles * 32, K] * w[tile's expert]^T).
+extern "C" int qt_expert_gemm_few(const void* x, const void* w, void* out, const int* tile_expert, int max_tiles, int experts, int n_out, int K, int act,
+                                  int* status, void* stream) {
+    QT_REQUIRE(max_tiles > 0 && experts > 0 && n_out > 0 && K > 0, "expert_gemm: bad sizes tiles=%d E=%d N=%d K=%d", max_tiles, experts, n_out, K);
+    QT_REQUIRE(K % 8 == 0, "expert_gemm: K=%d must be a multiple of 8 (16-byte rows for TMA)", K);
+    QT_REQUIRE((((uintptr_t)x | (uintptr_t)w) & 15) == 0, "expert_gemm: operands must be 16-byte aligned");
+    QT_REQUIRE(act < QT_ACT_COUNT, "expert_gemm: unknown activation code %d", act);
+    QT_REQUIRE(status != nullptr && tile_expert != nullptr, "expert_gemm: a status word and the tiles' experts are required");
+    cudaStream_t s = (cudaStream_t)stream;
+    if (act >= 0) return launch_few<true>(x, w, (__nv_bfloat16*)out, tile_expert, max_tiles, experts, n_out, K, act, status, s);
+    return launch_few<false>(x, w, (__nv_bfloat16*)out, tile_expert, max_tiles, experts, n_out, K, 0, status, s);
 }
 
 QT_DEFINE_LAST_ERROR(experts_tc)

@@ -117,6 +117,7 @@ _SIGNATURES = {
         "qt_experts_combine": [_c_ptr, _c_int, _c_ptr, _c_ptr, _c_int, _c_int, _c_int, _c_float, _c_ptr, _c_ptr, _c_int, _c_ll, _c_ptr, _c_ptr],
     },
     "experts_tc": {
+        "qt_expert_gemm_few": [_c_ptr, _c_ptr, _c_ptr, _c_ptr, _c_int, _c_int, _c_int, _c_int, _c_int, _c_ptr, _c_ptr],
         "qt_expert_gemm": [_c_ptr, _c_ptr, _c_ptr, _c_int, _c_ptr, _c_int, _c_int, _c_int, _c_int, _c_int, _c_ptr, _c_ptr],
     },
     "attention_mma": {
@@ -1388,9 +1389,18 @@ def experts_by_pair(x: torch.Tensor, token_ids: torch.Tensor | None, table: torc
 EXPERT_TILE_ROWS = 128      # rows of one tile of the tiled expert products (the MMA's M)
 
 
+_EXPERT_FEW_ROWS = 32       # rows of one tile where the experts have few rows each
+
+
+def expert_tile_rows(pairs: int, experts: int) -> int:
+    """Rows of a tile: 32 for up to 24 pairs an expert on average, else 128 (the whole feed-forward of 16 experts of 2,048 x 1,024 in tiles of
+    32 / 128 rows: 64 pairs 65 / 74 us, 384 pairs 68 / 76 us, 512 pairs 77 / 76 us)."""
+    return _EXPERT_FEW_ROWS if pairs <= 24 * experts else EXPERT_TILE_ROWS
+
+
 def expert_tiles(pairs: int, experts: int) -> int:
     """Tiles that hold ``pairs`` rows ordered by expert, however they fall: every expert's run ends in a tile of its own."""
-    return pairs // EXPERT_TILE_ROWS + experts
+    return pairs // expert_tile_rows(pairs, experts) + experts
 
 
 def experts_tiled_supported(x: torch.Tensor, up: torch.Tensor) -> bool:
@@ -1404,15 +1414,15 @@ def experts_tiled(x: torch.Tensor, token_ids: torch.Tensor | None, table: torch.
                   limit: float = 0.0, wide: torch.Tensor | None = None, base: GemmOut | None = None,
                   row_scale: torch.Tensor | None = None, in_weights: torch.Tensor | None = None) -> None:
     """The same result as ``experts_by_pair`` for many tokens: the (token, expert) pairs are ordered by expert on the
-    device, each expert's run padded to whole tiles of 128 rows, and both products run tile by tile on the tensor
+    device, each expert's run padded to whole tiles of 128 (few pairs: 32) rows, and both products run tile by tile on the tensor
     cores.  Scratch: ``ordered`` [rows, width], ``mid`` [rows, ff], ``y`` [rows, width] (bfloat16) with
-    rows = expert_tiles(T * top, E) * 128, and ``route`` (int32, T * top + rows + rows / 128 words); gated experts
+    rows = expert_tiles(T * top, E) * expert_tile_rows(T * top, E), and ``route`` (int32, T * top + rows + tiles words); gated experts
     also ``wide`` [rows, 2 ff] (their first product, before the gate kernel)."""
     tokens, width = x.shape
     experts, ff = up.shape[0], up.shape[1] // (2 if gated else 1)
     top = table.shape[1]
-    tiles = expert_tiles(tokens * top, experts)
-    rows = tiles * EXPERT_TILE_ROWS
+    tiles, tile_rows = expert_tiles(tokens * top, experts), expert_tile_rows(tokens * top, experts)
+    rows = tiles * tile_rows
     _need(x, "x", torch.bfloat16)
     if token_ids is not None:
         _need(token_ids, "token_ids", torch.int32, (tokens,))
@@ -1430,17 +1440,23 @@ def experts_tiled(x: torch.Tensor, token_ids: torch.Tensor | None, table: torch.
     pair_row, row_token, tile_expert = route[:tokens * top], route[tokens * top:tokens * top + rows], route[tokens * top + rows:]
     status = _status_word(x.device)
     _call("experts", "qt_experts_route", _ptr(x), _ptr(token_ids), _ptr(table), _ptr(ordered), _ptr(pair_row), _ptr(row_token),
-          _ptr(tile_expert), tokens, table.shape[0], top, experts, width, EXPERT_TILE_ROWS, tiles, _ptr(in_weights), _stream(), launches=2)
+          _ptr(tile_expert), tokens, table.shape[0], top, experts, width, tile_rows, tiles, _ptr(in_weights), _stream(), launches=2)
+
+    def product(rows_in, weight, rows_out, n_out, k, act):
+        if tile_rows == EXPERT_TILE_ROWS:
+            _call("experts_tc", "qt_expert_gemm", _ptr(rows_in), _ptr(weight), _ptr(rows_out), BF16, _ptr(tile_expert), tiles, experts, n_out, k, act, _ptr(status),
+                  _stream())
+        else:
+            _call("experts_tc", "qt_expert_gemm_few", _ptr(rows_in), _ptr(weight), _ptr(rows_out), _ptr(tile_expert), tiles, experts, n_out, k, act, _ptr(status),
+                  _stream())
+
     if gated:
         _need(wide, "wide", torch.bfloat16, (rows, 2 * ff))
-        _call("experts_tc", "qt_expert_gemm", _ptr(ordered), _ptr(up), _ptr(wide), BF16, _ptr(tile_expert), tiles, experts, 2 * ff, width,
-              -1, _ptr(status), _stream())
+        product(ordered, up, wide, 2 * ff, width, -1)
         swiglu(GemmOut(wide.view(1, rows, 2 * ff)), mid, 0, activation, limit)
     else:
-        _call("experts_tc", "qt_expert_gemm", _ptr(ordered), _ptr(up), _ptr(mid), BF16, _ptr(tile_expert), tiles, experts, ff, width,
-              activation_code(activation), _ptr(status), _stream())
-    _call("experts_tc", "qt_expert_gemm", _ptr(mid), _ptr(down), _ptr(y), BF16, _ptr(tile_expert), tiles, experts, width, ff,
-          -1, _ptr(status), _stream())
+        product(ordered, up, mid, ff, width, activation_code(activation))
+    product(mid, down, y, width, ff, -1)
     _call("experts", "qt_experts_combine", _ptr(y), BF16, _ptr(pair_row), _ptr(out), tokens, top, width, float(pair_weight),
           weights_ptr, base_ptr, base_splits, base_stride, scale_ptr, _stream())
 

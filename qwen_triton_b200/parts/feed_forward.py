@@ -209,7 +209,7 @@ class TableExperts:
         rows = pairs
         if self.tiled:
             tiles = kernels.expert_tiles(pairs, self.experts)
-            rows = tiles * kernels.EXPERT_TILE_ROWS
+            rows = tiles * kernels.expert_tile_rows(pairs, self.experts)
             ws.declare("experts.ordered", rows * self.hidden, runtime.dtype)
             ws.declare("experts.y", rows * self.hidden, runtime.dtype)
             ws.declare("experts.route", pairs + rows + tiles, torch.int32)
@@ -251,7 +251,7 @@ class TableExperts:
         pairs = tokens * self.top
         if self.tiled and pairs > min(_PAIRS_BY_PAIR, 2 * self.experts):
             tiles = kernels.expert_tiles(pairs, self.experts)
-            rows = tiles * kernels.EXPERT_TILE_ROWS
+            rows = tiles * kernels.expert_tile_rows(pairs, self.experts)
             kernels.experts_tiled(x, ctx.token_ids, self.table, self.up, self.down, ws.view("experts.ordered", rows, self.hidden),
                                   ws.view("experts.mid", rows, self.inter), ws.view("experts.y", rows, self.hidden),
                                   ws.view("experts.route", pairs + rows + tiles), out, self.activation, self.pair_weight)
@@ -344,7 +344,7 @@ class RoutedExperts:
         rows = pairs
         if self.tiled:
             tiles = kernels.expert_tiles(pairs, self.experts)
-            rows = tiles * kernels.EXPERT_TILE_ROWS
+            rows = tiles * kernels.expert_tile_rows(pairs, self.experts)
             ws.declare("experts.ordered", rows * self.hidden, runtime.dtype)
             ws.declare("experts.y", rows * self.hidden, runtime.dtype)
             ws.declare("experts.route", pairs + rows + tiles, torch.int32)
@@ -418,7 +418,7 @@ class RoutedExperts:
         pairs = tokens * self.top
         if self.tiled and pairs > min(_PAIRS_BY_PAIR, 2 * self.experts):
             tiles = kernels.expert_tiles(pairs, self.experts)
-            rows = tiles * kernels.EXPERT_TILE_ROWS
+            rows = tiles * kernels.expert_tile_rows(pairs, self.experts)
             kernels.experts_tiled(x, None, chosen, self.up, self.down, ws.view("experts.ordered", rows, self.hidden),
                                   ws.view("experts.mid", rows, self.inter), ws.view("experts.y", rows, self.hidden),
                                   ws.view("experts.route", pairs + rows + tiles), out, self.activation, pair_weight=1.0, pair_weights=out_weights,

@@ -877,3 +877,30 @@ def test_qk_heads_of_many_tokens_follow_the_few_token_form(in_dtype, out_dtype, 
         assert float((off - size * (2.0 ** -7 if out_dtype == torch.bfloat16 else 0.0)).max()) < 2e-6
         if out_dtype == torch.bfloat16:
             assert float((off > 0).double().mean()) < 0.02
+
+
+@pytest.mark.parametrize("gated", [True, False])
+@pytest.mark.parametrize("tokens, top, experts, width, ff, skew", [(1, 1, 1, 64, 8, False), (33, 1, 3, 72, 200, True), (60, 2, 5, 264, 136, False), (61, 2, 5, 264, 136, True),
+                                                                  (200, 4, 50, 128, 64, False), (64, 1, 4, 520, 1032, True)])
+def test_experts_in_tiles_of_few_and_many_rows(gated, tokens, top, experts, width, ff, skew):
+    """24 pairs an expert and less (tiles of 32 rows) and more (128): runs of more than a tile, experts without a row, features and K that
+    fill no tile; against 64 bits with the roundings between the products, each a 2^-8 of its value at most."""
+    dtype = torch.bfloat16
+    x, up = rand(tokens, width, seed=1, dtype=dtype), rand(experts, (2 if gated else 1) * ff, width, seed=2, scale=width ** -0.5, dtype=dtype)
+    down, pairs = rand(experts, width, ff, seed=3, scale=ff ** -0.5, dtype=dtype), rand(tokens, top, seed=6)
+    table = torch.stack([torch.arange(top) if skew else torch.randperm(experts, generator=gen(t))[:top] for t in range(tokens)]).int()
+    tiles, tile_rows = kernels.expert_tiles(tokens * top, experts), kernels.expert_tile_rows(tokens * top, experts)
+    rows = tiles * tile_rows
+    assert tile_rows == (32 if tokens * top <= 24 * experts else 128)
+    scratch = [torch.full((rows, n), float("nan"), dtype=dtype, device=DEV) for n in (width, ff, width, 2 * ff)]
+    out = torch.full((tokens, width), float("nan"), device=DEV)
+    kernels.experts_tiled(x, None, table.to(DEV), up, down, *scratch[:3], torch.empty(tokens * top + rows + tiles, dtype=torch.int32, device=DEV), out, "silu", pair_weights=pairs,
+                          gated=gated, wide=scratch[3] if gated else None)
+    kernels.check_status(DEV)
+    xd, upd, downd = x.double().cpu(), up.double().cpu(), down.double().cpu()
+    want = torch.zeros(tokens, width, dtype=torch.float64)
+    for t in range(tokens):
+        for j in range(top):
+            h = upd[table[t, j]] @ xd[t]
+            want[t] += float(pairs[t, j]) * (downd[table[t, j]] @ (h[:ff] * torch.sigmoid(h[:ff]) * (h[ff:] if gated else 1.0)))
+    assert float((out.cpu().double() - want).norm() / want.norm()) < 4 * 2.0 ** -8
