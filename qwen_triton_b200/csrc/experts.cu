@@ -381,22 +381,50 @@ __global__ void expert_gather_kernel(const uint4* __restrict__ x, const int* __r
     }
 }
 
-// out[t, :] = pair_weight * sum_k y[pair_row[t * top + k], :], in float, in the order of k.
-template <typename T>
-__global__ void expert_combine_kernel(const T* __restrict__ y, const int* __restrict__ pair_row, float* __restrict__ out, int top, int width,
+// out[t, :] = pair_weight * sum_k y[pair_row[t * top + k], :], in float, in the order of k.  Bound by the bytes of the rows; a thread takes V
+// neighbouring columns (4 where all rows lie on pieces of that size) and asks for the further term before the experts' rows.  1,999 tokens of 2
+// of 16 experts, 2,048 columns, a shared expert beside them: about 10 us; 21 us with one column a thread.
+template <typename T, int V>
+__global__ void __launch_bounds__(256) expert_combine_kernel(const T* __restrict__ y, const int* __restrict__ pair_row, float* __restrict__ out, int top, int width,
                                       float pair_weight, const float* __restrict__ pair_weights, const float* __restrict__ base,
                                       int base_splits, size_t base_stride, const float* __restrict__ row_scale) {
     pdl_launch_dependents();
     pdl_wait();
     const int t = blockIdx.x;
-    for (int c = blockIdx.y * blockDim.x + threadIdx.x; c < width; c += gridDim.y * blockDim.x) {
-        float acc = 0.f;
-        for (int k = 0; k < top; ++k)
-            acc += to_float(y[(size_t)pair_row[t * top + k] * width + c]) * (pair_weights ? pair_weights[(size_t)t * top + k] : 1.f);
-        if (!pair_weights) acc *= pair_weight;
+    for (int c = (blockIdx.y * 256 + threadIdx.x) * V; c < width; c += gridDim.y * 256 * V) {
         const size_t at = (size_t)t * width + c;
-        if (base) acc += (row_scale ? row_scale[t] : 1.f) * load_sum(base, at, base_splits, base_stride);
-        out[at] = acc;
+        float acc[V], more[V];
+#pragma unroll
+        for (int i = 0; i < V; ++i) acc[i] = more[i] = 0.f;
+        if (base) {
+            for (int s = 0; s < base_splits; ++s) {
+                if constexpr (V == 4) {
+                    const float4 b = *reinterpret_cast<const float4*>(base + at + (size_t)s * base_stride);
+                    more[0] += b.x; more[1] += b.y; more[2] += b.z; more[3] += b.w;
+                } else more[0] += base[at + (size_t)s * base_stride];
+            }
+        }
+        for (int k = 0; k < top; ++k) {
+            const T* row = y + (size_t)pair_row[t * top + k] * width + c;
+            const float weight = pair_weights ? pair_weights[(size_t)t * top + k] : 1.f;
+            if constexpr (V == 1) acc[0] += to_float(row[0]) * weight;
+            else if constexpr (sizeof(T) == 4) {
+                const float4 r = *reinterpret_cast<const float4*>(row);
+                acc[0] += r.x * weight; acc[1] += r.y * weight; acc[2] += r.z * weight; acc[3] += r.w * weight;
+            } else {
+                const uint2 raw = *reinterpret_cast<const uint2*>(row);
+                const __nv_bfloat162 lo = *reinterpret_cast<const __nv_bfloat162*>(&raw.x), hi = *reinterpret_cast<const __nv_bfloat162*>(&raw.y);
+                acc[0] += __low2float(lo) * weight; acc[1] += __high2float(lo) * weight; acc[2] += __low2float(hi) * weight; acc[3] += __high2float(hi) * weight;
+            }
+        }
+        const float scale = base && row_scale ? row_scale[t] : 1.f;
+#pragma unroll
+        for (int i = 0; i < V; ++i) {
+            if (!pair_weights) acc[i] *= pair_weight;
+            if (base) acc[i] += scale * more[i];
+        }
+        if constexpr (V == 4) *reinterpret_cast<float4*>(out + at) = make_float4(acc[0], acc[1], acc[2], acc[3]);
+        else out[at] = acc[0];
     }
 }
 
@@ -510,10 +538,14 @@ extern "C" int qt_experts_combine(const void* y, int dtype, const int* pair_row,
     if (n_tokens == 0) return QT_OK;
     cudaStream_t s = (cudaStream_t)stream;
     return QT_DISPATCH_DTYPE(dtype, "experts_combine", {
+        const bool fours = width % 4 == 0 && base_stride % 4 == 0 && (((uintptr_t)y | (uintptr_t)out | (uintptr_t)base) & 15) == 0;
         // few tokens: the columns of a row over several blocks, so that the launch fills the machine
-        const unsigned column_blocks = n_tokens >= 1024 ? 1u : (unsigned)((width + 255) / 256);
-        launch_kernel(expert_combine_kernel<T>, dim3(n_tokens, column_blocks), dim3(256), 0, s, (const T*)y, pair_row, out, top, width, pair_weight, pair_weights, base,
-                      base_splits, (size_t)base_stride, row_scale);
+        const int per_block = fours ? 1024 : 256;
+        const dim3 grid(n_tokens, n_tokens >= 1024 ? 1u : (unsigned)((width + per_block - 1) / per_block));
+        if (fours) launch_kernel(expert_combine_kernel<T, 4>, grid, dim3(256), 0, s, (const T*)y, pair_row, out, top, width, pair_weight, pair_weights, base,
+                                 base_splits, (size_t)base_stride, row_scale);
+        else launch_kernel(expert_combine_kernel<T, 1>, grid, dim3(256), 0, s, (const T*)y, pair_row, out, top, width, pair_weight, pair_weights, base,
+                           base_splits, (size_t)base_stride, row_scale);
         QT_CHECK_LAUNCH("expert_combine");
         return QT_OK;
     });

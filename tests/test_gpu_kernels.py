@@ -904,3 +904,23 @@ def test_experts_in_tiles_of_few_and_many_rows(gated, tokens, top, experts, widt
             h = upd[table[t, j]] @ xd[t]
             want[t] += float(pairs[t, j]) * (downd[table[t, j]] @ (h[:ff] * torch.sigmoid(h[:ff]) * (h[ff:] if gated else 1.0)))
     assert float((out.cpu().double() - want).norm() / want.norm()) < 4 * 2.0 ** -8
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("tokens, top, width", [(1, 1, 4), (5, 3, 1028), (1030, 2, 72), (3, 2, 37), (1024, 1, 1030)])
+@pytest.mark.parametrize("base, weights", [(0, True), (1, False), (3, True)])
+def test_expert_rows_combined(dtype, tokens, top, width, base, weights):
+    """Four columns a thread and one, rows over several blocks and one; sums of a few products in 32 bits."""
+    rows = tokens * top + 7
+    y = rand(rows, width, seed=1, dtype=dtype)
+    pair_row = torch.randperm(rows, generator=gen(2))[:tokens * top].int().to(DEV)
+    pairs, further, scale = rand(tokens, top, seed=3), rand(3, tokens, width, seed=4)[:max(base, 1)], rand(tokens, seed=5)
+    out = torch.full((tokens, width), float("nan"), device=DEV)
+    kernels._call("experts", "qt_experts_combine", kernels._ptr(y), kernels._code(y, "y"), kernels._ptr(pair_row), kernels._ptr(out), tokens, top, width, 0.25,
+                  kernels._ptr(pairs) if weights else None, kernels._ptr(further) if base else None, max(base, 1), further.stride(0) if base > 1 else 0,
+                  kernels._ptr(scale) if base == 3 else None, kernels._stream())
+    each = y.double()[pair_row.long()].view(tokens, top, width)
+    want = (each * pairs.double()[:, :, None]).sum(1) if weights else 0.25 * each.sum(1)
+    if base:
+        want = want + further.double().sum(0) * (scale.double()[:, None] if base == 3 else 1.0)
+    assert float((out.double() - want).abs().max()) < 2e-6 * max(1.0, float(want.abs().max()))
