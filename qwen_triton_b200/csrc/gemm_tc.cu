@@ -315,10 +315,11 @@ template <> __device__ __forceinline__ void store8<float>(float* dst, const floa
     reinterpret_cast<float4*>(dst)[1] = make_float4(f[4], f[5], f[6], f[7]);
 }
 template <> __device__ __forceinline__ void store8<__half>(__half* dst, const float (&f)[8]) {
-    __half h[8];
+    __half2 h[4];
 #pragma unroll
-    for (int i = 0; i < 8; ++i) h[i] = from_float<__half>(f[i]);
-    *reinterpret_cast<uint4*>(dst) = *reinterpret_cast<const uint4*>(h);
+    for (int i = 0; i < 4; ++i) h[i] = __halves2half2(from_float<__half>(f[2 * i]), from_float<__half>(f[2 * i + 1]));
+    *reinterpret_cast<uint4*>(dst) = make_uint4(reinterpret_cast<const uint32_t&>(h[0]), reinterpret_cast<const uint32_t&>(h[1]),
+                                                reinterpret_cast<const uint32_t&>(h[2]), reinterpret_cast<const uint32_t&>(h[3]));
 }
 template <> __device__ __forceinline__ void store8<__nv_bfloat16>(__nv_bfloat16* dst, const float (&f)[8]) {
     uint4 packed;
