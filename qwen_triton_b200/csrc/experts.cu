@@ -248,10 +248,8 @@ __global__ void __launch_bounds__(EV_WARPS * 32) expert_down_vec_kernel(const Ex
         lane_dots<T, FEATS>(row, (const T*)p.mid + ((size_t)t * p.top + k) * p.ff, 1.f, p.ff, lane, acc);
         const float weight = p.pair_weights ? p.pair_weights[(size_t)t * p.top + k] : 1.f;
 #pragma unroll
-        for (int j = 0; j < FEATS; ++j) total[j] += acc[j] * weight;
+        for (int j = 0; j < FEATS; ++j) total[j] += warp_sum(acc[j]) * weight;      // the weight on the finished sum, one rounding a pair
     }
-#pragma unroll
-    for (int j = 0; j < FEATS; ++j) total[j] = warp_sum(total[j]);
 #pragma unroll
     for (int j = 0; j < FEATS; ++j)
         if (lane == j && c0 + j < p.width) expert_put(p, t, c0 + j, total[j]);

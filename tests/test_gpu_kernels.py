@@ -331,6 +331,19 @@ def test_experts_by_pair(dtype, gated, tokens, top, experts, width, ff):
 
 
 @pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("tokens, width, ff", [(1, 64, 1000), (3, 520, 264), (20, 2056, 40), (5, 37, 44)])
+def test_experts_by_pair_weigh_finished_sums(dtype, tokens, width, ff):
+    """A pair's weight meets the finished sum, so a token of one expert is its weight times its result without one, bit for bit."""
+    x, up = rand(tokens, width, seed=1, dtype=dtype), rand(3, ff, width, seed=2, scale=width ** -0.5, dtype=dtype)
+    down, weights = rand(3, width, ff, seed=3, scale=ff ** -0.5, dtype=dtype), rand(tokens, 1, seed=4)
+    table, mid = (torch.arange(tokens) % 3).int()[:, None].contiguous().to(DEV), torch.empty(tokens, ff, dtype=dtype, device=DEV)
+    plain, weighed = torch.empty(tokens, width, device=DEV), torch.empty(tokens, width, device=DEV)
+    kernels.experts_by_pair(x, None, table, up, down, mid, plain, "silu", pair_weights=torch.ones_like(weights))
+    kernels.experts_by_pair(x, None, table, up, down, mid, weighed, "silu", pair_weights=weights)
+    assert torch.equal(weighed, plain * weights)
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("nq, nkv, d, window, ring, splits", [
     (6, 2, 80, None, 0, 1), (6, 2, 80, None, 0, 5), (4, 4, 16, 40, 128, 2), (16, 1, 128, None, 0, 3),
     (32, 8, 128, None, 0, 4), (5, 5, 112, 300, 0, 7), (10, 2, 48, None, 0, 64), (40, 2, 64, None, 0, 2), (8, 2, 96, 130, 256, 3)])
