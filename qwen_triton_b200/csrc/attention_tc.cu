@@ -40,7 +40,7 @@
 // used.  `sinks` (or `sink` alone: 0): the softmax's denominator has one more term, exp of the head's number, which is neither
 // scaled nor capped and has no value; it joins a row's sum once, at the end.
 //
-// DENSE (qt_attention_prefill_rows): prompts whose heads have keys and values of their own, formed for the step, in halves; keys of 128 or 192
+// DENSE (qt_attention_prefill_rows): prompts whose heads have keys and values of their own, formed for the step; keys of 128 or 192
 // elements, values of 64 or 128, a gate on the result ahead of its rounding.  Bound like the cached form by the softmax beside the MMAs: 2,048
 // tokens of 16 heads of 192 and 128 in 43 us (62 us with the gate's sums), 505 TFLOP/s; the same attention over cached rows of 576
 // and 512 elements (attention_latent.cu) 363 us.
@@ -50,7 +50,6 @@
 #include "tc_common.cuh"
 #include "score_cap.cuh"
 
-#include <cuda_fp16.h>
 #include <math.h>
 
 using namespace qt;
@@ -85,6 +84,8 @@ struct TcAttnParams {
     float softcap;                 // of the score cap (CAP)
     int keep_first;                // KEEP: keys at positions below this stay visible under the window
     int v_col;                     // DENSE: first value column of a row (key columns are in front: head * HD)
+    const float4* run_scale;       // DENSE: of a run of 64 rows, .y: its keys are meant times this, .z and .w: its values are meant over .z = 2^-.w
+    const float* q_scale;          // [T, nq]: queries are meant times this
     // DENSE: the result times sigmoid(gate[t, gate_offset + head * dv + c]), or with gate_per_head of column gate_offset + head; or null
     const float* gate; int gate_splits; size_t gate_split_stride; int gate_cols, gate_offset, gate_per_head;
 };
@@ -112,6 +113,8 @@ __device__ __forceinline__ float fast_exp2(float x) {
     asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
     return y;
 }
+// 2^e for a whole number e between -126 and 127
+__device__ __forceinline__ float exp2_of(float e) { return __uint_as_float((uint32_t)(127 + (int)e) << 23); }
 // Three-input maximum and two-wide float arithmetic (sm_100): half the instructions of the softmax's maximum, scaling
 // and row sum; every lane rounds as the one-wide form does.
 __device__ __forceinline__ float max3(float a, float b, float c) {
@@ -142,13 +145,12 @@ __device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
     asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
     return d;
 }
-__device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
-    __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
-    return *reinterpret_cast<uint32_t*>(&v);
-}
-
 __device__ __forceinline__ uint32_t pack_half(float lo, float hi) {
     __half2 v = __floats2half2_rn(lo, hi);
+    return *reinterpret_cast<uint32_t*>(&v);
+}
+__device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
+    __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
     return *reinterpret_cast<uint32_t*>(&v);
 }
 
@@ -174,7 +176,9 @@ __device__ __forceinline__ int cache_page(const int* table, int max_blocks, int 
 // an SM and one's softmax runs under the other's MMAs.
 // HD: elements of queries and keys, HDV of values.  DENSE: keys and values are not in a cache but columns of one matrix with a row per
 // token of this step (kv_row, below), and no token comes from before; queries, keys, values and P are then halves (11 bits of a number in
-// the place of bfloat16's 8: keys and values are rounded once more than the rows they are made from; P is at most 2^8).
+// the place of bfloat16's 8: keys and values are rounded once more than the rows they are made from), with powers of two per query and per
+// run of 64 keys that keep them within a half's range.  Those of queries and keys go into the factor on the scores; a weight is that of the
+// score plus the logarithm of its values' factor (relative to the first tile's), and the row's sum takes it back out.  P is at most 2^15: the row's maximum is taken 7 lower.
 // KEEP: a windowed query also sees the keys at positions below keep_first: their tiles come first, then the window's.
 template <int HD, int HDV, int BKEY, int PEN, int CAP, bool DENSE, bool KEEP>
 __global__ void __launch_bounds__(THREADS, BKEY == 64 ? 2 : 1) attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q,
@@ -350,9 +354,14 @@ __global__ void __launch_bounds__(THREADS, BKEY == 64 ? 2 : 1) attention_prefill
         const ScoreCap cap = CAP != CAP_NONE ? ScoreCap::make<CAP>(p.softcap, p.scale) : ScoreCap{};
         float m_run = -INFINITY, l_run = 0.f;              // the maximum this row scales by (scaled base-2 domain) and its sum
         pdl_wait();                                        // the output may still be read by an earlier kernel
+        const float first_run = DENSE ? p.run_scale[kv_row / PAGE + tile_begin].w : 0.f;
+        const float row_scale2 = DENSE && r < rows ? scale2 * p.q_scale[(size_t)(q_begin + q0 + r) * p.nq + head] : scale2;
         bool ok = true;
         for (int j = 0; j < n_tiles && ok; ++j) {
             const int s = j & 1;
+            float4 run = DENSE ? p.run_scale[kv_row / PAGE + tile_at(j)] : make_float4(1.f, 1.f, 1.f, 0.f);
+            if (DENSE) { run.z *= exp2_of(first_run); run.w -= first_run; }        // relative to the first tile's, which the result gets back
+            const float tile_scale2 = DENSE ? row_scale2 * run.y : scale2;
             if (!mbar_wait(s_full + 8 * s, (uint32_t)(j >> 1) & 1u, status, 3)) { ok = false; break; }
             tc_fence_after();
             const uint32_t s_addr = lane_addr + (s ? S_COL1 : S_COL0);
@@ -409,7 +418,7 @@ __global__ void __launch_bounds__(THREADS, BKEY == 64 ? 2 : 1) attention_prefill
             for (int q = 0; q < QUARTERS; ++q)
 #pragma unroll
                 for (int c = 0; c < 32; c += 2) mx[(c >> 1) & 3] = max3(mx[(c >> 1) & 3], __uint_as_float(v[q][c]), __uint_as_float(v[q][c + 1]));
-            const float m_tile = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3])) * scale2;
+            const float m_tile = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3])) * tile_scale2 + (DENSE ? run.w : 0.f);
             // the row's maximum moves only when the true one has run away from it
             const bool moves = m_tile > m_run + RESCALE_STEP;
             const float m_new = moves ? m_tile : m_run;
@@ -436,7 +445,8 @@ __global__ void __launch_bounds__(THREADS, BKEY == 64 ? 2 : 1) attention_prefill
             // P = 2^(s * scale2 - m) as bfloat16, two keys to a 32-bit column, over this row's scores in tensor memory
             // (they are in registers); the row sum
             uint64_t sum2[2] = {0ull, 0ull};               // two pairs of partial sums
-            const uint64_t scale22 = pair_f32(scale2, scale2), neg_m2 = pair_f32(-m_use, -m_use);
+            const float below = DENSE ? run.w + 7.f - m_use : -m_use;
+            const uint64_t scale22 = pair_f32(tile_scale2, tile_scale2), neg_m2 = pair_f32(below, below);
 #pragma unroll
             for (int h = 0; h < QUARTERS / 2; ++h) {       // 64 keys = 32 columns per store
                 uint32_t packed[32];
@@ -460,7 +470,8 @@ __global__ void __launch_bounds__(THREADS, BKEY == 64 ? 2 : 1) attention_prefill
             float sum[4];
             unpair_f32(sum2[0], sum[0], sum[2]);
             unpair_f32(sum2[1], sum[1], sum[3]);
-            l_run = l_run * alpha + (sum[0] + sum[1]) + (sum[2] + sum[3]);
+            if (DENSE) l_run = fmaf((sum[0] + sum[1]) + (sum[2] + sum[3]), run.z, l_run * alpha);
+            else l_run = l_run * alpha + (sum[0] + sum[1]) + (sum[2] + sum[3]);
             m_run = m_new;
         }
         if (ok && mbar_wait(pv_full + 8 * ((n_tiles - 1) & 1), (uint32_t)((n_tiles - 1) >> 1) & 1u, status, 3)) {
@@ -471,7 +482,7 @@ __global__ void __launch_bounds__(THREADS, BKEY == 64 ? 2 : 1) attention_prefill
                 factor = fast_exp2(m_run - top);
                 l_run = l_run * factor + fast_exp2(s2 - top);
             }
-            const float inv = factor / l_run;
+            const float inv = factor / l_run * (DENSE ? exp2_of(first_run) : 1.f);
             __nv_bfloat16* dst = p.out + ((size_t)(q_begin + q0 + r) * p.nq + head) * HDV;
 #pragma unroll 1
             for (int c0 = 0; c0 < HDV; c0 += 32) {
@@ -579,7 +590,7 @@ extern "C" int qt_attention_prefill_tc(const void* q, const void* k_cache, const
     rc = tensor_map(&map_v, v_cache, (uint64_t)n_pages * nv * PAGE, (uint64_t)d, PAGE);
     if (rc) return rc;
     TcAttnParams p{(__nv_bfloat16*)out, block_table, max_blocks, seq_start, seq_past, nq, nkv, ring_tokens, window, chunk, nv, scale, status, r1, r2,
-                   sink, sinks, softcap, keep_first, 0, nullptr, 1, 0, 0, 0, 0};
+                   sink, sinks, softcap, keep_first, 0, nullptr, nullptr, nullptr, 1, 0, 0, 0, 0};
     cudaStream_t s = (cudaStream_t)stream;
     // key tiles of one page, two blocks per SM: measured 12-22 % faster than tiles of two pages with one block per SM
 #define QT_LAUNCH_TC(PEN, CAP)                                                                      \
@@ -600,11 +611,12 @@ extern "C" int qt_attention_prefill_tc(const void* q, const void* k_cache, const
 #undef QT_LAUNCH_TC
 }
 
-// Causal attention of packed sequences that start at position 0, every head with keys and values of its own: q [n_tokens, heads, dk], kv
-// [kv_rows, heads * dk + heads * dv] (a row's keys by head, then its values by head) in halves, out [n_tokens, heads, dv] bfloat16.  The tokens of
-// sequence i are the rows from 64 (seq_start[i] / 64 + i) on; its last run of 64 rows is filled up with finite numbers.  gate [gate_splits, n_tokens,
+// Causal attention of packed sequences that start at position 0, every head with keys and values of its own: q [n_tokens, heads, dk] halves, kv
+// [kv_rows, heads * dk + heads * dv] (a row's keys by head, then its values by head) in halves, out [n_tokens, heads, dv] bfloat16.  The tokens of sequence i
+// are the rows from 64 (seq_start[i] / 64 + i) on; its last run of 64 rows is filled up with finite numbers.  Queries are meant times q_scale
+// [n_tokens, heads], the keys and values of a run of 64 rows by run_scale[run][4] as qt_latent_rows leaves it.  gate [gate_splits, n_tokens,
 // gate_cols] float or null: the result is multiplied by the sigmoid of the sums of the columns from gate_offset on (one a head or one an element).
-extern "C" int qt_attention_prefill_rows(const void* q, const void* kv, void* out, int n_tokens, int kv_rows, const int* seq_start, int n_seqs, int max_q_len,
+extern "C" int qt_attention_prefill_rows(const void* q, const float* q_scale, const void* kv, const float* run_scale, void* out, int n_tokens, int kv_rows, const int* seq_start, int n_seqs, int max_q_len,
                                          int heads, int dk, int dv, int window, float scale, const float* gate, int gate_splits, long long gate_split_stride,
                                          int gate_cols, int gate_offset, int gate_per_head, int* status, void* stream) {
     if (n_seqs == 0 || max_q_len == 0) return QT_OK;
@@ -613,6 +625,7 @@ extern "C" int qt_attention_prefill_rows(const void* q, const void* kv, void* ou
     QT_REQUIRE(n_seqs <= 65535 && (max_q_len + BQ - 1) / BQ <= 65535 && kv_rows >= (n_tokens / PAGE + n_seqs) * PAGE, "attention_prefill_rows: %d rows for %d tokens of %d sequences",
                kv_rows, n_tokens, n_seqs);
     QT_REQUIRE(status != nullptr && window >= 0 && scale > 0.f, "attention_prefill_rows: a status word and a positive scale are required");
+    QT_REQUIRE(q_scale && run_scale && ((uintptr_t)run_scale & 15) == 0, "attention_prefill_rows: the scales of queries and keys are required");
     QT_REQUIRE((((uintptr_t)q | (uintptr_t)kv | (uintptr_t)out) & 15) == 0, "attention_prefill_rows: operands must be 16-byte aligned");
     QT_REQUIRE(!gate || (gate_splits >= 1 && gate_offset >= 0 && gate_offset + heads * (gate_per_head ? 1 : dv) <= gate_cols &&
                          (gate_per_head || (((uintptr_t)gate & 15) == 0 && gate_offset % 4 == 0 && gate_cols % 4 == 0 && gate_split_stride % 4 == 0))),
@@ -622,7 +635,8 @@ extern "C" int qt_attention_prefill_rows(const void* q, const void* kv, void* ou
     if (rc) return rc;
     rc = tensor_map(&map_kv, kv, (uint64_t)kv_rows, (uint64_t)heads * (dk + dv), PAGE);
     if (rc) return rc;
-    TcAttnParams p{(__nv_bfloat16*)out, nullptr, 0, seq_start, nullptr, heads, heads, 0, window, 0, heads, scale, status, nullptr, nullptr, 0, nullptr, 0.f, 0, heads * dk, gate,
+    TcAttnParams p{(__nv_bfloat16*)out, nullptr, 0, seq_start, nullptr, heads, heads, 0, window, 0, heads, scale, status, nullptr, nullptr, 0, nullptr, 0.f, 0, heads * dk,
+                   (const float4*)run_scale, q_scale, gate,
                    gate_splits, (size_t)gate_split_stride, gate_cols, gate_offset, gate_per_head};
     cudaStream_t s = (cudaStream_t)stream;
     if (dk == 128 && dv == 64) return launch<128, 64, 64, PEN_NONE, CAP_NONE, true>(map_q, map_kv, map_kv, p, n_seqs, max_q_len, s);

@@ -23,7 +23,6 @@
 // element types of activations, weights and caches
 #define QT_F32 0
 #define QT_BF16 1
-#define QT_F16 2      // only where a kernel says so
 
 namespace qt {
 
@@ -55,6 +54,8 @@ static thread_local char g_error[512] = "";
 // anything a predecessor wrote (or writes anything a predecessor may still read), waits for the
 // predecessors to finish.  Work that depends on nothing earlier (set-up, weight prefetch) runs ahead of
 // that wait.  QT_B200_PDL=0 in the environment turns the launch attribute off; the wait is then a no-op.
+// What a predecessor wrote is read by ordinary loads: `__ldg`, and a `const T* __restrict__` parameter of a kernel, tell the compiler that
+// nobody writes there while the kernel runs, and it then moves such a read ahead of the wait where its address is known.
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 

@@ -42,7 +42,7 @@ __device__ __forceinline__ void tile_coords(int t, int w_tiles, int x_tiles, int
 }
 
 // What an epilogue does with the sums: store them; gate them (below); store an activation of them (bfloat16, one K range).
-constexpr int PLAIN = 0, GATED = 1, ACTIVATED = 2;
+constexpr int PLAIN = 0, GATED = 1, ACTIVATED = 2, KEYS_VALUES = 3;      // KEYS_VALUES: the pair kernel's alone (qt_gemm_tc_keys_values)
 
 // GATED: the weight's rows alternate 16 of a gate projection and 16 of an up projection; the 32 accumulator lanes of
 // an epilogue warp are then the gate rows (lanes 0..15) and the up rows (16..31) of the same 16 features, and the
@@ -337,7 +337,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_tc_pair_kernel(const __grid_c
                                                                   int M, int N, int kb_total, int kb_per_split, int splits,
                                                                   size_t split_stride, int act, float limit, int vector_stores, int tail_tiles,
                                                                   float* __restrict__ tail_scratch, int* tail_flags, const float* __restrict__ bias,
-                                                                  int* status) {
+                                                                  const float4* run_scale, int key_cols, int* status) {
     // instruction descriptor: float accumulator, bfloat16 A and B, both K-major, N = 256 weight rows, M = 256 tokens over the pair
     constexpr uint32_t IDESC = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(PAIR_W >> 3) << 17) | ((uint32_t)(PAIR_X >> 4) << 24);
     constexpr int S = PAIR_STAGES;
@@ -568,6 +568,16 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_tc_pair_kernel(const __grid_c
                                 if (f0 + 8 * h + j < features) dst[8 * h + j] = from_float<TO>(f[j]);
                         }
                     }
+                } else if (MODE == KEYS_VALUES) {          // pieces of 32 columns are all keys or all values
+                    const float4 scale = run_scale[m >> 6];
+                    const float factor = n0 + c < key_cols ? scale.x : scale.z;
+#pragma unroll
+                    for (int h = 0; h < 4; ++h) {
+                        float f[8];
+#pragma unroll
+                        for (int j = 0; j < 8; ++j) f[j] = __uint_as_float(v[8 * h + j]) * factor;
+                        store8<TO>(row + c + 8 * h, f);
+                    }
                 } else {
 #pragma unroll
                     for (int h = 0; h < 4; ++h) {
@@ -637,7 +647,7 @@ int pick_tail_tiles(long long n_tiles, int pairs, int kb_total, int tail, int ta
 template <typename TO, int MODE>
 int launch_pair(const CUtensorMap& map_w, const CUtensorMap& map_x, TO* out, int M, int N, int kb_total, int splits,
                 size_t split_stride, int act, float limit, int tail, float* tail_scratch, int* tail_flags, int tail_pairs, const float* bias, int* status,
-                cudaStream_t stream) {
+                cudaStream_t stream, const float4* run_scale = nullptr, int key_cols = 0) {
     const size_t smem = (size_t)PAIR_STAGES * PAIR_STAGE_BYTES + 1024 + (2 * PAIR_STAGES + 5) * 8 + 16;
     static int resident_pairs = 0;                           // pairs the device runs at once (one per TPC that can host a cluster)
     if (resident_pairs == 0) {
@@ -669,7 +679,7 @@ int launch_pair(const CUtensorMap& map_w, const CUtensorMap& map_x, TO* out, int
     const int per16 = 16 / (int)sizeof(TO), row_elems = MODE == GATED ? N / 2 : N;
     const int vector_stores = ((uintptr_t)out % 16 == 0 && row_elems % per16 == 0 && split_stride % per16 == 0) ? 1 : 0;
     launch_kernel_cluster(gemm_tc_pair_kernel<TO, MODE>, dim3(2 * pairs), dim3(THREADS), smem, stream, 2, map_w, map_x, out, M, N, kb_total,
-                          kb_per_split, splits, split_stride, act, limit, vector_stores, tail_tiles, tail_scratch, tail_flags, bias, status);
+                          kb_per_split, splits, split_stride, act, limit, vector_stores, tail_tiles, tail_scratch, tail_flags, bias, run_scale, key_cols, status);
     QT_CHECK_LAUNCH("gemm_tc_pair");
     return QT_OK;
 }
@@ -765,7 +775,7 @@ extern "C" int qt_gemm_tc(const void* x, const void* w, void* out, int out_dtype
     QT_FAIL(QT_ERR_ARG, "gemm_tc: unknown output type %d", out_dtype);
 }
 
-// The same product by pairs of blocks (see gemm_tc_pair_kernel): bfloat16 or float output (without `swiglu` and splits also halves), meant for many tokens (a
+// The same product by pairs of blocks (see gemm_tc_pair_kernel): bfloat16 or float output, meant for many tokens (a
 // pair covers 256 weight rows x 256 tokens); out[splits, M, N] in float when `splits` > 1, under the rule above.  With `swiglu` the weight's rows alternate 16 of a gate and
 // 16 of an up projection and `out` is [M, N / 2] = act(gate) * up (`act`: one of QT_ACT_*); `swiglu` 2: `out` [M, N] = act(product).  Codes in `status`: as above, 4 = the MMA issuer
 // waiting for the epilogues to free an accumulator.
@@ -798,10 +808,27 @@ extern "C" int qt_gemm_tc_pair(const void* x, const void* w, void* out, int out_
     if (out_dtype == QT_BF16 && swiglu == ACTIVATED)
         return launch_pair<__nv_bfloat16, ACTIVATED>(map_w, map_x, (__nv_bfloat16*)out, M, N, kb_total, 1, 0, act, 0.f, tail, tail_scratch, tail_flags, tail_pairs, bias, status, s);
     if (out_dtype == QT_BF16 && swiglu) return launch_pair<__nv_bfloat16, GATED>(map_w, map_x, (__nv_bfloat16*)out, M, N, kb_total, 1, 0, act, limit, tail, tail_scratch, tail_flags, tail_pairs, bias, status, s);
-    if (out_dtype == QT_F16 && !swiglu) return launch_pair<__half, PLAIN>(map_w, map_x, (__half*)out, M, N, kb_total, 1, 0, 0, 0.f, tail, tail_scratch, tail_flags, tail_pairs, bias, status, s);
     if (out_dtype == QT_BF16) return launch_pair<__nv_bfloat16, PLAIN>(map_w, map_x, (__nv_bfloat16*)out, M, N, kb_total, 1, 0, 0, 0.f, tail, tail_scratch, tail_flags, tail_pairs, bias, status, s);
     if (out_dtype == QT_F32 && !swiglu) return launch_pair<float, PLAIN>(map_w, map_x, (float*)out, M, N, kb_total, splits, (size_t)split_stride, 0, 0.f, tail, tail_scratch, tail_flags, tail_pairs, bias, status, s);
     QT_FAIL(QT_ERR_ARG, "gemm_tc_pair: output type %d%s is not offered", out_dtype, swiglu ? " with the SiLU-gated epilogue" : "");
+}
+
+// The same product into halves: out [M, N], the first `key_cols` columns (keys) multiplied by run_scale[m / 64].x, the others (values) by .z, powers of
+// two, before they are rounded.
+extern "C" int qt_gemm_tc_keys_values(const void* x, const void* w, void* out, int M, int N, int K, int key_cols, const float* run_scale, int* status,
+                                      void* stream) {
+    QT_REQUIRE(M > 0 && N > 0 && K > 0 && K % 8 == 0 && N % 32 == 0 && key_cols >= 0 && key_cols <= N && key_cols % 32 == 0,
+               "gemm_tc_keys_values: bad sizes M=%d N=%d (%d of keys) K=%d", M, N, key_cols, K);
+    QT_REQUIRE((((uintptr_t)x | (uintptr_t)w | (uintptr_t)out) & 15) == 0 && run_scale && ((uintptr_t)run_scale & 15) == 0 && status,
+               "gemm_tc_keys_values: operands must be 16-byte aligned, with scales and a status word");
+    QT_REQUIRE((long long)((M + PAIR_X - 1) / PAIR_X) * ((N + 2 * BW - 1) / (2 * BW)) < (1ll << 30), "gemm_tc_keys_values: M=%d x N=%d is too large for one launch", M, N);
+    CUtensorMap map_w, map_x;
+    int rc = tensor_map(&map_w, w, (uint64_t)N, (uint64_t)K, BW);
+    if (rc) return rc;
+    rc = tensor_map(&map_x, x, (uint64_t)M, (uint64_t)K, (uint32_t)PAIR_HALF);
+    if (rc) return rc;
+    return launch_pair<__half, KEYS_VALUES>(map_w, map_x, (__half*)out, M, N, (K + BK - 1) / BK, 1, 0, 0, 0.f, 0, nullptr, nullptr, 0, nullptr, status,
+                                                   (cudaStream_t)stream, (const float4*)run_scale, key_cols);
 }
 
 QT_DEFINE_LAST_ERROR(gemm_tc)

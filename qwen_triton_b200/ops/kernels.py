@@ -96,8 +96,8 @@ _SIGNATURES = {
                               _c_ptr, _c_ptr, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_ptr],
         "qt_latent_query_rot": [_c_ptr, _c_int, _c_int, _c_ll, _c_ptr, _c_int, _c_ptr, _c_ptr, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int,
                                 _c_int, _c_int, _c_ptr],
-        "qt_latent_rows": [_c_ptr, _c_ptr, _c_ptr, _c_int, _c_ptr, _c_int, _c_int, _c_int, _c_int, _c_int, _c_ptr],
-        "qt_latent_queries": [_c_ptr, _c_int, _c_int, _c_ll, _c_int, _c_ptr, _c_int, _c_ptr, _c_ptr, _c_int, _c_int, _c_int, _c_int, _c_int, _c_ptr],
+        "qt_latent_rows": [_c_ptr, _c_ptr, _c_ptr, _c_ptr, _c_int, _c_ptr, _c_int, _c_int, _c_int, _c_int, _c_float, _c_float, _c_int, _c_int, _c_ptr],
+        "qt_latent_queries": [_c_ptr, _c_int, _c_int, _c_ll, _c_int, _c_ptr, _c_int, _c_ptr, _c_ptr, _c_ptr, _c_int, _c_int, _c_int, _c_int, _c_int, _c_ptr],
         "qt_head_product": [_c_ptr, _c_int, _c_int, _c_ll, _c_ll, _c_ll, _c_int, _c_ptr, _c_int, _c_ptr, _c_int, _c_ll, _c_ll, _c_int,
                             _c_ptr, _c_int, _c_ll, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_ptr],
     },
@@ -132,7 +132,7 @@ _SIGNATURES = {
     "attention_tc": {
         "qt_attention_prefill_tc": [_c_ptr, _c_ptr, _c_ptr, _c_ptr, _c_int, _c_int, _c_ptr, _c_int, _c_ptr, _c_ptr, _c_int,
                                     _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_float, _c_ptr, _c_ptr, _c_int, _c_int, _c_int, _c_int, _c_ptr, _c_float, _c_int, _c_ptr, _c_ptr],
-        "qt_attention_prefill_rows": [_c_ptr, _c_ptr, _c_ptr, _c_int, _c_int, _c_ptr, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_float, _c_ptr,
+        "qt_attention_prefill_rows": [_c_ptr, _c_ptr, _c_ptr, _c_ptr, _c_ptr, _c_int, _c_int, _c_ptr, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_float, _c_ptr,
                                       _c_int, _c_ll, _c_int, _c_int, _c_int, _c_ptr, _c_ptr],
     },
     "gemm_f32": {
@@ -143,6 +143,7 @@ _SIGNATURES = {
     },
     "gemm_tc": {
         "qt_gemm_tc": [_c_ptr, _c_ptr, _c_ptr, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_ll, _c_int, _c_int, _c_int, _c_float, _c_ptr, _c_ptr, _c_ptr],
+        "qt_gemm_tc_keys_values": [_c_ptr, _c_ptr, _c_ptr, _c_int, _c_int, _c_int, _c_int, _c_ptr, _c_ptr, _c_ptr],
         "qt_gemm_tc_pair": [_c_ptr, _c_ptr, _c_ptr, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_float, _c_int, _c_ll, _c_int, _c_ptr,
                             _c_ptr, _c_int, _c_ptr, _c_ptr, _c_ptr],
         "qt_gemm_tc_pair_slots": [],
@@ -227,9 +228,6 @@ def _need(tensor: torch.Tensor, name: str, dtype=None, shape=None) -> None:
         raise KernelError(f"{name} must be contiguous")
     if shape is not None and tuple(tensor.shape) != tuple(shape):
         raise KernelError(f"{name} must have shape {tuple(shape)}, got {tuple(tensor.shape)}")
-
-
-_HALF_CODE = 2       # float16, for the kernels that name it
 
 
 def _code(tensor: torch.Tensor, name: str) -> int:
@@ -685,51 +683,72 @@ def rows_of_runs(tokens: int, n_seqs: int) -> int:
     return 64 * (tokens // 64 + n_seqs)
 
 
-def latent_rows(cache: torch.Tensor, rows: torch.Tensor, block_table: torch.Tensor, seq_start: torch.Tensor, n_seqs: int, max_tokens: int, page_tokens: int,
-                ring_tokens: int) -> None:
+def latent_rows(cache: torch.Tensor, rows: torch.Tensor, run_scale: torch.Tensor, rank: int, key_norm: float, value_norm: float, block_table: torch.Tensor, seq_start: torch.Tensor,
+                n_seqs: int, max_tokens: int, page_tokens: int, ring_tokens: int) -> None:
     """rows [rows_of_runs(T, sequences), row] = the cached latent rows [pages, 1, 64, row] of a step's sequences, all of which start at
-    position 0, in runs of 64 whose ends are zeros."""
+    position 0, in runs of 64 whose ends are zeros.  run_scale [runs, 4] (float) = per run the power of two that its keys are multiplied by as
+    halves, the inverse, that of its values, and the inverse's logarithm: a key's elements are bounded by the largest latent (the first ``rank``
+    elements) times ``key_norm`` and by the largest element behind them, a value's by the largest latent times ``value_norm``."""
     _need(cache, "cache", torch.bfloat16)
     _need(rows, "rows", torch.bfloat16, (rows.shape[0], cache.shape[3]))
+    _need(run_scale, "run_scale", torch.float32, (rows.shape[0] // 64, 4))
     _need(block_table, "block_table", torch.int32)
     _need(seq_start, "seq_start", torch.int32, (n_seqs + 1,))
     if block_table.shape[0] < n_seqs or cache.shape[1:3] != (1, 64):
         raise KernelError(f"latent_rows: cache {tuple(cache.shape)}, block table {tuple(block_table.shape)} for {n_seqs} sequences")
-    _call("latent", "qt_latent_rows", _ptr(cache), _ptr(rows), _ptr(block_table), block_table.shape[1], _ptr(seq_start), int(n_seqs), int(max_tokens),
-          cache.shape[3], int(page_tokens), int(ring_tokens), _stream())
+    _call("latent", "qt_latent_rows", _ptr(cache), _ptr(rows), _ptr(run_scale), _ptr(block_table), block_table.shape[1], _ptr(seq_start), int(n_seqs), int(max_tokens),
+          cache.shape[3], int(rank), float(key_norm), float(value_norm), int(page_tokens), int(ring_tokens), _stream())
 
 
-def latent_queries(q: GemmOut, cos_sin: torch.Tensor | None, token_pos: torch.Tensor, out: torch.Tensor, dim: int, rot: int) -> None:
+def keys_and_values(rows: torch.Tensor, weight: torch.Tensor, out: torch.Tensor, key_cols: int, run_scale: torch.Tensor) -> None:
+    """out [M, N] (halves) = rows [M, K] weight [N, K]^T, the first ``key_cols`` columns times run_scale[m // 64, 0], the others times
+    run_scale[m // 64, 2]."""
+    _need(rows, "rows", torch.bfloat16)
+    _need(weight, "weight", torch.bfloat16, (weight.shape[0], rows.shape[1]))
+    _need(out, "out", torch.float16, (rows.shape[0], weight.shape[0]))
+    _need(run_scale, "run_scale", torch.float32, (rows.shape[0] // 64, 4))
+    if rows.shape[0] % 64:
+        raise KernelError(f"keys_and_values: {rows.shape[0]} rows are not whole runs of 64")
+    _call("gemm_tc", "qt_gemm_tc_keys_values", _ptr(rows), _ptr(weight), _ptr(out), rows.shape[0], weight.shape[0], rows.shape[1], int(key_cols), _ptr(run_scale),
+          _ptr(_status_word(rows.device)), _stream())
+
+
+def latent_queries(q: GemmOut, cos_sin: torch.Tensor | None, token_pos: torch.Tensor, out: torch.Tensor, q_scale: torch.Tensor, dim: int, rot: int) -> None:
     """out [T, heads, row] (halves) = every head of ``q`` [*, T, heads (dim + rot)] (further columns behind are left alone): its ``dim``
-    elements, then its ``rot`` elements, the first ``cos_sin.shape[1]`` of them rotated by the token's position, then zeros."""
+    elements, then its ``rot`` elements, the first ``cos_sin.shape[1]`` of them rotated by the token's position, then zeros; all of them divided by
+    a power of two, q_scale [T, heads] (float)."""
     tokens, heads, row = out.shape
     _need(out, "out", torch.float16)
+    _need(q_scale, "q_scale", torch.float32, (tokens, heads))
     _need(token_pos, "token_pos", torch.int32, (tokens,))
     if q.rows != tokens or (q.tensor.dtype != torch.float32 and q.n_splits != 1):
         raise KernelError(f"latent_queries: q {tuple(q.tensor.shape)}, out {tuple(out.shape)}")
     if cos_sin is not None:
         _need(cos_sin, "cos_sin", torch.float32)
     _call("latent", "qt_latent_queries", _ptr(q.tensor), _code(q.tensor, "q"), q.n_splits, q.split_stride, q.cols, _ptr(cos_sin),
-          cos_sin.shape[1] if cos_sin is not None else 0, _ptr(token_pos), _ptr(out), tokens, heads, int(dim), int(rot), row, _stream())
+          cos_sin.shape[1] if cos_sin is not None else 0, _ptr(token_pos), _ptr(out), _ptr(q_scale), tokens, heads, int(dim), int(rot), row, _stream())
 
 
-def attention_prefill_rows(q: torch.Tensor, kv: torch.Tensor, out: torch.Tensor, seq_start: torch.Tensor, n_seqs: int, max_q_len: int, window: int | None,
-                           scale: float, gate: GemmOut | None = None, gate_offset: int = 0, gate_per_head: bool = False) -> None:
-    """Causal attention of packed sequences that start at position 0, on tcgen05: q [T, heads, 128 or 192] halves, out [T, heads, 64 or 128]
-    bfloat16, and kv (halves) [>= rows_of_runs(T, sequences), heads * (dk + dv)], a token's keys by head, then its values by head, in runs of 64 rows.  With ``gate`` (float sums [*, T, cols]) the
-    result is multiplied by sigmoid(gate[t, gate_offset + h * dv + n]), or with ``gate_per_head`` by sigmoid(gate[t, gate_offset + h]), before it is rounded."""
+def attention_prefill_rows(q: torch.Tensor, q_scale: torch.Tensor, kv: torch.Tensor, run_scale: torch.Tensor, out: torch.Tensor, seq_start: torch.Tensor, n_seqs: int,
+                           max_q_len: int, window: int | None, scale: float, gate: GemmOut | None = None, gate_offset: int = 0, gate_per_head: bool = False) -> None:
+    """Causal attention of packed sequences that start at position 0, on tcgen05: q [T, heads, 128 or 192] halves, meant times q_scale [T, heads];
+    kv [>= rows_of_runs(T, sequences), heads * (dk + dv)] halves, a token's keys by head, then its values by head, in runs of 64 rows with the
+    factors run_scale [runs, 4] (``latent_rows``); out [T, heads, 64 or 128] bfloat16.  With ``gate`` (float sums [*, T, cols]) the result is multiplied by
+    sigmoid(gate[t, gate_offset + h * dv + n]), or with ``gate_per_head`` by sigmoid(gate[t, gate_offset + h]), before it is rounded."""
     tokens, heads, dk = q.shape
     dv = out.shape[2]
     _need(q, "q", torch.float16)
+    _need(q_scale, "q_scale", torch.float32, (tokens, heads))
     _need(kv, "kv", torch.float16, (kv.shape[0], heads * (dk + dv)))
+    _need(run_scale, "run_scale", torch.float32, (kv.shape[0] // 64, 4))
     _need(out, "out", torch.bfloat16)
     _need(seq_start, "seq_start", torch.int32, (n_seqs + 1,))
     if gate is not None:
         _need(gate.tensor, "gate", torch.float32)
         if gate.rows != tokens:
             raise KernelError(f"attention_prefill_rows: a gate of {gate.rows} rows for {tokens} tokens")
-    _call("attention_tc", "qt_attention_prefill_rows", _ptr(q), _ptr(kv), _ptr(out), tokens, kv.shape[0], _ptr(seq_start), int(n_seqs), int(max_q_len), heads, dk, dv,
-          int(window or 0), float(scale), _ptr(gate.tensor) if gate is not None else None, gate.n_splits if gate is not None else 1,
+    _call("attention_tc", "qt_attention_prefill_rows", _ptr(q), _ptr(q_scale), _ptr(kv), _ptr(run_scale), _ptr(out), tokens, kv.shape[0], _ptr(seq_start), int(n_seqs),
+          int(max_q_len), heads, dk, dv, int(window or 0), float(scale), _ptr(gate.tensor) if gate is not None else None, gate.n_splits if gate is not None else 1,
           gate.split_stride if gate is not None else 0, gate.cols if gate is not None else 0, int(gate_offset), 1 if gate_per_head else 0,
           _ptr(_status_word(q.device)), _stream())
 
@@ -1667,12 +1686,11 @@ def gemm_tc_pair(a: torch.Tensor, w: torch.Tensor, out: GemmOut, swiglu: bool = 
         raise KernelError(f"gemm: a {tuple(a.shape)}, w {tuple(w.shape)}, out {tuple(out.tensor.shape)} do not fit")
     if rows == 0:
         return
-    halves = out.tensor.dtype == torch.float16 and not (swiglu or activate) and out.n_splits == 1
-    if not out.tensor.is_cuda or (out.tensor.dtype not in _CODES and not halves):
-        raise KernelError("gemm_tc_pair: the output must be a bfloat16 or float32 CUDA tensor (or, of the product alone, float16)")
+    if not out.tensor.is_cuda or out.tensor.dtype not in _CODES:
+        raise KernelError("gemm_tc_pair: the output must be a bfloat16 or float32 CUDA tensor")
     tail = pair_tail_mode() if tail is None else int(tail)
     slots, flags, pairs = _pair_tail(a.device) if tail != 0 and out.n_splits == 1 else (None, None, 0)
-    _call("gemm_tc", "qt_gemm_tc_pair", _ptr(a), _ptr(w), _ptr(out.tensor), _HALF_CODE if halves else _code(out.tensor, "out"), rows, w.shape[0], k,
+    _call("gemm_tc", "qt_gemm_tc_pair", _ptr(a), _ptr(w), _ptr(out.tensor), _code(out.tensor, "out"), rows, w.shape[0], k,
           1 if swiglu else 2 if activate else 0, activation_code(activation, swiglu) if swiglu or activate else 0, float(limit), out.n_splits, out.split_stride,
           tail, _ptr(slots) if slots is not None else None, _ptr(flags) if flags is not None else None, pairs,
           _ptr(_product_bias(bias, w)), _ptr(_status_word(a.device)), _stream())

@@ -23,7 +23,7 @@ query's and of the shared key part's matrices are put in that order, which chang
 
 Norms, rotation (float cos/sin table), scores, softmax and the gate are float; the query latent, the queries, the cache
 rows and the heads' outputs are rounded to the activation type between the products (in a prompt that forms keys and values per head, queries,
-keys and values to halves).
+keys and values to halves with a power of two per query and per 64 tokens, which keep more bits over the same range).
 
 Parameters: ``hidden_size``, ``num_heads``, ``head_dim``, ``rot_dim``, ``v_head_dim``, ``q_rank``, ``kv_rank``, ``scale``, ``eps``,
 ``position`` (a position part over ``rot_dim``; either pairing), ``window``, ``own_kv``, ``gate``, ``float_out``, and the tensor-name pieces ``dq``, ``uq``
@@ -100,9 +100,12 @@ class LatentAttention:
         self.most_runs = tokens // 64 + 64
         if self.expands:
             ws.declare("latent.rows", 64 * self.most_runs * self.row, runtime.dtype)
+            ws.declare("latent.run_scale", 4 * self.most_runs, torch.float32)
             ws.declare("latent.keys_values", 64 * self.most_runs * self.heads * (self.key + self.dv), torch.float16)
             ws.declare("latent.queries", tokens * self.heads * self.key, torch.float16)
+            ws.declare("latent.query_scale", tokens * self.heads, torch.float32)
         self.q_norm = self.kv_norm = self.uk_t = self.uv = self.expand = None
+        self.key_norm = self.value_norm = 0.0                  # the largest sum of magnitudes over a row of W_uk, of W_uv (and 1 %)
 
     # ------------------------------------------------------------------ weights
     @staticmethod
@@ -174,6 +177,7 @@ class LatentAttention:
             keys[:, self.d:self.d + self.rot, self.rank:] = torch.eye(self.rot, dtype=dtype, device=device)
             expand[self.heads * self.key:].view(self.heads, self.dv, self.row)[:, :, :self.rank] = self.uv
             self.expand = expand
+            self.key_norm, self.value_norm = (1.01 * float(w.float().abs().sum(dim=dim).max()) for w, dim in ((self.uk_t, 1), (self.uv, 2)))
         tables = self.runtime.options.setdefault("position_tables", {})
         key = self.position.key() + (self.runtime.max_positions,)
         if key not in tables:
@@ -213,18 +217,18 @@ class LatentAttention:
                 and tokens // 64 + ctx.n_seqs <= self.most_runs)
 
     def _over_own_keys(self, q_full, gate, gate_offset: int, ctx, cache, table):
-        """[T, heads, dv]: attention over every head's own keys and values, made from the cached rows.  They and the queries are halves:
-        in bfloat16 the one rounding that keys and values have more than latent rows puts the result 3 % further off."""
+        """[T, heads, dv]: attention over every head's own keys and values, made from the cached rows."""
         ws, tokens = self.runtime.workspace, q_full.rows
         count = kernels.rows_of_runs(tokens, ctx.n_seqs)
         rows = ws.view("latent.rows", count, self.row)
-        kernels.latent_rows(cache.k, rows, table, ctx.seq_start, ctx.n_seqs, ctx.max_q_len, cache.page_tokens, cache.ring_tokens)
-        keys_values = ws.view("latent.keys_values", 1, count, self.heads * (self.key + self.dv))
-        kernels.gemm_tc_pair(rows, self.expand, kernels.GemmOut(keys_values))
-        q = ws.view("latent.queries", tokens, self.heads, self.key)
-        kernels.latent_queries(q_full, self.cos_sin, ctx.token_pos, q, self.d, self.rot)
+        run_scale = ws.view("latent.run_scale", count // 64, 4)
+        kernels.latent_rows(cache.k, rows, run_scale, self.rank, self.key_norm, self.value_norm, table, ctx.seq_start, ctx.n_seqs, ctx.max_q_len, cache.page_tokens, cache.ring_tokens)
+        keys_values = ws.view("latent.keys_values", count, self.heads * (self.key + self.dv))
+        kernels.keys_and_values(rows, self.expand, keys_values, self.heads * self.key, run_scale)
+        q, q_scale = ws.view("latent.queries", tokens, self.heads, self.key), ws.view("latent.query_scale", tokens, self.heads)
+        kernels.latent_queries(q_full, self.cos_sin, ctx.token_pos, q, q_scale, self.d, self.rot)
         out = ws.view("latent.heads", tokens, self.heads, self.dv)
-        kernels.attention_prefill_rows(q, keys_values[0], out, ctx.seq_start, ctx.n_seqs, ctx.max_q_len, self.window, self.scale,
+        kernels.attention_prefill_rows(q, q_scale, keys_values, run_scale, out, ctx.seq_start, ctx.n_seqs, ctx.max_q_len, self.window, self.scale,
                                        gate=gate, gate_offset=gate_offset, gate_per_head=self.head_gate)
         return out
 

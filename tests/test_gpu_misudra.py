@@ -286,6 +286,74 @@ def test_prompts_over_keys_and_values_per_head(d, rot, turning, dv, rank, q_rank
     assert off["expanded"] < 5 * 2.0 ** -9 * 2 and off["expanded"] < 1.1 * off["rows"], off
 
 
+def _latent_mixer(tensors, dtype=torch.bfloat16, steps=512, **params):
+    """A latent mixer over a hidden size of 64 with these parameters and tensors, its buffers allocated."""
+    from qwen_triton_b200.config.spec import PartSpec
+    from qwen_triton_b200.parts.base import Runtime, Workspace
+    from qwen_triton_b200.parts.latent_attention import LatentAttention
+    device, rot = torch.device(DEV), params["rot_dim"]
+    runtime = Runtime(device=device, dtype=dtype, max_step_tokens=steps, max_positions=2048, workspace=Workspace(device), page_tokens=64)
+    params = {"hidden_size": 64, "float_out": True, "scale": (params["head_dim"] + rot) ** -0.5, "gate": False,
+              "position": PartSpec("rope", {"theta": 1e4, "rotary_dim": rot, "head_dim": rot, "pairing": "half"}), **params}
+    mixer = LatentAttention(params, "m", runtime)
+    if tensors is None:
+        tensors = {}
+        for name, spec in LatentAttention.expected_tensors(params, "m").items():
+            value = torch.randn(*spec.shape) * (1.0 if spec.role == "vector" else spec.shape[1] ** -0.5)
+            tensors[name] = value if spec.role == "vector" else value.bfloat16().float()
+    mixer.load(lambda name: tensors[name])
+    runtime.workspace.allocate()
+    return mixer, tensors
+
+
+def _latent_prompts(mixer, x, lengths, expanded=True, ring=0, cache=None):
+    """The mixer's results for prompts of these lengths, over keys and values per head or over latent rows."""
+    width = ring // 64 or -(-max(lengths) // 64)
+    step = _Prompts(list(lengths), width, list(reversed(range(width * len(lengths)))))
+    step.from_start = expanded
+    if cache is None:
+        cache = type("View", (), {})()
+        cache.k = torch.full((width * len(lengths), 1, 64, mixer.row), 1e4, dtype=x.dtype, device=DEV)
+        cache.v, cache.page_tokens, cache.ring_tokens, cache.writable, cache.group = cache.k, 64, ring, True, 0
+    out = mixer.forward(x.to(DEV), step, cache).value().cpu()
+    kernels.check_status(torch.device(DEV))
+    return out, cache
+
+
+@pytest.mark.parametrize("q_rank", [48, 0])
+@pytest.mark.parametrize("scores, values", [(24, 0), (-24, 0), (0, 30), (0, -30), (60, -60)])
+def test_prompts_over_keys_and_values_per_head_keep_the_range(q_rank, scores, values):
+    """Queries by 2^scores larger and keys by as much smaller, values by 2^values larger and the output's matrix by as much smaller: powers
+    of two, which round nothing anywhere, so the results are the same bits."""
+    torch.manual_seed(5)
+    params = {"num_heads": 3, "head_dim": 64, "rot_dim": 32, "v_head_dim": 64, "kv_rank": 128, "q_rank": q_rank}
+    mixer, tensors = _latent_mixer(None, **params)
+    lengths = (130, 64, 7)
+    x = torch.randn(sum(lengths), 64).bfloat16()
+    want, _ = _latent_prompts(mixer, x, lengths)
+    scaled = dict(tensors)
+    scaled["m.uq.weight" if q_rank else "m.q.weight"] = tensors["m.uq.weight" if q_rank else "m.q.weight"] * 2.0 ** scores
+    scaled["m.uk.weight"] = tensors["m.uk.weight"] * 2.0 ** -scores
+    scaled["m.dkv.weight"] = torch.cat((tensors["m.dkv.weight"][:128], tensors["m.dkv.weight"][128:] * 2.0 ** -scores))
+    scaled["m.uv.weight"], scaled["m.o.weight"] = tensors["m.uv.weight"] * 2.0 ** values, tensors["m.o.weight"] * 2.0 ** -values
+    got, _ = _latent_prompts(_latent_mixer(scaled, **params)[0], x, lengths)
+    assert bool(torch.isfinite(want).all()) and torch.equal(got, want)
+
+
+@pytest.mark.parametrize("spread", [0, 6, 12])
+def test_prompts_over_keys_and_values_per_head_of_uneven_tokens(spread):
+    """Tokens whose queries and shared key parts differ by up to 2^(2 spread), side by side in runs of 64, against the 32-bit mixer: no further
+    off than over latent rows (by more than a tenth, for single draws)."""
+    torch.manual_seed(spread)
+    params = {"num_heads": 4, "head_dim": 64, "rot_dim": 32, "v_head_dim": 64, "kv_rank": 128, "q_rank": 0}
+    mixer, tensors = _latent_mixer(None, **params)
+    lengths = (300, 129)
+    x = (torch.randn(sum(lengths), 64) * 2.0 ** torch.randint(-spread, spread + 1, (sum(lengths), 1))).bfloat16()
+    want = _latent_prompts(_latent_mixer(tensors, torch.float32, **params)[0], x.float(), lengths, expanded=False)[0].double()
+    off = {form: float((_latent_prompts(mixer, x, lengths, expanded=form)[0].double() - want).norm() / want.norm()) for form in (True, False)}
+    assert off[True] < 1.1 * off[False], off
+
+
 @pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("heads, rank, rot, window", [(3, 40, 16, 37), (20, 64, 32, 64), (40, 72, 24, 65), (1, 11, 6, 1), (70, 16, 8, 130), (5, 264, 8, 100),
                                                       (8, 32, 8, None)])
