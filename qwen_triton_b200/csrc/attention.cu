@@ -656,8 +656,8 @@ __global__ void __launch_bounds__(DEC_WARPS * 32) attention_decode_kernel(const 
 
 // One block per (sequence, head): out = sum_s acc_s e^{m_s - m} / sum_s l_s e^{m_s - m}; empty splits have m = -inf.
 template <typename T>
-__global__ void attention_combine_kernel(const float* __restrict__ part_acc, const float* __restrict__ part_ml,
-                                         T* __restrict__ out, int n_splits, int d, int sink, const float* __restrict__ sinks, int nq) {
+__global__ void attention_combine_kernel(const float* part_acc, const float* part_ml,
+                                         T* __restrict__ out, int n_splits, int d, int sink, const float* sinks, int nq) {
     pdl_launch_dependents();
     pdl_wait();
     const size_t item = blockIdx.x;   // seq * nq + head

@@ -656,9 +656,9 @@ __global__ void __launch_bounds__(32 * WS_MAX_WARPS) attention_decode_ws_kernel(
 
 // blockIdx.x is the (sequence, head), blockIdx.y a share of its columns: out = sum_s acc_s e^{m_s - m} / sum_s l_s e^{m_s - m};
 // empty splits have m = -inf.
-__global__ void attention_combine_mma_kernel(const float* __restrict__ part_acc, const float* __restrict__ part_ml,
+__global__ void attention_combine_mma_kernel(const float* part_acc, const float* part_ml,
                                              __nv_bfloat16* __restrict__ out, int n_splits, int d, int sink,
-                                             const float* __restrict__ sinks, int nq) {
+                                             const float* sinks, int nq) {
     pdl_launch_dependents();
     pdl_wait();
     constexpr int KEPT = 256;                                        // partial results whose factors the block keeps in shared memory

@@ -492,17 +492,17 @@ __global__ void __launch_bounds__(THREADS, BKEY == 64 ? 2 : 1) attention_prefill
                     if (DENSE && p.gate) {                // ahead of the one rounding of the result
                         const float* gate = p.gate + (size_t)(q_begin + q0 + r) * p.gate_cols + p.gate_offset + (p.gate_per_head ? head : head * HDV + c0);
                         if (p.gate_per_head) {
-                            float g = __ldg(gate);
-                            for (int sp = 1; sp < p.gate_splits; ++sp) g += __ldg(gate + sp * p.gate_split_stride);
+                            float g = *gate;
+                            for (int sp = 1; sp < p.gate_splits; ++sp) g += gate[sp * p.gate_split_stride];
                             const float f = 1.f / (1.f + expf(-g));
 #pragma unroll
                             for (int c = 0; c < 32; ++c) o[c] = __float_as_uint(__uint_as_float(o[c]) * f);
                         } else {
 #pragma unroll
                             for (int c = 0; c < 32; c += 4) {
-                                float4 g = __ldg(reinterpret_cast<const float4*>(gate + c));
+                                float4 g = *reinterpret_cast<const float4*>(gate + c);
                                 for (int sp = 1; sp < p.gate_splits; ++sp) {
-                                    const float4 more = __ldg(reinterpret_cast<const float4*>(gate + sp * p.gate_split_stride + c));
+                                    const float4 more = *reinterpret_cast<const float4*>(gate + sp * p.gate_split_stride + c);
                                     g.x += more.x; g.y += more.y; g.z += more.z; g.w += more.w;
                                 }
                                 o[c] = __float_as_uint(__uint_as_float(o[c]) / (1.f + expf(-g.x)));

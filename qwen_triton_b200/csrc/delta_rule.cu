@@ -114,8 +114,8 @@ __global__ void __launch_bounds__(128) delta_prepare_kernel(const PrepareParams 
 
 // kept[slot] <- the raw inputs of the sequence's last n_taps - 1 positions after this step.  One thread per
 // (sequence, channel): it reads what it needs of the old rows before it writes.
-__global__ void conv_keep_kernel(const float* __restrict__ proj, int n_splits, size_t split_stride, int proj_cols,
-                                 float* __restrict__ kept, const int* __restrict__ seq_start, const int* __restrict__ slots,
+__global__ void conv_keep_kernel(const float* proj, int n_splits, size_t split_stride, int proj_cols,
+                                 float* __restrict__ kept, const int* seq_start, const int* slots,
                                  int n_seqs, int channels, int n_taps) {
     pdl_launch_dependents();
     pdl_wait();
@@ -146,9 +146,9 @@ __device__ __forceinline__ float lowrank_value(float z, float rate) {
 }
 
 template <int MODE>
-__global__ void __launch_bounds__(256) lowrank_kernel(const float* __restrict__ proj, int n_splits, size_t split_stride, int proj_cols,
-                                                      int x_offset, int rank, const float* __restrict__ w, const float* __restrict__ bias,
-                                                      const float* __restrict__ rate_log, int per_rate, float power, float* __restrict__ out,
+__global__ void __launch_bounds__(256) lowrank_kernel(const float* proj, int n_splits, size_t split_stride, int proj_cols,
+                                                      int x_offset, int rank, const float* w, const float* bias,
+                                                      const float* rate_log, int per_rate, float power, float* __restrict__ out,
                                                       int n_tokens, int n_out) {
     pdl_launch_dependents();
     pdl_wait();
@@ -194,9 +194,9 @@ __global__ void __launch_bounds__(256) lowrank_kernel(const float* __restrict__ 
 // The same for a step of few tokens (up to 16 tiles of them): 64 outputs per block, so that many SMs get one, and the
 // columns cut into four ranges, one per 64 threads, whose sums meet in shared memory.
 template <int MODE>
-__global__ void __launch_bounds__(256) lowrank_few_kernel(const float* __restrict__ proj, int n_splits, size_t split_stride, int proj_cols,
-                                                          int x_offset, int rank, const float* __restrict__ w, const float* __restrict__ bias,
-                                                          const float* __restrict__ rate_log, int per_rate, float power, float* __restrict__ out,
+__global__ void __launch_bounds__(256) lowrank_few_kernel(const float* proj, int n_splits, size_t split_stride, int proj_cols,
+                                                          int x_offset, int rank, const float* w, const float* bias,
+                                                          const float* rate_log, int per_rate, float power, float* __restrict__ out,
                                                           int n_tokens, int n_out) {
     pdl_launch_dependents();
     pdl_wait();
@@ -829,8 +829,8 @@ __global__ void __launch_bounds__(WALK_THREADS) delta_chunk_walk_kernel(const Ch
 
 // out[t, h, :] = o / sqrt(mean(o^2) + eps) * w * gate[t, h, :].  One warp per (token, head).
 template <typename TO>
-__global__ void __launch_bounds__(128) gated_head_norm_kernel(const float* __restrict__ o, const float* __restrict__ gate,
-                                                              const float* __restrict__ w, float eps, TO* __restrict__ out,
+__global__ void __launch_bounds__(128) gated_head_norm_kernel(const float* o, const float* gate,
+                                                              const float* w, float eps, TO* __restrict__ out,
                                                               long long items, int vdim) {
     pdl_launch_dependents();
     pdl_wait();

@@ -13,8 +13,8 @@ using namespace qt;
 // residual[t, c, :] = table[ids[t], :] widened to float, times `scale` (1 for a plain gather), for every c of `copies` (a residual
 // of several parallel streams starts with all of them alike; 1: the plain stream).  One block per token.
 template <typename T>
-__global__ void embedding_kernel(float* __restrict__ residual, const T* __restrict__ table,
-                                 const int* __restrict__ ids, int hidden, int vocab, float scale, int copies) {
+__global__ void embedding_kernel(float* __restrict__ residual, const T* table,
+                                 const int* ids, int hidden, int vocab, float scale, int copies) {
     pdl_launch_dependents();
     pdl_wait();
     const int t = blockIdx.x;
@@ -32,8 +32,8 @@ __global__ void embedding_kernel(float* __restrict__ residual, const T* __restri
 // `start` (or null) takes a copy of the result in the table's type: the embedding's output, for a model whose layers
 // meet it again.  One block per token.
 template <typename T>
-__global__ void embedding_norm_kernel(float* __restrict__ residual, const T* __restrict__ table, const int* __restrict__ ids, int hidden,
-                                      int vocab, float scale, const float* __restrict__ norm_w, float eps, T* __restrict__ start) {
+__global__ void embedding_norm_kernel(float* __restrict__ residual, const T* table, const int* ids, int hidden,
+                                      int vocab, float scale, const float* norm_w, float eps, T* __restrict__ start) {
     pdl_launch_dependents();
     pdl_wait();
     __shared__ float scratch[32];
@@ -85,8 +85,8 @@ extern "C" int qt_embedding(float* residual, const void* table, const int* ids, 
 // out[t] = [x | start[t]] in the activation type, x = residual[t] + sum_s delta[s][t] in float; the stream is then zero:
 // what a map of these rows returns takes its place by the ordinary addition of the next norm.  One block per token.
 template <typename TD, typename TO>
-__global__ void stream_concat_kernel(float* __restrict__ residual, const TD* __restrict__ delta, int n_splits, size_t split_stride,
-                                     const TO* __restrict__ start, TO* __restrict__ out, int hidden) {
+__global__ void stream_concat_kernel(float* __restrict__ residual, const TD* delta, int n_splits, size_t split_stride,
+                                     const TO* start, TO* __restrict__ out, int hidden) {
     pdl_launch_dependents();
     pdl_wait();
     const size_t at = (size_t)blockIdx.x * hidden, to = 2 * at;
@@ -136,7 +136,7 @@ extern "C" int qt_stream_concat(float* residual, const void* delta, int delta_dt
 // out[t, :] += bias, on the float sums of a product before anything rounds them (the first plane, where a product is
 // split over K).  luozoupi/Qwen-Triton adds the bias of a linear layer with a kernel of its own as well
 // (kernels/matmul.py:99-111, modules/linear.py:31).
-__global__ void add_bias_kernel(float* __restrict__ out, const float* __restrict__ bias, int cols, size_t count) {
+__global__ void add_bias_kernel(float* __restrict__ out, const float* bias, int cols, size_t count) {
     pdl_launch_dependents();
     pdl_wait();
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < count; i += (size_t)gridDim.x * blockDim.x)
@@ -163,9 +163,9 @@ extern "C" int qt_add_bias(float* out, const float* bias, int rows, int cols, vo
 // Norm in groups: a row of `width` elements is `gridDim.y` equal consecutive parts of `hidden` elements, each
 // divided by its own root mean square (blockIdx.y is the part); one part is the plain norm.
 template <typename TD, typename TO>
-__global__ void add_rmsnorm_kernel(float* __restrict__ residual, const TD* __restrict__ delta, int n_splits,
-                                   size_t split_stride, const float* __restrict__ weight, float eps,
-                                   TO* __restrict__ out, const int* __restrict__ rows, int hidden, int width) {
+__global__ void add_rmsnorm_kernel(float* __restrict__ residual, const TD* delta, int n_splits,
+                                   size_t split_stride, const float* weight, float eps,
+                                   TO* __restrict__ out, const int* rows, int hidden, int width) {
     pdl_launch_dependents();
     pdl_wait();
     __shared__ float scratch[32];
@@ -231,9 +231,9 @@ __device__ __forceinline__ void add_splits4(float4& v, const TD* dp, int first, 
 }
 
 template <typename TD, typename TO, int BATCH, int MAX_THREADS, int MIN_BLOCKS>
-__global__ void __launch_bounds__(MAX_THREADS, MIN_BLOCKS) add_rmsnorm_vec_kernel(float* __restrict__ residual, const TD* __restrict__ delta, int n_splits,
-                                       size_t split_stride, const float* __restrict__ weight, float eps,
-                                       TO* __restrict__ out, const int* __restrict__ rows, int hidden, int width) {
+__global__ void __launch_bounds__(MAX_THREADS, MIN_BLOCKS) add_rmsnorm_vec_kernel(float* __restrict__ residual, const TD* delta, int n_splits,
+                                       size_t split_stride, const float* weight, float eps,
+                                       TO* __restrict__ out, const int* rows, int hidden, int width) {
     pdl_launch_dependents();
     pdl_wait();
     __shared__ float scratch[32];
@@ -277,9 +277,9 @@ __global__ void __launch_bounds__(MAX_THREADS, MIN_BLOCKS) add_rmsnorm_vec_kerne
 constexpr int NORM_CLUSTER = 8;
 
 template <typename TD, typename TO>
-__global__ void __launch_bounds__(1024, 1) add_rmsnorm_cluster_kernel(float* __restrict__ residual, const TD* __restrict__ delta, int n_splits,
-                                                                   size_t split_stride, const float* __restrict__ weight, float eps,
-                                                                   TO* __restrict__ out, const int* __restrict__ rows, int hidden) {
+__global__ void __launch_bounds__(1024, 1) add_rmsnorm_cluster_kernel(float* __restrict__ residual, const TD* delta, int n_splits,
+                                                                   size_t split_stride, const float* weight, float eps,
+                                                                   TO* __restrict__ out, const int* rows, int hidden) {
     pdl_launch_dependents();
     cluster_arrive_started();
     pdl_wait();
@@ -431,7 +431,7 @@ extern "C" int qt_add_dyt(float* residual, const float* delta_a, int splits_a, l
 // [map][head] (map-major), and the head's output is o = a1 - lambda * a2, divided by its root mean square over the
 // head's values (no weight), times `post`.  One warp per (token, head), float inside.
 template <typename T>
-__global__ void __launch_bounds__(128) map_difference_kernel(const T* __restrict__ ctx, T* __restrict__ out, long long tokens, int heads,
+__global__ void __launch_bounds__(128) map_difference_kernel(const T* ctx, T* __restrict__ out, long long tokens, int heads,
                                                              int dv, float lambda, float eps, float post) {
     pdl_launch_dependents();
     pdl_wait();
@@ -490,7 +490,7 @@ struct QkvParams {
 // The factors of a norm over the whole projection: row_inv[t] = {rsqrt(mean(q_t^2) + eps), rsqrt(mean(k_t^2) + eps)} over all
 // nq d (nkv d) elements of token t at once.  One block per token.
 template <typename TI>
-__global__ void qk_row_rms_kernel(const TI* __restrict__ qkv, int n_splits, size_t split_stride, size_t cols, int q_cols, int k_cols, float eps,
+__global__ void qk_row_rms_kernel(const TI* qkv, int n_splits, size_t split_stride, size_t cols, int q_cols, int k_cols, float eps,
                                   float* __restrict__ row_inv) {
     pdl_launch_dependents();
     pdl_wait();
@@ -1109,7 +1109,7 @@ extern "C" int qt_qkv_treat_write(const void* qkv, int in_dtype, int n_splits, l
 __device__ __forceinline__ size_t gate_column(int i, int group) { return group ? (size_t)(i / group) * 2 * group + i % group : (size_t)i; }
 
 template <typename TI, typename TO>
-__global__ void swiglu_kernel(const TI* __restrict__ gate_up, int n_splits, size_t split_stride, const float* __restrict__ bias,
+__global__ void swiglu_kernel(const TI* gate_up, int n_splits, size_t split_stride, const float* bias,
                               TO* __restrict__ out, long long total, int inter, int group, int act, float limit) {
     pdl_launch_dependents();
     pdl_wait();
@@ -1155,7 +1155,7 @@ template <typename TO> __device__ __forceinline__ float4 silu_mul4(const float4&
 
 // PT chunks per thread, all loads issued before the first store.
 template <typename TI, typename TO, int PT>
-__global__ void swiglu_vec_kernel(const TI* __restrict__ gate_up, int n_splits, size_t split_stride, const float* __restrict__ bias,
+__global__ void swiglu_vec_kernel(const TI* gate_up, int n_splits, size_t split_stride, const float* bias,
                                   TO* __restrict__ out, int inter, int group, int act, float limit) {
     pdl_launch_dependents();
     pdl_wait();

@@ -173,7 +173,7 @@ __device__ __forceinline__ void floats_of(const Eight<__nv_bfloat16>& r, float (
 
 // acc[j] += this lane's part of row[j] . (x times factor), n elements.
 template <typename T, int ROWS>
-__device__ __forceinline__ void lane_dots(const T* const (&row)[ROWS], const T* __restrict__ x, float factor, int n, int lane, float (&acc)[ROWS]) {
+__device__ __forceinline__ void lane_dots(const T* const (&row)[ROWS], const T* x, float factor, int n, int lane, float (&acc)[ROWS]) {
     constexpr int AT_ONCE = EV_BYTES / (ROWS * 8 * (int)sizeof(T)), TURNS = AT_ONCE < 1 ? 1 : AT_ONCE > 8 ? 8 : AT_ONCE;
     for (int i0 = lane * 8; i0 < n; i0 += 256 * TURNS) {
         Eight<T> w[TURNS][ROWS], v[TURNS];
@@ -362,8 +362,8 @@ __global__ void __launch_bounds__(1024) expert_route_kernel(const ExpertParams p
 
 // ordered[row, :] = x[row_token[row] / top, :] (zeros for padding rows), times the pair's input weight where there is one
 // (the product in float, rounded once).  One block per row, 16 bytes per thread and turn.
-__global__ void expert_gather_kernel(const uint4* __restrict__ x, const int* __restrict__ row_token, uint4* __restrict__ ordered, int chunks, int top,
-                                     const float* __restrict__ in_weights) {
+__global__ void expert_gather_kernel(const uint4* x, const int* row_token, uint4* __restrict__ ordered, int chunks, int top,
+                                     const float* in_weights) {
     pdl_launch_dependents();
     pdl_wait();
     const int row = blockIdx.x, pair = row_token[row], token = pair >= 0 ? pair / top : -1;
@@ -383,9 +383,9 @@ __global__ void expert_gather_kernel(const uint4* __restrict__ x, const int* __r
 // neighbouring columns (4 where all rows lie on pieces of that size) and asks for the further term before the experts' rows.  1,999 tokens of 2
 // of 16 experts, 2,048 columns, a shared expert beside them: about 10 us; 21 us with one column a thread.
 template <typename T, int V>
-__global__ void __launch_bounds__(256) expert_combine_kernel(const T* __restrict__ y, const int* __restrict__ pair_row, float* __restrict__ out, int top, int width,
-                                      float pair_weight, const float* __restrict__ pair_weights, const float* __restrict__ base,
-                                      int base_splits, size_t base_stride, const float* __restrict__ row_scale) {
+__global__ void __launch_bounds__(256) expert_combine_kernel(const T* y, const int* pair_row, float* __restrict__ out, int top, int width,
+                                      float pair_weight, const float* pair_weights, const float* base,
+                                      int base_splits, size_t base_stride, const float* row_scale) {
     pdl_launch_dependents();
     pdl_wait();
     const int t = blockIdx.x;
@@ -433,7 +433,7 @@ __global__ void __launch_bounds__(256) expert_combine_kernel(const T* __restrict
 // many equal runs of neighbours, a group's score is the largest in it, and only the experts of the `keep` best groups (of
 // equal ones the lower group first) can be chosen.
 // One warp per token; chosen [T, top], weights [T, top], gate [T] = sigmoid of the extra column.
-__global__ void __launch_bounds__(128) route_top_kernel(const float* __restrict__ logits, int n_splits, size_t split_stride, int cols,
+__global__ void __launch_bounds__(128) route_top_kernel(const float* logits, int n_splits, size_t split_stride, int cols,
                                                         int* __restrict__ chosen, float* __restrict__ weights, float* __restrict__ gate,
                                                         int n_tokens, int experts, int top, float scale, int normalize, int softmax, int groups,
                                                         int keep) {

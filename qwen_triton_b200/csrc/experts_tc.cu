@@ -43,7 +43,7 @@ __device__ __forceinline__ void store8(__nv_bfloat16* dst, const float (&f)[8]) 
 template <typename TO, bool ACT, int BN, int STAGES>
 __global__ void __launch_bounds__(THREADS) expert_gemm_kernel(const __grid_constant__ CUtensorMap map_x,
                                                               const __grid_constant__ CUtensorMap map_w, TO* __restrict__ out,
-                                                              const int* __restrict__ tile_expert, int n_out, int kb_total,
+                                                              const int* tile_expert, int n_out, int kb_total,
                                                               int w_tiles, int act, int* status) {
     constexpr uint32_t B_BYTES = BN * BK * 2, STAGE_BYTES = A_BYTES + B_BYTES;
     // instruction descriptor: float accumulator, bfloat16 A and B, both K-major, N = BN, M = 128
@@ -162,7 +162,7 @@ __device__ __forceinline__ void mbar_arrive(uint32_t bar) {
 template <typename TO, bool ACT>
 __global__ void __launch_bounds__(THREADS, 1) expert_gemm_persistent_kernel(const __grid_constant__ CUtensorMap map_x,
                                                                             const __grid_constant__ CUtensorMap map_w, TO* __restrict__ out,
-                                                                            const int* __restrict__ tile_expert, int n_out, int kb_total,
+                                                                            const int* tile_expert, int n_out, int kb_total,
                                                                             int w_tiles, int total_items, int act, int* status) {
     constexpr uint32_t IDESC = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(PBN >> 3) << 17) | ((uint32_t)(BM >> 4) << 24);
     extern __shared__ uint8_t smem_raw[];
@@ -322,7 +322,7 @@ constexpr uint32_t FEW_STAGE_BYTES = A_BYTES + FEW_ROWS * BK * 2;
 
 template <bool ACT>
 __global__ void __launch_bounds__(THREADS) expert_gemm_few_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_w,
-                                                                  __nv_bfloat16* __restrict__ out, const int* __restrict__ tile_expert, int n_out, int kb_total,
+                                                                  __nv_bfloat16* __restrict__ out, const int* tile_expert, int n_out, int kb_total,
                                                                   int w_tiles, int act, int* status) {
     // instruction descriptor: float accumulator, bfloat16 A (weights) and B (rows), both K-major, N = FEW_ROWS, M = 128
     constexpr uint32_t IDESC = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(FEW_ROWS >> 3) << 17) | ((uint32_t)(BM >> 4) << 24);

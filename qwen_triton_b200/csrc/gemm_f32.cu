@@ -41,7 +41,7 @@ __device__ __forceinline__ void copy16(float* to, const float* from, bool there)
 
 // TM x 8 results a thread, tiles of 8 TM x 128; grid (ranks x N tiles, M tiles); k_steps slices of 32 per rank
 template <int TM>
-__global__ void __launch_bounds__(GF_THREADS, 2) gemm_f32_tile_kernel(const float* __restrict__ a, const float* __restrict__ w, float* __restrict__ c,
+__global__ void __launch_bounds__(GF_THREADS, 2) gemm_f32_tile_kernel(const float* a, const float* w, float* __restrict__ c,
                                                                      int M, int N, int K, int ranks, int k_steps) {
     constexpr int BM = 8 * TM, STAGE = (BM + GF_BN) * GF_ROW;
     static_assert(GF_STAGES * STAGE >= BM * GF_BN, "a block's part of the result is exchanged in the ring's memory");
@@ -187,7 +187,7 @@ int launch_tiles(const float* a, const float* w, float* c, int M, int N, int K, 
 constexpr int GR_WARPS = 8, GR_ROWS = 4;
 
 template <int MT>
-__global__ void __launch_bounds__(GR_WARPS * 32) gemm_f32_rows_kernel(const float* __restrict__ a, const float* __restrict__ w, float* __restrict__ c,
+__global__ void __launch_bounds__(GR_WARPS * 32) gemm_f32_rows_kernel(const float* a, const float* w, float* __restrict__ c,
                                                                      int M, int N, int K, int shares) {
     constexpr int AHEAD = MT <= 2 ? 4 : 2;                                  // 16-byte pieces of each weight row in flight
     __shared__ float exchange[GR_WARPS][MT * GR_ROWS];

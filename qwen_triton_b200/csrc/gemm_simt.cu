@@ -8,7 +8,7 @@ using namespace qt;
 constexpr int GS_BM = 64, GS_BN = 64, GS_BK = 16, GS_THREADS = 256;
 
 template <typename TI, typename TO>
-__global__ void __launch_bounds__(GS_THREADS) gemm_simt_kernel(const TI* __restrict__ a, const TI* __restrict__ w,
+__global__ void __launch_bounds__(GS_THREADS) gemm_simt_kernel(const TI* a, const TI* w,
                                                               TO* __restrict__ c, int M, int N, int K) {
     pdl_launch_dependents();
     pdl_wait();

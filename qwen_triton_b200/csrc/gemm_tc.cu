@@ -52,7 +52,7 @@ template <int BX, typename TO, int MODE>
 __global__ void __launch_bounds__(THREADS) gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w,
                                                           const __grid_constant__ CUtensorMap map_x, TO* __restrict__ out,
                                                           int M, int N, int kb_total, int kb_per_split,
-                                                          size_t split_stride, int stages, int act, float limit, const float* __restrict__ bias, int* status) {
+                                                          size_t split_stride, int stages, int act, float limit, const float* bias, int* status) {
     constexpr uint32_t X_BYTES = BX * BK * 2;
     constexpr uint32_t STAGE_BYTES = W_BYTES + X_BYTES;
     constexpr uint32_t TMEM_COLS = BX < 32 ? 32 : BX;
@@ -336,7 +336,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_tc_pair_kernel(const __grid_c
                                                                   const __grid_constant__ CUtensorMap map_x, TO* __restrict__ out,
                                                                   int M, int N, int kb_total, int kb_per_split, int splits,
                                                                   size_t split_stride, int act, float limit, int vector_stores, int tail_tiles,
-                                                                  float* __restrict__ tail_scratch, int* tail_flags, const float* __restrict__ bias,
+                                                                  float* __restrict__ tail_scratch, int* tail_flags, const float* bias,
                                                                   const float4* run_scale, int key_cols, int* status) {
     // instruction descriptor: float accumulator, bfloat16 A and B, both K-major, N = 256 weight rows, M = 256 tokens over the pair
     constexpr uint32_t IDESC = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(PAIR_W >> 3) << 17) | ((uint32_t)(PAIR_X >> 4) << 24);

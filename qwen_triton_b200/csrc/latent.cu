@@ -112,8 +112,8 @@ extern "C" int qt_latent_prepare(const float* proj, int n_splits, long long spli
 // ----------------------------------------------------------------------------- the rotated part of the queries
 // q [splits, T, q_cols >= heads * (dim + rot)] -> out[t, h, out_offset + i] for i < rot.  One thread per (token, head, element).
 template <typename TI, typename TO>
-__global__ void latent_query_rot_kernel(const TI* __restrict__ q, int n_splits, size_t split_stride, const float* __restrict__ cos_sin,
-                                        int rotary_dim, const int* __restrict__ token_pos, TO* __restrict__ out, long long total,
+__global__ void latent_query_rot_kernel(const TI* q, int n_splits, size_t split_stride, const float* cos_sin,
+                                        int rotary_dim, const int* token_pos, TO* __restrict__ out, long long total,
                                         int heads, int dim, int rot, int q_cols, int out_row, int out_offset) {
     pdl_launch_dependents();
     pdl_wait();
@@ -179,8 +179,8 @@ __device__ __forceinline__ float2 into_halves(float largest) {
 // element is at most the largest of the latents (the first `rank` elements) times key_norm, or an element of the shared part behind
 // them; a value's at most the largest latent times value_norm.  2,048 tokens of 512 + 64 3.7 us (3.2 us without the largest elements).  grid (runs of the longest sequence, sequences).
 constexpr int LR_THREADS = 512;
-__global__ void __launch_bounds__(LR_THREADS) latent_rows_kernel(const uint4* __restrict__ cache, uint4* __restrict__ rows, float4* __restrict__ run_scale,
-                                                          const int* __restrict__ block_table, int max_blocks, const int* __restrict__ seq_start, int pieces,
+__global__ void __launch_bounds__(LR_THREADS) latent_rows_kernel(const uint4* cache, uint4* __restrict__ rows, float4* __restrict__ run_scale,
+                                                          const int* block_table, int max_blocks, const int* seq_start, int pieces,
                                                           int latent_pieces, float key_norm, float value_norm) {
     pdl_launch_dependents();
     pdl_wait();
@@ -250,20 +250,20 @@ __device__ __forceinline__ void sum_eight(const float* p, int n_splits, size_t s
 #pragma unroll
     for (int i = 0; i < 8; ++i) v[i] = 0.f;
     for (int s = 0; s < n_splits; ++s) {
-        const float4 a = __ldg(reinterpret_cast<const float4*>(p + (size_t)s * stride)), b = __ldg(reinterpret_cast<const float4*>(p + (size_t)s * stride) + 1);
+        const float4 a = *reinterpret_cast<const float4*>(p + (size_t)s * stride), b = reinterpret_cast<const float4*>(p + (size_t)s * stride)[1];
         v[0] += a.x; v[1] += a.y; v[2] += a.z; v[3] += a.w; v[4] += b.x; v[5] += b.y; v[6] += b.z; v[7] += b.w;
     }
 }
 __device__ __forceinline__ void sum_eight(const __nv_bfloat16* p, int, size_t, float (&v)[8]) {
-    const uint4 raw = __ldg(reinterpret_cast<const uint4*>(p));
+    const uint4 raw = *reinterpret_cast<const uint4*>(p);
     const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&raw);
 #pragma unroll
     for (int i = 0; i < 4; ++i) { v[2 * i] = __low2float(h[i]); v[2 * i + 1] = __high2float(h[i]); }
 }
 
 template <typename TI, int PIECES>
-__global__ void __launch_bounds__(256) latent_queries_kernel(const TI* __restrict__ q, int n_splits, size_t split_stride, int q_cols, const float* __restrict__ cos_sin,
-                                                             int rotary_dim, const int* __restrict__ token_pos, uint4* __restrict__ out, float* __restrict__ q_scale,
+__global__ void __launch_bounds__(256) latent_queries_kernel(const TI* q, int n_splits, size_t split_stride, int q_cols, const float* cos_sin,
+                                                             int rotary_dim, const int* token_pos, uint4* __restrict__ out, float* __restrict__ q_scale,
                                                              long long pairs, int heads, int dim, int rot) {
     pdl_launch_dependents();
     pdl_wait();
@@ -443,8 +443,8 @@ __global__ void __launch_bounds__(128) head_product_mma_kernel(const HeadProduct
                     if (tok < p.n_tokens && k < p.k) {
                         const float* at = (const float*)p.x + (size_t)((long long)tok * p.x_row + (long long)h * p.x_head + p.x_offset + k);
                         for (int sp = 0; sp < p.x_splits; ++sp) {
-                            const float4 a = __ldg(reinterpret_cast<const float4*>(at + (size_t)sp * p.x_split_stride));
-                            const float4 b = __ldg(reinterpret_cast<const float4*>(at + (size_t)sp * p.x_split_stride) + 1);
+                            const float4 a = *reinterpret_cast<const float4*>(at + (size_t)sp * p.x_split_stride);
+                            const float4 b = reinterpret_cast<const float4*>(at + (size_t)sp * p.x_split_stride)[1];
                             lo[j].x += a.x; lo[j].y += a.y; lo[j].z += a.z; lo[j].w += a.w;
                             hi[j].x += b.x; hi[j].y += b.y; hi[j].z += b.z; hi[j].w += b.w;
                         }
@@ -504,8 +504,8 @@ __global__ void __launch_bounds__(128) head_product_mma_kernel(const HeadProduct
                 for (int nt = 0; nt < 8; ++nt) {
                     const int n = n0 + nt * 8 + 2 * t;
                     const size_t at = (size_t)tok * p.gate_cols + p.gate_offset + (size_t)h * p.gate_head + (size_t)n * p.gate_elem;
-                    if (tok < p.n_tokens && n < p.n) gates[nt][2 * r] += __ldg(gate + at);
-                    if (tok < p.n_tokens && n + 1 < p.n) gates[nt][2 * r + 1] += __ldg(gate + at + p.gate_elem);
+                    if (tok < p.n_tokens && n < p.n) gates[nt][2 * r] += gate[at];
+                    if (tok < p.n_tokens && n + 1 < p.n) gates[nt][2 * r + 1] += gate[at + p.gate_elem];
                 }
             }
         }
@@ -568,7 +568,7 @@ __global__ void __launch_bounds__(128) head_product_few_kernel(const HeadProduct
             float4 lo = make_float4(0.f, 0.f, 0.f, 0.f), hi = lo;
             if (there)
                 for (int sp = 0; sp < p.x_splits; ++sp) {
-                    const float4 a = __ldg(reinterpret_cast<const float4*>(at + (size_t)sp * p.x_split_stride)), b = __ldg(reinterpret_cast<const float4*>(at + (size_t)sp * p.x_split_stride) + 1);
+                    const float4 a = *reinterpret_cast<const float4*>(at + (size_t)sp * p.x_split_stride), b = reinterpret_cast<const float4*>(at + (size_t)sp * p.x_split_stride)[1];
                     lo.x += a.x; lo.y += a.y; lo.z += a.z; lo.w += a.w;
                     hi.x += b.x; hi.y += b.y; hi.z += b.z; hi.w += b.w;
                 }
@@ -585,7 +585,7 @@ __global__ void __launch_bounds__(128) head_product_few_kernel(const HeadProduct
             for (int e = 0; e < 4 * NT; ++e) {
                 const int tok = warp * 16 + g + 8 * ((e >> 1) & 1), n = n0 + (e >> 2) * 8 + 2 * t + (e & 1);
                 if (tok < p.n_tokens && n < p.n)
-                    gates[e >> 2][e & 3] += __ldg(p.gate + (size_t)sp * p.gate_split_stride + (size_t)tok * p.gate_cols + p.gate_offset + (size_t)h * p.gate_head + (size_t)n * p.gate_elem);
+                    gates[e >> 2][e & 3] += p.gate[(size_t)sp * p.gate_split_stride + (size_t)tok * p.gate_cols + p.gate_offset + (size_t)h * p.gate_head + (size_t)n * p.gate_elem];
             }
     }
     cp_async_wait<0>();

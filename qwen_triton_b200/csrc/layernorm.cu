@@ -18,10 +18,10 @@
 using namespace qt;
 
 template <typename TD, typename TO>
-__global__ void add_layernorm_kernel(float* __restrict__ residual, const TD* __restrict__ delta, int n_splits, size_t split_stride,
-                                     const float* __restrict__ post_weight, const float* __restrict__ post_bias,
-                                     const float* __restrict__ weight, const float* __restrict__ bias, float eps,
-                                     TO* __restrict__ out, const int* __restrict__ rows, int hidden) {
+__global__ void add_layernorm_kernel(float* __restrict__ residual, const TD* delta, int n_splits, size_t split_stride,
+                                     const float* post_weight, const float* post_bias,
+                                     const float* weight, const float* bias, float eps,
+                                     TO* __restrict__ out, const int* rows, int hidden) {
     pdl_launch_dependents();
     pdl_wait();
     extern __shared__ float row[];            // [hidden]
@@ -91,10 +91,10 @@ __device__ __forceinline__ void store4(__nv_bfloat16* p, float4 v) {
 }
 
 template <typename TD, typename TO>
-__global__ void add_layernorm_vec_kernel(float* __restrict__ residual, const TD* __restrict__ delta, int n_splits, size_t split_stride,
-                                         const float* __restrict__ post_weight, const float* __restrict__ post_bias,
-                                         const float* __restrict__ weight, const float* __restrict__ bias, float eps,
-                                         TO* __restrict__ out, const int* __restrict__ rows, int hidden) {
+__global__ void add_layernorm_vec_kernel(float* __restrict__ residual, const TD* delta, int n_splits, size_t split_stride,
+                                         const float* post_weight, const float* post_bias,
+                                         const float* weight, const float* bias, float eps,
+                                         TO* __restrict__ out, const int* rows, int hidden) {
     pdl_launch_dependents();
     pdl_wait();
     __shared__ float scratch[32];
@@ -181,7 +181,7 @@ extern "C" int qt_add_layernorm(float* residual, const void* delta, int delta_dt
 
 // ----------------------------------------------------------------------------- activation on a product's sums
 template <typename TI, typename TO>
-__global__ void activation_kernel(const TI* __restrict__ in, int n_splits, size_t split_stride, TO* __restrict__ out, long long total, int act) {
+__global__ void activation_kernel(const TI* in, int n_splits, size_t split_stride, TO* __restrict__ out, long long total, int act) {
     pdl_launch_dependents();
     pdl_wait();
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x)
@@ -190,7 +190,7 @@ __global__ void activation_kernel(const TI* __restrict__ in, int n_splits, size_
 
 // Four elements a thread, for totals, strides and pointers that keep the alignment of a quad.
 template <typename TI, typename TO>
-__global__ void activation_vec_kernel(const TI* __restrict__ in, int n_splits, size_t split_stride, TO* __restrict__ out, long long quads, int act) {
+__global__ void activation_vec_kernel(const TI* in, int n_splits, size_t split_stride, TO* __restrict__ out, long long quads, int act) {
     pdl_launch_dependents();
     pdl_wait();
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < quads; i += (long long)gridDim.x * blockDim.x) {
@@ -237,7 +237,7 @@ extern "C" int qt_activation(const void* in, int in_dtype, int n_splits, long lo
 // out = wa * sum_s a[s] + wb * sum_s b[s], in float: two sublayers that run side by side on the same input and are
 // mixed with two constants before anything else happens to them.
 template <typename TA, typename TB>
-__global__ void weighted_sum_kernel(const TA* __restrict__ a, int a_splits, size_t a_stride, float wa, const TB* __restrict__ b, int b_splits,
+__global__ void weighted_sum_kernel(const TA* a, int a_splits, size_t a_stride, float wa, const TB* b, int b_splits,
                                     size_t b_stride, float wb, float* __restrict__ out, long long total) {
     pdl_launch_dependents();
     pdl_wait();

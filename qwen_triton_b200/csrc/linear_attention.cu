@@ -43,8 +43,8 @@ struct LinAttnParams {
 constexpr int LA_CONSTANT = 0, LA_PER_HEAD = 1, LA_PER_CHANNEL = 2;      // what a decay depends on besides its head
 
 __device__ __forceinline__ float la_raw(const LinAttnParams& p, size_t index) {
-    float x = __ldg(p.proj + index);
-    for (int s = 1; s < p.n_splits; ++s) x += __ldg(p.proj + index + (size_t)s * p.split_stride);
+    float x = p.proj[index];
+    for (int s = 1; s < p.n_splits; ++s) x += p.proj[index + (size_t)s * p.split_stride];
     return x;
 }
 __device__ __forceinline__ float la_act(const LinAttnParams& p, float x) { return p.act ? x / (1.f + expf(-x)) : x; }
@@ -54,15 +54,15 @@ template <int V> struct RotPack { float v[V]; };
 template <int V> __device__ __forceinline__ RotPack<V> rot_sum(const float* p, int n_splits, size_t stride) {
     RotPack<V> r;
     if constexpr (V == 4) {
-        float4 x = __ldg(reinterpret_cast<const float4*>(p));
+        float4 x = *reinterpret_cast<const float4*>(p);
         for (int s = 1; s < n_splits; ++s) {
-            const float4 y = __ldg(reinterpret_cast<const float4*>(p + (size_t)s * stride));
+            const float4 y = *reinterpret_cast<const float4*>(p + (size_t)s * stride);
             x.x += y.x; x.y += y.y; x.z += y.z; x.w += y.w;
         }
         r.v[0] = x.x; r.v[1] = x.y; r.v[2] = x.z; r.v[3] = x.w;
     } else {
-        r.v[0] = __ldg(p);
-        for (int s = 1; s < n_splits; ++s) r.v[0] += __ldg(p + (size_t)s * stride);
+        r.v[0] = *p;
+        for (int s = 1; s < n_splits; ++s) r.v[0] += p[(size_t)s * stride];
     }
     return r;
 }
@@ -76,7 +76,7 @@ template <int V> __device__ __forceinline__ void rot_put(float* p, const RotPack
 // Bound by the bytes it moves.  A thread takes V neighbouring columns (16-byte accesses where the rows allow) of row blockIdx.y, + gridDim.y, ..;
 // 1,999 rows of 6,144 columns: 19 us, 38 us with single floats whose place was divided out of one running index.
 template <int V>
-__global__ void __launch_bounds__(256) linear_attention_prepare_kernel(const float* __restrict__ proj, int n_splits, size_t split_stride, int proj_cols, int cols,
+__global__ void __launch_bounds__(256) linear_attention_prepare_kernel(const float* proj, int n_splits, size_t split_stride, int proj_cols, int cols,
                                                                        float* __restrict__ out, int n_tokens, int act) {
     pdl_launch_dependents();
     pdl_wait();
@@ -110,9 +110,9 @@ extern "C" int qt_linear_attention_prepare(const float* proj, int n_splits, long
 // holds (cos | sin, rd columns); the other columns pass.  A thread takes V neighbouring pairs, or V neighbouring columns that
 // do not turn; grid (blocks of a row's items, tokens).
 template <int V>
-__global__ void __launch_bounds__(256) linear_attention_rotate_kernel(const float* __restrict__ proj, int n_splits, size_t split_stride, int proj_cols, int cols,
-                                                                      float* __restrict__ out, int heads, int dim, int rd, const float* __restrict__ cos_sin,
-                                                                      int max_pos, const int* __restrict__ token_pos) {
+__global__ void __launch_bounds__(256) linear_attention_rotate_kernel(const float* proj, int n_splits, size_t split_stride, int proj_cols, int cols,
+                                                                      float* __restrict__ out, int heads, int dim, int rd, const float* cos_sin,
+                                                                      int max_pos, const int* token_pos) {
     pdl_launch_dependents();
     pdl_wait();
     const int item = blockIdx.x * 256 + threadIdx.x, half = rd / 2;
@@ -315,19 +315,19 @@ __global__ void __launch_bounds__(32 * LA_LANES) linear_attention_step_kernel(co
         decay[0] = constant;
         if (MODE != LA_CONSTANT) {
             const size_t th = (size_t)t * p.heads + head;
-            if (p.v_scale) v *= __ldg(p.v_scale + th);
-            if (MODE == LA_PER_HEAD) decay[0] = expf(__ldg(p.log_decay + th));
+            if (p.v_scale) v *= p.v_scale[th];
+            if (MODE == LA_PER_HEAD) decay[0] = expf(p.log_decay[th]);
             else if (vec && ((uintptr_t)p.log_decay & 15) == 0) {
 #pragma unroll
                 for (int i = 0; i < (MODE == LA_PER_CHANNEL ? RPL : 1); i += 4) {
-                    const float4 g = row0 + at(i) < p.dim ? __ldg(reinterpret_cast<const float4*>(p.log_decay + th * p.dim + row0 + at(i))) : make_float4(0.f, 0.f, 0.f, 0.f);
+                    const float4 g = row0 + at(i) < p.dim ? *reinterpret_cast<const float4*>(p.log_decay + th * p.dim + row0 + at(i)) : make_float4(0.f, 0.f, 0.f, 0.f);
                     const float e[4] = {g.x, g.y, g.z, g.w};
 #pragma unroll
                     for (int j = 0; j < 4; ++j) if (MODE == LA_PER_CHANNEL) decay[(i + j) % (MODE == LA_PER_CHANNEL ? RPL : 1)] = e[j];
                 }
             } else {
 #pragma unroll
-                for (int i = 0; i < (MODE == LA_PER_CHANNEL ? RPL : 1); ++i) decay[i] = row0 + at(i) < p.dim ? __ldg(p.log_decay + th * p.dim + row0 + at(i)) : 0.f;
+                for (int i = 0; i < (MODE == LA_PER_CHANNEL ? RPL : 1); ++i) decay[i] = row0 + at(i) < p.dim ? p.log_decay[th * p.dim + row0 + at(i)] : 0.f;
             }
         }
         float q[RPL], k[RPL];
@@ -336,8 +336,8 @@ __global__ void __launch_bounds__(32 * LA_LANES) linear_attention_step_kernel(co
 #pragma unroll
             for (int i = 0; i < RPL; i += 4) {
                 const bool has = row0 + at(i) < p.dim;
-                const float4 q4 = has ? __ldg(reinterpret_cast<const float4*>(p.proj + q_at + at(i))) : make_float4(0.f, 0.f, 0.f, 0.f);
-                const float4 k4 = has ? __ldg(reinterpret_cast<const float4*>(p.proj + k_at + at(i))) : make_float4(0.f, 0.f, 0.f, 0.f);
+                const float4 q4 = has ? *reinterpret_cast<const float4*>(p.proj + q_at + at(i)) : make_float4(0.f, 0.f, 0.f, 0.f);
+                const float4 k4 = has ? *reinterpret_cast<const float4*>(p.proj + k_at + at(i)) : make_float4(0.f, 0.f, 0.f, 0.f);
                 q[i] = q4.x; q[i + 1] = q4.y; q[i + 2] = q4.z; q[i + 3] = q4.w;
                 k[i] = k4.x; k[i + 1] = k4.y; k[i + 2] = k4.z; k[i + 3] = k4.w;
             }
@@ -507,14 +507,14 @@ __global__ void __launch_bounds__(256) linear_attention_step_rows_kernel(const L
         float v[COLS];
 #pragma unroll
         for (int j = 0; j < Q; ++j) {
-            q[j] = __ldg(reinterpret_cast<const float4*>(row + p.at_q + key_head * DIM + 4 * (lane + LANES * j)));
-            k[j] = __ldg(reinterpret_cast<const float4*>(row + p.at_k + key_head * DIM + 4 * (lane + LANES * j)));
-            if (MODE == LA_PER_CHANNEL) d[j] = __ldg(reinterpret_cast<const float4*>(p.log_decay + th * DIM + 4 * (lane + LANES * j)));
+            q[j] = *reinterpret_cast<const float4*>(row + p.at_q + key_head * DIM + 4 * (lane + LANES * j));
+            k[j] = *reinterpret_cast<const float4*>(row + p.at_k + key_head * DIM + 4 * (lane + LANES * j));
+            if (MODE == LA_PER_CHANNEL) d[j] = *reinterpret_cast<const float4*>(p.log_decay + th * DIM + 4 * (lane + LANES * j));
         }
 #pragma unroll
-        for (int c = 0; c < COLS; ++c) v[c] = col0 + GROUPS * c < p.vdim ? __ldg(row + p.at_v + (size_t)head * p.vdim + col0 + GROUPS * c) : 0.f;
-        const float whole = MODE == LA_CONSTANT ? p.decay[head] : MODE == LA_PER_HEAD ? expf(__ldg(p.log_decay + th)) : 0.f;
-        const float factor = MODE != LA_CONSTANT && p.v_scale ? __ldg(p.v_scale + th) : 1.f;
+        for (int c = 0; c < COLS; ++c) v[c] = col0 + GROUPS * c < p.vdim ? row[p.at_v + (size_t)head * p.vdim + col0 + GROUPS * c] : 0.f;
+        const float whole = MODE == LA_CONSTANT ? p.decay[head] : MODE == LA_PER_HEAD ? expf(p.log_decay[th]) : 0.f;
+        const float factor = MODE != LA_CONSTANT && p.v_scale ? p.v_scale[th] : 1.f;
 #pragma unroll
         for (int j = 0; j < Q; ++j) {
             if (MODE == LA_PER_CHANNEL) d[j] = make_float4(expf(d[j].x), expf(d[j].y), expf(d[j].z), expf(d[j].w));
@@ -642,7 +642,7 @@ __device__ __forceinline__ float gn_gate_sum(const GroupNormParams& p, size_t t,
     for (int s0 = 0; s0 < p.n_splits; s0 += 8) {                        // eight loads of a split product's planes in flight
         float v[8];
 #pragma unroll
-        for (int j = 0; j < 8; ++j) v[j] = s0 + j < p.n_splits ? __ldg(at + (size_t)(s0 + j) * p.split_stride) : 0.f;
+        for (int j = 0; j < 8; ++j) v[j] = s0 + j < p.n_splits ? at[(size_t)(s0 + j) * p.split_stride] : 0.f;
 #pragma unroll
         for (int j = 0; j < 8; ++j) g += v[j];
     }
@@ -654,8 +654,8 @@ __device__ __forceinline__ float gn_gate_value(const GroupNormParams& p, float g
 }
 __device__ __forceinline__ float gn_gate(const GroupNormParams& p, size_t t, int i) { return gn_gate_value(p, gn_gate_sum(p, t, i)); }
 __device__ __forceinline__ float gn_value(const GroupNormParams& p, size_t t, int i) {
-    float y = __ldg(p.o + t * p.width + i);
-    if (p.x) y += __ldg(p.skip + i / p.per_skip) * __ldg(p.x + t * p.x_cols + p.at_x + i);
+    float y = p.o[t * p.width + i];
+    if (p.x) y += __ldg(p.skip + i / p.per_skip) * p.x[t * p.x_cols + p.at_x + i];
     return y;
 }
 
@@ -683,15 +683,15 @@ __global__ void __launch_bounds__(WARP ? 128 : 1024) group_gate_norm_kernel(cons
     for (int j = 0; j < GN_CACHE; ++j) {
         const int i = first + j * step;
         const bool in = i < p.part;
-        y[j] = in ? __ldg(o + i) : 0.f;
-        if (ONE_PLANE) gate[j] = in && g ? __ldg(g + i) : 0.f;
+        y[j] = in ? o[i] : 0.f;
+        if (ONE_PLANE) gate[j] = in && g ? g[i] : 0.f;
         else gate[j] = in && g ? gn_gate_sum(p, t, base + i) : 0.f;
     }
     if (x) {
 #pragma unroll
         for (int j = 0; j < GN_CACHE; ++j) {
             const int i = first + j * step;
-            if (i < p.part) y[j] = fmaf(__ldg(p.skip + (base + i) / p.per_skip), __ldg(x + i), y[j]);
+            if (i < p.part) y[j] = fmaf(__ldg(p.skip + (base + i) / p.per_skip), x[i], y[j]);
         }
     }
 #pragma unroll

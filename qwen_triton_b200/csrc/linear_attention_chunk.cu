@@ -60,12 +60,12 @@ __device__ __forceinline__ Chunk chunk_of(const ChunkArgs& p, int seq, int c) {
 
 // Four consecutive floats from p on, `left` of which exist (zeros beyond); one 16-byte load where `vec` says the address allows it.
 __device__ __forceinline__ float4 load4(const float* p, int left, bool vec) {
-    if (vec && left >= 4) return __ldg(reinterpret_cast<const float4*>(p));
+    if (vec && left >= 4) return *reinterpret_cast<const float4*>(p);
     float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (left > 0) v.x = __ldg(p);
-    if (left > 1) v.y = __ldg(p + 1);
-    if (left > 2) v.z = __ldg(p + 2);
-    if (left > 3) v.w = __ldg(p + 3);
+    if (left > 0) v.x = *p;
+    if (left > 1) v.y = p[1];
+    if (left > 2) v.z = p[2];
+    if (left > 3) v.w = p[3];
     return v;
 }
 __device__ __forceinline__ void put4(float* p, const float4& v, int left, bool vec) {
@@ -169,7 +169,7 @@ __global__ void __launch_bounds__(PC_THREADS, 2) chunk_prepare_channel_kernel(co
         const int r = i / dim4, n = i % dim4;
         float v[SUB];
 #pragma unroll
-        for (int j = 0; j < SUB; ++j) v[j] = n < dim && r * SUB + j < ck.count ? __ldg(g + (size_t)(r * SUB + j) * g_row + n) : 0.f;
+        for (int j = 0; j < SUB; ++j) v[j] = n < dim && r * SUB + j < ck.count ? g[(size_t)(r * SUB + j) * g_row + n] : 0.f;
         float sum = 0.f;
 #pragma unroll
         for (int j = 0; j < SUB; ++j) { sum += v[j]; qs[(r * SUB + j) * ld + n] *= expf(sum); }
@@ -392,7 +392,7 @@ __global__ void __launch_bounds__(PT_THREADS) chunk_write_kernel(const ChunkArgs
     tile_product<TN, false, false>(ck.count,
         [&](int s, int i) {
             const float4 x = load4(v + (size_t)s * p.cols + i, s < ck.count ? p.vdim - m0 - i : 0, vec_v);
-            return factor && s < ck.count ? times(x, __ldg(factor + (size_t)s * p.heads)) : x;
+            return factor && s < ck.count ? times(x, factor[(size_t)s * p.heads]) : x;
         },
         [&](int s, int i) { return load4(k + (size_t)s * k_row + i, s < ck.count ? p.dim - n0 - i : 0, vec_k); }, acc, xs, ys);
     const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
@@ -491,7 +491,7 @@ __global__ void __launch_bounds__(PT_THREADS) chunk_read_kernel(const ChunkArgs 
     tile_product<TN, false, false>(ck.count, [&](int s, int t) { return load4(within + s * CT + t, s < ck.count ? 4 : 0, true); },
         [&](int s, int i) {
             const float4 x = load4(v + (size_t)s * p.cols + i, s < ck.count ? p.vdim - m0 - i : 0, vec_v);
-            return factor && s < ck.count ? times(x, __ldg(factor + (size_t)s * p.heads)) : x;
+            return factor && s < ck.count ? times(x, factor[(size_t)s * p.heads]) : x;
         }, acc, xs, ys);
 #pragma unroll
     for (int i = 0; i < 8; ++i) {

@@ -36,7 +36,7 @@ __device__ __forceinline__ void for_each_logit(const float* __restrict__ row, in
 }
 
 // One block per row.
-__global__ void __launch_bounds__(SMP_THREADS) argmax_kernel(const float* __restrict__ logits, int* __restrict__ out, int vocab) {
+__global__ void __launch_bounds__(SMP_THREADS) argmax_kernel(const float* logits, int* __restrict__ out, int vocab) {
     pdl_launch_dependents();
     pdl_wait();
     __shared__ float best_v[32];
@@ -170,8 +170,8 @@ __device__ __forceinline__ int sample_row(const float* __restrict__ row, float i
     return chosen;
 }
 
-__global__ void __launch_bounds__(SMP_THREADS) sample_kernel(const float* __restrict__ logits, const float* __restrict__ temperature,
-                                                            const float* __restrict__ uniform, int* __restrict__ out, int vocab) {
+__global__ void __launch_bounds__(SMP_THREADS) sample_kernel(const float* logits, const float* temperature,
+                                                            const float* uniform, int* __restrict__ out, int vocab) {
     pdl_launch_dependents();
     pdl_wait();
     const float* row = logits + (size_t)blockIdx.x * vocab;
@@ -389,8 +389,8 @@ __device__ TopState list_threshold(const unsigned int* list_key, const unsigned 
 }
 
 template <bool TOP>
-__global__ void __launch_bounds__(SMP_THREADS) sample_keyed_kernel(const float* __restrict__ logits, float inv_t, unsigned long long seed,
-                                                                  const int* __restrict__ keys, int* __restrict__ out, int vocab,
+__global__ void __launch_bounds__(SMP_THREADS) sample_keyed_kernel(const float* logits, float inv_t, unsigned long long seed,
+                                                                  const int* keys, int* __restrict__ out, int vocab,
                                                                   int top_k, float top_p) {
     pdl_launch_dependents();
     pdl_wait();
@@ -497,7 +497,7 @@ extern "C" int qt_sample_keyed(const float* logits, float temperature, long long
 // ids[i] holds a row number of `chosen` (or a negative number); it is replaced by the token chosen for that row
 // (0 for a negative number or a row that does not exist).  With this the next step can be launched before the host
 // has seen the tokens.  Tokens outside the vocabulary (the sampling kernels produce none) are clamped into it.
-__global__ void feed_tokens_kernel(int* __restrict__ ids, const int* __restrict__ chosen, int n, int n_chosen, int vocab) {
+__global__ void feed_tokens_kernel(int* __restrict__ ids, const int* chosen, int n, int n_chosen, int vocab) {
     pdl_launch_dependents();
     pdl_wait();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;

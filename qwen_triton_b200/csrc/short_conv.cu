@@ -77,8 +77,8 @@ __global__ void __launch_bounds__(128) conv_qk_write_kernel(const ConvParams p) 
 }
 
 // One thread per (sequence, channel): it reads what it needs of the old rows before it writes.
-__global__ void conv_keep_kernel(const float* __restrict__ proj, int n_splits, size_t split_stride, int proj_cols,
-                                 float* __restrict__ kept, const int* __restrict__ seq_start, const int* __restrict__ slots,
+__global__ void conv_keep_kernel(const float* proj, int n_splits, size_t split_stride, int proj_cols,
+                                 float* __restrict__ kept, const int* seq_start, const int* slots,
                                  int channels, int n_taps) {
     pdl_launch_dependents();
     pdl_wait();
@@ -259,7 +259,7 @@ extern "C" int qt_conv_act(const float* proj, int n_splits, long long split_stri
 
 // ----------------------------------------------------------------------------- sigmoid gate on the heads' outputs
 template <typename T>
-__global__ void gate_mul_kernel(T* __restrict__ x, const float* __restrict__ gate, int n_splits, size_t split_stride, int gate_cols,
+__global__ void gate_mul_kernel(T* __restrict__ x, const float* gate, int n_splits, size_t split_stride, int gate_cols,
                                 int gate_offset, long long total, int cols, int group) {
     pdl_launch_dependents();
     pdl_wait();
