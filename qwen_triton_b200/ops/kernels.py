@@ -942,15 +942,22 @@ def decay_scratch(max_step_tokens: int, heads: int, dim: int, vdim: int, per_cha
             "q_from": max_step_tokens * heads * wide, "k_to": max_step_tokens * heads * wide}
 
 
-def decay_chunks_pay(ctx, tokens: int, dim: int, max_step_tokens: int) -> bool:
-    """Whether a recurrence with a constant decay per head runs in chunks: from a longest portion of 64 tokens on (1,024 for up to 64 key
-    channels), where the scratch for ``max_step_tokens`` holds the step's chunks.  Token by token a step takes a time that grows
-    with its longest portion and a column's rows, in chunks it is four kernels whatever the length.  16 heads of 128 x 128, token
-    by token / in chunks: 2,048 tokens 763 / 117 us, 200 tokens 79 / 48, 100 tokens 42 / 51, 5 x 90 tokens 85 / 61, 32 x 64 tokens
-    218 / 128, 32 x 24 tokens 96 / 101; error against 64 bits at 64 tokens 3.1e-7 / 2.3e-7, at 2,048 7.5e-7 / 2.7e-7.  8 heads of
-    64 x 128: 2,048 tokens 453 / 55 us and 2.4e-7 / 2.3e-7; 400 tokens 92 / 40 us, but 2.0e-7 / 2.2e-7: eight rows a lane and a
-    short walk round less than two sums over 64."""
-    return ctx.max_q_len >= (64 if dim > 64 else 1024) and tokens // DECAY_CHUNK + ctx.n_seqs <= decay_chunks(max_step_tokens)
+def decay_chunks_pay(ctx, tokens: int, heads: int, dim: int, vdim: int, max_step_tokens: int, sms: int) -> bool:
+    """Whether a recurrence with a constant decay per head runs in chunks, by the times of both forms in microseconds, where the scratch for
+    ``max_step_tokens`` holds the step's chunks.  Token by token the longest portion's chain counts (a shorter one where the columns are few
+    enough for a warp each), and the states' columns times tokens; in chunks four kernels, and the states of every chunk, of which a sequence has at
+    least one.  Measured token by token / in chunks, 16 heads of 128 x 128: 64 tokens 37 / 58 us, 100 47 / 59, 128 51 / 57, 150 57 / 57, 200 70 / 64, 400
+    122 / 69, 1,024 284 / 94, 5 x 90 102 / 84, 32 x 64 232 / 143, one of 64 beside 31 of 3 50 / 103, one of 300 beside them 123 / 123; 16 heads of 256 x 128: 64 tokens
+    62 / 71, 100 84 / 71.  Of 90 such mixes of 8 to 32 heads the rule takes the slower form five times, by 8 % at most.  Error against 64 bits,
+    16 heads of 128 x 128: 64 tokens 3.1e-7 / 2.3e-7, 2,048 7.5e-7 / 2.7e-7.  Up to 64 key channels only from 1,024 tokens on: 8 heads of 64 x 128, 2,048
+    tokens 2.4e-7 / 2.3e-7, but 400 tokens 2.0e-7 / 2.2e-7 (eight rows a lane and a short walk round less than two sums over 64)."""
+    longest = ctx.max_q_len
+    if longest < (64 if dim > 64 else 1024) or tokens // DECAY_CHUNK + ctx.n_seqs > decay_chunks(max_step_tokens):
+        return False
+    work = heads * dim * vdim / 2 ** 18
+    warp_a_column = -(-vdim // 16) * heads * ctx.n_seqs < 2 * sms
+    walk = 14.0 + (0.23 if warp_a_column else 0.35) * -(-dim // 128) * longest + 0.1 * work * tokens
+    return walk > 54.0 + 2.6 * work * max(ctx.n_seqs, tokens / DECAY_CHUNK)
 
 
 def decayed_attention(rows: GemmOut, at_q: int, at_k: int, at_v: int, log_decay: torch.Tensor, state: torch.Tensor, out: torch.Tensor, ctx,

@@ -296,7 +296,7 @@ class LinearAttention:
         read = ws.view("linattn.read", tokens, self.heads, self.vdim)
         # q, k and v are summed and activated once, not by every block of the recurrence that reads them
         ready = kernels.linear_attention_prepare(proj, self.at_gate, ws.view("linattn.qkv", tokens, self.at_gate), self.act)
-        if self.chunked and kernels.decay_chunks_pay(ctx, tokens, self.dim, self.runtime.max_step_tokens):
+        if self.chunked and kernels.decay_chunks_pay(ctx, tokens, self.heads, self.dim, self.vdim, self.runtime.max_step_tokens, self.runtime.sm_count):
             kernels.decayed_attention(ready, 0, self.at_k, self.at_v, self.log_decay[:tokens], cache.state, read, ctx, self.dim,
                                       _decay_scratch_views(self), impl="chunks")
         else:

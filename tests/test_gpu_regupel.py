@@ -427,7 +427,7 @@ def test_linear_attention_with_a_decay_per_head_in_portions(heads, dim, vdim):
 
 @pytest.mark.parametrize("heads, dim, vdim, decay", [(3, 64, 40, [0.5, 1.0, 0.9961]), (2, 36, 33, [1e-30, 0.25]), (2, 128, 128, [0.999, 0.0])])
 def test_long_portions_in_chunks_follow_the_token_by_token_walk(heads, dim, vdim, decay):
-    """The mixer at and around the length from which it runs in chunks (64 tokens, 1,024 of up to 64 key channels; never with a decay of 0), with
+    """The mixer at and around the length from which it may run in chunks (64 tokens, 1,024 of up to 64 key channels; never with a decay of 0), with
     sequences that end on, before and behind a chunk's edge and a state left by the portion before, against 64 bits: both forms round
     in 32 bits, so nothing may be off by more than 2e-5 of the largest value (a few hundred additions of 2^-24 each)."""
     from qwen_triton_b200.parts.base import Runtime, Workspace
@@ -453,6 +453,38 @@ def test_long_portions_in_chunks_follow_the_token_by_token_walk(heads, dim, vdim
     done = [0, 0, 0]
     for counts in portions:
         step = _Step(counts, done, [2, 0, 1])
+        got = mixer.forward(torch.cat([x[d:d + c] for x, d, c in zip(xs, done, counts)]).to(DEV), step, cache).value().cpu().double()
+        wanted = torch.cat([w[d:d + c] for w, d, c in zip(want, done, counts)])
+        assert float((got - wanted).abs().max()) < 2e-5 * float(wanted.abs().max())
+        done = [d + c for d, c in zip(done, counts)]
+
+
+def test_wide_heads_in_chunks_behind_a_walk():
+    """More than 64 key channels: a short portion token by token, a long one behind it in chunks, a short one again; one state, 64 bits, the bound
+    of the test above."""
+    from qwen_triton_b200.parts.base import Runtime, Workspace
+    from qwen_triton_b200.parts.recurrent import LinearAttention
+    torch.manual_seed(3)
+    heads, dim, vdim, decay = 3, 136, 40, [0.5, 0.999, 1.0]
+    runtime = Runtime(device=torch.device(DEV), dtype=torch.float32, max_step_tokens=1024, max_positions=64, workspace=Workspace(torch.device(DEV)))
+    mixer = LinearAttention({"hidden_size": 32, "num_heads": heads, "head_dim": dim, "v_head_dim": vdim, "decay": decay, "gate": False}, "m", runtime)
+    tensors = {name: torch.randn(*spec.shape) * 0.3 for name, spec in LinearAttention.expected_tensors(mixer.params, "m").items()}
+    tensors["m.norm"] = torch.ones(heads * vdim)
+    mixer.load(lambda name: tensors[name])
+    runtime.workspace.allocate()
+    cache = type("View", (), {})()
+    cache.writable, cache.state = True, torch.zeros(3, heads, vdim, dim, device=DEV)
+    portions, chunked = ([70, 3], [449, 400], [65, 1]), (False, True, False)
+    xs = [torch.randn(sum(p[s] for p in portions), 32) for s in range(2)]
+    want = []
+    for x in xs:
+        q, k, v = (plain.silu(x.double() @ tensors[f"m.{n}.weight"].double().T).view(len(x), heads, -1) for n in ("q", "k", "v"))
+        o = plain.decayed_linear_attention(q, k, v, torch.tensor(decay).double()).reshape(len(x), -1)
+        want.append(plain.rms_divide(o, 1e-6) @ tensors["m.o.weight"].double().T)
+    done = [0, 0]
+    for counts, form in zip(portions, chunked):
+        step = _Step(counts, done, [1, 0])
+        assert kernels.decay_chunks_pay(step, sum(counts), heads, dim, vdim, 1024, runtime.sm_count) == form
         got = mixer.forward(torch.cat([x[d:d + c] for x, d, c in zip(xs, done, counts)]).to(DEV), step, cache).value().cpu().double()
         wanted = torch.cat([w[d:d + c] for w, d, c in zip(want, done, counts)])
         assert float((got - wanted).abs().max()) < 2e-5 * float(wanted.abs().max())

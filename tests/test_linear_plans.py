@@ -80,3 +80,30 @@ def test_the_fused_ring_is_as_deep_as_keeps_every_block_resident():
     assert [stages(6144, 4096, "qkv"), stages(4096, 4096, "attn_out"), stages(24576, 4096, "gate"), stages(4096, 12288, "mlp_out")] == [4, 4, 4, 5]
     assert [stages(10240, 5120, "qkv"), stages(5120, 8192, "attn_out"), stages(5120, 25600, "mlp_out")] == [0, 4, 4]
     assert stages(4096, 4096, "") == 0
+
+
+# (heads, key channels, value columns, portions, token by token, in chunks): measured, microseconds with cold caches
+_RECURRENCES = [
+    (16, 128, 128, [64], 36.6, 58.2), (16, 128, 128, [100], 46.9, 58.7), (16, 128, 128, [128], 51.2, 56.5), (16, 128, 128, [200], 69.7, 63.8),
+    (16, 128, 128, [1024], 284.4, 94.1), (16, 128, 128, [64] * 2, 44.8, 59.4), (16, 128, 128, [90] * 5, 102.4, 84.3), (16, 128, 128, [64] * 32, 232.3, 142.9),
+    (16, 128, 128, [64] + [3] * 31, 49.6, 103.1), (16, 128, 128, [128] + [3] * 31, 66.5, 108.4), (16, 128, 128, [64] + [20] * 31, 103.1, 117.7),
+    (32, 128, 128, [64], 41.4, 56.3), (32, 128, 128, [100], 57.7, 72.7), (32, 128, 128, [200], 96.9, 77.6), (32, 128, 128, [300] + [3] * 31, 151.5, 212.8),
+    (8, 128, 128, [150], 50.8, 56.1), (8, 128, 128, [200], 61.9, 55.9), (8, 128, 128, [300] + [3] * 31, 116.8, 88.6), (8, 128, 128, [128] + [3] * 31, 61.7, 84.4),
+    (16, 256, 128, [64], 62.3, 70.8), (16, 256, 128, [100], 84.1, 71.3), (16, 96, 128, [100], 42.8, 52.4), (16, 96, 128, [400], 119.9, 69.9)]
+
+
+@pytest.mark.parametrize("heads, dim, vdim, lengths, walk, chunks", _RECURRENCES)
+def test_recurrences_take_the_faster_form(heads, dim, vdim, lengths, walk, chunks):
+    """A short prompt, or many short portions beside a long one, keeps the walk; no choice costs more than a tenth."""
+    from types import SimpleNamespace
+    step = SimpleNamespace(max_q_len=max(lengths), n_seqs=len(lengths))
+    taken = chunks if kernels.decay_chunks_pay(step, sum(lengths), heads, dim, vdim, 4096, 148) else walk
+    assert taken <= 1.1 * min(walk, chunks)
+
+
+def test_recurrences_walk_where_chunks_are_less_exact_or_do_not_fit():
+    from types import SimpleNamespace
+    step = SimpleNamespace(max_q_len=1000, n_seqs=1)
+    assert not kernels.decay_chunks_pay(step, 1000, 8, 64, 128, 4096, 148)          # up to 64 key channels
+    assert kernels.decay_chunks_pay(SimpleNamespace(max_q_len=1024, n_seqs=1), 1024, 8, 64, 128, 4096, 148)
+    assert not kernels.decay_chunks_pay(SimpleNamespace(max_q_len=2000, n_seqs=100), 2099, 16, 128, 128, 2100, 148)      # more sequences than the scratch has ends for
