@@ -40,8 +40,27 @@ from .base import DeferredProduct, KVRequest, Runtime, part_class, register_mixe
 from .linear import Linear
 
 
-_EXPAND_TOKENS = 64      # longest portion from which a prompt forms keys and values per head
+_EXPAND_TOKENS = 64      # longest portion from which a prompt may form keys and values per head
 _MANY_TOKENS = 256       # steps of more tokens form the queries and the cache rows in products of their own (without a query latent)
+
+
+def own_keys_pay(heads: int, d: int, rot: int, dv: int, rank: int, window: int | None, longest: int, n_seqs: int, tokens: int) -> bool:
+    """Whether keys and values of every head's own take less time than the latent rows in a step of prompts, the longest of ``longest`` tokens (64
+    and more; the others are taken as equal).  Over latent rows a query and key cost 2 rank + rot multiplications and a head and token rank (d + dv)
+    in products per head; over its own keys a third of the former, at the price of three more kernels, a product over every run of 64
+    rows, and blocks for every sequence and head.  Microseconds over rows / over its own, all products of the layer in: 16 heads of 128 + 64
+    over rows of 512 + 64: 2,048 tokens 519 / 166, 400 122 / 98, 64 59 / 59, 32 x 64 214 / 167, 8 x 64 91 / 93, 64 beside 31 x 3 63 / 99, beside 31 x 17
+    107 / 122; 128 such heads: 1,000 tokens 1,261 / 435, 64 beside 31 x 3 162 / 485; 8 heads of 64 + 32 over 256 + 32: 2,048 tokens 174 / 94, 64 32 / 41; 16
+    heads of 128 + 64 over 64 + 64: 2,048 tokens 227 / 143, 400 76 / 89, 32 x 64 115 / 142.  The factors are fitted to 210 such pairs, of which ten
+    take the slower form by more than 3 % (by 18 % at most)."""
+    if longest < _EXPAND_TOKENS:
+        return False
+    rest = (tokens - longest) / (n_seqs - 1) if n_seqs > 1 else 0.0
+    pairs = longest * min(longest, 2 * (window or longest)) + (tokens - longest) * min(rest, 2 * (window or longest))
+    key = 128 if d + rot <= 128 else 192
+    saved = 3.0e-9 * heads * pairs * (2 * rank + rot) + 2.2e-8 * heads * tokens * rank * (d + dv) + 3.0e-5 * longest * (2 * rank + rot) + 0.01 * longest + 4.7e-4 * heads * tokens
+    spent = 9.6 + 4.5e-9 * heads * 64 * (tokens // 64 + n_seqs) * (key + dv) * (rank + rot) + 0.032 * heads * n_seqs
+    return saved > spent
 
 
 @register_mixer("latent_attention")
@@ -207,14 +226,10 @@ class LatentAttention:
 
     # ------------------------------------------------------------------ run
     def _expands_for(self, ctx, tokens: int) -> bool:
-        """Whether a step forms keys and values per head: where all its sequences start at position 0, one of them is long enough and the
-        scratch holds their runs.  Over latent rows a query and key cost rank + rot and rank multiplications, over keys and values
-        of its own d + rot and dv (a third), at the price of one product over the step's tokens.  16 heads of
-        128 + 64 over rows of 512 + 64, two layers with their own products, over rows / over keys and values of its own: 2,000 tokens
-        1,001 / 294 us, 2 x 600 tokens 374 / 200, 32 x 100 tokens 617 / 395, one of 64 tokens 159 / 145; 32 x 32 tokens 238 / 238, 32 x 17 tokens
-        168 / 204.  8 heads of 64 + 32 over 256 + 32: 2,000 tokens 124 / 64 us, 32 x 100 tokens 90 / 60, 32 x 17 tokens 44 / 44."""
-        return (self.expands and getattr(ctx, "from_start", False) and not ctx.is_decode and ctx.max_q_len >= _EXPAND_TOKENS
-                and tokens // 64 + ctx.n_seqs <= self.most_runs)
+        """Whether a step forms keys and values per head: where all its sequences start at position 0, the scratch holds their runs and it
+        pays."""
+        return (self.expands and getattr(ctx, "from_start", False) and not ctx.is_decode and tokens // 64 + ctx.n_seqs <= self.most_runs
+                and own_keys_pay(self.heads, self.d, self.rot, self.dv, self.rank, self.window, ctx.max_q_len, ctx.n_seqs, tokens))
 
     def _over_own_keys(self, q_full, gate, gate_offset: int, ctx, cache, table):
         """[T, heads, dv]: attention over every head's own keys and values, made from the cached rows."""

@@ -220,13 +220,14 @@ class _Prompts:
     (128, 64, 64, 128, 512, 96, False, None, False), (64, 32, 32, 64, 256, 0, "head", 70, False), (120, 16, 16, 64, 40, 40, True, None, True),
     (136, 8, 0, 128, 64, 0, True, 33, False), (8, 64, 32, 64, 512, 0, False, 1, False), (128, 0, 0, 128, 256, 0, True, None, False)])
 @pytest.mark.parametrize("lengths", [(17, 1, 64, 65, 127), (128, 129), (300,)])
-def test_prompts_over_keys_and_values_per_head(d, rot, turning, dv, rank, q_rank, gate, window, interleaved, lengths):
+def test_prompts_over_keys_and_values_per_head(d, rot, turning, dv, rank, q_rank, gate, window, interleaved, lengths, monkeypatch):
     """A prompt's keys and values formed per head against the attention over latent rows and against 64 bits, around the edges of its
     runs (64) and tiles (128), with unused pages full of large numbers: no further off than the form over latent rows (by more than a
     tenth, for single draws), and within what five roundings to 8 bits on the way (2^-9 each, at most, twice that through sharp scores) leave."""
     from qwen_triton_b200.config.spec import PartSpec
     from qwen_triton_b200.parts import latent_attention as module
     from qwen_triton_b200.parts.base import Runtime, Workspace
+    monkeypatch.setattr(module, "own_keys_pay", lambda *sizes: True)          # sizes at which latent rows would be faster, too
     torch.manual_seed(d + rank)
     device, hidden, heads, scale = torch.device(DEV), 64, 3, (d + rot) ** -0.5
     runtime = Runtime(device=device, dtype=torch.bfloat16, max_step_tokens=512, max_positions=512, workspace=Workspace(device), page_tokens=64)
@@ -309,13 +310,18 @@ def _latent_mixer(tensors, dtype=torch.bfloat16, steps=512, **params):
 def _latent_prompts(mixer, x, lengths, expanded=True, ring=0, cache=None):
     """The mixer's results for prompts of these lengths, over keys and values per head or over latent rows."""
     width = ring // 64 or -(-max(lengths) // 64)
+    from qwen_triton_b200.parts import latent_attention
     step = _Prompts(list(lengths), width, list(reversed(range(width * len(lengths)))))
     step.from_start = expanded
+    rule, latent_attention.own_keys_pay = latent_attention.own_keys_pay, lambda *sizes: True        # sizes at which latent rows would be faster, too
     if cache is None:
         cache = type("View", (), {})()
         cache.k = torch.full((width * len(lengths), 1, 64, mixer.row), 1e4, dtype=x.dtype, device=DEV)
         cache.v, cache.page_tokens, cache.ring_tokens, cache.writable, cache.group = cache.k, 64, ring, True, 0
-    out = mixer.forward(x.to(DEV), step, cache).value().cpu()
+    try:
+        out = mixer.forward(x.to(DEV), step, cache).value().cpu()
+    finally:
+        latent_attention.own_keys_pay = rule
     kernels.check_status(torch.device(DEV))
     return out, cache
 

@@ -107,3 +107,31 @@ def test_recurrences_walk_where_chunks_are_less_exact_or_do_not_fit():
     assert not kernels.decay_chunks_pay(step, 1000, 8, 64, 128, 4096, 148)          # up to 64 key channels
     assert kernels.decay_chunks_pay(SimpleNamespace(max_q_len=1024, n_seqs=1), 1024, 8, 64, 128, 4096, 148)
     assert not kernels.decay_chunks_pay(SimpleNamespace(max_q_len=2000, n_seqs=100), 2099, 16, 128, 128, 2100, 148)      # more sequences than the scratch has ends for
+
+
+# (heads, d, rot, dv, rank, longest, sequences, tokens, over latent rows, over keys and values per head): measured, microseconds
+_LATENT_PROMPTS = [
+    (16, 128, 64, 128, 512, 64, 1, 64, 59.2, 58.7), (16, 128, 64, 128, 512, 400, 1, 400, 121.6, 97.5), (16, 128, 64, 128, 512, 1000, 1, 1000, 199.4, 117.2),
+    (16, 128, 64, 128, 512, 2048, 1, 2048, 518.5, 165.8), (16, 128, 64, 128, 512, 64, 8, 512, 91.0, 93.4), (16, 128, 64, 128, 512, 64, 32, 2048, 213.5, 166.5),
+    (16, 128, 64, 128, 512, 128, 16, 2048, 223.8, 142.6), (16, 128, 64, 128, 512, 64, 32, 157, 62.7, 99.1), (16, 128, 64, 128, 512, 64, 32, 591, 106.5, 121.7),
+    (16, 128, 64, 128, 512, 64, 32, 1056, 131.7, 133.9), (128, 128, 64, 128, 512, 64, 1, 64, 89.2, 88.2), (128, 128, 64, 128, 512, 400, 1, 400, 448.4, 255.1),
+    (128, 128, 64, 128, 512, 1000, 1, 1000, 1260.7, 435.4), (128, 128, 64, 128, 512, 64, 8, 512, 407.3, 323.0), (128, 128, 64, 128, 512, 64, 32, 157, 161.6, 485.3),
+    (128, 128, 64, 128, 512, 64, 32, 591, 482.6, 660.3), (8, 64, 32, 64, 256, 64, 1, 64, 32.0, 41.2), (8, 64, 32, 64, 256, 400, 1, 400, 80.4, 71.1),
+    (8, 64, 32, 64, 256, 1000, 1, 1000, 113.4, 79.9), (8, 64, 32, 64, 256, 2048, 1, 2048, 174.1, 94.1), (8, 64, 32, 64, 256, 64, 8, 512, 61.2, 65.2),
+    (8, 64, 32, 64, 256, 64, 32, 2048, 78.9, 73.5), (8, 64, 32, 64, 256, 128, 16, 2048, 84.6, 72.3), (8, 64, 32, 64, 256, 64, 32, 157, 42.4, 46.9),
+    (8, 64, 32, 64, 256, 64, 32, 591, 61.7, 63.8), (8, 64, 32, 64, 256, 64, 32, 1056, 65.3, 64.8), (16, 64, 32, 64, 64, 64, 1, 64, 28.9, 41.8),
+    (16, 64, 32, 64, 64, 400, 1, 400, 69.1, 73.2), (16, 64, 32, 64, 64, 1000, 1, 1000, 89.2, 80.4), (16, 64, 32, 64, 64, 2048, 1, 2048, 193.5, 105.2),
+    (16, 64, 32, 64, 64, 64, 8, 512, 58.0, 66.6), (16, 64, 32, 64, 64, 64, 32, 2048, 89.3, 96.2), (16, 64, 32, 64, 64, 128, 16, 2048, 93.2, 82.2),
+    (16, 64, 32, 64, 64, 64, 32, 157, 39.1, 62.9), (16, 64, 32, 64, 64, 64, 32, 591, 64.1, 82.8), (16, 64, 32, 64, 64, 64, 32, 1056, 66.4, 85.8),
+    (16, 128, 64, 128, 64, 64, 1, 64, 30.9, 47.3), (16, 128, 64, 128, 64, 400, 1, 400, 75.6, 88.8), (16, 128, 64, 128, 64, 1000, 1, 1000, 107.2, 104.3),
+    (16, 128, 64, 128, 64, 2048, 1, 2048, 227.3, 143.2), (16, 128, 64, 128, 64, 64, 8, 512, 64.0, 83.0), (16, 128, 64, 128, 64, 64, 32, 2048, 114.5, 141.9),
+    (16, 128, 64, 128, 64, 128, 16, 2048, 118.4, 119.6), (16, 128, 64, 128, 64, 64, 32, 157, 41.6, 83.6), (16, 128, 64, 128, 64, 64, 32, 591, 71.0, 108.8),
+    (16, 128, 64, 128, 64, 64, 32, 1056, 81.9, 118.3)]
+
+
+@pytest.mark.parametrize("heads, d, rot, dv, rank, longest, n_seqs, tokens, rows, own", _LATENT_PROMPTS)
+def test_latent_prompts_take_the_faster_form(heads, d, rot, dv, rank, longest, n_seqs, tokens, rows, own):
+    """Small latents, short prompts and short portions beside a long one keep the latent rows; no choice costs more than a fifth."""
+    from qwen_triton_b200.parts.latent_attention import own_keys_pay
+    taken = own if own_keys_pay(heads, d, rot, dv, rank, None, longest, n_seqs, tokens) else rows
+    assert taken <= 1.2 * min(rows, own)
