@@ -122,26 +122,27 @@ class Workspace:
                 self._buffers[name] = torch.empty(max(numel, 1), dtype=dtype, device=self.device)
         self._views.clear()
 
-    def view(self, name: str, *shape: int) -> torch.Tensor:
-        """The leading elements of a buffer in ``shape``.  Views are kept by (name, shape): a step asks for the same
-        few dozen again and again, and making one costs two tensor operations on the host."""
-        key = (name, shape)
+    def view(self, name: str, *shape: int, dtype: torch.dtype | None = None) -> torch.Tensor:
+        """The leading elements of a buffer in ``shape``, read as ``dtype`` (of the same size) where it is given.  Views are kept by (name, shape):
+        a step asks for the same few dozen again and again, and making one costs two tensor operations on the host."""
+        key = (name, shape, dtype)
         found = self._views.get(key)
         if found is not None:
             return found
         if len(self._views) >= 4096:
             self._views.clear()
-        found = self._views[key] = self._make_view(name, shape)
+        found = self._views[key] = self._make_view(name, shape, dtype)
         return found
 
-    def _make_view(self, name: str, shape: tuple[int, ...]) -> torch.Tensor:
+    def _make_view(self, name: str, shape: tuple[int, ...], dtype: torch.dtype | None) -> torch.Tensor:
         count = 1
         for dim in shape:
             count *= dim
         buffer = self._buffers[name]
         if count > buffer.numel():
             raise ValueError(f"workspace buffer {name!r} holds {buffer.numel()} elements, {count} wanted")
-        return buffer[:count].view(*shape)
+        buffer = buffer[:count].view(*shape)
+        return buffer if dtype is None or dtype == buffer.dtype else buffer.view(dtype)
 
     def bytes(self) -> int:
         return sum(b.numel() * b.element_size() for b in self._buffers.values())

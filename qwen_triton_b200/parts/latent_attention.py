@@ -106,8 +106,6 @@ class LatentAttention:
         tokens = runtime.max_step_tokens
         if self.q_rank:
             ws.declare("latent.cq", tokens * self.q_rank, runtime.dtype)
-        ws.declare("latent.q", tokens * self.heads * self.row, runtime.dtype)
-        ws.declare("latent.ctx", tokens * self.heads * self.rank, runtime.dtype)
         ws.declare("latent.heads", tokens * self.heads * self.dv, runtime.dtype)
         ws.declare("attn.part_acc", _MAX_SPLIT_PAIRS * self.heads * self.rank, torch.float32)
         ws.declare("attn.part_ml", _MAX_SPLIT_PAIRS * self.heads * 2, torch.float32)
@@ -116,12 +114,13 @@ class LatentAttention:
         self.key = 128 if self.d + self.rot <= 128 else 192                     # a head's query and key there, filled up with zeros
         self.expands = (runtime.dtype == torch.bfloat16 and runtime.page_tokens == 64 and self.d + self.rot <= 192 and self.dv in (64, 128) and self.scale > 0
                         and self.d % 8 == 0 and self.rot % 8 == 0 and turning % 16 == 0 and self.row % 8 == 0 and self.at_kv % 8 == 0)
-        self.most_runs = tokens // 64 + 64
+        self.most_runs = tokens // 64 + min(64, tokens // 32)      # of sequences of 32 tokens and more on average: fewer do not pay
+        # queries and results of the form over latent rows; a step takes one form, so the other's queries, keys and values lie there too
+        ws.declare("latent.q", tokens * self.heads * (max(self.row, self.key) if self.expands else self.row), runtime.dtype)
+        ws.declare("latent.ctx", max(tokens * self.heads * self.rank, 64 * self.most_runs * self.heads * (self.key + self.dv) if self.expands else 0), runtime.dtype)
         if self.expands:
             ws.declare("latent.rows", 64 * self.most_runs * self.row, runtime.dtype)
             ws.declare("latent.run_scale", 4 * self.most_runs, torch.float32)
-            ws.declare("latent.keys_values", 64 * self.most_runs * self.heads * (self.key + self.dv), torch.float16)
-            ws.declare("latent.queries", tokens * self.heads * self.key, torch.float16)
             ws.declare("latent.query_scale", tokens * self.heads, torch.float32)
         self.q_norm = self.kv_norm = self.uk_t = self.uv = self.expand = None
         self.key_norm = self.value_norm = 0.0                  # the largest sum of magnitudes over a row of W_uk, of W_uv (and 1 %)
@@ -238,9 +237,9 @@ class LatentAttention:
         rows = ws.view("latent.rows", count, self.row)
         run_scale = ws.view("latent.run_scale", count // 64, 4)
         kernels.latent_rows(cache.k, rows, run_scale, self.rank, self.key_norm, self.value_norm, table, ctx.seq_start, ctx.n_seqs, ctx.max_q_len, cache.page_tokens, cache.ring_tokens)
-        keys_values = ws.view("latent.keys_values", count, self.heads * (self.key + self.dv))
+        keys_values = ws.view("latent.ctx", count, self.heads * (self.key + self.dv), dtype=torch.float16)
         kernels.keys_and_values(rows, self.expand, keys_values, self.heads * self.key, run_scale)
-        q, q_scale = ws.view("latent.queries", tokens, self.heads, self.key), ws.view("latent.query_scale", tokens, self.heads)
+        q, q_scale = ws.view("latent.q", tokens, self.heads, self.key, dtype=torch.float16), ws.view("latent.query_scale", tokens, self.heads)
         kernels.latent_queries(q_full, self.cos_sin, ctx.token_pos, q, q_scale, self.d, self.rot)
         out = ws.view("latent.heads", tokens, self.heads, self.dv)
         kernels.attention_prefill_rows(q, q_scale, keys_values, run_scale, out, ctx.seq_start, ctx.n_seqs, ctx.max_q_len, self.window, self.scale,

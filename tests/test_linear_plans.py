@@ -135,3 +135,21 @@ def test_latent_prompts_take_the_faster_form(heads, d, rot, dv, rank, longest, n
     from qwen_triton_b200.parts.latent_attention import own_keys_pay
     taken = own if own_keys_pay(heads, d, rot, dv, rank, None, longest, n_seqs, tokens) else rows
     assert taken <= 1.2 * min(rows, own)
+
+
+@pytest.mark.parametrize("heads, tokens", [(16, 4096), (128, 4096), (16, 256)])
+def test_latent_prompts_need_little_memory_of_their_own(heads, tokens):
+    """Queries, keys and values per head lie where the form over latent rows has its queries and results (a step takes one of the two): a fifth
+    more than that form alone at most."""
+    from qwen_triton_b200.config.spec import PartSpec
+    from qwen_triton_b200.parts.base import Runtime, Workspace
+    from qwen_triton_b200.parts.latent_attention import LatentAttention
+    params = {"hidden_size": 2048, "num_heads": heads, "head_dim": 128, "rot_dim": 64, "v_head_dim": 128, "q_rank": 768, "kv_rank": 512, "scale": 0.07,
+              "position": PartSpec("rope", {"theta": 1e4, "rotary_dim": 64, "head_dim": 64, "pairing": "half"})}
+    sizes = []
+    for page in (64, 128):                  # pages of 64: the form exists
+        runtime = Runtime(device=torch.device("cpu"), dtype=torch.bfloat16, max_step_tokens=tokens, max_positions=tokens, workspace=Workspace(torch.device("cpu")),
+                          page_tokens=page, sm_count=148)
+        assert LatentAttention(params, "m", runtime).expands == (page == 64)
+        sizes.append(sum(numel * dtype.itemsize for name, (numel, dtype) in runtime.workspace._need.items() if name.startswith("latent.")))
+    assert sizes[0] <= 1.2 * sizes[1], sizes
