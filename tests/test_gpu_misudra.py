@@ -346,6 +346,18 @@ def test_prompts_over_keys_and_values_per_head_keep_the_range(q_rank, scores, va
     assert bool(torch.isfinite(want).all()) and torch.equal(got, want)
 
 
+@pytest.mark.parametrize("window, chunk", [(100, 128), (1, 64), (65, 192)])
+def test_prompts_over_keys_and_values_per_head_in_a_ring(window, chunk):
+    """A windowed group's ring of pages, its block table cut to them, and a portion as long as the ring is made for: the bits of the same prompts
+    in pages of their own."""
+    torch.manual_seed(window)
+    mixer, _ = _latent_mixer(None, num_heads=3, head_dim=64, rot_dim=32, v_head_dim=64, kv_rank=128, q_rank=48, gate="head", window=window)
+    lengths = (chunk, 64, 5)
+    x = torch.randn(sum(lengths), 64).bfloat16()
+    ring = -(-(window + chunk - 1) // 64) * 64
+    assert torch.equal(_latent_prompts(mixer, x, lengths, ring=ring)[0], _latent_prompts(mixer, x, lengths)[0])
+
+
 @pytest.mark.parametrize("spread", [0, 6, 12])
 def test_prompts_over_keys_and_values_per_head_of_uneven_tokens(spread):
     """Tokens whose queries and shared key parts differ by up to 2^(2 spread), side by side in runs of 64, against the 32-bit mixer: no further
