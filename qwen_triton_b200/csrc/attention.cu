@@ -184,12 +184,8 @@ __global__ void __launch_bounds__(PF_WARPS * 32) attention_prefill_kernel(const 
 template <typename T, int DMAX>
 static int launch_prefill(const AttnParams& p, int max_q_len, cudaStream_t stream) {
     const size_t smem = ((size_t)PF_BQ * p.d + (size_t)PF_BK * (p.d + 1) + (size_t)PF_BK * p.dv + PF_BQ * PF_BK) * sizeof(float);
-    static bool configured = false;
-    if (!configured) {
-        cudaError_t err = cudaFuncSetAttribute(attention_prefill_kernel<T, DMAX>, cudaFuncAttributeMaxDynamicSharedMemorySize, (DMAX > 256 ? 200 : 100) * 1024);
-        if (err != cudaSuccess) QT_FAIL(QT_ERR_LAUNCH, "attention_prefill: cannot raise shared memory: %s", cudaGetErrorString(err));
-        configured = true;
-    }
+    const cudaError_t raised = raise_shared<attention_prefill_kernel<T, DMAX>>((DMAX > 256 ? 200 : 100) * 1024);
+    if (raised != cudaSuccess) QT_FAIL(QT_ERR_LAUNCH, "attention_prefill: cannot raise shared memory: %s", cudaGetErrorString(raised));
     dim3 grid((max_q_len + PF_BQ - 1) / PF_BQ, p.nq, p.n_seqs);
     launch_kernel(attention_prefill_kernel<T, DMAX>, dim3(grid), dim3(PF_WARPS * 32), smem, stream, p);
     QT_CHECK_LAUNCH("attention_prefill");
@@ -409,12 +405,8 @@ static bool prefill_f32_fits(const AttnParams& p) {
 
 static int launch_prefill_f32(const AttnParams& p, int max_q_len, cudaStream_t stream) {
     const size_t smem = ((size_t)(AF_BQ + AF_BK) * (p.d + 4) + (size_t)AF_BK * p.dv + (size_t)AF_BQ * (AF_BK + 4)) * sizeof(float);
-    static bool configured = false;
-    if (!configured) {
-        cudaError_t err = cudaFuncSetAttribute(attention_prefill_f32_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 100 * 1024);
-        if (err != cudaSuccess) QT_FAIL(QT_ERR_LAUNCH, "attention_prefill: cannot raise shared memory: %s", cudaGetErrorString(err));
-        configured = true;
-    }
+    const cudaError_t raised = raise_shared<attention_prefill_f32_kernel>(100 * 1024);
+    if (raised != cudaSuccess) QT_FAIL(QT_ERR_LAUNCH, "attention_prefill: cannot raise shared memory: %s", cudaGetErrorString(raised));
     launch_kernel(attention_prefill_f32_kernel, dim3((max_q_len + AF_BQ - 1) / AF_BQ, p.nq, p.n_seqs), dim3(AF_THREADS), smem, stream, p);
     QT_CHECK_LAUNCH("attention_prefill");
     return QT_OK;
@@ -684,12 +676,8 @@ template <typename T, int DMAX, int DEC_HEADS>
 static int launch_decode_heads(const DecodeParams& dp, cudaStream_t stream) {
     const AttnParams& p = dp.a;
     const size_t smem = ((size_t)DEC_HEADS * p.d + (size_t)DEC_WARPS * DEC_HEADS * p.dv + DEC_WARPS * DEC_HEADS * 2) * sizeof(float);
-    static bool configured = false;
-    if (!configured) {
-        cudaError_t err = cudaFuncSetAttribute(attention_decode_kernel<T, DMAX, DEC_HEADS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (DMAX > 256 ? 100 : 64) * 1024);
-        if (err != cudaSuccess) QT_FAIL(QT_ERR_LAUNCH, "attention_decode: cannot raise shared memory: %s", cudaGetErrorString(err));
-        configured = true;
-    }
+    const cudaError_t raised = raise_shared<attention_decode_kernel<T, DMAX, DEC_HEADS>>((DMAX > 256 ? 100 : 64) * 1024);
+    if (raised != cudaSuccess) QT_FAIL(QT_ERR_LAUNCH, "attention_decode: cannot raise shared memory: %s", cudaGetErrorString(raised));
     const int group = p.nq / p.nkv;
     dim3 grid(dp.n_splits, p.nkv * ((group + DEC_HEADS - 1) / DEC_HEADS), p.n_seqs);
     launch_kernel(attention_decode_kernel<T, DMAX, DEC_HEADS>, dim3(grid), dim3(DEC_WARPS * 32), smem, stream, dp);

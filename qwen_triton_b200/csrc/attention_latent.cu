@@ -336,9 +336,9 @@ __global__ void __launch_bounds__(LT_THREADS, 1) latent_attention_kernel(const L
     }
 }
 
-template <typename K>
-int raise_smem(K kernel, size_t bytes, const char* name) {
-    cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+template <auto KERNEL>
+int raise_smem(size_t bytes, const char* name) {
+    const cudaError_t err = raise_shared<KERNEL>((int)bytes);
     if (err != cudaSuccess) QT_FAIL(QT_ERR_LAUNCH, "%s: cannot raise shared memory to %zu: %s", name, bytes, cudaGetErrorString(err));
     return QT_OK;
 }
@@ -376,8 +376,8 @@ extern "C" int qt_attention_latent(const void* q, const void* cache, void* out, 
     int rc;
 #define QT_LAUNCH_LATENT_KP(NT, KP)                                                                                       \
     do {                                                                                                                 \
-        static bool ok = false;                                                                                          \
-        if (!ok) { rc = raise_smem(latent_attention_kernel<NT, KP>, 227 * 1024, "attention_latent"); if (rc) return rc; ok = true; } \
+        rc = raise_smem<latent_attention_kernel<NT, KP>>(227 * 1024, "attention_latent"); \
+        if (rc) return rc; \
         launch_kernel(latent_attention_kernel<NT, KP>, grid, dim3(LT_THREADS), smem, s, p);                               \
     } while (0)
 #define QT_LAUNCH_LATENT(NT)                                                                                              \

@@ -45,9 +45,9 @@ int decode_stages() {
     return stages;
 }
 
-template <typename K>
-int raise_smem(K kernel, size_t bytes, const char* name) {
-    cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+template <auto KERNEL>
+int raise_smem(size_t bytes, const char* name) {
+    const cudaError_t err = raise_shared<KERNEL>((int)bytes);
     if (err != cudaSuccess) QT_FAIL(QT_ERR_LAUNCH, "%s: cannot raise shared memory to %zu: %s", name, bytes, cudaGetErrorString(err));
     return QT_OK;
 }
@@ -75,12 +75,12 @@ extern "C" int qt_attention_decode_mma(const void* q, const void* k_cache, const
     dim3 grid(n_splits, nkv * ((group + 15) / 16), n_seqs);
     cudaStream_t s = (cudaStream_t)stream;
     if (d <= 64) {
-        static bool ok = false;
-        if (!ok) { rc = raise_smem(attention_decode_mma_kernel<64>, 100 * 1024, "attention_decode_mma"); if (rc) return rc; ok = true; }
+        rc = raise_smem<attention_decode_mma_kernel<64>>(100 * 1024, "attention_decode_mma");
+        if (rc) return rc;
         launch_kernel(attention_decode_mma_kernel<64>, dim3(grid), dim3(128), smem, s, p);
     } else {
-        static bool ok = false;
-        if (!ok) { rc = raise_smem(attention_decode_mma_kernel<128>, 128 * 1024, "attention_decode_mma"); if (rc) return rc; ok = true; }
+        rc = raise_smem<attention_decode_mma_kernel<128>>(128 * 1024, "attention_decode_mma");
+        if (rc) return rc;
         launch_kernel(attention_decode_mma_kernel<128>, dim3(grid), dim3(128), smem, s, p);
     }
     QT_CHECK_LAUNCH("attention_decode_mma");
@@ -129,8 +129,8 @@ extern "C" int qt_attention_decode_ws(const void* q, const void* k_cache, const 
     cudaStream_t s = (cudaStream_t)stream;
 #define QT_LAUNCH_WS(DMAX, EXACT, PEN, CAP)                                                                              \
     do {                                                                                                                 \
-        static bool ok = false;                                                                                          \
-        if (!ok) { rc = raise_smem(attention_decode_ws_kernel<DMAX, EXACT, PEN, CAP>, 227 * 1024, "attention_decode_ws"); if (rc) return rc; ok = true; } \
+        rc = raise_smem<attention_decode_ws_kernel<DMAX, EXACT, PEN, CAP>>(227 * 1024, "attention_decode_ws"); \
+        if (rc) return rc; \
         if (cluster) launch_kernel_cluster(attention_decode_ws_kernel<DMAX, EXACT, PEN, CAP>, grid, block, smem, s, (unsigned)n_splits, p); \
         else launch_kernel(attention_decode_ws_kernel<DMAX, EXACT, PEN, CAP>, grid, block, smem, s, p);                        \
     } while (0)
@@ -178,8 +178,8 @@ extern "C" int qt_attention_prefill_mma(const void* q, const void* k_cache, cons
     cudaStream_t s = (cudaStream_t)stream;
 #define QT_LAUNCH_PF(DMAX, PEN, CAP)                                                                                     \
     do {                                                                                                                 \
-        static bool ok = false;                                                                                          \
-        if (!ok) { rc = raise_smem(attention_prefill_mma_kernel<DMAX, PEN, CAP>, 100 * 1024, "attention_prefill_mma"); if (rc) return rc; ok = true; } \
+        rc = raise_smem<attention_prefill_mma_kernel<DMAX, PEN, CAP>>(100 * 1024, "attention_prefill_mma"); \
+        if (rc) return rc; \
         launch_kernel(attention_prefill_mma_kernel<DMAX, PEN, CAP>, dim3(grid), dim3(128), smem, s, p);                  \
     } while (0)
 #define QT_LAUNCH_PF_SIZE(PEN, CAP)                  \

@@ -542,12 +542,8 @@ int launch(const CUtensorMap& map_q, const CUtensorMap& map_k, const CUtensorMap
     // Q, two key tiles, the value tiles, alignment slack, barriers
     const size_t smem = (size_t)(HD / 64) * HALF_BYTES + 2 * (size_t)(HD / 64) * BKEY * 128 + (HD > 128 ? 1 : 2) * (size_t)(HDV / 64) * BKEY * 128 + ALIGN_SLACK<HD> +
                         128 + 64;
-    static bool configured = false;
-    if (!configured) {
-        cudaError_t err = cudaFuncSetAttribute(attention_prefill_tc_kernel<HD, HDV, BKEY, PEN, CAP, DENSE, KEEP>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
-        if (err != cudaSuccess) QT_FAIL(QT_ERR_LAUNCH, "attention_prefill_tc: cannot raise shared memory: %s", cudaGetErrorString(err));
-        configured = true;
-    }
+    const cudaError_t raised = raise_shared<attention_prefill_tc_kernel<HD, HDV, BKEY, PEN, CAP, DENSE, KEEP>>(227 * 1024);
+    if (raised != cudaSuccess) QT_FAIL(QT_ERR_LAUNCH, "attention_prefill_tc: cannot raise shared memory: %s", cudaGetErrorString(raised));
     dim3 grid(p.nq, (max_q_len + BQ - 1) / BQ, n_seqs);
     launch_kernel(attention_prefill_tc_kernel<HD, HDV, BKEY, PEN, CAP, DENSE, KEEP>, grid, dim3(THREADS), smem, stream, map_q, map_k, map_v, p);
     QT_CHECK_LAUNCH("attention_prefill_tc");

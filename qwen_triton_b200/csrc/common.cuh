@@ -72,6 +72,18 @@ inline int sm_count() {
     return counts[device];
 }
 
+// Lets a kernel ask for up to `bytes` of dynamic shared memory.  The runtime keeps that per device; it is told once per device and thread.
+template <auto KERNEL> inline cudaError_t raise_shared(int bytes) {
+    static thread_local int raised[64] = {};
+    int device = 0;
+    cudaError_t err = cudaGetDevice(&device);
+    if (err == cudaSuccess && (device < 0 || device >= 64)) err = cudaErrorInvalidDevice;
+    if (err != cudaSuccess || raised[device] >= bytes) return err;
+    err = cudaFuncSetAttribute(KERNEL, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    if (err == cudaSuccess) raised[device] = bytes;
+    return err;
+}
+
 inline bool pdl_enabled() {
     static int enabled = -1;
     if (enabled < 0) {

@@ -987,12 +987,8 @@ extern "C" int qt_lowrank(const float* proj, int n_splits, long long split_strid
 template <int R>
 static int launch_scan(const ScanParams& p, int n_seqs, cudaStream_t s) {
     const size_t smem = 2 * (size_t)SCAN_CHUNK * (3 * p.dim + SCAN_COLS + 1) * sizeof(float);
-    static bool configured = false;
-    if (!configured) {
-        cudaError_t err = cudaFuncSetAttribute(delta_scan_kernel<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, 208 * 1024);
-        if (err != cudaSuccess) QT_FAIL(QT_ERR_LAUNCH, "delta_scan: cannot raise shared memory: %s", cudaGetErrorString(err));
-        configured = true;
-    }
+    const cudaError_t raised = raise_shared<delta_scan_kernel<R>>(208 * 1024);
+    if (raised != cudaSuccess) QT_FAIL(QT_ERR_LAUNCH, "delta_scan: cannot raise shared memory: %s", cudaGetErrorString(raised));
     launch_kernel(delta_scan_kernel<R>, dim3((p.vdim + SCAN_COLS - 1) / SCAN_COLS, p.heads, n_seqs), dim3(SCAN_COLS * SCAN_LANES), smem, s, p);
     QT_CHECK_LAUNCH("delta_scan");
     return QT_OK;
@@ -1023,12 +1019,8 @@ extern "C" int qt_delta_scan(const float* q, const float* k, const float* v, con
 template <int R>
 static int launch_chunk_scan(const ChunkScanParams& p, int n_seqs, cudaStream_t s) {
     const size_t smem = 2 * ((size_t)CH * (3 * p.dim + 2 * CH + SCAN_COLS + 1) + p.dim) * sizeof(float);
-    static bool configured = false;
-    if (!configured) {
-        cudaError_t err = cudaFuncSetAttribute(delta_chunk_scan_kernel<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024);
-        if (err != cudaSuccess) QT_FAIL(QT_ERR_LAUNCH, "delta_chunk_scan: cannot raise shared memory: %s", cudaGetErrorString(err));
-        configured = true;
-    }
+    const cudaError_t raised = raise_shared<delta_chunk_scan_kernel<R>>(220 * 1024);
+    if (raised != cudaSuccess) QT_FAIL(QT_ERR_LAUNCH, "delta_chunk_scan: cannot raise shared memory: %s", cudaGetErrorString(raised));
     QT_REQUIRE(smem <= 220 * 1024, "delta_chunk_scan: %d key channels per head need more shared memory than a block has", p.dim);
     launch_kernel(delta_chunk_scan_kernel<R>, dim3((p.vdim + SCAN_COLS - 1) / SCAN_COLS, p.heads, n_seqs), dim3(SCAN_COLS * SCAN_LANES), smem, s, p);
     QT_CHECK_LAUNCH("delta_chunk_scan");
@@ -1038,12 +1030,8 @@ static int launch_chunk_scan(const ChunkScanParams& p, int n_seqs, cudaStream_t 
 template <int P>
 static int launch_chunk_walk(const ChunkScanParams& p, int n_seqs, cudaStream_t s) {
     const size_t smem = 2 * ((size_t)CH * (3 * 64 * P + AB + WALK_COLS) + 64 * P) * sizeof(float);
-    static bool configured = false;
-    if (!configured) {
-        cudaError_t err = cudaFuncSetAttribute(delta_chunk_walk_kernel<P>, cudaFuncAttributeMaxDynamicSharedMemorySize, 120 * 1024);
-        if (err != cudaSuccess) QT_FAIL(QT_ERR_LAUNCH, "delta_chunk_walk: cannot raise shared memory: %s", cudaGetErrorString(err));
-        configured = true;
-    }
+    const cudaError_t raised = raise_shared<delta_chunk_walk_kernel<P>>(120 * 1024);
+    if (raised != cudaSuccess) QT_FAIL(QT_ERR_LAUNCH, "delta_chunk_walk: cannot raise shared memory: %s", cudaGetErrorString(raised));
     // Blocks start while the kernel before still runs on most SMs; as much shared memory as it takes to keep them from piling up on
     // the first SMs that fall free (646 us in place of 255 us where two or three share an SM and others stand idle).
     const long long blocks = (long long)(p.vdim / WALK_COLS) * p.heads * n_seqs, per_sm = (blocks + sm_count() - 1) / sm_count();
@@ -1070,14 +1058,9 @@ extern "C" int qt_delta_scan_chunked(const float* q, const float* k, const float
     const bool walk = !plain_only && aligned && dim % 64 == 0 && dim <= 256 && vdim % WALK_COLS == 0;
     ChunkParams cp{q, k, log_decay, kt, qt, kb, gc, beta, ab, seq_start, heads, kv_heads, dim, walk ? 1 : 0};
     const size_t smem = 4 * (size_t)CH * dim * sizeof(float);
-    static bool configured = false;
-    if (!configured) {
-        cudaError_t err = cudaFuncSetAttribute(delta_chunk_prepare_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * 1024);
-        if (err == cudaSuccess) err = cudaFuncSetAttribute(delta_chunk_prepare_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * 1024);
-        if (err != cudaSuccess) QT_FAIL(QT_ERR_LAUNCH, "delta_chunk_prepare: cannot raise shared memory: %s", cudaGetErrorString(err));
-        configured = true;
-    }
     const bool fours = dim % 4 == 0 && (((uintptr_t)q | (uintptr_t)k | (uintptr_t)log_decay) & 15) == 0;
+    const cudaError_t raised = fours ? raise_shared<delta_chunk_prepare_kernel<4>>(64 * 1024) : raise_shared<delta_chunk_prepare_kernel<1>>(64 * 1024);
+    if (raised != cudaSuccess) QT_FAIL(QT_ERR_LAUNCH, "delta_chunk_prepare: cannot raise shared memory: %s", cudaGetErrorString(raised));
     const dim3 chunk_grid((max_tokens + CH - 1) / CH, heads, n_seqs);
     if (fours) launch_kernel(delta_chunk_prepare_kernel<4>, chunk_grid, dim3(128), smem, s, cp);
     else launch_kernel(delta_chunk_prepare_kernel<1>, chunk_grid, dim3(128), smem, s, cp);

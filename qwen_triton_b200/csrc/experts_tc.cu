@@ -296,12 +296,8 @@ int launch_persistent(const void* x, const void* w, TO* out, const int* tile_exp
     rc = tensor_map(&map_w, w, (uint64_t)experts * n_out, (uint64_t)K, PBN);
     if (rc) return rc;
     const size_t smem = (size_t)PSTAGES * P_STAGE_BYTES + 1024 + (2 * PSTAGES + 4) * 8 + 16;
-    static bool configured = false;
-    if (!configured) {
-        cudaError_t err = cudaFuncSetAttribute(expert_gemm_persistent_kernel<TO, ACT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (err != cudaSuccess) QT_FAIL(QT_ERR_LAUNCH, "expert_gemm: cannot raise shared memory: %s", cudaGetErrorString(err));
-        configured = true;
-    }
+    const cudaError_t raised = raise_shared<expert_gemm_persistent_kernel<TO, ACT>>((int)smem);
+    if (raised != cudaSuccess) QT_FAIL(QT_ERR_LAUNCH, "expert_gemm: cannot raise shared memory: %s", cudaGetErrorString(raised));
     const int w_tiles = (n_out + PBN - 1) / PBN, kb_total = (K + BK - 1) / BK;
     const long long items = (long long)max_tiles * w_tiles;
     QT_REQUIRE(items < (1ll << 31), "expert_gemm: too many tiles for one launch");
@@ -422,12 +418,8 @@ int launch_few(const void* x, const void* w, __nv_bfloat16* out, const int* tile
     rc = tensor_map(&map_w, w, (uint64_t)experts * n_out, (uint64_t)K, BM);
     if (rc) return rc;
     const size_t smem = (size_t)FEW_STAGES * FEW_STAGE_BYTES + 1024 + (2 * FEW_STAGES + 1) * 8 + 16;
-    static bool configured = false;
-    if (!configured) {
-        cudaError_t err = cudaFuncSetAttribute(expert_gemm_few_kernel<ACT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (err != cudaSuccess) QT_FAIL(QT_ERR_LAUNCH, "expert_gemm: cannot raise shared memory: %s", cudaGetErrorString(err));
-        configured = true;
-    }
+    const cudaError_t raised = raise_shared<expert_gemm_few_kernel<ACT>>((int)smem);
+    if (raised != cudaSuccess) QT_FAIL(QT_ERR_LAUNCH, "expert_gemm: cannot raise shared memory: %s", cudaGetErrorString(raised));
     const int w_tiles = (n_out + BM - 1) / BM, kb_total = (K + BK - 1) / BK;
     QT_REQUIRE((long long)max_tiles * w_tiles < (1ll << 31), "expert_gemm: too many tiles for one launch");
     launch_kernel(expert_gemm_few_kernel<ACT>, dim3((unsigned)(max_tiles * w_tiles)), dim3(THREADS), smem, stream, map_x, map_w, out, tile_expert, n_out, kb_total,
@@ -445,12 +437,8 @@ int launch_tile(const void* x, const void* w, TO* out, const int* tile_expert, i
     rc = tensor_map(&map_w, w, (uint64_t)experts * n_out, (uint64_t)K, BN);
     if (rc) return rc;
     const size_t smem = (size_t)STAGES * (A_BYTES + BN * BK * 2) + 1024 + (2 * STAGES + 1) * 8 + 16;
-    static bool configured = false;
-    if (!configured) {
-        cudaError_t err = cudaFuncSetAttribute(expert_gemm_kernel<TO, ACT, BN, STAGES>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (err != cudaSuccess) QT_FAIL(QT_ERR_LAUNCH, "expert_gemm: cannot raise shared memory: %s", cudaGetErrorString(err));
-        configured = true;
-    }
+    const cudaError_t raised = raise_shared<expert_gemm_kernel<TO, ACT, BN, STAGES>>((int)smem);
+    if (raised != cudaSuccess) QT_FAIL(QT_ERR_LAUNCH, "expert_gemm: cannot raise shared memory: %s", cudaGetErrorString(raised));
     const int w_tiles = (n_out + BN - 1) / BN, kb_total = (K + BK - 1) / BK;
     QT_REQUIRE((long long)max_tiles * w_tiles < (1ll << 31), "expert_gemm: too many tiles for one launch");
     launch_kernel(expert_gemm_kernel<TO, ACT, BN, STAGES>, dim3((unsigned)(max_tiles * w_tiles)), dim3(THREADS), smem, stream, map_x, map_w, out,

@@ -151,14 +151,8 @@ __global__ void __launch_bounds__(GF_THREADS, 2) gemm_f32_tile_kernel(const floa
 template <int TM>
 int launch_tiles(const float* a, const float* w, float* c, int M, int N, int K, cudaStream_t s) {
     constexpr int SMEM = GF_STAGES * (8 * TM + GF_BN) * GF_ROW * 4;
-    static thread_local bool opted[64] = {};
-    int device = 0;
-    if (cudaGetDevice(&device) != cudaSuccess || device < 0 || device >= 64) QT_FAIL(QT_ERR_LAUNCH, "gemm_f32: no current device");
-    if (!opted[device]) {
-        if (cudaFuncSetAttribute(gemm_f32_tile_kernel<TM>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM) != cudaSuccess)
-            QT_FAIL(QT_ERR_LAUNCH, "gemm_f32: %d bytes of shared memory: %s", SMEM, cudaGetErrorString(cudaGetLastError()));
-        opted[device] = true;
-    }
+    const cudaError_t raised = raise_shared<gemm_f32_tile_kernel<TM>>(SMEM);
+    if (raised != cudaSuccess) QT_FAIL(QT_ERR_LAUNCH, "gemm_f32: %d bytes of shared memory: %s", SMEM, cudaGetErrorString(raised));
     const long long tiles_n = (N + GF_BN - 1) / GF_BN, tiles_m = (M + 8 * TM - 1) / (8 * TM), slices = (K + GF_BK - 1) / GF_BK;
     QT_REQUIRE(tiles_m <= 65535, "gemm_f32: M=%d is too large for one launch", M);
     const int slots = 2 * sm_count();

@@ -235,12 +235,8 @@ int launch(const CUtensorMap& map_w, const CUtensorMap& map_x, FusedParams p, in
     if (stages < 2) stages = 2;
     p.stages = stages;
     const size_t smem = (size_t)stages * STAGE_BYTES + 1024 + (2 * stages + 1) * 8 + 16;
-    static bool configured = false;
-    if (!configured) {
-        cudaError_t err = cudaFuncSetAttribute(gemm_fused_kernel<BX, EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
-        if (err != cudaSuccess) QT_FAIL(QT_ERR_LAUNCH, "gemm_fused: cannot raise shared memory: %s", cudaGetErrorString(err));
-        configured = true;
-    }
+    const cudaError_t raised = raise_shared<gemm_fused_kernel<BX, EPI>>(227 * 1024);
+    if (raised != cudaSuccess) QT_FAIL(QT_ERR_LAUNCH, "gemm_fused: cannot raise shared memory: %s", cudaGetErrorString(raised));
     dim3 grid(((p.e.N + BW - 1) / BW) * p.splits, (p.e.M + BX - 1) / BX, 1);
     launch_kernel_cluster(gemm_fused_kernel<BX, EPI>, grid, dim3(THREADS), smem, stream, (unsigned)p.splits, map_w, map_x, p);
     QT_CHECK_LAUNCH("gemm_fused");

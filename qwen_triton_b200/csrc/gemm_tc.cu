@@ -649,10 +649,13 @@ int launch_pair(const CUtensorMap& map_w, const CUtensorMap& map_x, TO* out, int
                 size_t split_stride, int act, float limit, int tail, float* tail_scratch, int* tail_flags, int tail_pairs, const float* bias, int* status,
                 cudaStream_t stream, const float4* run_scale = nullptr, int key_cols = 0) {
     const size_t smem = (size_t)PAIR_STAGES * PAIR_STAGE_BYTES + 1024 + (2 * PAIR_STAGES + 5) * 8 + 16;
-    static int resident_pairs = 0;                           // pairs the device runs at once (one per TPC that can host a cluster)
+    const cudaError_t raised = raise_shared<gemm_tc_pair_kernel<TO, MODE>>(227 * 1024);       // (it also checks that there is a device below 64)
+    if (raised != cudaSuccess) QT_FAIL(QT_ERR_LAUNCH, "gemm_tc_pair: cannot raise shared memory: %s", cudaGetErrorString(raised));
+    static thread_local int resident[64] = {};               // pairs a device runs at once (one per TPC that can host a cluster)
+    int device = 0;
+    cudaGetDevice(&device);
+    int& resident_pairs = resident[device];
     if (resident_pairs == 0) {
-        cudaError_t err = cudaFuncSetAttribute(gemm_tc_pair_kernel<TO, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
-        if (err != cudaSuccess) QT_FAIL(QT_ERR_LAUNCH, "gemm_tc_pair: cannot raise shared memory: %s", cudaGetErrorString(err));
         cudaLaunchConfig_t config = {};
         config.gridDim = dim3(2 * (unsigned)sm_count());
         config.blockDim = dim3(THREADS);
@@ -665,7 +668,7 @@ int launch_pair(const CUtensorMap& map_w, const CUtensorMap& map_x, TO* out, int
         config.attrs = attribute;
         config.numAttrs = 1;
         int clusters = 0;
-        err = cudaOccupancyMaxActiveClusters(&clusters, gemm_tc_pair_kernel<TO, MODE>, &config);
+        const cudaError_t err = cudaOccupancyMaxActiveClusters(&clusters, gemm_tc_pair_kernel<TO, MODE>, &config);
         if (err != cudaSuccess || clusters < 1)
             QT_FAIL(QT_ERR_LAUNCH, "gemm_tc_pair: no cluster of two blocks fits the device (%s)", cudaGetErrorString(err));
         resident_pairs = clusters;
@@ -704,12 +707,8 @@ int launch(const CUtensorMap& map_w, const CUtensorMap& map_x, TO* out, int M, i
     if (stages > most) stages = most;
     if (stages < 2) stages = 2;
     const size_t smem = (size_t)stages * STAGE_BYTES + 1024 + (2 * stages + 1) * 8 + 16;
-    static bool configured = false;
-    if (!configured) {
-        cudaError_t err = cudaFuncSetAttribute(gemm_tc_kernel<BX, TO, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
-        if (err != cudaSuccess) QT_FAIL(QT_ERR_LAUNCH, "gemm_tc: cannot raise shared memory: %s", cudaGetErrorString(err));
-        configured = true;
-    }
+    const cudaError_t raised = raise_shared<gemm_tc_kernel<BX, TO, MODE>>(227 * 1024);
+    if (raised != cudaSuccess) QT_FAIL(QT_ERR_LAUNCH, "gemm_tc: cannot raise shared memory: %s", cudaGetErrorString(raised));
     const int kb_per_split = (kb_total + splits - 1) / splits;
     dim3 grid(((N + BW - 1) / BW) * ((M + BX - 1) / BX), 1, splits);
     launch_kernel(gemm_tc_kernel<BX, TO, MODE>, dim3(grid), dim3(THREADS), smem, stream, map_w, map_x, out, M, N, kb_total, kb_per_split, split_stride, stages, act, limit, bias, status);

@@ -622,12 +622,8 @@ constexpr int HF_MOST_TOKENS = 64, HF_MOST_K = 512;
 template <typename TI, int MT, int NT>
 static int launch_head_few(const HeadProductParams& p, cudaStream_t s) {
     const int k_padded = (p.k + 15) / 16 * 16;
-    static bool configured = false;
-    if (!configured) {
-        cudaError_t err = cudaFuncSetAttribute(head_product_few_kernel<TI, MT, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (16 * MT + 8 * NT) * (HF_MOST_K + 8) * 2);
-        if (err != cudaSuccess) QT_FAIL(QT_ERR_LAUNCH, "head_product: cannot raise shared memory: %s", cudaGetErrorString(err));
-        configured = true;
-    }
+    const cudaError_t raised = raise_shared<head_product_few_kernel<TI, MT, NT>>((16 * MT + 8 * NT) * (HF_MOST_K + 8) * 2);
+    if (raised != cudaSuccess) QT_FAIL(QT_ERR_LAUNCH, "head_product: cannot raise shared memory: %s", cudaGetErrorString(raised));
     launch_kernel(head_product_few_kernel<TI, MT, NT>, dim3((p.n + 8 * NT - 1) / (8 * NT), p.heads), dim3(128), (size_t)(16 * MT + 8 * NT) * (k_padded + 8) * 2, s, p, k_padded);
     QT_CHECK_LAUNCH("head_product_few");
     return QT_OK;

@@ -521,12 +521,8 @@ int run_chunks(const ChunkArgs& p, int n_seqs, int chunks, cudaStream_t s) {
     if (PER_CHANNEL) {
         const int dim4 = (p.dim + 3) / 4 * 4;
         const size_t smem = ((size_t)3 * CT * (dim4 + 4) + (size_t)(4 + 3 + 8) * dim4) * sizeof(float);
-        static bool configured = false;
-        if (!configured) {
-            cudaError_t err = cudaFuncSetAttribute(chunk_prepare_channel_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
-            if (err != cudaSuccess) QT_FAIL(QT_ERR_LAUNCH, "chunk_prepare: cannot raise shared memory: %s", cudaGetErrorString(err));
-            configured = true;
-        }
+        const cudaError_t raised = raise_shared<chunk_prepare_channel_kernel>(227 * 1024);
+        if (raised != cudaSuccess) QT_FAIL(QT_ERR_LAUNCH, "chunk_prepare: cannot raise shared memory: %s", cudaGetErrorString(raised));
         QT_REQUIRE(smem <= 227 * 1024, "decayed_attention_chunked: %d key channels need more shared memory than a block has", p.dim);
         const int vec = raw_q && raw_k && vec_q && vec_k && aligned4(p.log_decay, {p.dim});
         launch_kernel(chunk_prepare_channel_kernel, dim3(chunks, p.heads, n_seqs), dim3(PC_THREADS), smem, s, p, vec);

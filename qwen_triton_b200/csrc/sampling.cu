@@ -477,12 +477,8 @@ extern "C" int qt_sample_keyed(const float* logits, float temperature, long long
     if (rows == 0) return QT_OK;
     const bool top = (top_k > 0 && top_k < vocab) || top_p < 1.f;
     if (top) {
-        static bool configured = false;
-        if (!configured) {
-            cudaError_t err = cudaFuncSetAttribute(sample_keyed_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TOP_SMEM_ALL);
-            if (err != cudaSuccess) QT_FAIL(QT_ERR_LAUNCH, "sample: cannot raise shared memory: %s", cudaGetErrorString(err));
-            configured = true;
-        }
+        const cudaError_t raised = raise_shared<sample_keyed_kernel<true>>((int)TOP_SMEM_ALL);
+        if (raised != cudaSuccess) QT_FAIL(QT_ERR_LAUNCH, "sample: cannot raise shared memory: %s", cudaGetErrorString(raised));
         launch_kernel(sample_keyed_kernel<true>, dim3(rows), dim3(SMP_THREADS), TOP_SMEM_ALL, (cudaStream_t)stream, logits, 1.f / temperature,
                       (unsigned long long)seed, keys, out, vocab, top_k, top_p);
     } else {

@@ -19,3 +19,9 @@ def test_what_earlier_kernels_write_is_read_by_ordinary_loads(source):
         assert not re.search(r"const \w+\s*\*\s*__restrict__", signature), signature
     for call in re.finditer(r"__ldg\(", text):
         assert text[call.end():].startswith(WEIGHTS), text[call.start():call.start() + 80]
+
+
+@pytest.mark.parametrize("source", SOURCES, ids=lambda path: path.name)
+def test_what_the_runtime_keeps_per_device_is_not_kept_per_process(source):
+    """A kernel's limit of dynamic shared memory belongs to a device: raised once in a process, it is missing on the second device."""
+    assert not re.search(r"static bool \w+ = false;", source.read_text())
