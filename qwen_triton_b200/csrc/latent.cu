@@ -619,6 +619,18 @@ __global__ void __launch_bounds__(128) head_product_few_kernel(const HeadProduct
 
 constexpr int HF_MOST_TOKENS = 64, HF_MOST_K = 512;
 
+// Where all of K at once is the faster form: up to 16 tokens, and up to 32 unless float rows meet the longest K on the most heads.  Every block
+// of 32 outputs stages all rows again, so beyond 32 tokens only where that is little (few outputs a head and not too many blocks, or few blocks
+// at all).  In microseconds, ring / all at once, T tokens, heads x outputs x K: T 64, 16 x 512 x 128 3.9 / 4.8, 128 x 512 x 128 9.9 / 15.8, 16 x 128 x
+// 512 11.4 / 6.2, 64 x 128 x 512 14.1 / 9.7, 128 x 128 x 512 15.8 / 19.1 (from floats 26.9 / 37.4), 8 x 256 x 64 2.6 / 2.4, 16 x 256 x 256 4.2 / 5.7; T 32, 128 x
+// 512 x 128 9.6 / 9.3, 128 x 128 x 512 17.0 / 15.0 (from floats 22.5 / 24.5).
+static bool few_pays(const HeadProductParams& p, bool floats) {
+    const long long blocks = (long long)p.heads * ((p.n + 31) / 32);
+    if (p.n_tokens <= 16) return true;
+    if (p.n_tokens <= 32) return !floats || p.k <= 128 || blocks * p.k < (1 << 18);
+    return blocks <= 64 || (p.k >= 2 * p.n && blocks * p.k <= (1 << 17));
+}
+
 template <typename TI, int MT, int NT>
 static int launch_head_few(const HeadProductParams& p, cudaStream_t s) {
     const int k_padded = (p.k + 15) / 16 * 16;
@@ -659,7 +671,7 @@ extern "C" int qt_head_product(const void* x, int x_dtype, int x_splits, long lo
         ((x_dtype == QT_F32 && x_row % 4 == 0 && x_head % 4 == 0 && x_offset % 4 == 0 && x_split_stride % 4 == 0 && ((uintptr_t)x & 15) == 0) ||
          (x_dtype == QT_BF16 && x_splits == 1 && x_row % 8 == 0 && x_head % 8 == 0 && x_offset % 8 == 0 && ((uintptr_t)x & 15) == 0)) &&
         ((uintptr_t)w & 15) == 0) {
-        if (n_tokens <= HF_MOST_TOKENS && k <= HF_MOST_K) return x_dtype == QT_F32 ? head_few<float>(p, s) : head_few<__nv_bfloat16>(p, s);
+        if (n_tokens <= HF_MOST_TOKENS && k <= HF_MOST_K && few_pays(p, x_dtype == QT_F32)) return x_dtype == QT_F32 ? head_few<float>(p, s) : head_few<__nv_bfloat16>(p, s);
         dim3 tiles((n + HM_N - 1) / HM_N, (n_tokens + HM_T - 1) / HM_T, heads);
         if (x_dtype == QT_F32) launch_kernel(head_product_mma_kernel<float>, tiles, dim3(128), 0, s, p);
         else launch_kernel(head_product_mma_kernel<__nv_bfloat16>, tiles, dim3(128), 0, s, p);
