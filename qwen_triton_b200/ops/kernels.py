@@ -1095,13 +1095,21 @@ def _check_attention(q, k_cache, v_cache, out, block_table, num_kv_heads, page_t
     return tokens, num_heads, head_dim
 
 
+def _kept_on_tcgen05(head_dim: int, most_keys: int, window: int | None, keep_first: int) -> bool:
+    """Whether a prompt with kept first keys or a linear penalty is faster on tcgen05 than on mma.sync: with heads of 128 always; with heads of 64,
+    whose products weigh less beside the softmax, where a query sees enough keys.  16 heads of 64, mma.sync / tcgen05 in microseconds: penalty alone 2,048
+    tokens 87 / 46, 400 17 / 15, 128 8.4 / 10.6, 16 behind 500 21.5 / 15.7; a window of 512 beside 16 kept keys 600 tokens 25 / 21, 400 15.5 / 13.2; of 384 600 tokens
+    22 / 23; of 256 18.8 / 22.7; of 128 15.2 / 20.7.  16 heads of 128, a window of 100: 2,048 tokens 48 / 26, 64 8.3 / 7.3."""
+    return head_dim > 64 or (most_keys >= 288 and (window is None or window + keep_first >= 448))
+
+
 def _extended_choice(q, k_cache, v_cache, page_tokens: int, ring_tokens: int, scale: float, penalty, keep_first: int, sink: bool, v_dim,
-                     chunk, impl: str | None, mma: str, softcap: float | None = None) -> str | None:
+                     chunk, impl: str | None, mma: str, softcap: float | None = None, most_keys: int = 0, window: int | None = None) -> str | None:
     """The kernel for a call that asks for a linear distance penalty (``penalty`` = (slopes, None)), kept first keys, a
     softmax sink, a cap on the scores, or values that are the head of the cached key rows; None for a call that asks for none of
     these.  The mma.sync kernels (``mma`` names the caller's) compute the first four for values as wide as the keys (a cap goes
-    with no penalty), the tcgen05 prefill kernel each of them, kept keys and the linear penalty without a cap; the generic kernels compute
-    everything."""
+    with no penalty), the tcgen05 prefill kernel each of them, kept keys and the linear penalty without a cap and where that is faster; the generic
+    kernels compute everything."""
     if not ((penalty is not None and penalty[1] is None) or keep_first > 0 or sink or v_dim is not None or softcap is not None):
         return None
     fits = (v_dim is None and v_cache.shape[-1] == q.shape[2] and attention_mma_supported(q, page_tokens) and scale > 0
@@ -1109,7 +1117,8 @@ def _extended_choice(q, k_cache, v_cache, page_tokens: int, ring_tokens: int, sc
     plain = penalty is None and not keep_first
     kept = softcap is None and chunk is None and (penalty is None or penalty[1] is None)
     if mma == "mma" and impl in (None, "tc") and fits and (plain or kept) and attention_tc_supported(q, page_tokens):
-        return "tc"
+        if plain or impl == "tc" or _kept_on_tcgen05(q.shape[2], most_keys, window, keep_first):
+            return "tc"
     if impl in (None, mma) and fits:
         return mma
     if impl in (None, "generic"):
@@ -1208,7 +1217,8 @@ def attention_prefill(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Ten
                       num_kv_heads: int, page_tokens: int, ring_tokens: int, window: int | None, scale: float,
                       impl: str | None = None, penalty: tuple[torch.Tensor, torch.Tensor] | None = None,
                       chunk: int | None = None, keep_first: int = 0, sink: bool = False, v_dim: int | None = None,
-                      sinks: torch.Tensor | None = None, softcap: float | None = None, score_bound: float | None = None) -> None:
+                      sinks: torch.Tensor | None = None, softcap: float | None = None, score_bound: float | None = None,
+                      max_context: int | None = None) -> None:
     """Causal attention of packed sequences over the cache (which already holds this step's keys).
     ``chunk``: a query at position i sees key j only if i // chunk == j // chunk as well.  A value cache with fewer
     heads than the key cache serves key head g with value head g % (value heads).
@@ -1218,7 +1228,8 @@ def attention_prefill(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Ten
     ``keep_first``: a windowed query also sees the keys at positions below it.  ``sink``: the softmax has one more term
     of score 0 without a value, or, with ``sinks`` (float [heads]), of the head's own score, taken as it is (not scaled).  ``v_dim``: the values are the first ``v_dim`` elements of the rows of ``v_cache`` (which
     may be the key cache itself).  ``softcap``: scores pass softcap * tanh(score / softcap), the sink's does not; ``score_bound``: what the
-    caller knows no score's size to exceed (a cheaper form of the cap where that is within the cap)."""
+    caller knows no score's size to exceed (a cheaper form of the cap where that is within the cap).  ``max_context``: the longest sequence with
+    its past, where the caller knows it (some choices of a kernel go by it)."""
     _, num_heads, head_dim = _check_attention(q, k_cache, v_cache, out, block_table, num_kv_heads, page_tokens, penalty, v_dim)
     if sinks is not None:
         _need(sinks, "sinks", torch.float32, (num_heads,))
@@ -1235,7 +1246,8 @@ def attention_prefill(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Ten
         return
     if impl == "latent":
         raise KernelError("the tensor-core kernel for cached latent rows does not take this call")
-    extended = _extended_choice(q, k_cache, v_cache, page_tokens, ring_tokens, scale, penalty, keep_first, sink, v_dim, chunk, impl, "mma", softcap)
+    extended = _extended_choice(q, k_cache, v_cache, page_tokens, ring_tokens, scale, penalty, keep_first, sink, v_dim, chunk, impl, "mma", softcap,
+                                max_context or max_q_len, window)
     if extended is not None:
         impl = extended
     elif not _plain_attention(q, v_cache, penalty):

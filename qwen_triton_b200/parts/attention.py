@@ -381,7 +381,7 @@ class Attention:
             kernels.attention_prefill(q, cache.k, cache.v, out, table, ctx.seq_start, ctx.seq_past, ctx.max_q_len,
                                       self.nkv, cache.page_tokens, cache.ring_tokens, self.window, self.scale, penalty=penalty,
                                       chunk=self.chunk, keep_first=self.keep_first, sink=bool(self.sink), sinks=self.sinks, softcap=self.softcap,
-                                      score_bound=self.score_bound)
+                                      score_bound=self.score_bound, max_context=getattr(ctx, "max_context", None))
         if self.head_gate:
             kernels.gate_mul(out.view(tokens, self.nq * self.dv), proj, self.at_gate, group=self.dv)
         if self.maps > 1:

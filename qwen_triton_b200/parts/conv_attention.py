@@ -155,7 +155,7 @@ class ConvAttention:
         else:
             kernels.attention_prefill(q, keys.k, keys.k, out, table, ctx.seq_start, ctx.seq_past, ctx.max_q_len, self.nkv,
                                       keys.page_tokens, keys.ring_tokens, self.window, self.scale, penalty=penalty,
-                                      keep_first=self.keep_first, sink=self.sink)
+                                      keep_first=self.keep_first, sink=self.sink, max_context=getattr(ctx, "max_context", None))
         out = out.view(tokens, self.nq * self.d)
         if self.gated:
             kernels.gate_mul(out, proj, self.at_gate)

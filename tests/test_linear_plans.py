@@ -153,3 +153,13 @@ def test_latent_prompts_need_little_memory_of_their_own(heads, tokens):
         assert LatentAttention(params, "m", runtime).expands == (page == 64)
         sizes.append(sum(numel * dtype.itemsize for name, (numel, dtype) in runtime.workspace._need.items() if name.startswith("latent.")))
     assert sizes[0] <= 1.2 * sizes[1], sizes
+
+
+# (head size, longest context, window, kept keys, mma.sync, tcgen05): 16 heads, measured, microseconds
+@pytest.mark.parametrize("d, context, window, keep_first, mma, tc", [
+    (128, 64, 100, 16, 8.3, 7.3), (128, 2048, 100, 16, 48.0, 25.6), (128, 16, None, 0, 8.3, 6.4), (64, 2048, None, 0, 86.7, 46.1), (64, 400, None, 0, 17.4, 14.5),
+    (64, 128, None, 0, 8.4, 10.6), (64, 64, None, 0, 6.3, 6.9), (64, 516, None, 0, 21.5, 15.7), (64, 600, 512, 16, 24.8, 20.9), (64, 400, 512, 16, 15.5, 13.2),
+    (64, 200, 512, 16, 10.2, 10.9), (64, 600, 384, 16, 22.2, 23.0), (64, 600, 256, 16, 18.8, 22.7), (64, 600, 128, 16, 15.2, 20.7), (64, 1000, 100, 16, 17.0, 22.9)])
+def test_kept_keys_and_linear_penalties_take_the_faster_kernel(d, context, window, keep_first, mma, tc):
+    taken = tc if kernels._kept_on_tcgen05(d, context, window, keep_first) else mma
+    assert taken <= 1.05 * min(mma, tc)
