@@ -195,7 +195,8 @@ static int launch_prefill(const AttnParams& p, int max_q_len, cudaStream_t strea
 // ----------------------------------------------------------------------------- many tokens per sequence, 32-bit rows of whole 16-byte pieces
 // Heads of up to 128 elements, d, dv and value rows multiples of 4, 16-byte aligned operands; everything else as above.
 // grid (tiles of 32 queries, heads, sequences), the longest tiles first; 128 threads, tiles of 64 keys, two blocks an SM.
-// Bound by the FMA pipe and by reads of shared memory.  A warp owns 8 query rows in both products: in q k^T lane (half, t) holds rows
+// Bound by the latency of its loads and instructions (two blocks of 4 warps an SM; ncu, the prompts below: FMA pipe 28 % and shared memory 35 % busy while an SM is
+// active) and by the uneven ends of the longest tiles (SMs active 63 % of the time).  A warp owns 8 query rows in both products: in q k^T lane (half, t) holds rows
 // 2 warp + half + 8 i against keys t + 16 j (16 results, fma.rn.f32x2 along d, rows 4 floats apart so that neither operand's reads collide), in
 // P V it holds four value columns of all 8 rows.  So the softmax and P stay within the warp, and the block meets only where a
 // tile's keys or values change: the next keys arrive (cp.async) under P V, the next values under q k^T.

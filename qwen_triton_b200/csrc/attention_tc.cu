@@ -41,9 +41,8 @@
 // scaled nor capped and has no value; it joins a row's sum once, at the end.
 //
 // DENSE (qt_attention_prefill_rows): prompts whose heads have keys and values of their own, formed for the step; keys of 128 or 192
-// elements, values of 64 or 128, a gate on the result ahead of its rounding.  Bound like the cached form by the softmax beside the MMAs: 2,048
-// tokens of 16 heads of 192 and 128 in 43 us (62 us with the gate's sums), 505 TFLOP/s; the same attention over cached rows of 576
-// and 512 elements (attention_latent.cu) 363 us.
+// elements, values of 64 or 128, a gate on the result ahead of its rounding.  2,048 tokens of 16 heads of 192 and 128 with a gate per element in 62 us; the same
+// attention over cached rows of 576 and 512 elements (attention_latent.cu) 363 us.
 //
 // Counterpart in luozoupi/Qwen-Triton: kernels/flash_attention.py:54-152 (32 x 32 tl.dot tiles) and the masked
 // SDPA branch of modules/attention.py:110-123.

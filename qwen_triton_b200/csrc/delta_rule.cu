@@ -637,7 +637,7 @@ __global__ void __launch_bounds__(SCAN_COLS * SCAN_LANES) delta_chunk_scan_kerne
 }
 
 // The same walk for the usual sizes (dim = 64 P up to 256, vdim a multiple of 16).  A sequence's chunks follow one another, so what counts is
-// the time of one chunk: its instructions, its reads of shared memory and the chain from S0 to the next S.  A warp owns two columns of
+// the time of one chunk: above all its reads of shared memory (ncu, the prompt below: that pipe 80 % busy, FMA 31 %, issue slots 43 %) and the chain from S0 to the next S.  A warp owns two columns of
 // the state, a lane 2 P rows of each as P pairs of neighbouring rows (fma.rn.f32x2), so every 16 bytes of a key, a query or a decay that a
 // lane reads serve two columns, and everything but the chunk's data stays within the warp.  Per chunk: the sums over the rows, S0^T (e^L
 // k) and S0^T (e^L q), are reduced so that lane (h, l) ends with token l of column h (31 exchanges each); r = beta (v - S0^T (e^L k)) and

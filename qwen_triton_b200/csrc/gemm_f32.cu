@@ -5,8 +5,9 @@
 // operands lie in memory, so no value is duplicated or repacked; the even and the odd k of a sum are added at the end.
 //
 // gemm_f32_tile_kernel   tiles of 64 x 128 (16 x 128 and 32 x 128 for few rows), 128 threads of 8 x 8 results (2 x 8, 4 x 8), K slices of 32
-//   through a three-stage cp.async ring, two blocks an SM.  Bound by the FMA pipe and shared-memory reads: per 4 k a thread issues
-//   128 packed FMAs and 16 16-byte reads, free of bank conflicts (rows are 36 floats apart).  8 x 4 results a thread (12 reads for 64
+//   through a three-stage cp.async ring, two blocks an SM.  Per 4 k a thread issues 128 packed FMAs and 16 16-byte reads, nearly free of bank
+//   conflicts (rows are 36 floats apart).  549 rows, 6144 x 1024 (ncu): the FMA pipe busy 62 % of an SM's active cycles, shared memory 50 %; the rest are
+//   fixed latencies of the two warps a scheduler that 255 registers leave.  8 x 4 results a thread (12 reads for 64
 //   FMAs) ran at 35 TFLOP/s where 8 x 8 run at 41.  Up to eight blocks of a cluster share a tile's K and add their parts through
 //   distributed shared memory in the order of the ranks: for tiles that do not fill the SMs, and because a running sum over a K of
 //   thousands would lose low-order bits.  A slice's sums go into a second set of floats for the same reason.
