@@ -1,9 +1,9 @@
 // What follows a decode step's product, as device functions shared by the kernels that run it in their epilogue
-// (gemm_fused.cu: one launch per product; gemm_chain.cu: one persistent launch for a run of products).
+// (gemm_fused.cu: up to 128 tokens, tiles of 128 columns; gemm_few.cu: up to 16 tokens, tiles of 16 or 32).
 //
 //   STORE     out[m, n] = s_m * y (+ bias[n])           float or bfloat16 (the output head)
 //   RESIDUAL  r = residual[m, n] + y; residual[m, n] = r;  and, for the norm that follows, xw[m, n] = bf16(r * g[n])
-//             and sq_out[tile, m] = sum over the tile's 128 columns of r^2
+//             and sq_out[tile, m] = sum over the tile's columns of r^2
 //   SWIGLU    act[m, f] = a(s_m * gate) * (s_m * up), a = SiLU or another QT_ACT_*, the weight's rows alternating 16 of gate and 16 of up
 //   QKV       per head (head_dim divides 128): s_m * y, RMSNorm over the head with q or k weight, rotation by the
 //             cos/sin table at the token's position (pairs (i, i + rd/2) or (2i, 2i + 1)), then q to q_out and k, v
@@ -14,8 +14,8 @@
 // equals normalising the input.  sq_in == nullptr means s_m = 1.  Partial sums of squares are kept per tile and added
 // in a fixed order: results do not depend on scheduling.
 //
-// One warp finishes one (token, 128-column tile): lane l holds columns 4 l .. 4 l + 3 of the tile (for SWIGLU the
-// gate and up values of features 2 l, 2 l + 1).
+// W / 4 neighbouring lanes finish one (token, W-column tile): lane l of them holds columns 4 l .. 4 l + 3 of the tile (for
+// SWIGLU the gate and up values of features 2 l, 2 l + 1).  The whole warp calls; lanes that are not `live` store nothing.
 #pragma once
 
 #include "common.cuh"
@@ -54,12 +54,20 @@ __device__ __forceinline__ uint32_t pack2(float a, float b) {
 }
 __device__ __forceinline__ float4 ld4(const float* p) { return *reinterpret_cast<const float4*>(p); }
 
-// The factor of the deferred norm for token m: every lane of the warp gets it.
+// Sum over the LANES neighbouring lanes that share a token: each gets it.
+template <int LANES> __device__ __forceinline__ float lanes_sum(float v) {
+#pragma unroll
+    for (int off = LANES / 2; off > 0; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
+    return v;
+}
+
+// The factor of the deferred norm for token m: every lane of the token gets it.
+template <int LANES>
 __device__ __forceinline__ float row_scale(const EpilogueParams& p, int m, int lane) {
     if (p.sq_in == nullptr) return 1.f;
     float s = 0.f;
-    for (int i = lane; i < p.sq_tiles; i += 32) s += p.sq_in[(size_t)i * p.M + m];
-    return rsqrtf(warp_sum(s) * p.inv_hidden + p.eps);
+    for (int i = lane; i < p.sq_tiles; i += LANES) s += p.sq_in[(size_t)i * p.M + m];
+    return rsqrtf(lanes_sum<LANES>(s) * p.inv_hidden + p.eps);
 }
 
 // What the epilogue of one (token, tile) needs from global memory besides the product itself.  It depends only on
@@ -71,10 +79,10 @@ struct Operands {
     long long cache_at;     // QKV: element offset of this lane's piece in the key or value cache
 };
 
-template <int EPI>
+template <int EPI, int W = TILE>
 __device__ __forceinline__ Operands load_operands(const EpilogueParams& p, int m, int w0, int lane) {
     Operands o;
-    o.scale = row_scale(p, m, lane);
+    o.scale = row_scale<W / 4>(p, m, lane);
     o.a = o.b = o.c = make_float4(0.f, 0.f, 0.f, 0.f);
     o.pos = 0;
     o.cache_at = 0;
@@ -115,23 +123,24 @@ __device__ __forceinline__ int swiglu_gate_row(int lane) { const int f = 2 * lan
 
 // SWIGLU: g and u are the gate and up sums of features 2 lane, 2 lane + 1 of tile w_tile (gate rows (f / 16) * 32 + f % 16
 // of the tile, up rows 16 further).
-__device__ __forceinline__ void finish_swiglu(const EpilogueParams& p, const Operands& ops, float2 g, float2 u, int m, int w_tile, int lane) {
+template <int W = TILE>
+__device__ __forceinline__ void finish_swiglu(const EpilogueParams& p, const Operands& ops, float2 g, float2 u, int m, int w_tile, int lane, bool live = true) {
     g.x *= ops.scale; g.y *= ops.scale; u.x *= ops.scale; u.y *= ops.scale;
     if (p.bias) {
-        const int at = w_tile * TILE + swiglu_gate_row(lane);
+        const int at = w_tile * W + swiglu_gate_row(lane);
         if (at + 17 < p.N) { g.x += p.bias[at]; g.y += p.bias[at + 1]; u.x += p.bias[at + 16]; u.y += p.bias[at + 17]; }
     }
-    const int features = p.N >> 1, feature = w_tile * (TILE / 2) + 2 * lane;
-    if (feature < features) {
+    const int features = p.N >> 1, feature = w_tile * (W / 2) + 2 * lane;
+    if (live && feature < features) {
         const float a0 = gated_value<true>(g.x, u.x, p.act, p.limit), a1 = gated_value<true>(g.y, u.y, p.act, p.limit);
         *reinterpret_cast<uint32_t*>((__nv_bfloat16*)p.out + (size_t)m * features + feature) = pack2(a0, a1);
     }
 }
 
-// The other epilogues: v holds the sums of columns w_tile * 128 + 4 lane .. + 3 of token m.  The whole warp calls.
-template <int EPI>
-__device__ __forceinline__ void finish(const EpilogueParams& p, const Operands& ops, float4 v, int m, int w_tile, int lane) {
-    const int n_rows = p.N, n = w_tile * TILE + 4 * lane;
+// The other epilogues: v holds the sums of columns w_tile * W + 4 lane .. + 3 of token m.
+template <int EPI, int W = TILE>
+__device__ __forceinline__ void finish(const EpilogueParams& p, const Operands& ops, float4 v, int m, int w_tile, int lane, bool live = true) {
+    const int n_rows = live ? p.N : 0, n = w_tile * W + 4 * lane;
     if (EPI == EPI_STORE) {
         v.x *= ops.scale; v.y *= ops.scale; v.z *= ops.scale; v.w *= ops.scale;
         if (p.bias) {
@@ -166,10 +175,10 @@ __device__ __forceinline__ void finish(const EpilogueParams& p, const Operands& 
                     make_uint2(pack2(v.x * ops.b.x, v.y * ops.b.y), pack2(v.z * ops.b.z, v.w * ops.b.w));
         }
         if (p.norm_w) {
-            sq = warp_sum(sq);
-            if (lane == 0) p.sq_out[(size_t)w_tile * p.M + m] = sq;
+            sq = lanes_sum<W / 4>(sq);
+            if (lane == 0 && live) p.sq_out[(size_t)w_tile * p.M + m] = sq;
         }
-    } else if (EPI == EPI_QKV) {
+    } else if (EPI == EPI_QKV) {                            // W is 128: a head lies within the warp
         const int d = p.d, lanes_per_head = d >> 2;
         v.x *= ops.scale; v.y *= ops.scale; v.z *= ops.scale; v.w *= ops.scale;
         const int head = n / d, c = n - head * d;

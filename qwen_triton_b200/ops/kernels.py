@@ -156,6 +156,14 @@ _SIGNATURES = {
                           _c_ptr, _c_ptr, _c_ptr, _c_ptr, _c_ptr, _c_ptr, _c_int, _c_ptr, _c_ptr, _c_float,
                           _c_ptr, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_ptr, _c_ptr],
     },
+    "gemm_few": {
+        "qt_gemm_few": [_c_ptr, _c_ptr, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int,
+                        _c_ptr, _c_int, _c_int, _c_float, _c_ptr,
+                        _c_ptr, _c_int, _c_int, _c_float,
+                        _c_ptr, _c_ptr, _c_ptr, _c_ptr,
+                        _c_ptr, _c_ptr, _c_ptr, _c_ptr, _c_ptr, _c_ptr, _c_int, _c_ptr, _c_ptr, _c_float,
+                        _c_ptr, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_ptr],
+    },
     "sampling": {
         "qt_argmax": [_c_ptr, _c_ptr, _c_int, _c_int, _c_ptr],
         "qt_sample": [_c_ptr, _c_ptr, _c_ptr, _c_ptr, _c_int, _c_int, _c_ptr],
@@ -1782,6 +1790,15 @@ def fused_supported(w: torch.Tensor) -> bool:
     return w.dtype == torch.bfloat16 and w.dim() == 2 and w.shape[1] % 8 == 0 and w.data_ptr() % 16 == 0 and w.is_contiguous()
 
 
+FEW_MAX_ROWS = 16           # most tokens the kernel for few of them takes (csrc/gemm_few.cu)
+
+
+def few_supported(x, w: torch.Tensor) -> bool:
+    """Whether rows and weight can be read 32 bytes at a time, as the kernel for few tokens does."""
+    a = x.tensor if isinstance(x, ScaledRows) else x
+    return 0 < a.shape[0] <= FEW_MAX_ROWS and w.shape[1] % 16 == 0 and w.data_ptr() % 32 == 0 and a.data_ptr() % 32 == 0
+
+
 def fused_qkv_supported(head_dim: int, rotary_dim: int) -> bool:
     """The fused q/k-norm + rotation + cache write needs whole heads inside a 128-row weight tile and rotation
     pairs that four-element pieces can exchange."""
@@ -1791,7 +1808,7 @@ def fused_qkv_supported(head_dim: int, rotary_dim: int) -> bool:
 def _fused(x, w: torch.Tensor, splits: int, epilogue: int, *, out=None, residual=None, norm_w=None, xw=None, sq_out=None,
            q_out=None, k_cache=None, v_cache=None, token_seq=None, token_pos=None, block_table=None, q_w=None, k_w=None,
            qk_eps=0.0, cos_sin=None, nq=0, nkv=0, d=0, page_tokens=0, ring_tokens=0, write_kv=False, stages: int = 0,
-           act: int = 0, interleaved: bool = False, limit: float = 0.0, bias: torch.Tensor | None = None) -> None:
+           act: int = 0, interleaved: bool = False, limit: float = 0.0, bias: torch.Tensor | None = None, few: tuple[int, int] | None = None) -> None:
     scaled = x if isinstance(x, ScaledRows) else None
     a = scaled.tensor if scaled is not None else x
     _need(a, "x", torch.bfloat16)
@@ -1806,58 +1823,62 @@ def _fused(x, w: torch.Tensor, splits: int, epilogue: int, *, out=None, residual
         if scaled.sq.dim() != 2 or scaled.sq.shape[1] != rows:
             raise KernelError(f"gemm_fused: sums of squares {tuple(scaled.sq.shape)} for {rows} rows")
     rotary_dim, max_pos = (0, 0) if cos_sin is None else (cos_sin.shape[1], cos_sin.shape[0])
-    _call("gemm_fused", "qt_gemm_fused", _ptr(a), _ptr(w), rows, w.shape[0], k, tc_token_tile(rows), int(splits), int(stages), epilogue,
-          _ptr(scaled.sq) if scaled is not None else None, scaled.sq.shape[0] if scaled is not None else 0,
-          scaled.width if scaled is not None else 0, float(scaled.eps) if scaled is not None else 0.0, _ptr(_product_bias(bias, w)),
-          _ptr(out), _CODES.get(out.dtype, -1) if out is not None else 0, int(act), float(limit),
-          _ptr(residual), _ptr(norm_w), _ptr(xw), _ptr(sq_out),
-          _ptr(q_out), _ptr(k_cache), _ptr(v_cache), _ptr(token_seq), _ptr(token_pos), _ptr(block_table),
-          block_table.shape[1] if block_table is not None else 0, _ptr(q_w), _ptr(k_w), float(qk_eps),
-          _ptr(cos_sin), rotary_dim, max_pos, nq, nkv, d, page_tokens, ring_tokens, 1 if write_kv else 0,
-          1 if interleaved else 0, _ptr(_status_word(a.device)), _stream())
+    head = (_ptr(a), _ptr(w), rows, w.shape[0], k)
+    tail = (_ptr(scaled.sq) if scaled is not None else None, scaled.sq.shape[0] if scaled is not None else 0,
+            scaled.width if scaled is not None else 0, float(scaled.eps) if scaled is not None else 0.0, _ptr(_product_bias(bias, w)),
+            _ptr(out), _CODES.get(out.dtype, -1) if out is not None else 0, int(act), float(limit),
+            _ptr(residual), _ptr(norm_w), _ptr(xw), _ptr(sq_out),
+            _ptr(q_out), _ptr(k_cache), _ptr(v_cache), _ptr(token_seq), _ptr(token_pos), _ptr(block_table),
+            block_table.shape[1] if block_table is not None else 0, _ptr(q_w), _ptr(k_w), float(qk_eps),
+            _ptr(cos_sin), rotary_dim, max_pos, nq, nkv, d, page_tokens, ring_tokens, 1 if write_kv else 0, 1 if interleaved else 0)
+    if few is not None:
+        _call("gemm_few", "qt_gemm_few", *head, int(few[0]), int(few[1]), epilogue, *tail, _stream())
+    else:
+        _call("gemm_fused", "qt_gemm_fused", *head, tc_token_tile(rows), int(splits), int(stages), epilogue, *tail, _ptr(_status_word(a.device)), _stream())
 
 
 def gemm_fused_store(x, w: torch.Tensor, out: torch.Tensor, splits: int = 1, stages: int = 0, bias: torch.Tensor | None = None,
-                     activation: str | None = None) -> None:
+                     activation: str | None = None, few: tuple[int, int] | None = None) -> None:
     """out [M, N] (float or bfloat16) = x w^T (+ ``bias``, float), times the rows' deferred norm factor if ``x`` is ``ScaledRows``;
-    with ``activation`` that function of it."""
+    with ``activation`` that function of it.  ``few`` = (weight rows a block, warps a block): by the kernel for up to 16 tokens
+    (csrc/gemm_few.cu), here and in the products below."""
     _need(out, "out", shape=(x.shape[0], w.shape[0]))
     _fused(x, w, splits, _EPI_STORE if activation is None else _EPI_ACTIVATED, out=out, stages=stages, bias=bias,
-           act=0 if activation is None else activation_code(activation))
+           act=0 if activation is None else activation_code(activation), few=few)
 
 
 def gemm_fused_residual(x, w: torch.Tensor, residual: torch.Tensor, norm_weight: torch.Tensor | None = None,
                         eps: float = 0.0, xw: torch.Tensor | None = None, sq: torch.Tensor | None = None, splits: int = 1,
-                        stages: int = 0, bias: torch.Tensor | None = None) -> "ScaledRows | None":
+                        stages: int = 0, bias: torch.Tensor | None = None, few: tuple[int, int] | None = None) -> "ScaledRows | None":
     """residual [M, N] (float, in place) += x w^T (+ ``bias`` [N], float).  With ``norm_weight`` [N] the RMSNorm that follows is prepared in
     the same launch: ``xw`` [M, N] = bf16(residual * norm_weight) and ``sq`` [ceil(N / 128), M] = the rows' sums of
-    squares per 128 columns; returns them as ``ScaledRows`` for the product behind the norm."""
+    squares per 128 columns (with ``few``: per its weight rows); returns them as ``ScaledRows`` for the product behind the norm."""
     rows, n = x.shape[0], w.shape[0]
     _need(residual, "residual", torch.float32, (rows, n))
     if norm_weight is None:
-        _fused(x, w, splits, _EPI_RESIDUAL, residual=residual, stages=stages, bias=bias)
+        _fused(x, w, splits, _EPI_RESIDUAL, residual=residual, stages=stages, bias=bias, few=few)
         return None
     _need(norm_weight, "norm_weight", torch.float32, (n,))
     _need(xw, "xw", torch.bfloat16, (rows, n))
-    _need(sq, "sq", torch.float32, (-(-n // 128), rows))
-    _fused(x, w, splits, _EPI_RESIDUAL, residual=residual, norm_w=norm_weight, xw=xw, sq_out=sq, stages=stages, bias=bias)
+    _need(sq, "sq", torch.float32, (-(-n // (128 if few is None else few[0])), rows))
+    _fused(x, w, splits, _EPI_RESIDUAL, residual=residual, norm_w=norm_weight, xw=xw, sq_out=sq, stages=stages, bias=bias, few=few)
     return ScaledRows(xw, sq, n, float(eps))
 
 
 def gemm_fused_swiglu(x, w: torch.Tensor, out: torch.Tensor, splits: int = 1, stages: int = 0, activation: str = "silu",
-                      limit: float = 0.0, bias: torch.Tensor | None = None) -> None:
+                      limit: float = 0.0, bias: torch.Tensor | None = None, few: tuple[int, int] | None = None) -> None:
     """out [M, N / 2] (bfloat16) = act(gate) * up for a weight whose rows alternate SWIGLU_GROUP of gate and of up."""
     if w.shape[0] % (2 * SWIGLU_GROUP):
         raise KernelError(f"gemm_fused_swiglu: {w.shape[0]} rows are not gate and up rows in groups of {SWIGLU_GROUP}")
     _need(out, "out", torch.bfloat16, (x.shape[0], w.shape[0] // 2))
-    _fused(x, w, splits, _EPI_SWIGLU, out=out, stages=stages, act=activation_code(activation, True), limit=limit, bias=bias)
+    _fused(x, w, splits, _EPI_SWIGLU, out=out, stages=stages, act=activation_code(activation, True), limit=limit, bias=bias, few=few)
 
 
 def gemm_fused_qkv(x, w: torch.Tensor, q_out: torch.Tensor, k_cache: torch.Tensor | None, v_cache: torch.Tensor | None,
                    token_seq: torch.Tensor, token_pos: torch.Tensor, block_table: torch.Tensor | None,
                    q_weight: torch.Tensor | None, k_weight: torch.Tensor | None, eps: float, cos_sin: torch.Tensor | None,
                    num_heads: int, num_kv_heads: int, head_dim: int, page_tokens: int, ring_tokens: int,
-                   write_kv: bool = True, splits: int = 1, stages: int = 0, interleaved: bool = False) -> None:
+                   write_kv: bool = True, splits: int = 1, stages: int = 0, interleaved: bool = False, few: tuple[int, int] | None = None) -> None:
     """The fused projection [q; k; v] (or q alone) with per-head q/k RMSNorm, rotation and the cache write done in
     its epilogue: what ``gemm`` followed by ``qk_norm_rope_write`` does, in one launch."""
     rows = x.shape[0]
@@ -1881,4 +1902,4 @@ def gemm_fused_qkv(x, w: torch.Tensor, q_out: torch.Tensor, k_cache: torch.Tenso
     _fused(x, w, splits, _EPI_QKV, q_out=q_out, k_cache=k_cache if write_kv else None, v_cache=v_cache if write_kv else None,
            token_seq=token_seq, token_pos=token_pos, block_table=block_table if write_kv else None, q_w=q_weight, k_w=k_weight,
            qk_eps=eps, cos_sin=cos_sin, nq=num_heads, nkv=num_kv_heads, d=head_dim, page_tokens=page_tokens,
-           ring_tokens=ring_tokens, write_kv=write_kv, stages=stages, interleaved=interleaved)
+           ring_tokens=ring_tokens, write_kv=write_kv, stages=stages, interleaved=interleaved, few=few)

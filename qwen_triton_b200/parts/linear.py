@@ -24,6 +24,7 @@ _FUSED_BLOCKS_PER_SM = {3: 4, 4: 3, 5: 2}
 # barrier, the peers' sums); it grows with the rows, and beyond 16 it costs more than the small kernels it replaces
 # (8B shapes, 64 rows, replayed alone: q/k/v 15.8 us fused against 10.4 + 2.7 us, down 23.0 against 19.9 + 3.5 us).
 _FUSED_ROWS = int(os.environ.get("QT_B200_FUSED_ROWS", "16"))
+_FEW_WEIGHT = 8 << 20                  # most elements of a weight that few tokens read through csrc/gemm_few.cu (Linear.few_plan)
 # (most rows, blocks wanted in flight) for products bound by reading the weight.  Up to 16 rows the kernel's ring is
 # three stages deep and four blocks share an SM, which also lets the next product's blocks move in and fetch their
 # first weight tiles while this one drains; up to 64 rows two blocks with deeper rings measured better.  Up to 256
@@ -185,23 +186,43 @@ class Linear:
                 return stages
         return 0
 
+    def few_plan(self, x) -> tuple[int, int] | None:
+        """(weight rows a block, warps a block) where these rows take the kernel for few tokens (csrc/gemm_few.cu), else None.
+
+        It is the faster form where the launch before it and its own chain bound a product, not the weight's bytes: weights of up to
+        8 M elements (``_FEW_WEIGHT``).  Steps of the 0.6B shape (weights of 2 to 6 M) 20 to 31 % shorter at 1 to 16 sequences; of the 8B shape
+        (17 to 101 M) 4 % shorter at eight but 7 to 23 % longer at 1, 3 and 16, since its blocks keep fewer bytes in flight than a TMA ring.
+        Blocks of 32 rows for heads and gates; 16 rows otherwise, so that a thousand features still give 64 SMs a block (32 rows: one sequence
+        728 us a step instead of 634).  16 warps a block where their sums are short of the weight's arrival: beyond 8 tokens (797 us against 857 with
+        8), and where K is longest for its rows (570 to 590 against 634)."""
+        rows = x.shape[0]
+        if not 0 < rows <= kernels.FEW_MAX_ROWS or self.weight is None or self.weight.numel() > _FEW_WEIGHT or not kernels.few_supported(x, self.weight):
+            return None
+        wide = self.role in ("gate", "qkv")
+        return (32 if wide else 16), (8 if wide and rows <= 8 else 16)
+
+    def norm_tiles(self, x, width: int) -> int:
+        """Column ranges whose sums of squares ``into_residual`` hands on for rows of ``width`` elements."""
+        few = self.few_plan(x)
+        return -(-width // (128 if few is None else few[0]))
+
     def into_residual(self, x: torch.Tensor, residual: torch.Tensor, norm_weight: torch.Tensor | None = None, eps: float = 0.0,
                       xw: torch.Tensor | None = None, sq: torch.Tensor | None = None) -> "ScaledRows | None":
         """residual += x W^T, and the norm behind it prepared (see ``kernels.gemm_fused_residual``)."""
         return kernels.gemm_fused_residual(x, self.weight, residual, norm_weight, eps, xw, sq, splits=self._fused_splits(x.shape[0]),
-                                           stages=self._fused_stages(x.shape[0]), bias=self._loaded_bias())
+                                           stages=self._fused_stages(x.shape[0]), bias=self._loaded_bias(), few=self.few_plan(x))
 
     def into_swiglu(self, x, out: torch.Tensor, activation: str = "silu", limit: float = 0.0, bias: torch.Tensor | None = None) -> None:
         kernels.gemm_fused_swiglu(x, self.weight, out, splits=self._fused_splits(x.shape[0]), stages=self._fused_stages(x.shape[0]),
-                                  activation=activation, limit=limit, bias=bias)
+                                  activation=activation, limit=limit, bias=bias, few=self.few_plan(x))
 
     def into_activation(self, x, out: torch.Tensor, activation: str) -> None:
         """out = act(x W^T (+ bias)), the activation in the fused product's epilogue."""
         kernels.gemm_fused_store(x, self.weight, out, splits=self._fused_splits(x.shape[0]), stages=self._fused_stages(x.shape[0]), bias=self._loaded_bias(),
-                                 activation=activation)
+                                 activation=activation, few=self.few_plan(x))
 
     def into_qkv(self, x, *args, **kwargs) -> None:
-        kernels.gemm_fused_qkv(x, self.weight, *args, splits=self._fused_splits(x.shape[0]), stages=self._fused_stages(x.shape[0]), **kwargs)
+        kernels.gemm_fused_qkv(x, self.weight, *args, splits=self._fused_splits(x.shape[0]), stages=self._fused_stages(x.shape[0]), few=self.few_plan(x), **kwargs)
 
     def plan_splits(self, rows: int) -> int:
         """The number of K ranges that ``rows`` tokens are cut into by the plain products."""
@@ -213,7 +234,7 @@ class Linear:
             # rows whose norm factor is still to be applied: the fused product's plain store applies it
             if out is None:
                 out = self.runtime.workspace.view(f"{self.key}.out" if self.float_out else f"{self.key}.wide", rows, self.out_features)
-            kernels.gemm_fused_store(x, self.weight, out.view(rows, self.out_features), splits=self._fused_splits(rows), bias=self._loaded_bias())
+            kernels.gemm_fused_store(x, self.weight, out.view(rows, self.out_features), splits=self._fused_splits(rows), bias=self._loaded_bias(), few=self.few_plan(x))
             return GemmOut(out.view(1, rows, self.out_features))
         splits = self.plan_splits(rows)
         if out is None and splits > 1:
@@ -232,7 +253,7 @@ class Linear:
         if isinstance(x, ScaledRows) or not (self.float_out and self.fusable(rows)):
             return self(x)
         out = self.runtime.workspace.view(f"{self.key}.out", rows, self.out_features)
-        kernels.gemm_fused_store(x, self.weight, out, splits=self._fused_splits(rows), stages=self._fused_stages(rows), bias=self._loaded_bias())
+        kernels.gemm_fused_store(x, self.weight, out, splits=self._fused_splits(rows), stages=self._fused_stages(rows), bias=self._loaded_bias(), few=self.few_plan(x))
         return GemmOut(out.view(1, rows, self.out_features))
 
     def _loaded_bias(self) -> torch.Tensor | None:

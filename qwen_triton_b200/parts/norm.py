@@ -34,7 +34,8 @@ class RMSNorm:
         self.runtime = runtime
         self.weight: torch.Tensor | None = None
         runtime.workspace.declare("normed", runtime.max_step_tokens * self.size, runtime.dtype)
-        runtime.workspace.declare("normed.sq", -(-self.size // 128) * kernels.FUSED_MAX_ROWS, torch.float32)
+        # column ranges of at least 16 for up to FEW_MAX_ROWS rows, of 128 beyond
+        runtime.workspace.declare("normed.sq", max(-(-self.size // 128) * kernels.FUSED_MAX_ROWS, -(-self.size // 16) * kernels.FEW_MAX_ROWS), torch.float32)
 
     @classmethod
     def expected_tensors(cls, params, name: str) -> dict[str, TensorSpec]:
@@ -84,7 +85,7 @@ class RMSNorm:
                 stream.pending = deferred.run()
             elif rows is None and lazy and self.offers_scaled_rows:
                 xw = ws.view("normed", count, self.size)
-                sq = ws.view("normed.sq", -(-self.size // 128), count)
+                sq = ws.view("normed.sq", deferred.linear.norm_tiles(deferred.x, self.size), count)
                 return deferred.linear.into_residual(deferred.x, stream.residual, self.weight, self.eps, xw, sq)
             else:
                 deferred.linear.into_residual(deferred.x, stream.residual)
