@@ -155,9 +155,6 @@ __global__ void __launch_bounds__(THREADS) expert_gemm_kernel(const __grid_const
 constexpr int PBN = 256, PSTAGES = 4;
 constexpr uint32_t P_B_BYTES = PBN * BK * 2, P_STAGE_BYTES = A_BYTES + P_B_BYTES;
 
-__device__ __forceinline__ void mbar_arrive(uint32_t bar) {
-    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
-}
 
 template <typename TO, bool ACT>
 __global__ void __launch_bounds__(THREADS, 1) expert_gemm_persistent_kernel(const __grid_constant__ CUtensorMap map_x,

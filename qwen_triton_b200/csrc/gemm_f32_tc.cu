@@ -1,0 +1,311 @@
+// C[M, N] = A[M, K] * W[N, K]^T of float operands on the fifth-generation tensor cores, exact in what it multiplies: the 32-bit path's
+// products of more than a few rows.
+//
+// A float of 24 bits is the sum of three bfloat16 numbers (round to nearest, subtract, twice more: 8 + 8 + 8 bits, nothing is lost), and a product of
+// two bfloat16 numbers is exact in the float that tcgen05.mma adds it to.  Of the nine products of pieces six are formed: 1.1, 1.2, 2.1, 2.2,
+// 1.3, 3.1; the others are below 2^-25 of the operands' product and of either sign.  What could lose bits is the adding: the tensor pipe
+// does not round to nearest, so an accumulator takes one K slice of 64 (small products first) and is then added, rounded to nearest, to sums in registers.
+//
+// A block forms 128 x 128 results.  Eight warps load the next slice's floats into registers, split them and store the pieces where the MMAs read
+// them, two stages deep: A's in tensor memory, a row a thread (from shared memory both operands of 128 x 128 x 16 are 128 bytes a clock, all it
+// gives, and a slice took twice its 1,536 cycles of the tensor pipe), W's as swizzled tiles.  One thread issues 24 MMAs a slice, and the eight
+// warps add a finished slice's accumulator up while the next one is multiplied.  Up to eight blocks of a cluster share K where the tiles do not fill
+// the SMs, and add up through distributed shared memory in the order of the ranks.
+//
+// Infinities, NaN and numbers that round to an infinite bfloat16 have no such pieces: a block that meets one forms its results again with FMAs.
+#include "tc_common.cuh"
+
+using namespace qt;
+using namespace qt_tc;
+
+namespace {
+
+constexpr int TILE = 128, BK = 64;                     // rows of either operand a block takes, K elements of a slice
+constexpr int WORK_WARPS = 8, THREADS = (WORK_WARPS + 1) * 32;
+constexpr uint32_t PIECE_BYTES = TILE * BK * 2;        // one piece of W: [128 rows][64] bfloat16, 128-byte swizzle
+constexpr uint32_t STAGE_BYTES = 3 * PIECE_BYTES;
+constexpr int A_COLS = BK / 2;                         // one piece of A in tensor memory: row i in lane i, two elements a column
+constexpr uint32_t TMEM_A = 2 * TILE, TMEM_COLS = 512; // two accumulators, two stages of A's pieces
+constexpr int UNITS = 8;                               // runs of eight elements a thread splits per slice
+constexpr int MOST_RANKS = 8, PARK_ROW = TILE + 4;
+constexpr uint32_t IDESC = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(TILE >> 3) << 17) | ((uint32_t)(TILE >> 4) << 24);
+static_assert(TILE * PARK_ROW * 4 <= 2 * STAGE_BYTES, "a block's part of the result is parked in the stages' memory");
+
+// What the truncated additions of a slice leave out on average, of its sum.
+constexpr float SHORTFALL = 0.f;
+
+struct Params {
+    const float* a; const float* w; float* c;
+    int M, N, K, ranks, slices_per_rank;
+    int* status;
+};
+
+__device__ __forceinline__ uint32_t pack_rn(float lo, float hi) {
+    uint32_t d;
+    asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(d) : "f"(hi), "f"(lo));
+    return d;
+}
+__device__ __forceinline__ float low_of(uint32_t v) { return __uint_as_float(v << 16); }
+__device__ __forceinline__ float high_of(uint32_t v) { return __uint_as_float(v & 0xffff0000u); }
+__device__ __forceinline__ void store16(uint32_t at, const uint32_t (&v)[4]) {
+    asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(at), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]) : "memory");
+}
+__device__ __forceinline__ void store_columns(uint32_t taddr, const uint32_t (&v)[16]) {
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};"
+                 ::"r"(taddr), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]),
+                   "r"(v[8]), "r"(v[9]), "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15]) : "memory");
+}
+__device__ __forceinline__ float4 load4(const float* p) {
+    float4 v;
+    asm volatile("ld.global.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p) : "memory");
+    return v;
+}
+__device__ __forceinline__ float4 peer4(uint32_t addr) {
+    float4 v;
+    asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr) : "memory");
+    return v;
+}
+
+__global__ void __launch_bounds__(THREADS, 1) gemm_f32_tc_kernel(const __grid_constant__ Params p) {
+    extern __shared__ uint8_t smem_raw[];
+    const uint32_t raw = smem_u32(smem_raw), base = (raw + 1023u) & ~1023u;
+    uint8_t* smem = smem_raw + (base - raw);
+    const uint32_t bars = base + 2 * STAGE_BYTES;      // full[2], empty[2], summed[2] (an accumulator is complete), added[2] (and read)
+    const uint32_t full = bars, empty = bars + 16, summed = bars + 32, added = bars + 48;
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + 2 * STAGE_BYTES + 64);
+    int* odd = reinterpret_cast<int*>(smem + 2 * STAGE_BYTES + 68);         // a number without pieces was met
+
+    pdl_launch_dependents();
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int rank = p.ranks > 1 ? (int)cluster_ctarank() : 0;
+    const int n0 = (int)(blockIdx.x / (unsigned)p.ranks) * TILE, m0 = blockIdx.y * TILE;
+    const int k_begin = rank * p.slices_per_rank * BK, k_end = min(p.K, k_begin + p.slices_per_rank * BK);
+    const int slices = (k_end - k_begin + BK - 1) / BK;                     // >= 1: the host sizes the ranks so
+    int* status = p.status;
+
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < 2; ++s) {
+            mbar_init(full + 8 * s, WORK_WARPS); mbar_init(empty + 8 * s, 1);
+            mbar_init(summed + 8 * s, 1); mbar_init(added + 8 * s, WORK_WARPS);
+        }
+        *odd = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == WORK_WARPS) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(TMEM_COLS) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem_base = *tmem_slot;
+
+    if (warp == WORK_WARPS) {
+        if (lane == 0) {
+            const uint64_t desc0 = operand_desc(base);
+            for (int i = 0; i < slices; ++i) {
+                const int s = i & 1;
+                const uint32_t turn = (uint32_t)(i >> 1) & 1u;
+                if (!mbar_wait(full + 8 * s, turn, status, 2)) break;
+                if (!mbar_wait(added + 8 * s, turn ^ 1u, status, 4)) break;
+                tc_fence_after();
+                const uint64_t w0 = desc0 + (uint64_t)(s * (STAGE_BYTES >> 4));
+                const uint32_t acc = tmem_base + s * TILE, a0 = tmem_base + TMEM_A + s * 3 * A_COLS;
+                auto product = [&](int x, int y, bool first) {
+#pragma unroll
+                    for (int k = 0; k < BK / 16; ++k)
+                        umma_bf16_a_tmem(acc, a0 + x * A_COLS + 8 * k, w0 + y * (PIECE_BYTES >> 4) + 2 * k, IDESC, first && k == 0 ? 0u : 1u);
+                };
+                product(0, 2, true); product(2, 0, false); product(1, 1, false);
+                product(0, 1, false); product(1, 0, false); product(0, 0, false);
+                umma_commit(empty + 8 * s);
+                umma_commit(summed + 8 * s);
+            }
+        }
+        __syncwarp();
+    } else {
+        // Warps 0 to 3: a thread holds a row of A's slice, unit u is its elements 8 u .. 8 u + 7.  Warps 4 to 7: unit u of a thread is eight
+        // neighbouring elements of row 16 u + (thread / 8) of W's.
+        const bool of_a = warp < 4;
+        const int chunk = threadIdx.x & 7, w_row = (threadIdx.x & 127) >> 3;
+        float v[UNITS][8];
+        auto ask = [&](int u, int slice) {
+            const int at = of_a ? m0 + (int)threadIdx.x : n0 + 16 * u + w_row, k = k_begin + slice * BK + 8 * (of_a ? u : chunk);
+            const bool there = at < (of_a ? p.M : p.N);
+            const float* from = (of_a ? p.a : p.w) + (size_t)at * p.K + k;
+            const float4 x = there && k < k_end ? load4(from) : make_float4(0.f, 0.f, 0.f, 0.f);              // K is a multiple of 4
+            const float4 y = there && k + 4 < k_end ? load4(from + 4) : make_float4(0.f, 0.f, 0.f, 0.f);
+            v[u][0] = x.x; v[u][1] = x.y; v[u][2] = x.z; v[u][3] = x.w; v[u][4] = y.x; v[u][5] = y.y; v[u][6] = y.z; v[u][7] = y.w;
+        };
+        float sums[64];                                                     // row 32 (warp % 4) + lane, columns 64 (warp / 4) ..
+#pragma unroll
+        for (int j = 0; j < 64; ++j) sums[j] = 0.f;
+        const uint32_t mine = tmem_base + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)(warp >> 2) * 64u;
+        auto add = [&](int i) {
+            const int s = i & 1;
+            if (!mbar_wait(summed + 8 * s, (uint32_t)(i >> 1) & 1u, status, 3)) return false;
+            tc_fence_after();
+#pragma unroll
+            for (int part = 0; part < 4; ++part) {
+                uint32_t x[16];
+                tmem_load16(mine + s * TILE + 16 * part, x);
+#pragma unroll
+                for (int j = 0; j < 16; ++j) sums[16 * part + j] += __uint_as_float(x[j]);
+            }
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(added + 8 * s);
+            return true;
+        };
+        if (of_a) pdl_wait();                                               // weights depend on no earlier kernel
+#pragma unroll
+        for (int u = 0; u < UNITS; ++u) ask(u, 0);
+        if (!of_a) pdl_wait();
+        float none = 0.f;                                                   // stays 0 while every number has its pieces
+        // the next piece of a unit: its numbers rounded, and what is left of them
+        auto piece_of = [&](int u, uint32_t* h, bool first, bool last) {
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                float& lo = v[u][2 * j];
+                float& hi = v[u][2 * j + 1];
+                h[j] = pack_rn(lo, hi);
+                if (last) continue;
+                lo -= low_of(h[j]); hi -= high_of(h[j]);
+                if (first) { none = fmaf(0.f, lo, none); none = fmaf(0.f, hi, none); }
+            }
+        };
+        bool ok = true;
+        for (int i = 0; i < slices && ok; ++i) {
+            const int s = i & 1;
+            ok = mbar_wait(empty + 8 * s, ((uint32_t)(i >> 1) & 1u) ^ 1u, status, 1);
+            if (!ok) break;
+            if (of_a) {
+                tc_fence_after();
+#pragma unroll
+                for (int part = 0; part < 2; ++part)
+#pragma unroll
+                    for (int piece = 0; piece < 3; ++piece) {
+                        uint32_t h[16];
+#pragma unroll
+                        for (int u = 0; u < 4; ++u) {
+                            piece_of(4 * part + u, h + 4 * u, piece == 0, piece == 2);
+                            if (piece == 2 && i + 1 < slices) ask(4 * part + u, i + 1);
+                        }
+                        store_columns(tmem_base + ((uint32_t)(warp * 32) << 16) + TMEM_A + (s * 3 + piece) * A_COLS + 16 * part, h);
+                    }
+                tmem_wait_st();
+                tc_fence_before();
+            } else {
+#pragma unroll
+                for (int u = 0; u < UNITS; ++u) {
+                    uint32_t h[3][4];
+#pragma unroll
+                    for (int piece = 0; piece < 3; ++piece) piece_of(u, h[piece], piece == 0, piece == 2);
+                    if (i + 1 < slices) ask(u, i + 1);
+                    const int row = 16 * u + w_row;
+                    const uint32_t at = base + s * STAGE_BYTES + (uint32_t)(row * 128 + ((chunk ^ (row & 7)) << 4));
+#pragma unroll
+                    for (int piece = 0; piece < 3; ++piece) store16(at + piece * PIECE_BYTES, h[piece]);
+                }
+                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            }
+            __syncwarp();
+            if (lane == 0) mbar_arrive(full + 8 * s);
+            if (i > 0) ok = add(i - 1);
+        }
+        if (ok) ok = add(slices - 1);
+        if (none != 0.f) atomicOr(odd, 1);                                  // NaN
+        asm volatile("bar.sync 1, %0;" ::"n"(WORK_WARPS * 32) : "memory");
+        const int row = (warp & 3) * 32 + lane, col0 = (warp >> 2) * 64, m = m0 + row;
+#pragma unroll
+        for (int j = 0; j < 64; ++j) sums[j] = fmaf(sums[j], SHORTFALL, sums[j]);
+        if (*(volatile int*)odd != 0) {
+            const float* x = p.a + (size_t)min(m, p.M - 1) * p.K;
+#pragma unroll 1
+            for (int j0 = 0; j0 < 64; ++j0) {
+                const float* y = p.w + (size_t)min(n0 + col0 + j0, p.N - 1) * p.K;
+                float sum = 0.f;
+                for (int k = k_begin; k < k_end; ++k) sum = fmaf(x[k], y[k], sum);
+#pragma unroll
+                for (int j = 0; j < 64; ++j) if (j == j0) sums[j] = sum;    // registers have no index
+            }
+        }
+        if (p.ranks > 1) {                                                  // every MMA has read the stages: they are free
+            float* park = reinterpret_cast<float*>(smem) + row * PARK_ROW + col0;
+#pragma unroll
+            for (int j = 0; j < 64; j += 4) *reinterpret_cast<float4*>(park + j) = make_float4(sums[j], sums[j + 1], sums[j + 2], sums[j + 3]);
+        } else if (m < p.M && ok) {
+            float* to = p.c + (size_t)m * p.N + n0 + col0;
+#pragma unroll
+            for (int j = 0; j < 64; j += 4) {
+                if (n0 + col0 + j + 3 < p.N && (p.N & 3) == 0) *reinterpret_cast<float4*>(to + j) = make_float4(sums[j], sums[j + 1], sums[j + 2], sums[j + 3]);
+                else
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) if (n0 + col0 + j + e < p.N) to[j + e] = sums[j + e];
+            }
+        }
+    }
+    // The tensor memory goes back before a block waits for its peers: one that waits for tensor memory then waits for none that waits for it.
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    if (*(volatile int*)status != 0) {                                      // a wait gave up: let MMAs in flight finish first
+        const unsigned long long t0 = global_timer();
+        while (global_timer() - t0 < 2000000ull) __nanosleep(1000);
+    }
+    if (warp == WORK_WARPS) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(TMEM_COLS) : "memory");
+    if (p.ranks > 1) {
+        cluster_sync_all();
+        // a block finishes every ranks-th row: a warp a row, four columns a lane
+        if (*(volatile int*)status == 0 && warp < WORK_WARPS) {
+            for (int row = rank + p.ranks * warp; row < TILE && m0 + row < p.M; row += p.ranks * WORK_WARPS) {
+                const uint32_t off = (uint32_t)(row * PARK_ROW + 4 * lane) * 4u;
+                float4 part[MOST_RANKS];
+#pragma unroll
+                for (int r = 0; r < MOST_RANKS; ++r) if (r < p.ranks) part[r] = peer4(map_to_cta(base, (uint32_t)r) + off);
+                float4 sum = part[0];
+#pragma unroll
+                for (int r = 1; r < MOST_RANKS; ++r) if (r < p.ranks) { sum.x += part[r].x; sum.y += part[r].y; sum.z += part[r].z; sum.w += part[r].w; }
+                const int n = n0 + 4 * lane;
+                float* to = p.c + (size_t)(m0 + row) * p.N + n;
+                if (n + 3 < p.N && (p.N & 3) == 0) *reinterpret_cast<float4*>(to) = sum;
+                else {
+                    const float e[4] = {sum.x, sum.y, sum.z, sum.w};
+                    for (int j = 0; j < 4; ++j) if (n + j < p.N) to[j] = e[j];
+                }
+            }
+        }
+        cluster_sync_all();                                                 // nobody leaves while its sums are read
+    }
+}
+
+}  // namespace
+
+// a [M, K], w [N, K], c [M, N] float; K a multiple of 4, a and w 16-byte aligned, c too where N is a multiple of 4; `status` as in qt_gemm_tc.
+extern "C" int qt_gemm_f32_tc(const float* a, const float* w, float* c, int M, int N, int K, int* status, void* stream) {
+    QT_REQUIRE(M >= 0 && N > 0 && K > 0, "gemm_f32_tc: bad sizes M=%d N=%d K=%d", M, N, K);
+    QT_REQUIRE(K % 4 == 0 && (((uintptr_t)a | (uintptr_t)w) & 15) == 0 && (N % 4 != 0 || ((uintptr_t)c & 15) == 0), "gemm_f32_tc: rows must be 16-byte aligned (K=%d)", K);
+    QT_REQUIRE(status != nullptr, "gemm_f32_tc: a status word is required");
+    const int n_tiles = (N + TILE - 1) / TILE, m_tiles = (M + TILE - 1) / TILE, slices = (K + BK - 1) / BK;
+    QT_REQUIRE(m_tiles <= 65535, "gemm_f32_tc: M=%d is too many rows", M);
+    if (M == 0) return QT_OK;
+    // Waves of blocks, one to an SM, times a block's slices and what it does besides (about two slices' time, three with peers).
+    const int sms = sm_count();
+    int ranks = 1, per = slices;
+    long long best = -1;
+    for (int r = 1; r <= MOST_RANKS; ++r) {
+        const int each = (slices + r - 1) / r;
+        if ((r - 1) * each >= slices) continue;                             // a rank without slices
+        const long long cost = (((long long)n_tiles * m_tiles * r + sms - 1) / sms) * (each + (r > 1 ? 3 : 2));
+        if (best < 0 || cost < best) { best = cost; ranks = r; per = each; }
+    }
+    const Params p{a, w, c, M, N, K, ranks, per, status};
+    const size_t smem = 2 * STAGE_BYTES + 1024 + 80;
+    const cudaError_t raised = raise_shared<gemm_f32_tc_kernel>(227 * 1024);
+    if (raised != cudaSuccess) QT_FAIL(QT_ERR_LAUNCH, "gemm_f32_tc: cannot raise shared memory: %s", cudaGetErrorString(raised));
+    launch_kernel_cluster(gemm_f32_tc_kernel, dim3((unsigned)(n_tiles * ranks), (unsigned)m_tiles), dim3(THREADS), smem, (cudaStream_t)stream, (unsigned)ranks, p);
+    QT_CHECK_LAUNCH("gemm_f32_tc");
+    return QT_OK;
+}
+
+QT_DEFINE_LAST_ERROR(gemm_f32_tc)

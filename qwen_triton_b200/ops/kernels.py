@@ -138,6 +138,9 @@ _SIGNATURES = {
     "gemm_f32": {
         "qt_gemm_f32": [_c_ptr, _c_ptr, _c_ptr, _c_int, _c_int, _c_int, _c_ptr],
     },
+    "gemm_f32_tc": {
+        "qt_gemm_f32_tc": [_c_ptr, _c_ptr, _c_ptr, _c_int, _c_int, _c_int, _c_ptr, _c_ptr],
+    },
     "gemm_simt": {
         "qt_gemm_simt": [_c_ptr, _c_ptr, _c_int, _c_ptr, _c_int, _c_int, _c_int, _c_int, _c_ptr],
     },
@@ -1532,6 +1535,17 @@ def gemm_f32(a: torch.Tensor, w: torch.Tensor, out: GemmOut) -> None:
         raise KernelError(f"gemm: a {tuple(a.shape)}, w {tuple(w.shape)}, out {tuple(out.tensor.shape)} do not fit")
     _need(out.tensor, "out", torch.float32)
     _call("gemm_f32", "qt_gemm_f32", _ptr(a), _ptr(w), _ptr(out.tensor), a.shape[0], w.shape[0], a.shape[1], _stream())
+
+
+def gemm_f32_tc(a: torch.Tensor, w: torch.Tensor, out: GemmOut) -> None:
+    """out = a [M, K] @ w [N, K]^T of float operands on the tcgen05 tensor cores, each split into three bfloat16 pieces without loss; K a
+    multiple of 4, 16-byte aligned operands."""
+    _need(a, "a", torch.float32)
+    _need(w, "w", torch.float32)
+    if a.shape[1] != w.shape[1] or out.n_splits != 1 or (out.rows, out.cols) != (a.shape[0], w.shape[0]):
+        raise KernelError(f"gemm: a {tuple(a.shape)}, w {tuple(w.shape)}, out {tuple(out.tensor.shape)} do not fit")
+    _need(out.tensor, "out", torch.float32)
+    _call("gemm_f32_tc", "qt_gemm_f32_tc", _ptr(a), _ptr(w), _ptr(out.tensor), a.shape[0], w.shape[0], a.shape[1], _ptr(_status_word(a.device)), _stream())
 
 
 # ----------------------------------------------------------------------------- sampling
