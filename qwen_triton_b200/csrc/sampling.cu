@@ -35,44 +35,63 @@ __device__ __forceinline__ void for_each_logit(const float* __restrict__ row, in
     if (tail + me < end) f(tail + me, row[tail + me]);
 }
 
-// One block per row.
-__global__ void __launch_bounds__(SMP_THREADS) argmax_kernel(const float* logits, int* __restrict__ out, int vocab) {
+// A cluster of blocks per row, each with a part of the ids; the first block takes the best of theirs.  One block alone draws 60 GB/s of a row.
+constexpr int ARGMAX_BLOCKS = 8;
+
+struct Best { float v; int i; };
+__device__ __forceinline__ Best better(Best a, Best b) { return b.v > a.v || (b.v == a.v && b.i < a.i) ? b : a; }
+__device__ __forceinline__ Best warp_best(Best mine) {
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) {
+        Best other;
+        other.v = __shfl_xor_sync(0xffffffffu, mine.v, off);
+        other.i = __shfl_xor_sync(0xffffffffu, mine.i, off);
+        mine = better(mine, other);
+    }
+    return mine;
+}
+
+__global__ void __launch_bounds__(SMP_THREADS) argmax_kernel(const float* logits, int* __restrict__ out, int vocab, int blocks) {
     pdl_launch_dependents();
+    const int at = blockIdx.x / blocks, part = blockIdx.x - at * blocks;
+    if (blocks > 1) cluster_arrive_started();
     pdl_wait();
     __shared__ float best_v[32];
     __shared__ int best_i[32];
-    const float* row = logits + (size_t)blockIdx.x * vocab;
-    float v = -INFINITY;
-    int idx = 0x7fffffff;
-    for_each_logit(row, 0, vocab, threadIdx.x, blockDim.x, [&](int i, float x) {
-        if (x > v || (x == v && i < idx)) { v = x; idx = i; }
-    });
-    auto better = [](float av, int ai, float bv, int bi) { return bv > av || (bv == av && bi < ai); };
-#pragma unroll
-    for (int off = 16; off > 0; off >>= 1) {
-        const float ov = __shfl_xor_sync(0xffffffffu, v, off);
-        const int oi = __shfl_xor_sync(0xffffffffu, idx, off);
-        if (better(v, idx, ov, oi)) { v = ov; idx = oi; }
-    }
+    __shared__ float part_v[ARGMAX_BLOCKS], part_i[ARGMAX_BLOCKS];       // the first block's: what the parts found, ids as their bits
+    const int per = ((vocab + blocks - 1) / blocks + 3) & ~3;
+    const float* row = logits + (size_t)at * vocab;
+    const Best none = {-INFINITY, 0x7fffffff};
+    Best best = none;
+    for_each_logit(row, part * per, min(vocab, (part + 1) * per), threadIdx.x, blockDim.x, [&](int i, float x) { best = better(best, Best{x, i}); });
+    best = warp_best(best);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    if (lane == 0) { best_v[warp] = v; best_i[warp] = idx; }
+    if (lane == 0) { best_v[warp] = best.v; best_i[warp] = best.i; }
     __syncthreads();
+    if (blocks > 1) cluster_wait_started();
     if (warp == 0) {
-        v = best_v[lane]; idx = best_i[lane];
-#pragma unroll
-        for (int off = 16; off > 0; off >>= 1) {
-            const float ov = __shfl_xor_sync(0xffffffffu, v, off);
-            const int oi = __shfl_xor_sync(0xffffffffu, idx, off);
-            if (better(v, idx, ov, oi)) { v = ov; idx = oi; }
+        best = warp_best(Best{best_v[lane], best_i[lane]});
+        if (blocks == 1) {
+            if (lane == 0) out[at] = best.i == none.i ? 0 : best.i;
+        } else if (lane == 0) {
+            cluster_store_float(&part_v[part], 0, best.v);
+            cluster_store_float(&part_i[part], 0, __int_as_float(best.i));
         }
-        if (lane == 0) out[blockIdx.x] = idx == 0x7fffffff ? 0 : idx;
+    }
+    if (blocks == 1) return;
+    cluster_barrier();
+    if (part == 0 && warp == 0) {
+        best = warp_best(lane < blocks ? Best{part_v[lane], __float_as_int(part_i[lane])} : none);
+        if (lane == 0) out[at] = best.i == none.i ? 0 : best.i;
     }
 }
 
 extern "C" int qt_argmax(const float* logits, int* out, int rows, int vocab, void* stream) {
     QT_REQUIRE(rows >= 0 && vocab > 0, "argmax: bad sizes rows=%d vocab=%d", rows, vocab);
     if (rows == 0) return QT_OK;
-    launch_kernel(argmax_kernel, dim3(rows), dim3(SMP_THREADS), 0, (cudaStream_t)stream, logits, out, vocab);
+    int blocks = ARGMAX_BLOCKS;                                          // two blocks fit an SM; a part is at least one turn of a block's loads
+    while (blocks > 1 && ((long long)rows * blocks > 2 * sm_count() || vocab / blocks < 4 * SMP_THREADS)) blocks /= 2;
+    launch_kernel_cluster(argmax_kernel, dim3(rows * blocks), dim3(SMP_THREADS), 0, (cudaStream_t)stream, (unsigned)blocks, logits, out, vocab, blocks);
     QT_CHECK_LAUNCH("argmax");
     return QT_OK;
 }
