@@ -13,8 +13,11 @@
 // an expert may be gated (its first matrix holds [gate; up] rows, mid = gate(g, u)), and a further term
 // row_scale[t] * base[t] (a shared expert behind a gate of one number per token) may be added to the sum.
 #include "common.cuh"
+#include "few_tokens.cuh"
 
 #include <math.h>
+
+#include <type_traits>
 
 using namespace qt;
 
@@ -281,6 +284,231 @@ template <typename T> static int launch_expert_rows(const ExpertParams& p, cudaS
     return QT_OK;
 }
 
+// ----------------------------------------------------------------------------- few tokens: per expert that any of them chose
+// The same two passes in bfloat16 for up to 32 pairs, an expert's weights read once for all of its pairs (the passes above read them once
+// a pair: 8 tokens of one of 8 experts read twice as many bytes as there are, through L2).  The pairs form groups, of one expert and up to
+// eight pairs each; a group's pairs are the N of mma.sync, the weights its M (few_tokens.cuh).  A pair's weight, on the input or on the
+// output, multiplies float sums.
+constexpr int EG_PAIRS = 32;               // a lane a pair
+constexpr int EG_WARPS = 8;
+constexpr int EG_STEP = 32;                // K elements of a warp's turn: 8 a lane
+constexpr int EG_RANKS = 4;                // most blocks that share K in the second pass
+
+struct PairGroups {
+    int expert[EG_PAIRS];
+    int pair[EG_PAIRS][8];                 // -1 beyond a group's pairs
+    int count;
+};
+// One warp: groups in the order of their first pairs.
+__device__ __forceinline__ void group_pairs(const ExpertParams& p, PairGroups& groups, int lane) {
+    const int pairs = p.n_tokens * p.top;
+    const int e = lane < pairs ? expert_of(p, lane / p.top, lane % p.top) : -1;
+    const unsigned same = __match_any_sync(0xffffffffu, e), before = (1u << lane) - 1u;
+    const int rank = __popc(same & before);
+    const unsigned leaders = __ballot_sync(0xffffffffu, e >= 0 && rank % 8 == 0);
+    unsigned mine = same;                                     // my group's first pair is the (rank / 8 * 8)-th of my expert's
+    for (int skip = rank / 8 * 8; skip > 0; --skip) mine &= mine - 1u;
+    const int leader = __ffs(mine) - 1, group = __popc(leaders & ((1u << leader) - 1u));
+    for (int i = 0; i < 8; ++i) groups.pair[lane][i] = -1;
+    __syncwarp();
+    if (e >= 0) {
+        groups.pair[group][rank % 8] = lane;
+        groups.expert[group] = e;
+    }
+    if (lane == 0) groups.count = __popc(leaders);
+}
+
+// An item is 16 features of a gated expert (32 of another) for the pairs of a group; a block takes every gridDim.x-th of them, and asks for the
+// next item's weights while it finishes one.
+template <bool GATED>
+__global__ void __launch_bounds__(EG_WARPS * 32, 2) expert_up_groups_kernel(const ExpertParams p) {
+    constexpr int DEPTH = 4, FEATS = GATED ? 16 : 32;
+    __shared__ PairGroups groups;
+    __shared__ __align__(16) float sums[2][EG_WARPS][8][36];
+    pdl_launch_dependents();
+    pdl_wait();
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+    if (warp == 0) group_pairs(p, groups, lane);
+    __syncthreads();
+    const int K = p.width, blocks = (p.ff + FEATS - 1) / FEATS, total = blocks * groups.count;
+    const int turns = (K + EG_STEP - 1) / EG_STEP, per = (turns + EG_WARPS - 1) / EG_WARPS;      // of an item, the same for every warp
+    const int items = (int)blockIdx.x < total ? (total - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x : 0;
+    const int mine = items * per;
+    qt_few::Line<8> a[DEPTH][2][2], b[DEPTH];
+    auto ask = [&](int slot, int i) {
+        const int n = i / per, item = (int)blockIdx.x + n * (int)gridDim.x, group = item / blocks, f0 = (item - group * blocks) * FEATS;
+        const int k = (warp + (i - n * per) * EG_WARPS) * EG_STEP + 8 * t, pair = groups.pair[group][g];
+        const __nv_bfloat16* w = (const __nv_bfloat16*)p.up + (size_t)groups.expert[group] * (GATED ? 2 : 1) * p.ff * K + k;
+#pragma unroll
+        for (int r = 0; r < 2; ++r)
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {                     // rows beyond the last repeat it; their sums are not stored
+                const int row = GATED ? r * p.ff + min(f0 + 8 * h + g, p.ff - 1) : min(f0 + 16 * r + 8 * h + g, p.ff - 1);
+                if (k < K) a[slot][r][h] = qt_few::load_weight<8>(w + (size_t)row * K);
+                else a[slot][r][h] = qt_few::Line<8>{};
+            }
+        if (k < K && pair >= 0) b[slot] = qt_few::load_rows<8>((const __nv_bfloat16*)p.x + (size_t)(pair / p.top) * K + k);
+        else b[slot] = qt_few::Line<8>{};
+    };
+    // the block's sums of an item, and its features
+    auto finish = [&](int n) {
+        const float (*part)[8][36] = sums[n & 1];
+        const int item = (int)blockIdx.x + n * (int)gridDim.x, group = item / blocks, f0 = (item - group * blocks) * FEATS;
+        const int slot = threadIdx.x / 8, l = threadIdx.x % 8, of = groups.pair[group][slot];
+        if (of < 0) return;
+        const float weight = p.in_weights ? p.in_weights[of] : 1.f;
+        __nv_bfloat16* mid = (__nv_bfloat16*)p.mid + (size_t)of * p.ff;
+        if (GATED) {
+            float2 gate = make_float2(0.f, 0.f), up = make_float2(0.f, 0.f);
+#pragma unroll
+            for (int s = 0; s < EG_WARPS; ++s) {
+                const float2 gs = *reinterpret_cast<const float2*>(&part[s][slot][2 * l]), us = *reinterpret_cast<const float2*>(&part[s][slot][2 * l + 16]);
+                gate.x += gs.x; gate.y += gs.y; up.x += us.x; up.y += us.y;
+            }
+            const int f = f0 + 2 * l;                         // ff is a multiple of 8
+            if (f < p.ff)
+                *reinterpret_cast<__nv_bfloat162*>(mid + f) = __floats2bfloat162_rn(gated_value<false>(gate.x * weight, up.x * weight, p.act, p.limit),
+                                                                                    gated_value<false>(gate.y * weight, up.y * weight, p.act, p.limit));
+        } else {
+            float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+            for (int s = 0; s < EG_WARPS; ++s) {
+                const float4 x = *reinterpret_cast<const float4*>(&part[s][slot][4 * l]);
+                v.x += x.x; v.y += x.y; v.z += x.z; v.w += x.w;
+            }
+            const int f = f0 + 4 * l;
+            if (f < p.ff) {
+                *reinterpret_cast<__nv_bfloat162*>(mid + f) = __floats2bfloat162_rn(gate_activation<false>(v.x * weight, p.act), gate_activation<false>(v.y * weight, p.act));
+                *reinterpret_cast<__nv_bfloat162*>(mid + f + 2) = __floats2bfloat162_rn(gate_activation<false>(v.z * weight, p.act), gate_activation<false>(v.w * weight, p.act));
+            }
+        }
+    };
+    float c[2][4] = {};
+#pragma unroll
+    for (int u = 0; u < DEPTH; ++u)
+        if (u < mine) ask(u, u);
+    for (int i0 = 0; i0 < mine; i0 += DEPTH) {
+#pragma unroll
+        for (int u = 0; u < DEPTH; ++u) {
+            const int i = i0 + u;
+            if (i >= mine) break;
+            qt_few::turn_product<2>(c, a[u], b[u]);
+            if (i + DEPTH < mine) ask(u, i + DEPTH);
+            if ((i + 1) % per == 0) {                         // the item's last turn
+                const int n = i / per;
+#pragma unroll
+                for (int r = 0; r < 2; ++r)
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) {
+                        sums[n & 1][warp][2 * t + (e & 1)][16 * r + g + 8 * (e >> 1)] = c[r][e];
+                        c[r][e] = 0.f;
+                    }
+                __syncthreads();                              // two sets of sums: the next item's go into the other
+                if (threadIdx.x < 64) finish(n);
+            }
+        }
+    }
+}
+
+// grid (blocks of 16 columns x RANKS): a cluster's blocks share K, every block walks all groups; a token's sums meet in the block that
+// finishes it.
+template <int RANKS>
+__global__ void __launch_bounds__(EG_WARPS * 32, 2) expert_down_groups_kernel(const ExpertParams p) {
+    constexpr int DEPTH = 8;
+    __shared__ PairGroups groups;
+    __shared__ __align__(16) float sums[EG_WARPS][EG_PAIRS][16];
+    __shared__ __align__(16) float parts[RANKS][EG_PAIRS][16];
+    pdl_launch_dependents();
+    if (RANKS > 1) cluster_arrive_started();
+    pdl_wait();
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+    const int rank = blockIdx.x % RANKS, c0 = blockIdx.x / RANKS * 16, K = p.ff, pairs = p.n_tokens * p.top;
+    if (warp == 0) group_pairs(p, groups, lane);
+    __syncthreads();
+    const int first = rank + RANKS * warp, stride = RANKS * EG_WARPS;
+    const int turns = (K + EG_STEP - 1) / EG_STEP, per = first < turns ? (turns - first + stride - 1) / stride : 0;   // of a group
+    const int mine = per * groups.count;
+    qt_few::Line<8> a[DEPTH][1][2], b[DEPTH];
+    auto ask = [&](int slot, int i) {                         // turns of the groups one after the other
+        const int group = i / per, k = (first + (i - group * per) * stride) * EG_STEP + 8 * t, pair = groups.pair[group][g];
+        const __nv_bfloat16* w = (const __nv_bfloat16*)p.down + (size_t)groups.expert[group] * p.width * K + k;
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            if (k < K) a[slot][0][h] = qt_few::load_weight<8>(w + (size_t)min(c0 + 8 * h + g, p.width - 1) * K);
+            else a[slot][0][h] = qt_few::Line<8>{};
+        }
+        if (k < K && pair >= 0) b[slot] = qt_few::load_rows<8>((const __nv_bfloat16*)p.mid + (size_t)pair * K + k);
+        else b[slot] = qt_few::Line<8>{};
+    };
+    float c[1][4] = {};
+    auto put = [&](int group) {
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            const int pair = groups.pair[group][2 * t + (e & 1)];
+            if (pair >= 0) sums[warp][pair][g + 8 * (e >> 1)] = c[0][e];
+            c[0][e] = 0.f;
+        }
+    };
+#pragma unroll
+    for (int u = 0; u < DEPTH; ++u)
+        if (u < mine) ask(u, u);
+    for (int i0 = 0; i0 < mine; i0 += DEPTH) {
+#pragma unroll
+        for (int u = 0; u < DEPTH; ++u) {
+            const int i = i0 + u;
+            if (i >= mine) break;
+            qt_few::turn_product<1>(c, a[u], b[u]);
+            if (i + DEPTH < mine) ask(u, i + DEPTH);
+            if ((i + 1) % per == 0) put(i / per);
+        }
+    }
+    if (per == 0)
+        for (int group = 0; group < groups.count; ++group) put(group);
+    __syncthreads();
+    if (RANKS > 1) cluster_wait_started();
+    for (int item = threadIdx.x; item < pairs * 4; item += EG_WARPS * 32) {
+        const int pair = item / 4, at = item % 4 * 4;
+        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+        for (int s = 0; s < EG_WARPS; ++s) {
+            const float4 part = *reinterpret_cast<const float4*>(&sums[s][pair][at]);
+            v.x += part.x; v.y += part.y; v.z += part.z; v.w += part.w;
+        }
+        if (RANKS > 1) qt_few::cluster_store4(&parts[rank][pair][at], (uint32_t)(pair / p.top % RANKS), v);
+        else *reinterpret_cast<float4*>(&parts[0][pair][at]) = v;
+    }
+    if (RANKS > 1) cluster_barrier();
+    else __syncthreads();
+    for (int item = threadIdx.x; item < (p.n_tokens + RANKS - 1) / RANKS * 16; item += EG_WARPS * 32) {
+        const int token = rank + item / 16 * RANKS, col = item % 16;
+        if (token >= p.n_tokens || c0 + col >= p.width) continue;
+        float total = 0.f;
+        for (int k = 0; k < p.top; ++k) {                     // in the order of the table's row
+            const int pair = token * p.top + k;
+            float v = 0.f;
+#pragma unroll
+            for (int s = 0; s < RANKS; ++s) v += parts[s][pair][col];
+            total += v * (p.pair_weights ? p.pair_weights[pair] : 1.f);
+        }
+        expert_put(p, token, c0 + col, total);
+    }
+}
+
+static int launch_expert_groups(const ExpertParams& p, cudaStream_t s) {
+    const int feats = p.gated ? 16 : 32, items = (p.ff + feats - 1) / feats * p.n_tokens * p.top;
+    const dim3 block(EG_WARPS * 32), up(items < 2 * sm_count() ? items : 2 * sm_count());
+    if (p.gated) launch_kernel(expert_up_groups_kernel<true>, up, block, 0, s, p);
+    else launch_kernel(expert_up_groups_kernel<false>, up, block, 0, s, p);
+    QT_CHECK_LAUNCH("expert_up");
+    // as many blocks to a column as leave every warp of theirs two turns of a group
+    const int turns = (p.ff + EG_STEP - 1) / EG_STEP, columns = (p.width + 15) / 16;
+    if (turns >= 2 * EG_RANKS * EG_WARPS) launch_kernel_cluster(expert_down_groups_kernel<EG_RANKS>, dim3(columns * EG_RANKS), block, 0, s, EG_RANKS, p);
+    else if (turns >= 4 * EG_WARPS) launch_kernel_cluster(expert_down_groups_kernel<2>, dim3(columns * 2), block, 0, s, 2, p);
+    else launch_kernel(expert_down_groups_kernel<1>, dim3(columns), block, 0, s, p);
+    QT_CHECK_LAUNCH("expert_down");
+    return QT_OK;
+}
+
 static int check_experts(const char* name, int n_tokens, int vocab, int top, int experts, int width, int ff, int act) {
     QT_REQUIRE(n_tokens >= 0 && vocab > 0 && top > 0 && experts > 0 && top <= experts, "%s: bad routing sizes T=%d V=%d top=%d E=%d", name, n_tokens, vocab, top, experts);
     QT_REQUIRE(width > 0 && ff > 0, "%s: bad sizes width=%d ff=%d", name, width, ff);
@@ -305,6 +533,8 @@ extern "C" int qt_experts_by_pair(const void* x, const int* token_ids, const int
         const size_t smem_up = (size_t)width * sizeof(float), smem_down = (size_t)top * ff * sizeof(float);
         const dim3 grid_up(n_tokens * top, (ff + per_block - 1) / per_block), grid_down(n_tokens, (width + per_block - 1) / per_block);
         // 16-byte loads: rows of both weights, of x and of mid start on 16-byte boundaries
+        if (std::is_same<T, __nv_bfloat16>::value && n_tokens * top <= EG_PAIRS && width % 8 == 0 && ff % 8 == 0 &&
+            (((uintptr_t)up | (uintptr_t)down | (uintptr_t)x | (uintptr_t)mid) & 15) == 0) return launch_expert_groups(p, s);
         if (width % 8 == 0 && ff % 8 == 0 && (((uintptr_t)up | (uintptr_t)down | (uintptr_t)x | (uintptr_t)mid) & 15) == 0) return launch_expert_rows<T>(p, s);
         if (smem_up > 48 * 1024) cudaFuncSetAttribute(expert_up_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_up);
         if (smem_down > 48 * 1024) cudaFuncSetAttribute(expert_down_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_down);
