@@ -236,6 +236,11 @@ class Linear:
                 out = self.runtime.workspace.view(f"{self.key}.out" if self.float_out else f"{self.key}.wide", rows, self.out_features)
             kernels.gemm_fused_store(x, self.weight, out.view(rows, self.out_features), splits=self._fused_splits(rows), bias=self._loaded_bias(), few=self.few_plan(x))
             return GemmOut(out.view(1, rows, self.out_features))
+        few = self.few_plan(x) if out is None and self.fused_plans else None
+        if few is not None:                # one finished plane, where the products below would hand partial sums to the consumer
+            plane = self.runtime.workspace.view(f"{self.key}.out" if self.float_out else f"{self.key}.wide", rows, self.out_features)
+            kernels.gemm_fused_store(x, self.weight, plane, bias=self._loaded_bias(), few=few)
+            return GemmOut(plane.view(1, rows, self.out_features))
         splits = self.plan_splits(rows)
         if out is None and splits > 1:
             result = GemmOut(self.runtime.workspace.view(f"{self.key}.partial", splits, rows, self.out_features))
