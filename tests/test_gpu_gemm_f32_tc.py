@@ -1,0 +1,46 @@
+"""Float products on the tensor cores (csrc/gemm_f32_tc.cu) against 64 bits: edges of tiles, slices and ranks, numbers of very different
+sizes, and numbers that have no bfloat16 pieces."""
+import pytest
+import torch
+
+from qwen_triton_b200.ops import kernels
+from qwen_triton_b200.ops.kernels import GemmOut
+from test_gpu_kernels import DEV, rand
+
+pytestmark = pytest.mark.gpu
+
+
+def both(a, w):
+    out = [torch.full((1, a.shape[0], w.shape[0]), float("nan"), device=DEV) for _ in range(2)]
+    kernels.gemm_f32_tc(a, w, GemmOut(out[0]))
+    kernels.gemm_f32(a, w, GemmOut(out[1]))
+    kernels.check_status(DEV)
+    return out[0][0], out[1][0]
+
+
+@pytest.mark.parametrize("m, n, k", [(1, 1, 4), (9, 64, 4), (128, 128, 64), (129, 130, 68), (33, 200, 2052), (300, 131, 1000), (549, 1024, 1024), (40, 513, 12288)])
+@pytest.mark.parametrize("kind", ["normal", "positive", "wide"])
+def test_errors_against_64_bits(m, n, k, kind):
+    a, w = rand(m, k, seed=1), rand(n, k, seed=2, scale=0.02)
+    if kind == "positive":
+        a, w = a.abs(), w.abs()
+    if kind == "wide":
+        a = a * torch.exp(6 * rand(m, k, seed=3))
+    want = a.double() @ w.double().T
+    got, _ = both(a, w)
+    # Products are exact but for pieces below 2^-25 of them; a slice of 64 is four truncated additions of its large products (at most an ulp, 2^-23 of
+    # what is summed so far, each), and K / 64 slices are rounded additions: 8 x 2^-24 of the absolute sums bounds both with room.
+    assert bool(((got.double() - want).abs() <= 8 * 2.0 ** -24 * (a.double().abs() @ w.double().abs().T)).all())
+    assert float((got.double() - want).norm()) <= 2e-7 * float(want.norm())
+
+
+def test_numbers_without_pieces_are_multiplied_as_floats():
+    a, w = rand(140, 256, seed=4), rand(200, 256, seed=5)
+    a[3, 5], a[7, 9], a[130, 3], w[150, 7], w[151, 3] = float("inf"), float("nan"), 3.4e38, -float("inf"), 1.0
+    got, want = both(a, w)
+    assert torch.equal(torch.isnan(got), torch.isnan(want))
+    finite = torch.isfinite(want)
+    assert torch.equal(finite, torch.isfinite(got))
+    assert torch.equal(got[~finite & ~torch.isnan(want)], want[~finite & ~torch.isnan(want)])
+    exact = a.double() @ w.double().T
+    assert bool(((got.double() - exact).abs()[finite] <= 2.0 ** -20 * (a.double().abs() @ w.double().abs().T)[finite]).all())
