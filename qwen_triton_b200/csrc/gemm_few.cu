@@ -167,22 +167,15 @@ int dispatch(const void* w, const void* x, int K, int warps, const EpilogueParam
         if (warps == 16) return launch<EPI, RT, 1, 16, 16, DEPTH>(w, x, K, e, stream);
         return launch<EPI, RT, 1, 8, 16, DEPTH>(w, x, K, e, stream);
     }
-    if (e.M <= 16) {
-        if (warps == 16) return launch<EPI, RT, 2, 16, 16, DEPTH2>(w, x, K, e, stream);
-        return launch<EPI, RT, 2, 8, 16, DEPTH2>(w, x, K, e, stream);
-    }
-    if constexpr (EPI == EPI_STORE) {                               // four tiles of tokens: 16 bytes a lane, for the registers
-        if (e.M <= 24) return launch<EPI, RT, 3, 8, 8, RT == 1 ? 4 : 2>(w, x, K, e, stream);
-        return launch<EPI, RT, 4, 8, 8, RT == 1 ? 3 : 2>(w, x, K, e, stream);
-    }
-    QT_FAIL(QT_ERR_ARG, "gemm_few: %d tokens (up to 32 for the plain store, up to 16 otherwise)", e.M);
+    if (warps == 16) return launch<EPI, RT, 2, 16, 16, DEPTH2>(w, x, K, e, stream);
+    return launch<EPI, RT, 2, 8, 16, DEPTH2>(w, x, K, e, stream);
 }
 
 }  // namespace
 
-// x [M, K] bfloat16 (M up to 16, or 32 if the product is only stored), w [N, K] bfloat16, K a multiple of 16 and both 32-byte aligned.  `epilogue` picks what is done with
+// x [M, K] bfloat16 (M up to 16), w [N, K] bfloat16, K a multiple of 16 and both 32-byte aligned.  `epilogue` picks what is done with
 // the product and which of the pointers are read, as in qt_gemm_fused; `block_rows` (16, or 32 as q/k/v and the gate always take) is
-// how many rows of w a block holds, and the width of the tiles whose sums of squares sq_out receives; `warps` (8 or 16; beyond 16 tokens 8) share K.
+// how many rows of w a block holds, and the width of the tiles whose sums of squares sq_out receives; `warps` (8 or 16) share K.
 extern "C" int qt_gemm_few(const void* x, const void* w, int M, int N, int K, int block_rows, int warps, int epilogue,
                            const float* sq_in, int sq_tiles, int norm_width, float eps, const float* bias,
                            void* out, int out_dtype, int act, float limit,
@@ -191,7 +184,7 @@ extern "C" int qt_gemm_few(const void* x, const void* w, int M, int N, int K, in
                            const int* block_table, int max_blocks, const float* q_w, const float* k_w, float qk_eps,
                            const float* cos_sin, int rotary_dim, int max_pos, int nq, int nkv, int d, int page_tokens,
                            int ring_tokens, int write_kv, int interleaved, void* stream) {
-    QT_REQUIRE(M > 0 && M <= (epilogue == EPI_STORE || epilogue == EPI_ACTIVATED ? 32 : 16) && N > 0 && K > 0, "gemm_few: bad sizes M=%d N=%d K=%d (up to 16 tokens, 32 for the store)", M, N, K);
+    QT_REQUIRE(M > 0 && M <= 16 && N > 0 && K > 0, "gemm_few: bad sizes M=%d N=%d K=%d (up to 16 tokens)", M, N, K);
     QT_REQUIRE(K % 16 == 0 && (uintptr_t)x % 32 == 0 && (uintptr_t)w % 32 == 0, "gemm_few: rows must start on 32-byte boundaries (K=%d)", K);
     QT_REQUIRE(warps == 8 || warps == 16, "gemm_few: %d warps (8 or 16)", warps);
     QT_REQUIRE(block_rows == 32 || (block_rows == 16 && epilogue != EPI_SWIGLU && epilogue != EPI_QKV), "gemm_few: blocks of %d rows for epilogue %d", block_rows, epilogue);

@@ -1805,13 +1805,12 @@ def fused_supported(w: torch.Tensor) -> bool:
 
 
 FEW_MAX_ROWS = 16           # most tokens the kernel for few of them takes (csrc/gemm_few.cu)
-FEW_MAX_STORED_ROWS = 32    # and most where the product is only stored
 
 
 def few_supported(x, w: torch.Tensor) -> bool:
     """Whether rows and weight can be read 32 bytes at a time, as the kernel for few tokens does."""
     a = x.tensor if isinstance(x, ScaledRows) else x
-    return 0 < a.shape[0] <= FEW_MAX_STORED_ROWS and w.shape[1] % 16 == 0 and w.data_ptr() % 32 == 0 and a.data_ptr() % 32 == 0
+    return 0 < a.shape[0] <= FEW_MAX_ROWS and w.shape[1] % 16 == 0 and w.data_ptr() % 32 == 0 and a.data_ptr() % 32 == 0
 
 
 def fused_qkv_supported(head_dim: int, rotary_dim: int) -> bool:

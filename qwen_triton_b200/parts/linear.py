@@ -186,7 +186,7 @@ class Linear:
                 return stages
         return 0
 
-    def few_plan(self, x, most: int = kernels.FEW_MAX_ROWS) -> tuple[int, int] | None:
+    def few_plan(self, x) -> tuple[int, int] | None:
         """(weight rows a block, warps a block) where these rows take the kernel for few tokens (csrc/gemm_few.cu), else None.
 
         It is the faster form where the launch before it and its own chain bound a product, not the weight's bytes: weights of up to
@@ -196,10 +196,8 @@ class Linear:
         728 us a step instead of 634).  16 warps a block where their sums are short of the weight's arrival: beyond 8 tokens (797 us against 857 with
         8), and where K is longest for its rows (570 to 590 against 634)."""
         rows = x.shape[0]
-        if not 0 < rows <= most or self.weight is None or self.weight.numel() > _FEW_WEIGHT or not kernels.few_supported(x, self.weight):
+        if not 0 < rows <= kernels.FEW_MAX_ROWS or self.weight is None or self.weight.numel() > _FEW_WEIGHT or not kernels.few_supported(x, self.weight):
             return None
-        if rows > kernels.FEW_MAX_ROWS:    # every block reads all of the tokens: half as many blocks where that still gives every SM one
-            return (32 if self.out_features >= 32 * self.runtime.sm_count else 16), 8
         wide = self.role in ("gate", "qkv")
         return (32 if wide else 16), (8 if wide and rows <= 8 else 16)
 
@@ -238,7 +236,7 @@ class Linear:
                 out = self.runtime.workspace.view(f"{self.key}.out" if self.float_out else f"{self.key}.wide", rows, self.out_features)
             kernels.gemm_fused_store(x, self.weight, out.view(rows, self.out_features), splits=self._fused_splits(rows), bias=self._loaded_bias(), few=self.few_plan(x))
             return GemmOut(out.view(1, rows, self.out_features))
-        few = self.few_plan(x, kernels.FEW_MAX_STORED_ROWS) if out is None and self.fused_plans else None
+        few = self.few_plan(x) if out is None and self.fused_plans else None
         if few is not None:                # one finished plane, where the products below would hand partial sums to the consumer
             plane = self.runtime.workspace.view(f"{self.key}.out" if self.float_out else f"{self.key}.wide", rows, self.out_features)
             kernels.gemm_fused_store(x, self.weight, plane, bias=self._loaded_bias(), few=few)

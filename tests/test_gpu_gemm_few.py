@@ -13,7 +13,7 @@ BF16 = torch.bfloat16
 FORMS = [(16, 8), (32, 8), (32, 16), (16, 16)]
 
 
-@pytest.mark.parametrize("rows, n, k", [(1, 503, 96), (8, 4096, 1024), (16, 130, 512), (9, 33, 2064), (3, 15, 16), (5, 128, 4112), (1, 1024, 3072), (17, 200, 1040), (32, 136, 2048)])
+@pytest.mark.parametrize("rows, n, k", [(1, 503, 96), (8, 4096, 1024), (16, 130, 512), (9, 33, 2064), (3, 15, 16), (5, 128, 4112), (1, 1024, 3072)])
 @pytest.mark.parametrize("few", FORMS)
 @pytest.mark.parametrize("out_dtype", [torch.float32, BF16])
 def test_store(rows, n, k, few, out_dtype):
@@ -87,9 +87,7 @@ def test_qkv_equals_the_product_for_more_tokens(nq, nkv, d, rotary, ring, own_kv
 def test_what_it_refuses():
     x, w, out = rand(4, 64, seed=1, dtype=BF16), rand(256, 64, seed=2, dtype=BF16), torch.empty(4, 256, device=DEV)
     with pytest.raises(kernels.KernelError, match="up to 16 tokens"):
-        kernels.gemm_fused_store(rand(33, 64, seed=1, dtype=BF16), w, torch.empty(33, 256, device=DEV), few=(32, 8))
-    with pytest.raises(kernels.KernelError, match="up to 16 tokens"):
-        kernels.gemm_fused_residual(rand(17, 64, seed=1, dtype=BF16), w, torch.empty(17, 256, device=DEV), few=(32, 8))
+        kernels.gemm_fused_store(rand(17, 64, seed=1, dtype=BF16), w, torch.empty(17, 256, device=DEV), few=(32, 8))
     with pytest.raises(kernels.KernelError, match="32-byte"):
         kernels.gemm_fused_store(rand(4, 72, seed=1, dtype=BF16), rand(256, 72, seed=2, dtype=BF16), out, few=(32, 8))
     with pytest.raises(kernels.KernelError, match="rows for epilogue"):
