@@ -608,9 +608,7 @@ __global__ void qk_norm_rope_write_kernel(const QkvParams p) {
 // a lane holds the E-element pieces (j, j + d/2) of a rotation pair in registers and nothing passes through shared
 // memory.  One warp takes HEADS_PER_WARP consecutive heads of one token, so that position, page and cos/sin are
 // looked up once.  Same arithmetic as the kernel above: float norm, weight, then rotation.
-constexpr int HEADS_PER_WARP = 4;
-// Blocks of four warps an SM: what the registers of two runs leave room for.
-constexpr int pairs_blocks(size_t element, int rounds) { return (element == 2 ? 7 : 5) / rounds; }
+constexpr int HEADS_PER_WARP = 4, PAIRS_BLOCKS = 8;                     // blocks of four warps an SM
 
 template <int E> struct Piece;
 template <> struct Piece<1> { float v[1]; };
@@ -643,7 +641,7 @@ template <int E> __device__ __forceinline__ void store_piece(__nv_bfloat16* p, c
 template <typename T, int E> struct alignas(sizeof(T) * E) Raw { T v[E]; };
 
 template <typename TI, typename TO, int E, int IT>
-__global__ void __launch_bounds__(128, pairs_blocks(sizeof(TI), IT)) qk_norm_rope_pairs_kernel(const QkvParams p, int runs) {
+__global__ void __launch_bounds__(128, IT == 1 ? PAIRS_BLOCKS : PAIRS_BLOCKS / 2) qk_norm_rope_pairs_kernel(const QkvParams p, int runs) {
     pdl_launch_dependents();
     const int lane = threadIdx.x & 31, stride = gridDim.x * 4, items = p.n_tokens * runs;
     int item = blockIdx.x * 4 + (threadIdx.x >> 5);
@@ -690,19 +688,19 @@ __global__ void __launch_bounds__(128, pairs_blocks(sizeof(TI), IT)) qk_norm_rop
             const int page = p.block_table[(size_t)p.token_seq[t] * p.max_blocks + slot_pos / p.page_tokens];
             r.cache_row = ((size_t)page * p.nkv * p.page_tokens + (slot_pos % p.page_tokens)) * (size_t)p.d;
         }
-        if constexpr (sizeof(TI) == 4) {                                // partial sums are floats
-            for (int s = 1; s < p.n_splits; ++s)
+        if constexpr (sizeof(TI) == 4)                                  // partial sums are floats
+        for (int s = 1; s < p.n_splits; ++s) {
 #pragma unroll
-                for (int hh = 0; hh < HEADS_PER_WARP; ++hh) {
-                    const TI* src = in + (head0 + hh < heads_total ? hh : 0) * p.d + (size_t)s * p.split_stride;
+            for (int hh = 0; hh < HEADS_PER_WARP; ++hh) {
+                const TI* src = in + (head0 + hh < heads_total ? hh : 0) * p.d + (size_t)s * p.split_stride;
 #pragma unroll
-                    for (int it = 0; it < IT; ++it) {
-                        const int j = (it * 32 + lane) * E;
-                        const Piece<E> dl = load_piece<E>(src + j), dh = load_piece<E>(src + half + j);
+                for (int it = 0; it < IT; ++it) {
+                    const int j = (it * 32 + lane) * E;
+                    const Piece<E> dl = load_piece<E>(src + j), dh = load_piece<E>(src + half + j);
 #pragma unroll
-                        for (int e = 0; e < E; ++e) { r.lo[hh][it].v[e] += dl.v[e]; r.hi[hh][it].v[e] += dh.v[e]; }
-                    }
+                    for (int e = 0; e < E; ++e) { r.lo[hh][it].v[e] += dl.v[e]; r.hi[hh][it].v[e] += dh.v[e]; }
                 }
+            }
         }
     };
     if (item >= items) return;
@@ -909,7 +907,7 @@ extern "C" int qt_qk_norm_rope_write(const void* qkv, int in_dtype, int n_splits
     if (pe && !own_values && !(unit_norm && (q_weight || k_weight)) && !whole_norm && !extra_cols && pair_aligned && n_tokens >= 256 && (long long)n_tokens * (nq + 2 * nkv) < (1ll << 30) && (in_dtype == QT_F32 || (in_dtype == QT_BF16 && n_splits == 1)) && out_dtype == QT_BF16) {
         const int heads_total = nq + (kv_in_proj ? 2 * nkv : 0);
         const int runs = ((write_kv ? heads_total : nq) + HEADS_PER_WARP - 1) / HEADS_PER_WARP;
-        const long long blocks = ((long long)n_tokens * runs + 3) / 4, resident = (long long)pairs_blocks(in_dtype == QT_F32 ? 4 : 2, pit) * sm_count();
+        const long long blocks = ((long long)n_tokens * runs + 3) / 4, resident = (long long)(pit == 1 ? PAIRS_BLOCKS : PAIRS_BLOCKS / 2) * sm_count();
         const dim3 pgrid((unsigned)(blocks < resident ? blocks : resident));
 #define QT_LAUNCH_PAIRS(TI, E, IT) launch_kernel(qk_norm_rope_pairs_kernel<TI, __nv_bfloat16, E, IT>, pgrid, dim3(128), 0, s, p, runs)
         if (in_dtype == QT_BF16) {
