@@ -608,7 +608,7 @@ __global__ void qk_norm_rope_write_kernel(const QkvParams p) {
 // a lane holds the E-element pieces (j, j + d/2) of a rotation pair in registers and nothing passes through shared
 // memory.  One warp takes HEADS_PER_WARP consecutive heads of one token, so that position, page and cos/sin are
 // looked up once.  Same arithmetic as the kernel above: float norm, weight, then rotation.
-constexpr int HEADS_PER_WARP = 4, PAIRS_BLOCKS = 8;                     // blocks of four warps an SM
+constexpr int HEADS_PER_WARP = 4;
 
 template <int E> struct Piece;
 template <> struct Piece<1> { float v[1]; };
@@ -635,60 +635,33 @@ template <int E> __device__ __forceinline__ void store_piece(__nv_bfloat16* p, c
     else p[0] = __float2bfloat16_rn(r.v[0]);
 }
 
-// What bounds it is a chain of lookups (position, then its cos and sin and its page, beside the heads themselves), not bytes: blocks that take
-// one run of heads each and leave wait it out once a wave.  So the grid is what is resident at once and a warp walks the runs (item = token x
-// runs + run), asking for the next run's lookups and heads while it finishes one.
-template <typename T, int E> struct alignas(sizeof(T) * E) Raw { T v[E]; };
-
+// blockIdx.x is the token, blockIdx.y * 4 + warp the run of heads.
 template <typename TI, typename TO, int E, int IT>
-__global__ void __launch_bounds__(128, IT == 1 ? PAIRS_BLOCKS : PAIRS_BLOCKS / 2) qk_norm_rope_pairs_kernel(const QkvParams p, int runs) {
+__global__ void __launch_bounds__(128) qk_norm_rope_pairs_kernel(const QkvParams p) {
     pdl_launch_dependents();
-    const int lane = threadIdx.x & 31, stride = gridDim.x * 4, items = p.n_tokens * runs;
-    int item = blockIdx.x * 4 + (threadIdx.x >> 5);
+    pdl_wait();
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int heads_total = p.nq + (p.kv_in_proj ? 2 * p.nkv : 0);
+    const int t = blockIdx.x;
+    const int head0 = (blockIdx.y * 4 + warp) * HEADS_PER_WARP;
+    if (head0 >= heads_total || (head0 >= p.nq && !p.write_kv)) return;
     const int half = p.d >> 1;
-    Piece<E> wq_lo[IT], wq_hi[IT], wk_lo[IT], wk_hi[IT];                // the norm weights: the same for every item
-#pragma unroll
-    for (int it = 0; it < IT; ++it) {
-        const int j = (it * 32 + lane) * E;
-        if (p.q_weight) { wq_lo[it] = load_piece<E>(p.q_weight + j); wq_hi[it] = load_piece<E>(p.q_weight + half + j); }
-        if (p.k_weight) { wk_lo[it] = load_piece<E>(p.k_weight + j); wk_hi[it] = load_piece<E>(p.k_weight + half + j); }
-    }
-    struct Run {
-        Raw<TI, E> lo[HEADS_PER_WARP][IT], hi[HEADS_PER_WARP][IT];      // as they are stored: half the registers of floats
-        Piece<E> c[IT], sn[IT];
-        size_t cache_row;    // element offset of (page, kv head 0, token) in the caches
-    };
-    // positions, pages and tables come with the step, not from the kernel before
-    auto position = [&](int i) { return i < items ? p.token_pos[i / runs] : 0; };
-    // every load of a run is issued before the first store of the one before it (the compiler cannot move loads across the
+    const TI* in = (const TI*)p.qkv + ((size_t)t * heads_total + head0) * p.d;
+
+    // every load of the warp's heads is issued before the first store (the compiler cannot move loads across the
     // stores itself: it does not know that the projection and the outputs are different memory)
-    auto fetch = [&](Run& r, int i, int pos) {
-        const int t = i / runs, head0 = (i - t * runs) * HEADS_PER_WARP;
-        const TI* in = (const TI*)p.qkv + ((size_t)t * heads_total + head0) * p.d;
+    Piece<E> lo[HEADS_PER_WARP][IT], hi[HEADS_PER_WARP][IT];
 #pragma unroll
-        for (int hh = 0; hh < HEADS_PER_WARP; ++hh) {
-            const TI* src = in + (head0 + hh < heads_total ? hh : 0) * p.d;
-#pragma unroll
-            for (int it = 0; it < IT; ++it) {
-                const int j = (it * 32 + lane) * E;
-                r.lo[hh][it] = *reinterpret_cast<const Raw<TI, E>*>(src + j);
-                r.hi[hh][it] = *reinterpret_cast<const Raw<TI, E>*>(src + half + j);
-            }
-        }
-        const float* cs = p.cos_sin + (size_t)(pos < p.max_pos ? pos : p.max_pos - 1) * p.d;
+    for (int hh = 0; hh < HEADS_PER_WARP; ++hh) {
+        const TI* src = in + (head0 + hh < heads_total ? hh : 0) * p.d;
 #pragma unroll
         for (int it = 0; it < IT; ++it) {
-            r.c[it] = load_piece<E>(cs + (it * 32 + lane) * E);
-            r.sn[it] = load_piece<E>(cs + half + (it * 32 + lane) * E);
+            const int j = (it * 32 + lane) * E;
+            lo[hh][it] = load_piece<E>(src + j);
+            hi[hh][it] = load_piece<E>(src + half + j);
         }
-        r.cache_row = 0;
-        if (p.write_kv && head0 + HEADS_PER_WARP > p.nq) {
-            const int slot_pos = p.ring_tokens > 0 ? pos % p.ring_tokens : pos;
-            const int page = p.block_table[(size_t)p.token_seq[t] * p.max_blocks + slot_pos / p.page_tokens];
-            r.cache_row = ((size_t)page * p.nkv * p.page_tokens + (slot_pos % p.page_tokens)) * (size_t)p.d;
-        }
-        if constexpr (sizeof(TI) == 4)                                  // partial sums are floats
+    }
+    if (p.n_splits > 1) {
         for (int s = 1; s < p.n_splits; ++s) {
 #pragma unroll
             for (int hh = 0; hh < HEADS_PER_WARP; ++hh) {
@@ -698,80 +671,76 @@ __global__ void __launch_bounds__(128, IT == 1 ? PAIRS_BLOCKS : PAIRS_BLOCKS / 2
                     const int j = (it * 32 + lane) * E;
                     const Piece<E> dl = load_piece<E>(src + j), dh = load_piece<E>(src + half + j);
 #pragma unroll
-                    for (int e = 0; e < E; ++e) { r.lo[hh][it].v[e] += dl.v[e]; r.hi[hh][it].v[e] += dh.v[e]; }
+                    for (int e = 0; e < E; ++e) { lo[hh][it].v[e] += dl.v[e]; hi[hh][it].v[e] += dh.v[e]; }
                 }
             }
         }
-    };
-    if (item >= items) return;
-    int next_pos = position(item + stride);
-    Run run;
-    {
-        const int pos = position(item);
-        pdl_wait();
-        fetch(run, item, pos);
+    }
+    // what all heads of the token share: position, cos and sin, the cache page, the norm weights
+    const int pos = p.token_pos[t];
+    const float* cs = p.cos_sin + (size_t)(pos < p.max_pos ? pos : p.max_pos - 1) * p.d;
+    Piece<E> c[IT], sn[IT], wq_lo[IT], wq_hi[IT], wk_lo[IT], wk_hi[IT];
+#pragma unroll
+    for (int it = 0; it < IT; ++it) {
+        const int j = (it * 32 + lane) * E;
+        c[it] = load_piece<E>(cs + j);
+        sn[it] = load_piece<E>(cs + half + j);
+        if (p.q_weight) { wq_lo[it] = load_piece<E>(p.q_weight + j); wq_hi[it] = load_piece<E>(p.q_weight + half + j); }
+        if (p.k_weight) { wk_lo[it] = load_piece<E>(p.k_weight + j); wk_hi[it] = load_piece<E>(p.k_weight + half + j); }
+    }
+    size_t cache_row = 0;    // element offset of (page, kv head 0, token) in the caches
+    if (p.write_kv && head0 + HEADS_PER_WARP > p.nq) {
+        const int slot_pos = p.ring_tokens > 0 ? pos % p.ring_tokens : pos;
+        const int page = p.block_table[(size_t)p.token_seq[t] * p.max_blocks + slot_pos / p.page_tokens];
+        cache_row = ((size_t)page * p.nkv * p.page_tokens + (slot_pos % p.page_tokens)) * (size_t)p.d;
     }
     const size_t head_stride = (size_t)p.page_tokens * p.d;
     const float inv_d = 1.f / (float)p.d;
-    for (; item < items; item += stride) {
-        const Run now = run;
-        if (item + stride < items) {
-            const int pos = next_pos;
-            next_pos = position(item + 2 * stride);
-            fetch(run, item + stride, pos);
-        }
-        const int t = item / runs, head0 = (item - t * runs) * HEADS_PER_WARP;
 #pragma unroll
-        for (int hh = 0; hh < HEADS_PER_WARP; ++hh) {
-            const int head = head0 + hh;
-            if (head >= heads_total) break;
-            const bool is_q = head < p.nq, is_k = !is_q && head < p.nq + p.nkv;
-            if (!is_q && !p.write_kv) break;
-            TO* dst;
-            if (is_q) dst = (TO*)p.q_out + ((size_t)t * p.nq + head) * p.d;
-            else if (is_k) dst = (TO*)p.k_cache + now.cache_row + (size_t)(head - p.nq) * head_stride;
-            else dst = (TO*)p.v_cache + now.cache_row + (size_t)(head - p.nq - p.nkv) * head_stride;
-            const bool weighted = is_q ? p.q_weight != nullptr : (is_k && p.k_weight != nullptr);
-            const bool normed = weighted || (p.unit_norm && (is_q || is_k));
-            Piece<E> lo[IT], hi[IT];
+    for (int hh = 0; hh < HEADS_PER_WARP; ++hh) {
+        const int head = head0 + hh;
+        if (head >= heads_total) break;
+        const bool is_q = head < p.nq, is_k = !is_q && head < p.nq + p.nkv;
+        if (!is_q && !p.write_kv) break;
+        TO* dst;
+        if (is_q) dst = (TO*)p.q_out + ((size_t)t * p.nq + head) * p.d;
+        else if (is_k) dst = (TO*)p.k_cache + cache_row + (size_t)(head - p.nq) * head_stride;
+        else dst = (TO*)p.v_cache + cache_row + (size_t)(head - p.nq - p.nkv) * head_stride;
+        const bool weighted = is_q ? p.q_weight != nullptr : (is_k && p.k_weight != nullptr);
+        const bool normed = weighted || (p.unit_norm && (is_q || is_k));
+        float inv = 1.f;
+        if (normed) {
+            float sq = 0.f;
 #pragma unroll
             for (int it = 0; it < IT; ++it)
 #pragma unroll
-                for (int e = 0; e < E; ++e) { lo[it].v[e] = to_float(now.lo[hh][it].v[e]); hi[it].v[e] = to_float(now.hi[hh][it].v[e]); }
-            float inv = 1.f;
-            if (normed) {
-                float sq = 0.f;
+                for (int e = 0; e < E; ++e) sq += lo[hh][it].v[e] * lo[hh][it].v[e] + hi[hh][it].v[e] * hi[hh][it].v[e];
+            inv = rsqrtf(warp_sum(sq) * inv_d + p.eps);
+        }
 #pragma unroll
-                for (int it = 0; it < IT; ++it)
+        for (int it = 0; it < IT; ++it) {
+            const int j = (it * 32 + lane) * E;
+            Piece<E> a = lo[hh][it], b = hi[hh][it];
+            if (normed && !weighted) {
 #pragma unroll
-                    for (int e = 0; e < E; ++e) sq += lo[it].v[e] * lo[it].v[e] + hi[it].v[e] * hi[it].v[e];
-                inv = rsqrtf(warp_sum(sq) * inv_d + p.eps);
-            }
+                for (int e = 0; e < E; ++e) { a.v[e] *= inv; b.v[e] *= inv; }
+            } else if (normed) {
 #pragma unroll
-            for (int it = 0; it < IT; ++it) {
-                const int j = (it * 32 + lane) * E;
-                Piece<E> a = lo[it], b = hi[it];
-                if (normed && !weighted) {
-#pragma unroll
-                    for (int e = 0; e < E; ++e) { a.v[e] *= inv; b.v[e] *= inv; }
-                } else if (normed) {
-#pragma unroll
-                    for (int e = 0; e < E; ++e) {
-                        a.v[e] = a.v[e] * inv * (is_q ? wq_lo[it].v[e] : wk_lo[it].v[e]);
-                        b.v[e] = b.v[e] * inv * (is_q ? wq_hi[it].v[e] : wk_hi[it].v[e]);
-                    }
+                for (int e = 0; e < E; ++e) {
+                    a.v[e] = a.v[e] * inv * (is_q ? wq_lo[it].v[e] : wk_lo[it].v[e]);
+                    b.v[e] = b.v[e] * inv * (is_q ? wq_hi[it].v[e] : wk_hi[it].v[e]);
                 }
-                if (is_q || is_k) {
-#pragma unroll
-                    for (int e = 0; e < E; ++e) {
-                        const float ya = a.v[e] * now.c[it].v[e] - b.v[e] * now.sn[it].v[e];
-                        const float yb = b.v[e] * now.c[it].v[e] + a.v[e] * now.sn[it].v[e];
-                        a.v[e] = ya; b.v[e] = yb;
-                    }
-                }
-                store_piece<E>(dst + j, a);
-                store_piece<E>(dst + half + j, b);
             }
+            if (is_q || is_k) {
+#pragma unroll
+                for (int e = 0; e < E; ++e) {
+                    const float ya = a.v[e] * c[it].v[e] - b.v[e] * sn[it].v[e];
+                    const float yb = b.v[e] * c[it].v[e] + a.v[e] * sn[it].v[e];
+                    a.v[e] = ya; b.v[e] = yb;
+                }
+            }
+            store_piece<E>(dst + j, a);
+            store_piece<E>(dst + half + j, b);
         }
     }
 }
@@ -904,12 +873,10 @@ extern "C" int qt_qk_norm_rope_write(const void* qkv, int in_dtype, int n_splits
     const bool pair_aligned = split_stride % 2 == 0 && ((uintptr_t)qkv % 8 == 0) && ((uintptr_t)q_out % 8 == 0) && ((uintptr_t)cos_sin % 8 == 0) &&
                               (!q_weight || (uintptr_t)q_weight % 8 == 0) && (!k_weight || (uintptr_t)k_weight % 8 == 0) &&
                               (!write_kv || (((uintptr_t)k_cache % 8 == 0) && ((uintptr_t)v_cache % 8 == 0)));
-    if (pe && !own_values && !(unit_norm && (q_weight || k_weight)) && !whole_norm && !extra_cols && pair_aligned && n_tokens >= 256 && (long long)n_tokens * (nq + 2 * nkv) < (1ll << 30) && (in_dtype == QT_F32 || (in_dtype == QT_BF16 && n_splits == 1)) && out_dtype == QT_BF16) {
+    if (pe && !own_values && !(unit_norm && (q_weight || k_weight)) && !whole_norm && !extra_cols && pair_aligned && n_tokens >= 256 && nq + 2 * nkv <= 65535 * 16 && (in_dtype == QT_F32 || in_dtype == QT_BF16) && out_dtype == QT_BF16) {
         const int heads_total = nq + (kv_in_proj ? 2 * nkv : 0);
-        const int runs = ((write_kv ? heads_total : nq) + HEADS_PER_WARP - 1) / HEADS_PER_WARP;
-        const long long blocks = ((long long)n_tokens * runs + 3) / 4, resident = (long long)(pit == 1 ? PAIRS_BLOCKS : PAIRS_BLOCKS / 2) * sm_count();
-        const dim3 pgrid((unsigned)(blocks < resident ? blocks : resident));
-#define QT_LAUNCH_PAIRS(TI, E, IT) launch_kernel(qk_norm_rope_pairs_kernel<TI, __nv_bfloat16, E, IT>, pgrid, dim3(128), 0, s, p, runs)
+        const dim3 pgrid((unsigned)n_tokens, (unsigned)((heads_total + warps * HEADS_PER_WARP - 1) / (warps * HEADS_PER_WARP)));
+#define QT_LAUNCH_PAIRS(TI, E, IT) launch_kernel(qk_norm_rope_pairs_kernel<TI, __nv_bfloat16, E, IT>, pgrid, dim3(warps * 32), 0, s, p)
         if (in_dtype == QT_BF16) {
             if (pe == 2 && pit == 1) QT_LAUNCH_PAIRS(__nv_bfloat16, 2, 1);
             else if (pe == 2) QT_LAUNCH_PAIRS(__nv_bfloat16, 2, 2);
