@@ -291,7 +291,7 @@ template <typename T> static int launch_expert_rows(const ExpertParams& p, cudaS
 // output, multiplies float sums.
 constexpr int EG_PAIRS = 32;               // a lane a pair
 constexpr int EG_WARPS = 8;
-constexpr int EG_STEP = 32;                // K elements of a warp's turn: 8 a lane
+constexpr int EG_STEP = 64;                // K elements of a warp's turn: 16 a lane
 constexpr int EG_RANKS = 4;                // most blocks that share K in the second pass
 
 struct PairGroups {
@@ -318,70 +318,42 @@ __device__ __forceinline__ void group_pairs(const ExpertParams& p, PairGroups& g
     if (lane == 0) groups.count = __popc(leaders);
 }
 
-// An item is 16 features of a gated expert (32 of another) for the pairs of a group; a block takes every gridDim.x-th of them, and asks for the
-// next item's weights while it finishes one.
+// grid (feature blocks, pairs): block (i, g) forms 16 features of a gated expert, 32 of another, for the pairs of group g.  (Fewer blocks that walk
+// several of these, the next one's weights asked for ahead, took 3 us longer at every size.)
 template <bool GATED>
 __global__ void __launch_bounds__(EG_WARPS * 32, 2) expert_up_groups_kernel(const ExpertParams p) {
-    constexpr int DEPTH = 4, FEATS = GATED ? 16 : 32;
+    constexpr int DEPTH = 2, FEATS = GATED ? 16 : 32;
     __shared__ PairGroups groups;
-    __shared__ __align__(16) float sums[2][EG_WARPS][8][36];
+    __shared__ __align__(16) float sums[EG_WARPS][8][36];
     pdl_launch_dependents();
     pdl_wait();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
     if (warp == 0) group_pairs(p, groups, lane);
     __syncthreads();
-    const int K = p.width, blocks = (p.ff + FEATS - 1) / FEATS, total = blocks * groups.count;
-    const int turns = (K + EG_STEP - 1) / EG_STEP, per = (turns + EG_WARPS - 1) / EG_WARPS;      // of an item, the same for every warp
-    const int items = (int)blockIdx.x < total ? (total - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x : 0;
-    const int mine = items * per;
-    qt_few::Line<8> a[DEPTH][2][2], b[DEPTH];
+    if ((int)blockIdx.y >= groups.count) return;
+    const int f0 = blockIdx.x * FEATS, K = p.width;
+    const __nv_bfloat16* w = (const __nv_bfloat16*)p.up + (size_t)groups.expert[blockIdx.y] * (GATED ? 2 : 1) * p.ff * K;
+    const int pair = groups.pair[blockIdx.y][g];
+    const __nv_bfloat16* x = (const __nv_bfloat16*)p.x + (size_t)(pair < 0 ? 0 : pair / p.top) * K;
+    const __nv_bfloat16* row[2][2];                           // rows beyond the last repeat it; their sums are not stored
+#pragma unroll
+    for (int r = 0; r < 2; ++r)
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+            row[r][h] = w + (size_t)(GATED ? r * p.ff + min(f0 + 8 * h + g, p.ff - 1) : min(f0 + 16 * r + 8 * h + g, p.ff - 1)) * K;
+    const int turns = (K + EG_STEP - 1) / EG_STEP, mine = (turns - warp + EG_WARPS - 1) / EG_WARPS;
+    qt_few::Line<16> a[DEPTH][2][2], b[DEPTH];
     auto ask = [&](int slot, int i) {
-        const int n = i / per, item = (int)blockIdx.x + n * (int)gridDim.x, group = item / blocks, f0 = (item - group * blocks) * FEATS;
-        const int k = (warp + (i - n * per) * EG_WARPS) * EG_STEP + 8 * t, pair = groups.pair[group][g];
-        const __nv_bfloat16* w = (const __nv_bfloat16*)p.up + (size_t)groups.expert[group] * (GATED ? 2 : 1) * p.ff * K + k;
+        const int k = (warp + i * EG_WARPS) * EG_STEP + 16 * t;
 #pragma unroll
         for (int r = 0; r < 2; ++r)
 #pragma unroll
-            for (int h = 0; h < 2; ++h) {                     // rows beyond the last repeat it; their sums are not stored
-                const int row = GATED ? r * p.ff + min(f0 + 8 * h + g, p.ff - 1) : min(f0 + 16 * r + 8 * h + g, p.ff - 1);
-                if (k < K) a[slot][r][h] = qt_few::load_weight<8>(w + (size_t)row * K);
-                else a[slot][r][h] = qt_few::Line<8>{};
+            for (int h = 0; h < 2; ++h) {
+                if (k < K) a[slot][r][h] = qt_few::load_weight<16>(row[r][h] + k);
+                else a[slot][r][h] = qt_few::Line<16>{};
             }
-        if (k < K && pair >= 0) b[slot] = qt_few::load_rows<8>((const __nv_bfloat16*)p.x + (size_t)(pair / p.top) * K + k);
-        else b[slot] = qt_few::Line<8>{};
-    };
-    // the block's sums of an item, and its features
-    auto finish = [&](int n) {
-        const float (*part)[8][36] = sums[n & 1];
-        const int item = (int)blockIdx.x + n * (int)gridDim.x, group = item / blocks, f0 = (item - group * blocks) * FEATS;
-        const int slot = threadIdx.x / 8, l = threadIdx.x % 8, of = groups.pair[group][slot];
-        if (of < 0) return;
-        const float weight = p.in_weights ? p.in_weights[of] : 1.f;
-        __nv_bfloat16* mid = (__nv_bfloat16*)p.mid + (size_t)of * p.ff;
-        if (GATED) {
-            float2 gate = make_float2(0.f, 0.f), up = make_float2(0.f, 0.f);
-#pragma unroll
-            for (int s = 0; s < EG_WARPS; ++s) {
-                const float2 gs = *reinterpret_cast<const float2*>(&part[s][slot][2 * l]), us = *reinterpret_cast<const float2*>(&part[s][slot][2 * l + 16]);
-                gate.x += gs.x; gate.y += gs.y; up.x += us.x; up.y += us.y;
-            }
-            const int f = f0 + 2 * l;                         // ff is a multiple of 8
-            if (f < p.ff)
-                *reinterpret_cast<__nv_bfloat162*>(mid + f) = __floats2bfloat162_rn(gated_value<false>(gate.x * weight, up.x * weight, p.act, p.limit),
-                                                                                    gated_value<false>(gate.y * weight, up.y * weight, p.act, p.limit));
-        } else {
-            float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll
-            for (int s = 0; s < EG_WARPS; ++s) {
-                const float4 x = *reinterpret_cast<const float4*>(&part[s][slot][4 * l]);
-                v.x += x.x; v.y += x.y; v.z += x.z; v.w += x.w;
-            }
-            const int f = f0 + 4 * l;
-            if (f < p.ff) {
-                *reinterpret_cast<__nv_bfloat162*>(mid + f) = __floats2bfloat162_rn(gate_activation<false>(v.x * weight, p.act), gate_activation<false>(v.y * weight, p.act));
-                *reinterpret_cast<__nv_bfloat162*>(mid + f + 2) = __floats2bfloat162_rn(gate_activation<false>(v.z * weight, p.act), gate_activation<false>(v.w * weight, p.act));
-            }
-        }
+        if (k < K && pair >= 0) b[slot] = qt_few::load_rows<16>(x + k);
+        else b[slot] = qt_few::Line<16>{};
     };
     float c[2][4] = {};
 #pragma unroll
@@ -390,22 +362,43 @@ __global__ void __launch_bounds__(EG_WARPS * 32, 2) expert_up_groups_kernel(cons
     for (int i0 = 0; i0 < mine; i0 += DEPTH) {
 #pragma unroll
         for (int u = 0; u < DEPTH; ++u) {
-            const int i = i0 + u;
-            if (i >= mine) break;
+            if (i0 + u >= mine) break;
             qt_few::turn_product<2>(c, a[u], b[u]);
-            if (i + DEPTH < mine) ask(u, i + DEPTH);
-            if ((i + 1) % per == 0) {                         // the item's last turn
-                const int n = i / per;
+            if (i0 + u + DEPTH < mine) ask(u, i0 + u + DEPTH);
+        }
+    }
 #pragma unroll
-                for (int r = 0; r < 2; ++r)
+    for (int r = 0; r < 2; ++r)
 #pragma unroll
-                    for (int e = 0; e < 4; ++e) {
-                        sums[n & 1][warp][2 * t + (e & 1)][16 * r + g + 8 * (e >> 1)] = c[r][e];
-                        c[r][e] = 0.f;
-                    }
-                __syncthreads();                              // two sets of sums: the next item's go into the other
-                if (threadIdx.x < 64) finish(n);
-            }
+        for (int e = 0; e < 4; ++e) sums[warp][2 * t + (e & 1)][16 * r + g + 8 * (e >> 1)] = c[r][e];
+    __syncthreads();
+    if (threadIdx.x >= 64) return;
+    const int slot = threadIdx.x / 8, l = threadIdx.x % 8, of = groups.pair[blockIdx.y][slot];
+    if (of < 0) return;
+    const float weight = p.in_weights ? p.in_weights[of] : 1.f;
+    __nv_bfloat16* mid = (__nv_bfloat16*)p.mid + (size_t)of * p.ff;
+    if (GATED) {
+        float2 gate = make_float2(0.f, 0.f), up = make_float2(0.f, 0.f);
+#pragma unroll
+        for (int s = 0; s < EG_WARPS; ++s) {
+            const float2 gs = *reinterpret_cast<const float2*>(&sums[s][slot][2 * l]), us = *reinterpret_cast<const float2*>(&sums[s][slot][2 * l + 16]);
+            gate.x += gs.x; gate.y += gs.y; up.x += us.x; up.y += us.y;
+        }
+        const int f = f0 + 2 * l;                             // ff is a multiple of 16
+        if (f < p.ff)
+            *reinterpret_cast<__nv_bfloat162*>(mid + f) = __floats2bfloat162_rn(gated_value<false>(gate.x * weight, up.x * weight, p.act, p.limit),
+                                                                                gated_value<false>(gate.y * weight, up.y * weight, p.act, p.limit));
+    } else {
+        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+        for (int s = 0; s < EG_WARPS; ++s) {
+            const float4 part = *reinterpret_cast<const float4*>(&sums[s][slot][4 * l]);
+            v.x += part.x; v.y += part.y; v.z += part.z; v.w += part.w;
+        }
+        const int f = f0 + 4 * l;
+        if (f < p.ff) {
+            *reinterpret_cast<__nv_bfloat162*>(mid + f) = __floats2bfloat162_rn(gate_activation<false>(v.x * weight, p.act), gate_activation<false>(v.y * weight, p.act));
+            *reinterpret_cast<__nv_bfloat162*>(mid + f + 2) = __floats2bfloat162_rn(gate_activation<false>(v.z * weight, p.act), gate_activation<false>(v.w * weight, p.act));
         }
     }
 }
@@ -414,7 +407,7 @@ __global__ void __launch_bounds__(EG_WARPS * 32, 2) expert_up_groups_kernel(cons
 // finishes it.
 template <int RANKS>
 __global__ void __launch_bounds__(EG_WARPS * 32, 2) expert_down_groups_kernel(const ExpertParams p) {
-    constexpr int DEPTH = 8;
+    constexpr int DEPTH = 4;
     __shared__ PairGroups groups;
     __shared__ __align__(16) float sums[EG_WARPS][EG_PAIRS][16];
     __shared__ __align__(16) float parts[RANKS][EG_PAIRS][16];
@@ -428,17 +421,17 @@ __global__ void __launch_bounds__(EG_WARPS * 32, 2) expert_down_groups_kernel(co
     const int first = rank + RANKS * warp, stride = RANKS * EG_WARPS;
     const int turns = (K + EG_STEP - 1) / EG_STEP, per = first < turns ? (turns - first + stride - 1) / stride : 0;   // of a group
     const int mine = per * groups.count;
-    qt_few::Line<8> a[DEPTH][1][2], b[DEPTH];
+    qt_few::Line<16> a[DEPTH][1][2], b[DEPTH];
     auto ask = [&](int slot, int i) {                         // turns of the groups one after the other
-        const int group = i / per, k = (first + (i - group * per) * stride) * EG_STEP + 8 * t, pair = groups.pair[group][g];
+        const int group = i / per, k = (first + (i - group * per) * stride) * EG_STEP + 16 * t, pair = groups.pair[group][g];
         const __nv_bfloat16* w = (const __nv_bfloat16*)p.down + (size_t)groups.expert[group] * p.width * K + k;
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
-            if (k < K) a[slot][0][h] = qt_few::load_weight<8>(w + (size_t)min(c0 + 8 * h + g, p.width - 1) * K);
-            else a[slot][0][h] = qt_few::Line<8>{};
+            if (k < K) a[slot][0][h] = qt_few::load_weight<16>(w + (size_t)min(c0 + 8 * h + g, p.width - 1) * K);
+            else a[slot][0][h] = qt_few::Line<16>{};
         }
-        if (k < K && pair >= 0) b[slot] = qt_few::load_rows<8>((const __nv_bfloat16*)p.mid + (size_t)pair * K + k);
-        else b[slot] = qt_few::Line<8>{};
+        if (k < K && pair >= 0) b[slot] = qt_few::load_rows<16>((const __nv_bfloat16*)p.mid + (size_t)pair * K + k);
+        else b[slot] = qt_few::Line<16>{};
     };
     float c[1][4] = {};
     auto put = [&](int group) {
@@ -495,15 +488,15 @@ __global__ void __launch_bounds__(EG_WARPS * 32, 2) expert_down_groups_kernel(co
 }
 
 static int launch_expert_groups(const ExpertParams& p, cudaStream_t s) {
-    const int feats = p.gated ? 16 : 32, items = (p.ff + feats - 1) / feats * p.n_tokens * p.top;
-    const dim3 block(EG_WARPS * 32), up(items < 2 * sm_count() ? items : 2 * sm_count());
+    const int feats = p.gated ? 16 : 32;
+    const dim3 block(EG_WARPS * 32), up((p.ff + feats - 1) / feats, p.n_tokens * p.top);
     if (p.gated) launch_kernel(expert_up_groups_kernel<true>, up, block, 0, s, p);
     else launch_kernel(expert_up_groups_kernel<false>, up, block, 0, s, p);
     QT_CHECK_LAUNCH("expert_up");
-    // as many blocks to a column as leave every warp of theirs two turns of a group
+    // as many blocks to a column as leave every warp of theirs a turn of a group
     const int turns = (p.ff + EG_STEP - 1) / EG_STEP, columns = (p.width + 15) / 16;
-    if (turns >= 2 * EG_RANKS * EG_WARPS) launch_kernel_cluster(expert_down_groups_kernel<EG_RANKS>, dim3(columns * EG_RANKS), block, 0, s, EG_RANKS, p);
-    else if (turns >= 4 * EG_WARPS) launch_kernel_cluster(expert_down_groups_kernel<2>, dim3(columns * 2), block, 0, s, 2, p);
+    if (turns >= EG_RANKS * EG_WARPS) launch_kernel_cluster(expert_down_groups_kernel<EG_RANKS>, dim3(columns * EG_RANKS), block, 0, s, EG_RANKS, p);
+    else if (turns >= 2 * EG_WARPS) launch_kernel_cluster(expert_down_groups_kernel<2>, dim3(columns * 2), block, 0, s, 2, p);
     else launch_kernel(expert_down_groups_kernel<1>, dim3(columns), block, 0, s, p);
     QT_CHECK_LAUNCH("expert_down");
     return QT_OK;
@@ -532,9 +525,10 @@ extern "C" int qt_experts_by_pair(const void* x, const int* token_ids, const int
     return QT_DISPATCH_DTYPE(dtype, "experts_by_pair", {
         const size_t smem_up = (size_t)width * sizeof(float), smem_down = (size_t)top * ff * sizeof(float);
         const dim3 grid_up(n_tokens * top, (ff + per_block - 1) / per_block), grid_down(n_tokens, (width + per_block - 1) / per_block);
+        // Per expert where the pairs are at least as many as the experts, so that some share one.
+        if (std::is_same<T, __nv_bfloat16>::value && n_tokens * top <= EG_PAIRS && n_tokens * top >= experts && width % 16 == 0 && ff % 16 == 0 &&
+            (((uintptr_t)up | (uintptr_t)down | (uintptr_t)x | (uintptr_t)mid) & 31) == 0) return launch_expert_groups(p, s);
         // 16-byte loads: rows of both weights, of x and of mid start on 16-byte boundaries
-        if (std::is_same<T, __nv_bfloat16>::value && n_tokens * top <= EG_PAIRS && width % 8 == 0 && ff % 8 == 0 &&
-            (((uintptr_t)up | (uintptr_t)down | (uintptr_t)x | (uintptr_t)mid) & 15) == 0) return launch_expert_groups(p, s);
         if (width % 8 == 0 && ff % 8 == 0 && (((uintptr_t)up | (uintptr_t)down | (uintptr_t)x | (uintptr_t)mid) & 15) == 0) return launch_expert_rows<T>(p, s);
         if (smem_up > 48 * 1024) cudaFuncSetAttribute(expert_up_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_up);
         if (smem_down > 48 * 1024) cudaFuncSetAttribute(expert_down_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_down);

@@ -6,9 +6,9 @@
 // 1.3, 3.1; the others are below 2^-25 of the operands' product and of either sign.  What could lose bits is the adding: the tensor pipe
 // does not round to nearest, so an accumulator takes one K slice of 64 (small products first) and is then added, rounded to nearest, to sums in registers.
 //
-// A block forms 128 x 128 results.  Eight warps load the next slice's floats into registers, split them and store the pieces where the MMAs read
-// them, two stages deep: A's in tensor memory, a row a thread (from shared memory both operands of 128 x 128 x 16 are 128 bytes a clock, all it
-// gives, and a slice took twice its 1,536 cycles of the tensor pipe), W's as swizzled tiles.  One thread issues 24 MMAs a slice, and the eight
+// A block forms 128 x 128 results.  Sixteen warps load the next slice's floats into registers, split them and store the pieces where the MMAs read
+// them, two stages deep: A's in tensor memory, half a row a thread (from shared memory both operands of 128 x 128 x 16 would be 128 bytes a clock, all it
+// gives), W's as swizzled tiles.  One thread issues 24 MMAs a slice (1,536 cycles of the tensor pipe), and the sixteen
 // warps add a finished slice's accumulator up while the next one is multiplied.  Up to eight blocks of a cluster share K where the tiles do not fill
 // the SMs, and add up through distributed shared memory in the order of the ranks.
 //
@@ -21,18 +21,19 @@ using namespace qt_tc;
 namespace {
 
 constexpr int TILE = 128, BK = 64;                     // rows of either operand a block takes, K elements of a slice
-constexpr int WORK_WARPS = 8, THREADS = (WORK_WARPS + 1) * 32;
+constexpr int WORK_WARPS = 16, THREADS = (WORK_WARPS + 1) * 32;
 constexpr uint32_t PIECE_BYTES = TILE * BK * 2;        // one piece of W: [128 rows][64] bfloat16, 128-byte swizzle
 constexpr uint32_t STAGE_BYTES = 3 * PIECE_BYTES;
 constexpr int A_COLS = BK / 2;                         // one piece of A in tensor memory: row i in lane i, two elements a column
 constexpr uint32_t TMEM_A = 2 * TILE, TMEM_COLS = 512; // two accumulators, two stages of A's pieces
-constexpr int UNITS = 8;                               // runs of eight elements a thread splits per slice
+constexpr int UNITS = 4;                               // runs of eight elements a thread splits per slice
+constexpr int COLS = 32;                               // results a thread keeps the sums of
 constexpr int MOST_RANKS = 8, PARK_ROW = TILE + 4;
 constexpr uint32_t IDESC = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(TILE >> 3) << 17) | ((uint32_t)(TILE >> 4) << 24);
 static_assert(TILE * PARK_ROW * 4 <= 2 * STAGE_BYTES, "a block's part of the result is parked in the stages' memory");
 
-// What the truncated additions of a slice leave out on average, of its sum.
-constexpr float SHORTFALL = 0.f;
+// What the truncated additions leave out on average, of the sum: 4.7e-8 for operands of one sign and 6.0e-8 for either, alike for every K from 64 to 12,288.
+constexpr float SHORTFALL = 5.4e-8f;
 
 struct Params {
     const float* a; const float* w; float* c;
@@ -124,33 +125,38 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_f32_tc_kernel(const __grid_co
         }
         __syncwarp();
     } else {
-        // Warps 0 to 3: a thread holds a row of A's slice, unit u is its elements 8 u .. 8 u + 7.  Warps 4 to 7: unit u of a thread is eight
-        // neighbouring elements of row 16 u + (thread / 8) of W's.
-        const bool of_a = warp < 4;
-        const int chunk = threadIdx.x & 7, w_row = (threadIdx.x & 127) >> 3;
+        // Warps 0 to 7: a thread holds half a row of A's slice (warps 0 to 3 the first), unit u is its elements 8 u .. 8 u + 7.  Warps 8 to 15: unit u
+        // of a thread is eight neighbouring elements of row 32 u + (thread / 8) of W's.
+        const bool of_a = warp < 8;
+        const int chunk = threadIdx.x & 7, w_row = (threadIdx.x & 255) >> 3, a_row = threadIdx.x & 127, a_half = (warp >> 2) & 1;
         float v[UNITS][8];
         auto ask = [&](int u, int slice) {
-            const int at = of_a ? m0 + (int)threadIdx.x : n0 + 16 * u + w_row, k = k_begin + slice * BK + 8 * (of_a ? u : chunk);
+            const int at = of_a ? m0 + a_row : n0 + 32 * u + w_row, k = k_begin + slice * BK + 8 * (of_a ? 4 * a_half + u : chunk);
             const bool there = at < (of_a ? p.M : p.N);
             const float* from = (of_a ? p.a : p.w) + (size_t)at * p.K + k;
             const float4 x = there && k < k_end ? load4(from) : make_float4(0.f, 0.f, 0.f, 0.f);              // K is a multiple of 4
             const float4 y = there && k + 4 < k_end ? load4(from + 4) : make_float4(0.f, 0.f, 0.f, 0.f);
             v[u][0] = x.x; v[u][1] = x.y; v[u][2] = x.z; v[u][3] = x.w; v[u][4] = y.x; v[u][5] = y.y; v[u][6] = y.z; v[u][7] = y.w;
         };
-        float sums[64];                                                     // row 32 (warp % 4) + lane, columns 64 (warp / 4) ..
+        float sums[COLS];                                                   // row 32 (warp % 4) + lane, columns 32 (warp / 4) ..
 #pragma unroll
-        for (int j = 0; j < 64; ++j) sums[j] = 0.f;
-        const uint32_t mine = tmem_base + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)(warp >> 2) * 64u;
-        auto add = [&](int i) {
+        for (int j = 0; j < COLS; ++j) sums[j] = 0.f;
+        const uint32_t mine = tmem_base + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)(warp >> 2) * COLS;
+        auto add = [&](int i, bool last) {
             const int s = i & 1;
             if (!mbar_wait(summed + 8 * s, (uint32_t)(i >> 1) & 1u, status, 3)) return false;
             tc_fence_after();
 #pragma unroll
-            for (int part = 0; part < 4; ++part) {
+            for (int part = 0; part < COLS / 16; ++part) {
                 uint32_t x[16];
                 tmem_load16(mine + s * TILE + 16 * part, x);
 #pragma unroll
-                for (int j = 0; j < 16; ++j) sums[16 * part + j] += __uint_as_float(x[j]);
+                for (int j = 0; j < 16; ++j) {
+                    float& sum = sums[16 * part + j];
+                    float y = __uint_as_float(x[j]);
+                    if (last) y = fmaf(SHORTFALL, sum + y, y);              // of the whole sum, ahead of its last rounding
+                    sum += y;
+                }
             }
             tc_fence_before();
             __syncwarp();
@@ -182,17 +188,15 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_f32_tc_kernel(const __grid_co
             if (of_a) {
                 tc_fence_after();
 #pragma unroll
-                for (int part = 0; part < 2; ++part)
+                for (int piece = 0; piece < 3; ++piece) {
+                    uint32_t h[16];
 #pragma unroll
-                    for (int piece = 0; piece < 3; ++piece) {
-                        uint32_t h[16];
-#pragma unroll
-                        for (int u = 0; u < 4; ++u) {
-                            piece_of(4 * part + u, h + 4 * u, piece == 0, piece == 2);
-                            if (piece == 2 && i + 1 < slices) ask(4 * part + u, i + 1);
-                        }
-                        store_columns(tmem_base + ((uint32_t)(warp * 32) << 16) + TMEM_A + (s * 3 + piece) * A_COLS + 16 * part, h);
+                    for (int u = 0; u < UNITS; ++u) {
+                        piece_of(u, h + 4 * u, piece == 0, piece == 2);
+                        if (piece == 2 && i + 1 < slices) ask(u, i + 1);
                     }
+                    store_columns(tmem_base + ((uint32_t)((warp & 3) * 32) << 16) + TMEM_A + (s * 3 + piece) * A_COLS + 16 * a_half, h);
+                }
                 tmem_wait_st();
                 tc_fence_before();
             } else {
@@ -202,7 +206,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_f32_tc_kernel(const __grid_co
 #pragma unroll
                     for (int piece = 0; piece < 3; ++piece) piece_of(u, h[piece], piece == 0, piece == 2);
                     if (i + 1 < slices) ask(u, i + 1);
-                    const int row = 16 * u + w_row;
+                    const int row = 32 * u + w_row;
                     const uint32_t at = base + s * STAGE_BYTES + (uint32_t)(row * 128 + ((chunk ^ (row & 7)) << 4));
 #pragma unroll
                     for (int piece = 0; piece < 3; ++piece) store16(at + piece * PIECE_BYTES, h[piece]);
@@ -211,33 +215,31 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_f32_tc_kernel(const __grid_co
             }
             __syncwarp();
             if (lane == 0) mbar_arrive(full + 8 * s);
-            if (i > 0) ok = add(i - 1);
+            if (i > 0) ok = add(i - 1, false);
         }
-        if (ok) ok = add(slices - 1);
+        if (ok) ok = add(slices - 1, true);
         if (none != 0.f) atomicOr(odd, 1);                                  // NaN
         asm volatile("bar.sync 1, %0;" ::"n"(WORK_WARPS * 32) : "memory");
-        const int row = (warp & 3) * 32 + lane, col0 = (warp >> 2) * 64, m = m0 + row;
-#pragma unroll
-        for (int j = 0; j < 64; ++j) sums[j] = fmaf(sums[j], SHORTFALL, sums[j]);
+        const int row = (warp & 3) * 32 + lane, col0 = (warp >> 2) * COLS, m = m0 + row;
         if (*(volatile int*)odd != 0) {
             const float* x = p.a + (size_t)min(m, p.M - 1) * p.K;
 #pragma unroll 1
-            for (int j0 = 0; j0 < 64; ++j0) {
+            for (int j0 = 0; j0 < COLS; ++j0) {
                 const float* y = p.w + (size_t)min(n0 + col0 + j0, p.N - 1) * p.K;
                 float sum = 0.f;
                 for (int k = k_begin; k < k_end; ++k) sum = fmaf(x[k], y[k], sum);
 #pragma unroll
-                for (int j = 0; j < 64; ++j) if (j == j0) sums[j] = sum;    // registers have no index
+                for (int j = 0; j < COLS; ++j) if (j == j0) sums[j] = sum;    // registers have no index
             }
         }
         if (p.ranks > 1) {                                                  // every MMA has read the stages: they are free
             float* park = reinterpret_cast<float*>(smem) + row * PARK_ROW + col0;
 #pragma unroll
-            for (int j = 0; j < 64; j += 4) *reinterpret_cast<float4*>(park + j) = make_float4(sums[j], sums[j + 1], sums[j + 2], sums[j + 3]);
+            for (int j = 0; j < COLS; j += 4) *reinterpret_cast<float4*>(park + j) = make_float4(sums[j], sums[j + 1], sums[j + 2], sums[j + 3]);
         } else if (m < p.M && ok) {
             float* to = p.c + (size_t)m * p.N + n0 + col0;
 #pragma unroll
-            for (int j = 0; j < 64; j += 4) {
+            for (int j = 0; j < COLS; j += 4) {
                 if (n0 + col0 + j + 3 < p.N && (p.N & 3) == 0) *reinterpret_cast<float4*>(to + j) = make_float4(sums[j], sums[j + 1], sums[j + 2], sums[j + 3]);
                 else
 #pragma unroll

@@ -1537,6 +1537,11 @@ def gemm_f32(a: torch.Tensor, w: torch.Tensor, out: GemmOut) -> None:
     _call("gemm_f32", "qt_gemm_f32", _ptr(a), _ptr(w), _ptr(out.tensor), a.shape[0], w.shape[0], a.shape[1], _stream())
 
 
+def gemm_f32_on_tc(a: torch.Tensor, w: torch.Tensor, out: GemmOut) -> bool:
+    """Whether a float product that ``gemm_f32`` takes runs on the tensor cores instead: more than 32 rows."""
+    return a.shape[0] > 32 and (w.shape[0] % 4 != 0 or out.tensor.data_ptr() % 16 == 0)
+
+
 def gemm_f32_tc(a: torch.Tensor, w: torch.Tensor, out: GemmOut) -> None:
     """out = a [M, K] @ w [N, K]^T of float operands on the tcgen05 tensor cores, each split into three bfloat16 pieces without loss; K a
     multiple of 4, 16-byte aligned operands."""
@@ -1749,7 +1754,7 @@ def gemm_uses_pairs(a: torch.Tensor, w: torch.Tensor) -> bool:
 
 def gemm(a: torch.Tensor, w: torch.Tensor, out: GemmOut, bias: torch.Tensor | None = None) -> None:
     """out = a @ w^T (+ ``bias`` [N], float, for float results) with the kernel that fits the element type and shape (a static choice):
-    tensor cores for bfloat16 with 16-byte aligned rows; on the FMA pipe the packed float32 kernels, and the plain one for what is left
+    tensor cores for bfloat16 with 16-byte aligned rows, and for float32 of more than a few rows (exact pieces); on the FMA pipe the packed float32 kernels, and the plain one for what is left
     (float32 rows that are not 16-byte aligned, bfloat16 that the tensor cores' loads cannot take)."""
     if gemm_tc_supported(a, w):
         if gemm_uses_pairs(a, w):
@@ -1758,7 +1763,7 @@ def gemm(a: torch.Tensor, w: torch.Tensor, out: GemmOut, bias: torch.Tensor | No
             gemm_tc(a, w, out, bias=bias)
     elif out.n_splits == 1:
         if gemm_f32_supported(a, w, out):
-            gemm_f32(a, w, out)
+            (gemm_f32_tc if gemm_f32_on_tc(a, w, out) else gemm_f32)(a, w, out)
         else:
             gemm_simt(a, w, out)
         if bias is not None and out.rows:
