@@ -542,7 +542,7 @@ __global__ void __launch_bounds__(DEC_WARPS * 32) attention_decode_kernel(const 
         if (valid) {
             const T* krow = kc + cache_offset(table, key, p.ring_tokens, p.page_tokens, p.nkv, kvh, d);
             if (dp.fours) {
-                constexpr int AHEAD = DMAX <= 128 ? 16 : 8;         // pieces of the key asked for before the first is used
+                constexpr int AHEAD = 8;                    // pieces of the key asked for before the first is used
                 for (int c0 = 0; c0 < d; c0 += 4 * AHEAD) {
                     float4 kv[AHEAD];
 #pragma unroll
@@ -589,7 +589,7 @@ __global__ void __launch_bounds__(DEC_WARPS * 32) attention_decode_kernel(const 
         // every lane knows where its key's value lies; VALUES_AHEAD of them are asked for before the first is used
         const int n_keys = min(32, k_end - k0);
         const unsigned long long mine = valid ? cache_offset(table, key, p.ring_tokens, p.page_tokens, p.nv, vh, p.v_row) : 0;
-        constexpr int VALUES_AHEAD = DMAX <= 128 ? 16 : DMAX <= 256 ? 4 : 1;
+        constexpr int VALUES_AHEAD = DMAX <= 128 ? 8 : DMAX <= 256 ? 4 : 1;
         for (int kk = 0; kk < n_keys; kk += VALUES_AHEAD) {
             float v[VALUES_AHEAD][DMAX / 32];
 #pragma unroll

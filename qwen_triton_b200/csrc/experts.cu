@@ -525,8 +525,10 @@ extern "C" int qt_experts_by_pair(const void* x, const int* token_ids, const int
     return QT_DISPATCH_DTYPE(dtype, "experts_by_pair", {
         const size_t smem_up = (size_t)width * sizeof(float), smem_down = (size_t)top * ff * sizeof(float);
         const dim3 grid_up(n_tokens * top, (ff + per_block - 1) / per_block), grid_down(n_tokens, (width + per_block - 1) / per_block);
-        // Per expert where the pairs are at least as many as the experts, so that some share one.
-        if (std::is_same<T, __nv_bfloat16>::value && n_tokens * top <= EG_PAIRS && n_tokens * top >= experts && width % 16 == 0 && ff % 16 == 0 &&
+        // Per expert where the pairs are at least as many as the experts, so that some share one, and where an expert's bytes outweigh the longer way to
+        // them (groups, a cluster's sums).  Both passes, by pair / per expert: 8, 16, 32 tokens of one of 8 experts of 1,024 x 2,048 18 / 15, 33 / 25, 54 / 28 us; 8,
+        // 12, 16 tokens of 2 of 16 of 2,048 x 1,024 34 / 31, 44 / 35, 55 / 39 us; but of 1,024 x 512 10 / 14 us, 8 tokens of 4 of 32 of 2,048 x 768 48 / 54 us.
+        if (std::is_same<T, __nv_bfloat16>::value && n_tokens * top <= EG_PAIRS && n_tokens * top >= experts && (long long)width * ff >= (2ll << 20) && width % 16 == 0 && ff % 16 == 0 &&
             (((uintptr_t)up | (uintptr_t)down | (uintptr_t)x | (uintptr_t)mid) & 31) == 0) return launch_expert_groups(p, s);
         // 16-byte loads: rows of both weights, of x and of mid start on 16-byte boundaries
         if (width % 8 == 0 && ff % 8 == 0 && (((uintptr_t)up | (uintptr_t)down | (uintptr_t)x | (uintptr_t)mid) & 15) == 0) return launch_expert_rows<T>(p, s);

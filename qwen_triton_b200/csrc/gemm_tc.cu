@@ -331,32 +331,6 @@ template <> __device__ __forceinline__ void store8<__nv_bfloat16>(__nv_bfloat16*
     *reinterpret_cast<uint4*>(dst) = packed;
 }
 
-// 16 results to a 32-byte boundary.  A thread of the pair kernel's epilogue has a row of its own, so an instruction of the warp touches 32 rows,
-// and whole sectors halve what the memory system is asked for.
-__device__ __forceinline__ void store32(void* dst, const uint32_t (&v)[8]) {
-    asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};"
-                 ::"l"(dst), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]) : "memory");
-}
-template <typename TO> __device__ __forceinline__ void store16(TO* dst, const float (&f)[16]) {
-    if constexpr (sizeof(TO) == 4) {
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            uint32_t v[8];
-#pragma unroll
-            for (int j = 0; j < 8; ++j) v[j] = __float_as_uint(f[8 * h + j]);
-            store32(dst + 8 * h, v);
-        }
-    } else {
-        uint32_t v[8];
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-            const __nv_bfloat162 h = __floats2bfloat162_rn(f[2 * j], f[2 * j + 1]);
-            v[j] = *reinterpret_cast<const uint32_t*>(&h);
-        }
-        store32(dst, v);
-    }
-}
-
 template <typename TO, int MODE>
 __global__ void __launch_bounds__(THREADS, 1) gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_w,
                                                                   const __grid_constant__ CUtensorMap map_x, TO* __restrict__ out,
@@ -580,13 +554,6 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_tc_pair_kernel(const __grid_c
                     // columns c .. c + 15 are the gate rows of 16 features, c + 16 .. c + 31 the up rows of the same
                     const int f0 = (n0 + c) >> 1;
                     TO* dst = row + (c >> 1);
-                    if (vector_stores == 2 && f0 + 16 <= features) {
-                        float f[16];
-#pragma unroll
-                        for (int j = 0; j < 16; ++j) f[j] = gated_value<true>(__uint_as_float(v[j]), __uint_as_float(v[16 + j]), act, limit);
-                        store16<TO>(dst, f);
-                        continue;
-                    }
 #pragma unroll
                     for (int h = 0; h < 2; ++h) {
                         float f[8];
@@ -612,19 +579,6 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_tc_pair_kernel(const __grid_c
                         store8<TO>(row + c + 8 * h, f);
                     }
                 } else {
-                    if (vector_stores == 2 && n0 + c + 32 <= N) {
-#pragma unroll
-                        for (int h = 0; h < 2; ++h) {
-                            float f[16];
-#pragma unroll
-                            for (int j = 0; j < 16; ++j) {
-                                const float y = __uint_as_float(v[16 * h + j]);
-                                f[j] = MODE == ACTIVATED ? gate_activation<true>(y, act) : y;
-                            }
-                            store16<TO>(row + c + 16 * h, f);
-                        }
-                        continue;
-                    }
 #pragma unroll
                     for (int h = 0; h < 4; ++h) {
                         float f[8];
@@ -724,10 +678,9 @@ int launch_pair(const CUtensorMap& map_w, const CUtensorMap& map_x, TO* out, int
     const int kb_per_split = (kb_total + splits - 1) / splits;
     const int tail_tiles = splits == 1 && tail_scratch && tail_flags ? pick_tail_tiles(items, resident_pairs, kb_total, tail, tail_pairs) : 0;
     if (tail_tiles) pairs = (unsigned)resident_pairs;        // fewer tiles than pairs: all of them by K ranges over every pair
-    // stores of 32 bytes (2) or 16 (1) need every output row (and plane) to start on such a boundary
-    const int row_elems = MODE == GATED ? N / 2 : N;
-    const auto rows_at = [&](int bytes) { const int per = bytes / (int)sizeof(TO); return (uintptr_t)out % bytes == 0 && row_elems % per == 0 && split_stride % per == 0; };
-    const int vector_stores = rows_at(32) ? 2 : rows_at(16) ? 1 : 0;
+    // 16-byte stores need every output row (and plane) to start on a 16-byte boundary
+    const int per16 = 16 / (int)sizeof(TO), row_elems = MODE == GATED ? N / 2 : N;
+    const int vector_stores = ((uintptr_t)out % 16 == 0 && row_elems % per16 == 0 && split_stride % per16 == 0) ? 1 : 0;
     launch_kernel_cluster(gemm_tc_pair_kernel<TO, MODE>, dim3(2 * pairs), dim3(THREADS), smem, stream, 2, map_w, map_x, out, M, N, kb_total,
                           kb_per_split, splits, split_stride, act, limit, vector_stores, tail_tiles, tail_scratch, tail_flags, bias, run_scale, key_cols, status);
     QT_CHECK_LAUNCH("gemm_tc_pair");
