@@ -8,9 +8,15 @@
 //
 // A block forms 128 x 128 results.  Sixteen warps load the next slice's floats into registers, split them and store the pieces where the MMAs read
 // them, two stages deep: A's in tensor memory, half a row a thread (from shared memory both operands of 128 x 128 x 16 would be 128 bytes a clock, all it
-// gives), W's as swizzled tiles.  One thread issues 24 MMAs a slice (1,536 cycles of the tensor pipe), and the sixteen
+// gives), W's as swizzled tiles.  A's floats come by TMA: a row a thread read straight from memory is 32 lines an instruction, 2,048 cycles a slice.  One thread issues 24 MMAs a slice (1,536 cycles of the tensor pipe), and the sixteen
 // warps add a finished slice's accumulator up while the next one is multiplied.  Up to eight blocks of a cluster share K where the tiles do not fill
 // the SMs, and add up through distributed shared memory in the order of the ranks.
+//
+// What bounds it now is the splitting: a slice takes 1.9 us (3,300 cycles), and with one product in the place of six 0.9 of that.
+//
+// N x K, rows, us before (gemm_f32.cu) / here: 4096 x 1024 64 19.5 / 13.5, 549 120 / 57, 4,096 802 / 229; 6144 x 1024 549 177 / 67; 1024 x 3072 549 111 / 34; 4096 x 12288 4,096
+// 9,928 / 2,622 (157 TFLOP/s); up to 32 rows the FMA pipe's kernels are as fast or faster.  Error against 64 bits over the result's norm, before / here: random signs, 1,024
+// to 12,288 of K 1.05e-7 to 1.62e-7 / 0.78e-7 to 1.19e-7; operands of one sign 0.43e-7 to 0.63e-7 / 0.46e-7 to 0.62e-7.
 //
 // Infinities, NaN and numbers that round to an infinite bfloat16 have no such pieces: a block that meets one forms its results again with FMAs.
 #include "tc_common.cuh"
@@ -21,7 +27,9 @@ using namespace qt_tc;
 namespace {
 
 constexpr int TILE = 128, BK = 64;                     // rows of either operand a block takes, K elements of a slice
-constexpr int WORK_WARPS = 16, THREADS = (WORK_WARPS + 1) * 32;
+constexpr int WORK_WARPS = 16, MMA_WARP = 16, COPY_WARP = 17, THREADS = 18 * 32;
+constexpr int A_STAGES = 3;                            // slices of A as floats, ahead of their splitting
+constexpr uint32_t A_HALF_BYTES = TILE * 128, A_STAGE_BYTES = 2 * A_HALF_BYTES;      // [128 rows][32 floats] twice, 128-byte swizzle
 constexpr uint32_t PIECE_BYTES = TILE * BK * 2;        // one piece of W: [128 rows][64] bfloat16, 128-byte swizzle
 constexpr uint32_t STAGE_BYTES = 3 * PIECE_BYTES;
 constexpr int A_COLS = BK / 2;                         // one piece of A in tensor memory: row i in lane i, two elements a column
@@ -67,14 +75,16 @@ __device__ __forceinline__ float4 peer4(uint32_t addr) {
     return v;
 }
 
-__global__ void __launch_bounds__(THREADS, 1) gemm_f32_tc_kernel(const __grid_constant__ Params p) {
+__global__ void __launch_bounds__(THREADS, 1) gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ Params p) {
     extern __shared__ uint8_t smem_raw[];
     const uint32_t raw = smem_u32(smem_raw), base = (raw + 1023u) & ~1023u;
     uint8_t* smem = smem_raw + (base - raw);
-    const uint32_t bars = base + 2 * STAGE_BYTES;      // full[2], empty[2], summed[2] (an accumulator is complete), added[2] (and read)
-    const uint32_t full = bars, empty = bars + 16, summed = bars + 32, added = bars + 48;
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + 2 * STAGE_BYTES + 64);
-    int* odd = reinterpret_cast<int*>(smem + 2 * STAGE_BYTES + 68);         // a number without pieces was met
+    const uint32_t a_floats = base + 2 * STAGE_BYTES;
+    // full[2], empty[2], summed[2] (an accumulator is complete), added[2] (and read), arrived[3] (floats of A), taken[3]
+    constexpr uint32_t BARS = 2 * STAGE_BYTES + A_STAGES * A_STAGE_BYTES;
+    const uint32_t bars = base + BARS, full = bars, empty = bars + 16, summed = bars + 32, added = bars + 48, arrived = bars + 64, taken = arrived + 8 * A_STAGES;
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + BARS + 64 + 16 * A_STAGES);
+    int* odd = reinterpret_cast<int*>(tmem_slot + 1);                       // a number without pieces was met
 
     pdl_launch_dependents();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -89,10 +99,11 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_f32_tc_kernel(const __grid_co
             mbar_init(full + 8 * s, WORK_WARPS); mbar_init(empty + 8 * s, 1);
             mbar_init(summed + 8 * s, 1); mbar_init(added + 8 * s, WORK_WARPS);
         }
+        for (int s = 0; s < A_STAGES; ++s) { mbar_init(arrived + 8 * s, 1); mbar_init(taken + 8 * s, WORK_WARPS / 2); }
         *odd = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    if (warp == WORK_WARPS) {
+    if (warp == MMA_WARP) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(TMEM_COLS) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
@@ -101,7 +112,20 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_f32_tc_kernel(const __grid_co
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
 
-    if (warp == WORK_WARPS) {
+    if (warp == COPY_WARP) {
+        if (lane == 0) {
+            prefetch_tensor_map(&map_a);
+            pdl_wait();
+            for (int i = 0, s = 0, turn = 0; i < slices; ++i) {
+                if (!mbar_wait(taken + 8 * s, (uint32_t)turn ^ 1u, status, 1)) break;
+                mbar_expect_tx(arrived + 8 * s, A_STAGE_BYTES);
+                for (int h = 0; h < 2; ++h)                                 // the map counts 16-bit elements, two a float
+                    tma_load_2d(a_floats + s * A_STAGE_BYTES + h * A_HALF_BYTES, &map_a, arrived + 8 * s, 2 * (k_begin + i * BK + 32 * h), m0);
+                if (++s == A_STAGES) { s = 0; turn ^= 1; }
+            }
+        }
+        __syncwarp();
+    } else if (warp == MMA_WARP) {
         if (lane == 0) {
             const uint64_t desc0 = operand_desc(base);
             for (int i = 0; i < slices; ++i) {
@@ -130,13 +154,14 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_f32_tc_kernel(const __grid_co
         const bool of_a = warp < 8;
         const int chunk = threadIdx.x & 7, w_row = (threadIdx.x & 255) >> 3, a_row = threadIdx.x & 127, a_half = (warp >> 2) & 1;
         float v[UNITS][8];
-        auto ask = [&](int u, int slice) {
-            const int at = of_a ? m0 + a_row : n0 + 32 * u + w_row, k = k_begin + slice * BK + 8 * (of_a ? 4 * a_half + u : chunk);
-            const bool there = at < (of_a ? p.M : p.N);
-            const float* from = (of_a ? p.a : p.w) + (size_t)at * p.K + k;
-            const float4 x = there && k < k_end ? load4(from) : make_float4(0.f, 0.f, 0.f, 0.f);              // K is a multiple of 4
-            const float4 y = there && k + 4 < k_end ? load4(from + 4) : make_float4(0.f, 0.f, 0.f, 0.f);
+        auto put = [&](int u, const float4& x, const float4& y) {
             v[u][0] = x.x; v[u][1] = x.y; v[u][2] = x.z; v[u][3] = x.w; v[u][4] = y.x; v[u][5] = y.y; v[u][6] = y.z; v[u][7] = y.w;
+        };
+        auto ask = [&](int u, int slice) {                                  // of W
+            const int at = n0 + 32 * u + w_row, k = k_begin + slice * BK + 8 * chunk;
+            const float* from = p.w + (size_t)at * p.K + k;
+            const float4 none = make_float4(0.f, 0.f, 0.f, 0.f);
+            put(u, at < p.N && k < k_end ? load4(from) : none, at < p.N && k + 4 < k_end ? load4(from + 4) : none);              // K is a multiple of 4
         };
         float sums[COLS];                                                   // row 32 (warp % 4) + lane, columns 32 (warp / 4) ..
 #pragma unroll
@@ -163,10 +188,13 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_f32_tc_kernel(const __grid_co
             if (lane == 0) mbar_arrive(added + 8 * s);
             return true;
         };
-        if (of_a) pdl_wait();                                               // weights depend on no earlier kernel
+        if (!of_a) {                                                        // weights depend on no earlier kernel
 #pragma unroll
-        for (int u = 0; u < UNITS; ++u) ask(u, 0);
-        if (!of_a) pdl_wait();
+            for (int u = 0; u < UNITS; ++u) ask(u, 0);
+        }
+        pdl_wait();                                                         // the result may still be read by one
+        int a_stage = 0;
+        uint32_t a_turn = 0;
         float none = 0.f;                                                   // stays 0 while every number has its pieces
         // the next piece of a unit: its numbers rounded, and what is left of them
         auto piece_of = [&](int u, uint32_t* h, bool first, bool last) {
@@ -186,6 +214,15 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_f32_tc_kernel(const __grid_co
             ok = mbar_wait(empty + 8 * s, ((uint32_t)(i >> 1) & 1u) ^ 1u, status, 1);
             if (!ok) break;
             if (of_a) {
+                ok = mbar_wait(arrived + 8 * a_stage, a_turn, status, 3);
+                if (!ok) break;
+                const uint8_t* floats = smem + 2 * STAGE_BYTES + a_stage * A_STAGE_BYTES + a_half * A_HALF_BYTES + a_row * 128;
+#pragma unroll
+                for (int u = 0; u < UNITS; ++u)                             // a row's 16-byte pieces lie in the swizzle's order
+                    put(u, *reinterpret_cast<const float4*>(floats + (((2 * u) ^ (a_row & 7)) << 4)), *reinterpret_cast<const float4*>(floats + (((2 * u + 1) ^ (a_row & 7)) << 4)));
+                __syncwarp();
+                if (lane == 0) mbar_arrive(taken + 8 * a_stage);
+                if (++a_stage == A_STAGES) { a_stage = 0; a_turn ^= 1u; }
                 tc_fence_after();
 #pragma unroll
                 for (int piece = 0; piece < 3; ++piece) {
@@ -193,7 +230,6 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_f32_tc_kernel(const __grid_co
 #pragma unroll
                     for (int u = 0; u < UNITS; ++u) {
                         piece_of(u, h + 4 * u, piece == 0, piece == 2);
-                        if (piece == 2 && i + 1 < slices) ask(u, i + 1);
                     }
                     store_columns(tmem_base + ((uint32_t)((warp & 3) * 32) << 16) + TMEM_A + (s * 3 + piece) * A_COLS + 16 * a_half, h);
                 }
@@ -255,7 +291,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_f32_tc_kernel(const __grid_co
         const unsigned long long t0 = global_timer();
         while (global_timer() - t0 < 2000000ull) __nanosleep(1000);
     }
-    if (warp == WORK_WARPS) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(TMEM_COLS) : "memory");
+    if (warp == MMA_WARP) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(TMEM_COLS) : "memory");
     if (p.ranks > 1) {
         cluster_sync_all();
         // a block finishes every ranks-th row: a warp a row, four columns a lane
@@ -301,11 +337,14 @@ extern "C" int qt_gemm_f32_tc(const float* a, const float* w, float* c, int M, i
         const long long cost = (((long long)n_tiles * m_tiles * r + sms - 1) / sms) * (each + (r > 1 ? 3 : 2));
         if (best < 0 || cost < best) { best = cost; ranks = r; per = each; }
     }
+    CUtensorMap map_a;
+    const int rc = tensor_map(&map_a, a, (uint64_t)M, 2 * (uint64_t)K, TILE);     // floats as pairs of 16-bit elements: only copied
+    if (rc) return rc;
     const Params p{a, w, c, M, N, K, ranks, per, status};
-    const size_t smem = 2 * STAGE_BYTES + 1024 + 80;
+    const size_t smem = 2 * STAGE_BYTES + A_STAGES * A_STAGE_BYTES + 1024 + 64 + 16 * A_STAGES + 16;
     const cudaError_t raised = raise_shared<gemm_f32_tc_kernel>(227 * 1024);
     if (raised != cudaSuccess) QT_FAIL(QT_ERR_LAUNCH, "gemm_f32_tc: cannot raise shared memory: %s", cudaGetErrorString(raised));
-    launch_kernel_cluster(gemm_f32_tc_kernel, dim3((unsigned)(n_tiles * ranks), (unsigned)m_tiles), dim3(THREADS), smem, (cudaStream_t)stream, (unsigned)ranks, p);
+    launch_kernel_cluster(gemm_f32_tc_kernel, dim3((unsigned)(n_tiles * ranks), (unsigned)m_tiles), dim3(THREADS), smem, (cudaStream_t)stream, (unsigned)ranks, map_a, p);
     QT_CHECK_LAUNCH("gemm_f32_tc");
     return QT_OK;
 }

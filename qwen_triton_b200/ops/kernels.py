@@ -1538,7 +1538,8 @@ def gemm_f32(a: torch.Tensor, w: torch.Tensor, out: GemmOut) -> None:
 
 
 def gemm_f32_on_tc(a: torch.Tensor, w: torch.Tensor, out: GemmOut) -> bool:
-    """Whether a float product that ``gemm_f32`` takes runs on the tensor cores instead: more than 32 rows."""
+    """Whether a float product that ``gemm_f32`` takes runs on the tensor cores instead: more than 32 rows (N x K 6144 x 1024, FMA pipe / tensor cores:
+    32 rows 20.4 / 29.7 us, 33 34.7 / 29.7, 549 177 / 67; 64 x 64 33 rows 5.5 / 5.0)."""
     return a.shape[0] > 32 and (w.shape[0] % 4 != 0 or out.tensor.data_ptr() % 16 == 0)
 
 
