@@ -1,0 +1,43 @@
+"""Which products of few tokens run where (host decisions, no device)."""
+import pytest
+import torch
+
+from qwen_triton_b200.ops import kernels
+from qwen_triton_b200.ops.kernels import GemmOut, ScaledRows
+from qwen_triton_b200.parts import linear
+from test_linear_plans import _Runtime
+
+
+def _linear(out_features, in_features, role="attn_out", dtype=torch.bfloat16):
+    made = linear.Linear("x", out_features, in_features, _Runtime(dtype, 64), role=role)
+    made.weight = torch.zeros(out_features, in_features, dtype=dtype)
+    return made
+
+
+@pytest.mark.parametrize("rows, role, plan", [(1, "gate", (32, 8)), (8, "qkv", (32, 8)), (9, "gate", (32, 16)), (16, "attn_out", (16, 16)), (17, "attn_out", None), (1, "", (16, 16))])
+def test_few_tokens_on_a_small_weight(rows, role, plan):
+    x = torch.zeros(rows, 1024, dtype=torch.bfloat16)
+    assert _linear(4096, 1024, role).few_plan(x) == plan
+    assert _linear(4096, 1024, role).few_plan(ScaledRows(x, torch.zeros(8, rows), 1024, 1e-6)) == plan
+
+
+def test_what_keeps_the_ring():
+    x = torch.zeros(4, 4096, dtype=torch.bfloat16)
+    assert _linear(4096, 4096).few_plan(x) is None                               # 16 M elements: bound by its bytes
+    assert _linear(2048, 4096).few_plan(x) == (16, 16)                           # 8 M
+    assert _linear(512, 1000).few_plan(torch.zeros(4, 1000, dtype=torch.bfloat16)) is None     # rows off 32-byte boundaries
+    shifted = torch.zeros(4 * 1024 + 8, dtype=torch.bfloat16)[8:].view(4, 1024)
+    assert _linear(512, 1024).few_plan(shifted) is None or shifted.data_ptr() % 32 == 0
+
+
+def test_the_sums_of_squares_follow_the_kernel():
+    few, many = torch.zeros(8, 2048, dtype=torch.bfloat16), torch.zeros(17, 2048, dtype=torch.bfloat16)
+    made = _linear(1024, 2048)
+    assert made.norm_tiles(few, 1024) == 64 and made.norm_tiles(many, 1024) == 8
+    assert _linear(1000, 2048).norm_tiles(few, 1000) == 63
+
+
+@pytest.mark.parametrize("rows, on", [(1, False), (32, False), (33, True), (549, True)])
+def test_float_products_on_the_tensor_cores(rows, on):
+    a, w = torch.zeros(rows, 64), torch.zeros(128, 64)
+    assert kernels.gemm_f32_on_tc(a, w, GemmOut(torch.zeros(1, rows, 128))) is on

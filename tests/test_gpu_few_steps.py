@@ -1,0 +1,67 @@
+"""Steps of few tokens: the greedy choice over a cluster, decode attention in the order of the lengths, experts read once for their pairs."""
+import pytest
+import torch
+
+from qwen_triton_b200.ops import kernels
+from qwen_triton_b200.ops.kernels import GemmOut
+from test_gpu_kernels import DEV, PAGE, rand
+
+pytestmark = pytest.mark.gpu
+BF16 = torch.bfloat16
+
+
+@pytest.mark.parametrize("rows, vocab", [(1, 151936), (3, 151937), (40, 32768), (64, 16384), (2, 4099)])
+def test_greedy_choice_over_parts_of_a_row(rows, vocab):
+    logits = rand(rows, vocab, seed=1)
+    places = [(7 * i * i + 13) % (vocab - 1) for i in range(rows)]
+    for i, at in enumerate(places):
+        logits[i, at], logits[i, vocab - 1] = 50.0, 50.0                     # a tie with another part's last id: the lower one
+    logits[0, :] = -float("inf")
+    if rows > 1:
+        logits[1, : vocab // 2] = float("nan")                               # never chosen
+        logits[1, vocab - 1] = 60.0
+    out = torch.empty(rows, dtype=torch.int32, device=DEV)
+    kernels.argmax(logits, out)
+    assert out.tolist() == [0] + ([vocab - 1] if rows > 1 else []) + places[2:]
+
+
+@pytest.mark.parametrize("window", [None, 70])
+def test_decode_attention_does_not_depend_on_the_order_of_the_lengths(window):
+    """More blocks than are resident at once are handed out longest first; eight sequences at a time are not."""
+    seqs, nq, nkv, d = 41, 16, 8, 128
+    lengths = torch.tensor([1 + (i * 7919) % 193 for i in range(seqs)], dtype=torch.int32, device=DEV)
+    width = -(-193 // PAGE)
+    k, v = rand(seqs * width, nkv, PAGE, d, seed=2, dtype=BF16), rand(seqs * width, nkv, PAGE, d, seed=3, dtype=BF16)
+    table = torch.arange(seqs * width, dtype=torch.int32, device=DEV).view(seqs, width)
+    q = rand(seqs, nq, d, seed=4, dtype=BF16)
+    whole, parts = torch.full_like(q, float("nan")), torch.full_like(q, float("nan"))
+    kernels.attention_decode(q, k, v, whole, table, lengths, nkv, PAGE, 0, window, d ** -0.5, 1, None, None, warps=3)
+    for i in range(0, seqs, 8):
+        some = slice(i, min(i + 8, seqs))
+        kernels.attention_decode(q[some], k, v, parts[some], table[some].contiguous(), lengths[some], nkv, PAGE, 0, window, d ** -0.5, 1, None, None, warps=3)
+    assert torch.equal(whole, parts)
+
+
+@pytest.mark.parametrize("experts, top, width, ff, tokens, skew", [(8, 1, 1024, 2048, 8, False), (4, 2, 2048, 1040, 15, False), (3, 1, 2064, 1024, 32, True),
+                                                                   (2, 2, 1040, 2032, 1, False), (16, 2, 2048, 1024, 16, True)])
+@pytest.mark.parametrize("gated", [True, False])
+@pytest.mark.parametrize("weights", ["output", "input", "none"])
+def test_experts_read_once_for_all_of_their_pairs(experts, top, width, ff, tokens, skew, gated, weights):
+    """Groups of one pair to four groups of eight of one expert; features and columns that end inside a block."""
+    x, up, down = rand(tokens, width, seed=1, dtype=BF16), rand(experts, (2 if gated else 1) * ff, width, seed=2, scale=0.03, dtype=BF16), \
+        rand(experts, width, ff, seed=3, scale=0.03, dtype=BF16)
+    table = torch.stack([torch.arange(top) if skew else torch.randperm(experts, generator=torch.Generator().manual_seed(t))[:top] for t in range(tokens)]).int().to(DEV)
+    pair = 0.5 + rand(tokens, top, seed=5).abs()
+    base, scale = rand(2, tokens, width, seed=6), rand(tokens, seed=7)
+    mid, out = torch.empty(tokens * top, ff, dtype=BF16, device=DEV), torch.full((tokens, width), float("nan"), device=DEV)
+    kernels.experts_by_pair(x, None, table, up, down, mid, out, "silu", pair_weight=0.7, pair_weights=pair if weights == "output" else None, gated=gated,
+                            in_weights=pair if weights == "input" else None, base=GemmOut(base), row_scale=scale)
+    want = scale[:, None].double() * base.double().sum(0)
+    for t in range(tokens):
+        for k in range(top):
+            e, share = int(table[t, k]), float(pair[t, k])
+            h = up[e].double() @ x[t].double() * (share if weights == "input" else 1.0)
+            act = torch.nn.functional.silu(h[:ff]) * h[ff:] if gated else torch.nn.functional.silu(h)
+            want[t] += (down[e].double() @ act.to(BF16).double()) * (share if weights == "output" else 0.7)
+    # the activations are rounded to bfloat16 (2^-9 of each; here some round the other way than the 64-bit ones), the rest are float sums
+    assert float((out.double() - want).norm()) <= 2.0 ** -9 * float(want.norm())
