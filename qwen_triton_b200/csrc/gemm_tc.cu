@@ -331,6 +331,53 @@ template <> __device__ __forceinline__ void store8<__nv_bfloat16>(__nv_bfloat16*
     *reinterpret_cast<uint4*>(dst) = packed;
 }
 
+// 16 results to a 32-byte boundary.  A thread of the pair kernel's epilogue has a row of its own, so an instruction of the warp touches 32 rows,
+// and whole sectors halve what the memory system is asked for.  With 16-byte stores / so, N x K of 2,956 rows: 4096 x 1024 25.3 / 21.5 us, 1024 x 3072 in float planes 24.5 / 20.6;
+// the float products of the Bizurax design's prompts 54 / 48 us each.
+__device__ __forceinline__ void store32(void* dst, const uint32_t (&v)[8]) {
+    asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};"
+                 ::"l"(dst), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]) : "memory");
+}
+template <typename TO> __device__ __forceinline__ void store16(TO* dst, const float (&f)[16]) {
+    if constexpr (sizeof(TO) == 4) {
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            uint32_t v[8];
+#pragma unroll
+            for (int j = 0; j < 8; ++j) v[j] = __float_as_uint(f[8 * h + j]);
+            store32(dst + 8 * h, v);
+        }
+    } else {
+        static_assert(sizeof(TO) == 2, "");
+        uint32_t v[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            const TO pair[2] = {from_float<TO>(f[2 * j]), from_float<TO>(f[2 * j + 1])};
+            v[j] = (uint32_t)reinterpret_cast<const uint16_t&>(pair[0]) | (uint32_t)reinterpret_cast<const uint16_t&>(pair[1]) << 16;
+        }
+        store32(dst, v);
+    }
+}
+
+// Up to 16 neighbouring results of a row, `left` of which are inside it.  (The results are formed once, whatever stores them: a second copy of the
+// gates' arithmetic does not fit the instruction cache beside the first, and the gated product took 2.4 times as long.)
+template <typename TO> __device__ __forceinline__ void store_run(TO* dst, const float (&f)[16], int left, int vector_stores) {
+    if (vector_stores == 2 && left >= 16) { store16<TO>(dst, f); return; }
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        if (vector_stores && left >= 8 * h + 8) {
+            float part[8];
+#pragma unroll
+            for (int j = 0; j < 8; ++j) part[j] = f[8 * h + j];
+            store8<TO>(dst + 8 * h, part);
+        } else {
+#pragma unroll
+            for (int j = 0; j < 8; ++j)
+                if (8 * h + j < left) dst[8 * h + j] = from_float<TO>(f[8 * h + j]);
+        }
+    }
+}
+
 template <typename TO, int MODE>
 __global__ void __launch_bounds__(THREADS, 1) gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_w,
                                                                   const __grid_constant__ CUtensorMap map_x, TO* __restrict__ out,
@@ -554,20 +601,10 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_tc_pair_kernel(const __grid_c
                     // columns c .. c + 15 are the gate rows of 16 features, c + 16 .. c + 31 the up rows of the same
                     const int f0 = (n0 + c) >> 1;
                     TO* dst = row + (c >> 1);
+                    float f[16];
 #pragma unroll
-                    for (int h = 0; h < 2; ++h) {
-                        float f[8];
-#pragma unroll
-                        for (int j = 0; j < 8; ++j)
-                            f[j] = gated_value<true>(__uint_as_float(v[8 * h + j]), __uint_as_float(v[16 + 8 * h + j]), act, limit);
-                        if (vector_stores && f0 + 8 * h + 8 <= features) {
-                            store8<TO>(dst + 8 * h, f);
-                        } else {
-#pragma unroll
-                            for (int j = 0; j < 8; ++j)
-                                if (f0 + 8 * h + j < features) dst[8 * h + j] = from_float<TO>(f[j]);
-                        }
-                    }
+                    for (int j = 0; j < 16; ++j) f[j] = gated_value<true>(__uint_as_float(v[j]), __uint_as_float(v[16 + j]), act, limit);
+                    store_run<TO>(dst, f, features - f0, vector_stores);
                 } else if (MODE == KEYS_VALUES) {          // pieces of 32 columns are all keys or all values
                     const float4 scale = run_scale[m >> 6];
                     const float factor = n0 + c < key_cols ? scale.x : scale.z;
@@ -580,20 +617,14 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_tc_pair_kernel(const __grid_c
                     }
                 } else {
 #pragma unroll
-                    for (int h = 0; h < 4; ++h) {
-                        float f[8];
+                    for (int h = 0; h < 2; ++h) {
+                        float f[16];
 #pragma unroll
-                        for (int j = 0; j < 8; ++j) {
-                            const float y = __uint_as_float(v[8 * h + j]);
+                        for (int j = 0; j < 16; ++j) {
+                            const float y = __uint_as_float(v[16 * h + j]);
                             f[j] = MODE == ACTIVATED ? gate_activation<true>(y, act) : y;
                         }
-                        if (vector_stores && n0 + c + 8 * h + 8 <= N) {
-                            store8<TO>(row + c + 8 * h, f);
-                        } else {
-#pragma unroll
-                            for (int j = 0; j < 8; ++j)
-                                if (n0 + c + 8 * h + j < N) row[c + 8 * h + j] = from_float<TO>(f[j]);
-                        }
+                        store_run<TO>(row + c + 16 * h, f, N - n0 - c - 16 * h, vector_stores);
                     }
                 }
             }
@@ -678,9 +709,10 @@ int launch_pair(const CUtensorMap& map_w, const CUtensorMap& map_x, TO* out, int
     const int kb_per_split = (kb_total + splits - 1) / splits;
     const int tail_tiles = splits == 1 && tail_scratch && tail_flags ? pick_tail_tiles(items, resident_pairs, kb_total, tail, tail_pairs) : 0;
     if (tail_tiles) pairs = (unsigned)resident_pairs;        // fewer tiles than pairs: all of them by K ranges over every pair
-    // 16-byte stores need every output row (and plane) to start on a 16-byte boundary
-    const int per16 = 16 / (int)sizeof(TO), row_elems = MODE == GATED ? N / 2 : N;
-    const int vector_stores = ((uintptr_t)out % 16 == 0 && row_elems % per16 == 0 && split_stride % per16 == 0) ? 1 : 0;
+    // stores of 32 bytes (2) or 16 (1) need every output row (and plane) to start on such a boundary
+    const int row_elems = MODE == GATED ? N / 2 : N;
+    const auto rows_at = [&](int bytes) { const int per = bytes / (int)sizeof(TO); return (uintptr_t)out % bytes == 0 && row_elems % per == 0 && split_stride % per == 0; };
+    const int vector_stores = rows_at(32) ? 2 : rows_at(16) ? 1 : 0;
     launch_kernel_cluster(gemm_tc_pair_kernel<TO, MODE>, dim3(2 * pairs), dim3(THREADS), smem, stream, 2, map_w, map_x, out, M, N, kb_total,
                           kb_per_split, splits, split_stride, act, limit, vector_stores, tail_tiles, tail_scratch, tail_flags, bias, run_scale, key_cols, status);
     QT_CHECK_LAUNCH("gemm_tc_pair");
