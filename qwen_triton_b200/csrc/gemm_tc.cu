@@ -359,8 +359,7 @@ template <typename TO> __device__ __forceinline__ void store16(TO* dst, const fl
     }
 }
 
-// Up to 16 neighbouring results of a row, `left` of which are inside it.  (The results are formed once, whatever stores them: a second copy of the
-// gates' arithmetic does not fit the instruction cache beside the first, and the gated product took 2.4 times as long.)
+// Up to 16 neighbouring results of a row, `left` of which are inside it.
 template <typename TO> __device__ __forceinline__ void store_run(TO* dst, const float (&f)[16], int left, int vector_stores) {
     if (vector_stores == 2 && left >= 16) { store16<TO>(dst, f); return; }
 #pragma unroll
@@ -601,10 +600,20 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_tc_pair_kernel(const __grid_c
                     // columns c .. c + 15 are the gate rows of 16 features, c + 16 .. c + 31 the up rows of the same
                     const int f0 = (n0 + c) >> 1;
                     TO* dst = row + (c >> 1);
-                    float f[16];
 #pragma unroll
-                    for (int j = 0; j < 16; ++j) f[j] = gated_value<true>(__uint_as_float(v[j]), __uint_as_float(v[16 + j]), act, limit);
-                    store_run<TO>(dst, f, features - f0, vector_stores);
+                    for (int h = 0; h < 2; ++h) {            // eight at a time: sixteen gates formed ahead of their store took 2.4 times as long
+                        float f[8];
+#pragma unroll
+                        for (int j = 0; j < 8; ++j)
+                            f[j] = gated_value<true>(__uint_as_float(v[8 * h + j]), __uint_as_float(v[16 + 8 * h + j]), act, limit);
+                        if (vector_stores && f0 + 8 * h + 8 <= features) {
+                            store8<TO>(dst + 8 * h, f);
+                        } else {
+#pragma unroll
+                            for (int j = 0; j < 8; ++j)
+                                if (f0 + 8 * h + j < features) dst[8 * h + j] = from_float<TO>(f[j]);
+                        }
+                    }
                 } else if (MODE == KEYS_VALUES) {          // pieces of 32 columns are all keys or all values
                     const float4 scale = run_scale[m >> 6];
                     const float factor = n0 + c < key_cols ? scale.x : scale.z;
