@@ -1,5 +1,6 @@
 // C[M, N] = A[M, K] * W[N, K]^T in true float on the FMA pipe (no tensor cores, no reduced-precision mode): the 32-bit path's
-// products wherever rows are 16-byte aligned (K % 4 == 0).  gemm_simt.cu keeps the other alignments and bfloat16 operands.
+// products of up to 32 rows wherever these are 16-byte aligned (K % 4 == 0); more rows are gemm_f32_tc.cu's.  gemm_simt.cu keeps the other alignments and
+// bfloat16 operands.
 //
 // Both kernels multiply with fma.rn.f32x2 along K: a 16-byte piece of a row is two pairs of neighbouring k, which is how both
 // operands lie in memory, so no value is duplicated or repacked; the even and the odd k of a sum are added at the end.
