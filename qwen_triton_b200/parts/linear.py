@@ -201,6 +201,13 @@ class Linear:
         wide = self.role in ("gate", "qkv")
         return (32 if wide else 16), (8 if wide and rows <= 8 else 16)
 
+    def plain_few_plan(self, x) -> tuple[int, int] | None:
+        """``few_plan`` for a product that nothing is fused to.  The switches that give the small kernels back (``QT_B200_FUSED``, whose list of roles
+        names no product without one, and ``QT_B200_FUSED_ROWS``) give this product's partial sums back too."""
+        if not self.fused_plans or x.shape[0] > _FUSED_ROWS or not kernels.fused_enabled(self.role):
+            return None
+        return self.few_plan(x)
+
     def norm_tiles(self, x, width: int) -> int:
         """Column ranges whose sums of squares ``into_residual`` hands on for rows of ``width`` elements."""
         few = self.few_plan(x)
@@ -236,7 +243,7 @@ class Linear:
                 out = self.runtime.workspace.view(f"{self.key}.out" if self.float_out else f"{self.key}.wide", rows, self.out_features)
             kernels.gemm_fused_store(x, self.weight, out.view(rows, self.out_features), splits=self._fused_splits(rows), bias=self._loaded_bias(), few=self.few_plan(x))
             return GemmOut(out.view(1, rows, self.out_features))
-        few = self.few_plan(x) if out is None and self.fused_plans else None
+        few = self.plain_few_plan(x) if out is None else None
         if few is not None:                # one finished plane, where the products below would hand partial sums to the consumer
             plane = self.runtime.workspace.view(f"{self.key}.out" if self.float_out else f"{self.key}.wide", rows, self.out_features)
             kernels.gemm_fused_store(x, self.weight, plane, bias=self._loaded_bias(), few=few)

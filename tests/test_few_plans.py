@@ -30,6 +30,28 @@ def test_what_keeps_the_ring():
     assert _linear(512, 1024).few_plan(shifted) is None or shifted.data_ptr() % 32 == 0
 
 
+@pytest.mark.parametrize("setting, role, few", [("1", "", True), ("1", "qkv", True), ("0", "", False), ("0", "attn_out", False), ("qkv,gate", "qkv", True),
+                                                ("qkv,gate", "mlp_out", False), ("qkv,gate", "", False)])
+def test_plain_products_follow_the_switch_of_the_fused_ones(monkeypatch, setting, role, few):
+    monkeypatch.setenv("QT_B200_FUSED", setting)
+    x = torch.zeros(4, 1024, dtype=torch.bfloat16)
+    assert (_linear(4096, 1024, role).plain_few_plan(x) is not None) is few
+    monkeypatch.setattr(linear, "_FUSED_ROWS", 3)
+    assert _linear(4096, 1024, role).plain_few_plan(x) is None
+
+
+def test_the_product_itself_asks_the_switch(monkeypatch):
+    made, taken = _linear(512, 1024, ""), []
+    made.runtime.workspace.view = lambda name, *shape: torch.empty(shape)
+    monkeypatch.setattr(kernels, "gemm_fused_store", lambda *args, **kwargs: taken.append("few"))
+    monkeypatch.setattr(kernels, "gemm", lambda *args, **kwargs: taken.append("plain"))
+    x = torch.zeros(4, 1024, dtype=torch.bfloat16)
+    for setting in ("1", "0"):
+        monkeypatch.setenv("QT_B200_FUSED", setting)
+        made(x)
+    assert taken == ["few", "plain"]
+
+
 def test_the_sums_of_squares_follow_the_kernel():
     few, many = torch.zeros(8, 2048, dtype=torch.bfloat16), torch.zeros(17, 2048, dtype=torch.bfloat16)
     made = _linear(1024, 2048)
