@@ -93,13 +93,15 @@ extern "C" int qt_attention_decode_mma(const void* q, const void* k_cache, const
 
 // The decode kernel that gives every warp a key range of its own: `n_splits` blocks of `warps` warps per
 // (sequence, kv head).  Two to eight blocks form a cluster and merge in the first block's shared memory (one
-// launch, no scratch); more go through scratch and the combine kernel.
+// launch, no scratch); more go through scratch and the combine kernel.  `order` (or null) holds every sequence's number
+// and its length of seq_len, the most keys first.
 extern "C" int qt_attention_decode_ws(const void* q, const void* k_cache, const void* v_cache, void* out,
                                       const int* block_table, int max_blocks, const int* seq_len, int n_seqs, int nq,
                                       int nkv, int d, int page_tokens, int ring_tokens, int window, float scale,
                                       int n_splits, int warps, float* part_acc, float* part_ml, const float* r1, const float* r2,
                                       int chunk, int nv, int keep_first, int sink, const float* sinks, float softcap, int cap_small,
-                                      void* stream) {
+                                      const int* order, void* stream) {
+    QT_REQUIRE((uintptr_t)order % 8 == 0, "attention_decode_ws: the order of the sequences must start on an 8-byte boundary");
     QT_REQUIRE(chunk >= 0 && nv >= 0 && (nv == 0 || nkv % nv == 0), "attention_decode_ws: chunk=%d, %d value heads for %d key heads", chunk, nv, nkv);
     if (n_seqs == 0) return QT_OK;
     int rc = check("attention_decode_ws", n_seqs, nq, nkv, d, page_tokens, ring_tokens, window);
@@ -126,10 +128,12 @@ extern "C" int qt_attention_decode_ws(const void* q, const void* k_cache, const 
                 n_splits, part_acc, part_ml, 2, cluster ? 1 : 0, r1, r2, chunk, nv, keep_first, sink, sinks, softcap};
     const size_t smem = rings + (cluster ? inboxes : 0);
     dim3 grid(n_splits, nkv * ((group + 15) / 16), n_seqs), block(32 * warps);
-    // Blocks beyond those resident at once start when others end: the longest sequences first, so that none is left over at the end
-    // (64 sequences of 1,024 to 2,048 tokens, 36 layers: a step of 6,451 us is 6,310 with this and the quicker greedy choice).
+    // Blocks beyond those resident at once start when others end: the longest sequences first, so that none is left over at the end.  The host orders
+    // them once a step, and a block reads its sequence and length where it would read the length (whole steps without an order / with one: 64 sequences
+    // of 1,024 to 2,048 tokens on the 8B shape 6,578 / 6,427 us; of 2,048 each 7,109 / 7,134, where every block ranking all lengths by itself took 7,236; of
+    // 200 each on the 0.6B shape 1,602 / 1,603, 1,636 so).  A mask in chunks leaves a sequence as many keys as it has behind its last boundary, whatever its length.
     const long long resident = (long long)(227 * 1024 / (smem + 1024)) * sm_count();
-    p.longest_first = n_seqs > 1 && n_seqs <= WS_MOST_ORDERED && (long long)grid.x * grid.y * grid.z > resident;
+    if (chunk == 0 && (long long)grid.x * grid.y * grid.z > resident) p.order = reinterpret_cast<const int2*>(order);
     cudaStream_t s = (cudaStream_t)stream;
 #define QT_LAUNCH_WS(DMAX, EXACT, PEN, CAP)                                                                              \
     do {                                                                                                                 \

@@ -64,8 +64,8 @@ struct MmaParams {
     const float* sinks = nullptr;
     // softcap (kernels instantiated with a CAP): scores pass softcap tanh(s / softcap) first; the sink's does not.
     float softcap = 0.f;
-    // decode, one range per warp: the sequences with the most keys are handed out first (more blocks than are resident at once).
-    int longest_first = 0;
+    // decode, one range per warp: {sequence, its length} in the order in which the blocks take them, or null for the order they come in.
+    const int2* order = nullptr;
 };
 
 // The factor on a row's accumulator and its new denominator when the sink term joins a softmax whose running maximum
@@ -394,26 +394,6 @@ struct WarpTileCopy {
     }
 };
 
-// The sequence whose place is `place` among the step's when the one with the most keys comes first.  The whole block calls; `lens` holds n_seqs + 1
-// words of shared memory that are free again behind it.
-constexpr int WS_MOST_ORDERED = 128;
-__device__ __forceinline__ int sequence_by_length(const MmaParams& p, int place, int* lens) {
-    const int most = p.window > 0 ? p.window + p.keep_first : 0x7fffffff;
-    for (int i = threadIdx.x; i < p.n_seqs; i += blockDim.x) lens[i] = min(p.seq_len[i], most);
-    __syncthreads();
-    for (int i = threadIdx.x; i < p.n_seqs; i += blockDim.x) {
-        const int mine = lens[i];
-        int longer = 0;
-#pragma unroll 8
-        for (int j = 0; j < p.n_seqs; ++j) longer += lens[j] > mine || (lens[j] == mine && j < i) ? 1 : 0;
-        if (longer == place) lens[p.n_seqs] = i;                     // one thread of the block: the places are all different
-    }
-    __syncthreads();
-    const int seq = lens[p.n_seqs];
-    __syncthreads();
-    return seq;
-}
-
 template <int DMAX, bool EXACT, bool PEN = false, int CAP = CAP_NONE>
 __global__ void __launch_bounds__(32 * WS_MAX_WARPS) attention_decode_ws_kernel(const MmaParams p) {
     pdl_launch_dependents();
@@ -430,7 +410,8 @@ __global__ void __launch_bounds__(32 * WS_MAX_WARPS) attention_decode_ws_kernel(
     const int rows = min(16, group - h0);
     const int head_base = kvh * group + h0;
     const int split = blockIdx.x;
-    const int seq = p.longest_first ? sequence_by_length(p, blockIdx.z, reinterpret_cast<int*>(smem_raw)) : blockIdx.z;
+    const int2 mine = p.order ? p.order[blockIdx.z] : make_int2(blockIdx.z, p.seq_len[blockIdx.z]);      // one read either way
+    const int seq = mine.x, len = mine.y;
     const int stream = split * warps + warp, n_streams = gridDim.x * warps;
 
     __nv_bfloat16* q_s = reinterpret_cast<__nv_bfloat16*>(smem_raw);                 // [16][lds]
@@ -438,7 +419,6 @@ __global__ void __launch_bounds__(32 * WS_MAX_WARPS) attention_decode_ws_kernel(
     const uint32_t q_bytes = 16u * lds * 2u;
     const uint32_t ring0 = smem_u32(smem_raw) + q_bytes + (uint32_t)warp * 4u * tile_bytes;   // [stage][K tile, V tile]
 
-    const int len = p.seq_len[seq];
     const int lo = max(p.window > 0 ? max(0, len - p.window) : 0, chunk_start(len - 1, p.chunk));
     const int nv = p.nv > 0 ? p.nv : p.nkv, vh = kvh % nv;
     const int first_tile = lo / WS_TILE, last_tile = (len - 1) / WS_TILE;

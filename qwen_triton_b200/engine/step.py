@@ -62,6 +62,7 @@ class StepContext:
         self.is_decode = False
         self.token_ids = self.token_seq = self.token_pos = None
         self.seq_start = self.seq_past = self.seq_len = self.slots = self.want_rows = None
+        self.order = None          # [sequences, 2]: number and length, the longest first (planned one-token passes)
         self._tables: dict[int, torch.Tensor] = {}
         self._decode_plans: dict[tuple, "_DecodePlan"] = {}
 
@@ -70,7 +71,7 @@ class StepContext:
 
     @staticmethod
     def meta_size(max_tokens: int, max_seqs: int, table_widths: list[int]) -> int:
-        return 4 * max_tokens + 5 * max_seqs + 8 + max_seqs * sum(table_widths) + 64
+        return 4 * max_tokens + 7 * max_seqs + 8 + max_seqs * sum(table_widths) + 64
 
     def fill(self, slots: list[int], tokens: list[list[int]], past: list[int], want_rows: list[int],
              tables: list[np.ndarray], max_context: int | None = None) -> None:
@@ -107,6 +108,7 @@ class StepContext:
         (self.token_ids, self.token_seq, self.token_pos, self.seq_start, self.seq_past, self.seq_len,
          self.slots, self.want_rows) = views[:8]
         self._tables = {g: views[8 + g].view(n_seqs, tables[g].shape[1]) for g in range(len(tables))}
+        self.order = None
         self.n_tokens, self.n_seqs, self.n_want = n_tokens, n_seqs, len(want_rows)
         self.max_q_len = max(q_lens) if q_lens else 0
         self.max_context = max_context if max_context is not None else (int(seq_len.max()) if n_seqs else 0)
@@ -128,6 +130,8 @@ class StepContext:
         array[2 * n:3 * n] = past
         array[plan.at_past:plan.at_past + n] = past
         np.add(array[plan.at_past:plan.at_past + n], 1, out=array[plan.at_len:plan.at_len + n])
+        if n > 1:
+            longest_first(array[plan.at_len:plan.at_len + n], array[plan.at_order:plan.at_order + 2 * n].reshape(n, 2))
         array[plan.at_slots:plan.at_slots + n] = slots
         for offset, table in zip(plan.at_tables, tables):
             array[offset:offset + table.size] = table.reshape(-1)
@@ -149,11 +153,17 @@ class StepContext:
         self.meta_bytes = 4 * plan.total
         (self.token_ids, self.token_seq, self.token_pos, self.seq_start, self.seq_past, self.seq_len,
          self.slots, self.want_rows) = plan.views[:8]
-        self._tables = plan.tables
+        self._tables, self.order = plan.tables, plan.order
         self.n_tokens = self.n_seqs = self.n_want = n
         self.max_q_len = 1
         self.max_context = max_context
         self.is_decode, self.from_start = True, False
+
+
+def longest_first(lengths: np.ndarray, into: np.ndarray) -> None:
+    """Every sequence's number and length, the longest first, equal ones as they come."""
+    into[:, 0] = np.argsort(-lengths, kind="stable")
+    into[:, 1] = lengths[into[:, 0]]
 
 
 class _DecodePlan:
@@ -165,13 +175,15 @@ class _DecodePlan:
         self.n = n
         sizes = [n, n, n, n + 1, n, n, n, n] + [n * w for w in widths]
         offsets = np.concatenate(([0], np.cumsum(sizes))).tolist()
-        self.total = offsets[-1]
+        self.at_order = -(-offsets[-1] // 2) * 2                      # read eight bytes at a time
+        self.total = self.at_order + (2 * n if n > 1 else 0)
         if self.total > meta.numel():
             raise ValueError(f"step metadata of {self.total} words exceeds the buffer of {meta.numel()}")
         self.at_past, self.at_len, self.at_slots = offsets[4], offsets[5], offsets[6]
         self.at_tables = offsets[8:8 + len(widths)]
         self.views = [meta[offsets[i]:offsets[i + 1]] for i in range(len(sizes))]
         self.tables = {g: self.views[8 + g].view(n, w) for g, w in enumerate(widths)}
+        self.order = meta[self.at_order:self.total].view(n, 2) if n > 1 else None
         self.buffers = []
         for _ in range(self.RING):
             host = torch.zeros(self.total, dtype=torch.int32, pin_memory=True)

@@ -125,7 +125,7 @@ _SIGNATURES = {
                                     _c_int, _c_int, _c_int, _c_float, _c_int, _c_ptr, _c_ptr, _c_ptr],
         "qt_attention_decode_ws": [_c_ptr, _c_ptr, _c_ptr, _c_ptr, _c_ptr, _c_int, _c_ptr, _c_int, _c_int, _c_int, _c_int,
                                    _c_int, _c_int, _c_int, _c_float, _c_int, _c_int, _c_ptr, _c_ptr, _c_ptr, _c_ptr, _c_int, _c_int,
-                                   _c_int, _c_int, _c_ptr, _c_float, _c_int, _c_ptr],
+                                   _c_int, _c_int, _c_ptr, _c_float, _c_int, _c_ptr, _c_ptr],
         "qt_attention_prefill_mma": [_c_ptr, _c_ptr, _c_ptr, _c_ptr, _c_ptr, _c_int, _c_ptr, _c_ptr, _c_int, _c_int, _c_int,
                                      _c_int, _c_int, _c_int, _c_int, _c_int, _c_float, _c_ptr, _c_ptr, _c_int, _c_int, _c_int, _c_int, _c_ptr, _c_float, _c_int, _c_ptr],
     },
@@ -1309,8 +1309,9 @@ def attention_decode(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tens
                      part_acc: torch.Tensor | None, part_ml: torch.Tensor | None, impl: str | None = None,
                      warps: int = 1, penalty: tuple[torch.Tensor, torch.Tensor] | None = None, chunk: int | None = None,
                      keep_first: int = 0, sink: bool = False, v_dim: int | None = None, sinks: torch.Tensor | None = None,
-                     softcap: float | None = None, score_bound: float | None = None) -> None:
-    """One query token per sequence; ``seq_len`` counts the keys it sees (its own included).
+                     softcap: float | None = None, score_bound: float | None = None, order: torch.Tensor | None = None) -> None:
+    """One query token per sequence; ``seq_len`` counts the keys it sees (its own included).  ``order`` [sequences, 2] (int32) may name
+    every sequence and its ``seq_len``, the longest first: "ws" hands its blocks out so where not all are resident at once.
 
     With ``n_splits`` > 1 the keys of each sequence are cut into that many ranges whose partial
     results pass through ``part_acc`` (float, >= B nq splits d) and ``part_ml`` (float, >= B nq splits 2).
@@ -1320,6 +1321,8 @@ def attention_decode(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tens
     """
     n_seqs, num_heads, head_dim = _check_attention(q, k_cache, v_cache, out, block_table, num_kv_heads, page_tokens, penalty, v_dim)
     _need(seq_len, "seq_len", torch.int32, (n_seqs,))
+    if order is not None:
+        _need(order, "order", torch.int32, (n_seqs, 2))
     if sinks is not None:
         _need(sinks, "sinks", torch.float32, (num_heads,))
         sink = True
@@ -1361,7 +1364,7 @@ def attention_decode(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tens
     if picked == "ws":
         _call("attention_mma", "qt_attention_decode_ws", *common, int(warps), _ptr(part_acc), _ptr(part_ml),
               _ptr(penalty[0]) if penalty else None, _ptr(penalty[1]) if penalty else None, int(chunk or 0), v_cache.shape[1],
-              int(keep_first), 1 if sink else 0, _ptr(sinks), cap, cap_small, _stream(), launches=launches)
+              int(keep_first), 1 if sink else 0, _ptr(sinks), cap, cap_small, _ptr(order), _stream(), launches=launches)
     elif picked == "mma":
         _call("attention_mma", "qt_attention_decode_mma", *common, _ptr(part_acc), _ptr(part_ml), _stream(), launches=launches)
     else:

@@ -376,7 +376,7 @@ class Attention:
                                      ws.view("attn.part_acc", _MAX_SPLIT_PAIRS * self.nq * self.dv),
                                      ws.view("attn.part_ml", _MAX_SPLIT_PAIRS * self.nq * 2), warps=warps, penalty=penalty,
                                      chunk=self.chunk, keep_first=self.keep_first, sink=bool(self.sink), sinks=self.sinks, softcap=self.softcap,
-                                     score_bound=self.score_bound)
+                                     score_bound=self.score_bound, order=ctx.order)
         else:
             kernels.attention_prefill(q, cache.k, cache.v, out, table, ctx.seq_start, ctx.seq_past, ctx.max_q_len,
                                       self.nkv, cache.page_tokens, cache.ring_tokens, self.window, self.scale, penalty=penalty,

@@ -151,7 +151,7 @@ class ConvAttention:
             kernels.attention_decode(q, keys.k, keys.k, out, table, ctx.seq_len, self.nkv, keys.page_tokens, keys.ring_tokens, self.window,
                                      self.scale, self._splits(ctx), ws.view("attn.part_acc", _MAX_SPLIT_PAIRS * self.nq * self.d),
                                      ws.view("attn.part_ml", _MAX_SPLIT_PAIRS * self.nq * 2), penalty=penalty, keep_first=self.keep_first,
-                                     sink=self.sink)
+                                     sink=self.sink, order=ctx.order)
         else:
             kernels.attention_prefill(q, keys.k, keys.k, out, table, ctx.seq_start, ctx.seq_past, ctx.max_q_len, self.nkv,
                                       keys.page_tokens, keys.ring_tokens, self.window, self.scale, penalty=penalty,

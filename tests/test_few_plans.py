@@ -1,7 +1,9 @@
 """Which products of few tokens run where (host decisions, no device)."""
+import numpy as np
 import pytest
 import torch
 
+from qwen_triton_b200.engine.step import StepContext, longest_first
 from qwen_triton_b200.ops import kernels
 from qwen_triton_b200.ops.kernels import GemmOut, ScaledRows
 from qwen_triton_b200.parts import linear
@@ -63,3 +65,16 @@ def test_the_sums_of_squares_follow_the_kernel():
 def test_float_products_on_the_tensor_cores(rows, on):
     a, w = torch.zeros(rows, 64), torch.zeros(128, 64)
     assert kernels.gemm_f32_on_tc(a, w, GemmOut(torch.zeros(1, rows, 128))) is on
+
+
+@pytest.mark.parametrize("lengths, places", [([5, 5, 5], [0, 1, 2]), ([1, 700, 3, 700, 2], [1, 3, 2, 4, 0]), ([9, 1], [0, 1])])
+def test_the_longest_sequences_come_first(lengths, places):
+    into = np.full((len(lengths), 2), -1, dtype=np.int32)
+    longest_first(np.array(lengths, dtype=np.int32), into)
+    assert into[:, 0].tolist() == places and into[:, 1].tolist() == [lengths[i] for i in places]
+
+
+def test_the_step_metadata_has_room_for_the_order():
+    for n in (2, 3, 48, 256):
+        # a one-token pass of n of the 2 n tokens a pass may have: ids, sequences, positions, starts, pasts, lengths, slots, wanted rows, tables, order
+        assert 8 * n + 1 + n * (16 + 32) + 1 + 2 * n <= StepContext.meta_size(2 * n, n, [16, 32])

@@ -1,7 +1,9 @@
 """Steps of few tokens: the greedy choice over a cluster, decode attention in the order of the lengths, experts read once for their pairs."""
+import numpy as np
 import pytest
 import torch
 
+from qwen_triton_b200.engine.step import longest_first
 from qwen_triton_b200.ops import kernels
 from qwen_triton_b200.ops.kernels import GemmOut
 from test_gpu_kernels import DEV, PAGE, rand
@@ -40,6 +42,31 @@ def test_decode_attention_does_not_depend_on_the_order_of_the_lengths(window):
         some = slice(i, min(i + 8, seqs))
         kernels.attention_decode(q[some], k, v, parts[some], table[some].contiguous(), lengths[some], nkv, PAGE, 0, window, d ** -0.5, 1, None, None, warps=3)
     assert torch.equal(whole, parts)
+
+
+@pytest.mark.parametrize("seqs, mask, splits", [(41, {}, 1), (41, {"window": 70}, 1), (41, {"window": 70, "keep_first": 40}, 1), (41, {"chunk": 64}, 1), (41, {}, 3),
+                                                (130, {}, 1), (3, {}, 2)])
+def test_decode_attention_in_a_given_order(seqs, mask, splits):
+    """The same results whatever order the sequences are handed out in: one block a sequence and head, several that merge in a cluster, more
+    sequences than a block's threads, fewer blocks than are resident (the order is not read)."""
+    nq, nkv, d = 16, 8, 128
+    lengths = [1 + (i * 7919) % 193 for i in range(seqs)]
+    seq_len = torch.tensor(lengths, dtype=torch.int32, device=DEV)
+    width = -(-193 // PAGE)
+    k, v = rand(seqs * width, nkv, PAGE, d, seed=2, dtype=BF16), rand(seqs * width, nkv, PAGE, d, seed=3, dtype=BF16)
+    table = torch.arange(seqs * width, dtype=torch.int32, device=DEV).view(seqs, width)
+    q = rand(seqs, nq, d, seed=4, dtype=BF16)
+    order = np.empty((seqs, 2), dtype=np.int32)
+    longest_first(np.array(lengths, dtype=np.int32), order)
+    results = []
+    for given in (None, order, order[::-1].copy()):
+        out = torch.full_like(q, float("nan"))
+        kernels.attention_decode(q, k, v, out, table, seq_len, nkv, PAGE, 0, mask.get("window"), d ** -0.5, splits, rand(seqs * nq * splits * d, seed=5),
+                                 rand(seqs * nq * splits * 2, seed=6), impl="ws", warps=3, chunk=mask.get("chunk"), keep_first=mask.get("keep_first", 0),
+                                 order=None if given is None else torch.from_numpy(given).to(DEV))
+        results.append(out)
+    assert torch.isfinite(results[0]).all()
+    assert torch.equal(results[0], results[1]) and torch.equal(results[0], results[2])
 
 
 @pytest.mark.parametrize("experts, top, width, ff, tokens, skew", [(8, 1, 1024, 2048, 8, False), (4, 2, 2048, 1040, 15, False), (3, 1, 2064, 1024, 32, True),
