@@ -193,12 +193,16 @@ class Linear:
         8 M elements (``_FEW_WEIGHT``).  Steps of the 0.6B shape (weights of 2 to 6 M) 20 to 31 % shorter at 1 to 16 sequences; of the 8B shape
         (17 to 101 M) 4 % shorter at eight but 7 to 23 % longer at 1, 3 and 16, since its blocks keep fewer bytes in flight than a TMA ring.
         Blocks of 32 rows for heads and gates; 16 rows otherwise, so that a thousand features still give 64 SMs a block (32 rows: one sequence
-        728 us a step instead of 634).  16 warps a block where their sums are short of the weight's arrival: beyond 8 tokens (797 us against 857 with
+        728 us a step instead of 634), as long as all of these are resident at once, two an SM: a second wave costs more than the ring (one to 16 rows, ring / this,
+        plain: 4096 x 1024 3.8 to 4.1 / 3.6 to 3.9 us, but 6144 x 1024 4.2 to 4.5 / 5.3 to 5.7, 8192 x 512 3.7 to 4.1 / 6.0 to 6.3).
+        16 warps a block where their sums are short of the weight's arrival: beyond 8 tokens (797 us against 857 with
         8), and where K is longest for its rows (570 to 590 against 634)."""
         rows = x.shape[0]
         if not 0 < rows <= kernels.FEW_MAX_ROWS or self.weight is None or self.weight.numel() > _FEW_WEIGHT or not kernels.few_supported(x, self.weight):
             return None
         wide = self.role in ("gate", "qkv")
+        if not wide and -(-self.out_features // 16) > 2 * self.runtime.sm_count:
+            return None
         return (32 if wide else 16), (8 if wide and rows <= 8 else 16)
 
     def plain_few_plan(self, x) -> tuple[int, int] | None:

@@ -54,6 +54,11 @@ def test_the_product_itself_asks_the_switch(monkeypatch):
     assert taken == ["few", "plain"]
 
 
+@pytest.mark.parametrize("out_features, role, few", [(4736, "", True), (4737, "", False), (8192, "mlp_out", False), (8192, "gate", True), (6144, "qkv", True)])
+def test_a_second_wave_of_blocks_keeps_the_ring(out_features, role, few):
+    assert (_linear(out_features, 512, role).few_plan(torch.zeros(4, 512, dtype=torch.bfloat16)) is not None) is few
+
+
 def test_the_sums_of_squares_follow_the_kernel():
     few, many = torch.zeros(8, 2048, dtype=torch.bfloat16), torch.zeros(17, 2048, dtype=torch.bfloat16)
     made = _linear(1024, 2048)
