@@ -14,9 +14,12 @@
 //
 // What bounds it now is the splitting: a slice takes 1.9 us (3,300 cycles), and with one product in the place of six 0.9 of that.
 //
-// N x K, rows, us before (gemm_f32.cu) / here: 4096 x 1024 64 19.5 / 13.5, 549 120 / 57, 4,096 802 / 229; 6144 x 1024 549 177 / 67; 1024 x 3072 549 111 / 34; 4096 x 12288 4,096
-// 9,928 / 2,622 (157 TFLOP/s); up to 32 rows the FMA pipe's kernels are as fast or faster.  Error against 64 bits over the result's norm, before / here: random signs, 1,024
-// to 12,288 of K 1.05e-7 to 1.62e-7 / 0.78e-7 to 1.19e-7; operands of one sign 0.43e-7 to 0.63e-7 / 0.46e-7 to 0.62e-7.
+// N x K, rows, us before (gemm_f32.cu) / here, L2 flushed ahead of each: 4096 x 1024 64 27 / 21, 549 129 / 64, 4,096 807 / 236; 6144 x 1024 549 184 / 74; 1024 x 3072 549 117 / 39; 4096 x 12288
+// 549 1,458 / 512, 4,096 9,940 / 2,290 (180 TFLOP/s); up to 32 rows the FMA pipe's kernels are as fast or faster.
+//
+// What is exact in float stays so (one number a row, powers of two, whole numbers up to 2^24).  Error against 64 bits over the result's norm, before / here, 64 to 12,288 of K: random signs
+// 0.84e-7 to 1.61e-7 / 0.78e-7 to 1.40e-7; operands of one sign 0.40e-7 to 0.63e-7 / 0.86e-7 to 0.98e-7, of which 0.79e-7 is the mean of the large instructions' cuts towards zero.  A factor for that
+// mean would round off sums that nothing was cut from; accumulators read back every 32 or 16 of K (0.60e-7 to 0.83e-7, 0.56e-7 to 0.91e-7) cost 10 to 25 % and 35 to 140 % of the time.
 //
 // Infinities, NaN and numbers that round to an infinite bfloat16 have no such pieces: a block that meets one forms its results again with FMAs.
 #include "tc_common.cuh"
@@ -40,8 +43,6 @@ constexpr int MOST_RANKS = 8, PARK_ROW = TILE + 4;
 constexpr uint32_t IDESC = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(TILE >> 3) << 17) | ((uint32_t)(TILE >> 4) << 24);
 static_assert(TILE * PARK_ROW * 4 <= 2 * STAGE_BYTES, "a block's part of the result is parked in the stages' memory");
 
-// What the truncated additions leave out on average, of the sum: 4.7e-8 for operands of one sign and 6.0e-8 for either, alike for every K from 64 to 12,288.
-constexpr float SHORTFALL = 5.4e-8f;
 
 struct Params {
     const float* a; const float* w; float* c;
@@ -167,7 +168,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_f32_tc_kernel(const __grid_co
 #pragma unroll
         for (int j = 0; j < COLS; ++j) sums[j] = 0.f;
         const uint32_t mine = tmem_base + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)(warp >> 2) * COLS;
-        auto add = [&](int i, bool last) {
+        auto add = [&](int i) {
             const int s = i & 1;
             if (!mbar_wait(summed + 8 * s, (uint32_t)(i >> 1) & 1u, status, 3)) return false;
             tc_fence_after();
@@ -176,12 +177,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_f32_tc_kernel(const __grid_co
                 uint32_t x[16];
                 tmem_load16(mine + s * TILE + 16 * part, x);
 #pragma unroll
-                for (int j = 0; j < 16; ++j) {
-                    float& sum = sums[16 * part + j];
-                    float y = __uint_as_float(x[j]);
-                    if (last) y = fmaf(SHORTFALL, sum + y, y);              // of the whole sum, ahead of its last rounding
-                    sum += y;
-                }
+                for (int j = 0; j < 16; ++j) sums[16 * part + j] += __uint_as_float(x[j]);
             }
             tc_fence_before();
             __syncwarp();
@@ -251,9 +247,9 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_f32_tc_kernel(const __grid_co
             }
             __syncwarp();
             if (lane == 0) mbar_arrive(full + 8 * s);
-            if (i > 0) ok = add(i - 1, false);
+            if (i > 0) ok = add(i - 1);
         }
-        if (ok) ok = add(slices - 1, true);
+        if (ok) ok = add(slices - 1);
         if (none != 0.f) atomicOr(odd, 1);                                  // NaN
         asm volatile("bar.sync 1, %0;" ::"n"(WORK_WARPS * 32) : "memory");
         const int row = (warp & 3) * 32 + lane, col0 = (warp >> 2) * COLS, m = m0 + row;

@@ -45,3 +45,38 @@ def test_numbers_without_pieces_are_multiplied_as_floats():
     assert torch.equal(got[~finite & ~torch.isnan(want)], want[~finite & ~torch.isnan(want)])
     exact = a.double() @ w.double().T
     assert bool(((got.double() - exact).abs()[finite] <= 2.0 ** -20 * (a.double().abs() @ w.double().abs().T)[finite]).all())
+
+
+def guarded(a, w):
+    """The product, written ahead of a row that nothing may touch."""
+    m, n = a.shape[0], w.shape[0]
+    held = torch.full((m + 1, n), 7.25, device=DEV)
+    kernels.gemm_f32_tc(a, w, GemmOut(held[:m].unsqueeze(0)))
+    kernels.check_status(DEV)
+    assert bool((held[m] == 7.25).all())
+    return held[:m]
+
+
+@pytest.mark.parametrize("m, n, k", [(33, 3, 4), (129, 131, 64), (40, 70, 68), (300, 129, 1000), (35, 513, 2052), (130, 1024, 4096)])
+def test_what_can_be_exact_is(m, n, k):
+    """Sums of one number, and of whole numbers below 2^24, in one slice, several, and several ranks."""
+    a = rand(m, k, seed=1) * torch.exp(3 * rand(m, k, seed=2))                       # all 24 bits of a mantissa
+    places = torch.arange(n, device=DEV) * 7 % k
+    w = torch.zeros(n, k, device=DEV)
+    w[torch.arange(n, device=DEV), places] = torch.exp2((torch.arange(n, device=DEV) % 19 - 9).float())
+    assert torch.equal(guarded(a, w), a[:, places] * w.sum(1))
+    assert torch.equal(guarded(w, a), (a[:, places] * w.sum(1)).T)
+    whole, signs = (rand(m, k, seed=3) * 30).round(), (rand(n, k, seed=4) * 20).round()
+    assert torch.equal(guarded(whole, signs), (whole.double() @ signs.double().T).float())
+    large = (rand(m, k, seed=5) * 2 ** 21).round()                                   # three pieces each
+    assert torch.equal(guarded(large, torch.sign(w)), large[:, places])
+
+
+@pytest.mark.parametrize("k", [64, 1024, 4096])
+def test_operands_of_one_sign_lose_no_more_than_the_pipe_cuts(k):
+    """Cuts go towards zero: of a slice's four large instructions each takes half a unit of the sum so far (a quarter of the slice's to all of it) on average, at
+    most 2.5 x 2^-24 together; what is rounded to nearest has no mean."""
+    a, w = rand(300, k, seed=1).abs(), rand(500, k, seed=2).abs()
+    want = a.double() @ w.double().T
+    mean = float(((guarded(a, w).double() - want) / want).mean())
+    assert -2.5 * 2.0 ** -24 <= mean <= 2.0 ** -28
