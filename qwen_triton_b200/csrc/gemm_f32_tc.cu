@@ -21,7 +21,8 @@
 // 0.84e-7 to 1.61e-7 / 0.78e-7 to 1.40e-7; operands of one sign 0.40e-7 to 0.63e-7 / 0.86e-7 to 0.98e-7, of which 0.79e-7 is the mean of the large instructions' cuts towards zero.  A factor for that
 // mean would round off sums that nothing was cut from; accumulators read back every 32 or 16 of K (0.60e-7 to 0.83e-7, 0.56e-7 to 0.91e-7) cost 10 to 25 % and 35 to 140 % of the time.
 //
-// Infinities, NaN and numbers that round to an infinite bfloat16 have no such pieces: a block that meets one forms its results again with FMAs.
+// Infinities, NaN and numbers that round to an infinite bfloat16 have no such pieces: a block that meets one forms its results again with FMAs (float_results:
+// 4096 x 1024, 549 rows with a NaN in each 420 us; 4096 x 12288, 4,096 rows 26 ms).
 #include "tc_common.cuh"
 
 using namespace qt;
@@ -39,10 +40,10 @@ constexpr int A_COLS = BK / 2;                         // one piece of A in tens
 constexpr uint32_t TMEM_A = 2 * TILE, TMEM_COLS = 512; // two accumulators, two stages of A's pieces
 constexpr int UNITS = 4;                               // runs of eight elements a thread splits per slice
 constexpr int COLS = 32;                               // results a thread keeps the sums of
-constexpr int MOST_RANKS = 8, PARK_ROW = TILE + 4;
+constexpr int MOST_RANKS = 8, PARK_ROW = TILE + 4, FLOAT_ROW = BK + 4;
 constexpr uint32_t IDESC = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(TILE >> 3) << 17) | ((uint32_t)(TILE >> 4) << 24);
 static_assert(TILE * PARK_ROW * 4 <= 2 * STAGE_BYTES, "a block's part of the result is parked in the stages' memory");
-
+static_assert(2 * TILE * FLOAT_ROW * 4 <= A_STAGES * A_STAGE_BYTES, "a slice of both operands as floats lies in the memory of A's");
 
 struct Params {
     const float* a; const float* w; float* c;
@@ -50,6 +51,18 @@ struct Params {
     int* status;
 };
 
+// mbar_wait without its call: the working warps hold sums and floats across their waits, which a call has them store and load again.
+__device__ __forceinline__ bool wait_here(uint32_t bar, uint32_t parity, int* status, int code) {
+    unsigned long long start = 0;
+    for (uint32_t spins = 0; !mbar_try_wait(bar, parity);) {
+        if ((++spins & 0x3ffu) != 0) continue;
+        if (*(volatile int*)status != 0) return false;
+        const unsigned long long now = global_timer();
+        if (start == 0) start = now;
+        else if (now - start > WAIT_LIMIT_NS) { atomicCAS(status, 0, code); return false; }
+    }
+    return true;
+}
 __device__ __forceinline__ uint32_t pack_rn(float lo, float hi) {
     uint32_t d;
     asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(d) : "f"(hi), "f"(lo));
@@ -74,6 +87,55 @@ __device__ __forceinline__ float4 peer4(uint32_t addr) {
     float4 v;
     asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr) : "memory");
     return v;
+}
+
+// A block's results by FMAs, for numbers that are not the sum of three bfloat16 pieces, written over those of the pieces: to C, or to where a block with peers
+// parks them.  The sixteen working warps call; `tiles` receives a slice of A's rows and of W's after the other.  Sums of 16, of a slice, and of all slices.
+__device__ __noinline__ void float_results(const Params& p, int m0, int n0, int k_begin, int k_end, float* tiles, float* park) {
+    const int row = threadIdx.x & 127, col0 = (int)(threadIdx.x >> 7) * COLS;
+    float sums[COLS] = {};
+#pragma unroll 1
+    for (int k0 = k_begin; k0 < k_end; k0 += BK) {
+        asm volatile("bar.sync 1, %0;" ::"n"(WORK_WARPS * 32) : "memory");
+#pragma unroll 4
+        for (int i = threadIdx.x; i < 2 * TILE * BK / 4; i += WORK_WARPS * 32) {
+            const int r = i / (BK / 4), k = k0 + i % (BK / 4) * 4, at = r < TILE ? m0 + r : n0 + r - TILE;
+            const bool there = at < (r < TILE ? p.M : p.N) && k < k_end;
+            const float4 v = there ? load4((r < TILE ? p.a : p.w) + (size_t)at * p.K + k) : make_float4(0.f, 0.f, 0.f, 0.f);
+            *reinterpret_cast<float4*>(tiles + r * FLOAT_ROW + i % (BK / 4) * 4) = v;
+        }
+        asm volatile("bar.sync 1, %0;" ::"n"(WORK_WARPS * 32) : "memory");
+        const float *x = tiles + row * FLOAT_ROW, *y = tiles + (TILE + col0) * FLOAT_ROW;
+#pragma unroll
+        for (int j0 = 0; j0 < COLS; j0 += 16) {
+            float slice[16] = {};
+#pragma unroll 1
+            for (int k1 = 0; k1 < BK; k1 += 16) {
+                float part[16] = {};
+#pragma unroll 1
+                for (int k = k1; k < k1 + 16; k += 4) {
+                    const float4 u = *reinterpret_cast<const float4*>(x + k);
+#pragma unroll
+                    for (int j = 0; j < 16; ++j) {
+                        const float4 v = *reinterpret_cast<const float4*>(y + (j0 + j) * FLOAT_ROW + k);
+                        part[j] = fmaf(u.w, v.w, fmaf(u.z, v.z, fmaf(u.y, v.y, fmaf(u.x, v.x, part[j]))));
+                    }
+                }
+#pragma unroll
+                for (int j = 0; j < 16; ++j) slice[j] += part[j];
+            }
+#pragma unroll
+            for (int j = 0; j < 16; ++j) sums[j0 + j] += slice[j];
+        }
+    }
+    if (p.ranks > 1) {
+#pragma unroll
+        for (int j = 0; j < COLS; ++j) park[row * PARK_ROW + col0 + j] = sums[j];
+    } else if (m0 + row < p.M) {
+#pragma unroll
+        for (int j = 0; j < COLS; ++j)
+            if (n0 + col0 + j < p.N) p.c[(size_t)(m0 + row) * p.N + n0 + col0 + j] = sums[j];
+    }
 }
 
 __global__ void __launch_bounds__(THREADS, 1) gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ Params p) {
@@ -118,7 +180,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_f32_tc_kernel(const __grid_co
             prefetch_tensor_map(&map_a);
             pdl_wait();
             for (int i = 0, s = 0, turn = 0; i < slices; ++i) {
-                if (!mbar_wait(taken + 8 * s, (uint32_t)turn ^ 1u, status, 1)) break;
+                if (!wait_here(taken + 8 * s, (uint32_t)turn ^ 1u, status, 1)) break;
                 mbar_expect_tx(arrived + 8 * s, A_STAGE_BYTES);
                 for (int h = 0; h < 2; ++h)                                 // the map counts 16-bit elements, two a float
                     tma_load_2d(a_floats + s * A_STAGE_BYTES + h * A_HALF_BYTES, &map_a, arrived + 8 * s, 2 * (k_begin + i * BK + 32 * h), m0);
@@ -132,8 +194,8 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_f32_tc_kernel(const __grid_co
             for (int i = 0; i < slices; ++i) {
                 const int s = i & 1;
                 const uint32_t turn = (uint32_t)(i >> 1) & 1u;
-                if (!mbar_wait(full + 8 * s, turn, status, 2)) break;
-                if (!mbar_wait(added + 8 * s, turn ^ 1u, status, 4)) break;
+                if (!wait_here(full + 8 * s, turn, status, 2)) break;
+                if (!wait_here(added + 8 * s, turn ^ 1u, status, 4)) break;
                 tc_fence_after();
                 const uint64_t w0 = desc0 + (uint64_t)(s * (STAGE_BYTES >> 4));
                 const uint32_t acc = tmem_base + s * TILE, a0 = tmem_base + TMEM_A + s * 3 * A_COLS;
@@ -170,7 +232,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_f32_tc_kernel(const __grid_co
         const uint32_t mine = tmem_base + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)(warp >> 2) * COLS;
         auto add = [&](int i) {
             const int s = i & 1;
-            if (!mbar_wait(summed + 8 * s, (uint32_t)(i >> 1) & 1u, status, 3)) return false;
+            if (!wait_here(summed + 8 * s, (uint32_t)(i >> 1) & 1u, status, 3)) return false;
             tc_fence_after();
 #pragma unroll
             for (int part = 0; part < COLS / 16; ++part) {
@@ -207,10 +269,10 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_f32_tc_kernel(const __grid_co
         bool ok = true;
         for (int i = 0; i < slices && ok; ++i) {
             const int s = i & 1;
-            ok = mbar_wait(empty + 8 * s, ((uint32_t)(i >> 1) & 1u) ^ 1u, status, 1);
+            ok = wait_here(empty + 8 * s, ((uint32_t)(i >> 1) & 1u) ^ 1u, status, 1);
             if (!ok) break;
             if (of_a) {
-                ok = mbar_wait(arrived + 8 * a_stage, a_turn, status, 3);
+                ok = wait_here(arrived + 8 * a_stage, a_turn, status, 3);
                 if (!ok) break;
                 const uint8_t* floats = smem + 2 * STAGE_BYTES + a_stage * A_STAGE_BYTES + a_half * A_HALF_BYTES + a_row * 128;
 #pragma unroll
@@ -250,20 +312,9 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_f32_tc_kernel(const __grid_co
             if (i > 0) ok = add(i - 1);
         }
         if (ok) ok = add(slices - 1);
-        if (none != 0.f) atomicOr(odd, 1);                                  // NaN
+        if (none != 0.f || !ok) atomicOr(odd, ok ? 1 : 2);
         asm volatile("bar.sync 1, %0;" ::"n"(WORK_WARPS * 32) : "memory");
         const int row = (warp & 3) * 32 + lane, col0 = (warp >> 2) * COLS, m = m0 + row;
-        if (*(volatile int*)odd != 0) {
-            const float* x = p.a + (size_t)min(m, p.M - 1) * p.K;
-#pragma unroll 1
-            for (int j0 = 0; j0 < COLS; ++j0) {
-                const float* y = p.w + (size_t)min(n0 + col0 + j0, p.N - 1) * p.K;
-                float sum = 0.f;
-                for (int k = k_begin; k < k_end; ++k) sum = fmaf(x[k], y[k], sum);
-#pragma unroll
-                for (int j = 0; j < COLS; ++j) if (j == j0) sums[j] = sum;    // registers have no index
-            }
-        }
         if (p.ranks > 1) {                                                  // every MMA has read the stages: they are free
             float* park = reinterpret_cast<float*>(smem) + row * PARK_ROW + col0;
 #pragma unroll
@@ -283,6 +334,8 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_f32_tc_kernel(const __grid_co
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
+    if (warp < WORK_WARPS && *(volatile int*)odd == 1)                      // A's floats have all been read: the slices lie in their place
+        float_results(p, m0, n0, k_begin, k_end, reinterpret_cast<float*>(smem + 2 * STAGE_BYTES), reinterpret_cast<float*>(smem));
     if (*(volatile int*)status != 0) {                                      // a wait gave up: let MMAs in flight finish first
         const unsigned long long t0 = global_timer();
         while (global_timer() - t0 < 2000000ull) __nanosleep(1000);
