@@ -21,7 +21,8 @@
 // 0.84e-7 to 1.61e-7 / 0.78e-7 to 1.40e-7; operands of one sign 0.40e-7 to 0.63e-7 / 0.86e-7 to 0.98e-7, of which 0.79e-7 is the mean of the large instructions' cuts towards zero.  A factor for that
 // mean would round off sums that nothing was cut from; accumulators read back every 32 or 16 of K (0.60e-7 to 0.83e-7, 0.56e-7 to 0.91e-7) cost 10 to 25 % and 35 to 140 % of the time.
 //
-// Infinities, NaN and numbers that round to an infinite bfloat16 have no such pieces: a block that meets one forms its results again with FMAs (float_results:
+// Infinities, NaN, numbers that round to an infinite bfloat16 and those whose last piece lies below bfloat16's smallest (under 2^-110, at the earliest 2^-102) have no
+// such pieces: a block that meets one forms its results again with FMAs (float_results:
 // 4096 x 1024, 549 rows with a NaN in each 420 us; 4096 x 12288, 4,096 rows 26 ms).
 #include "tc_common.cuh"
 
@@ -254,6 +255,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_f32_tc_kernel(const __grid_co
         int a_stage = 0;
         uint32_t a_turn = 0;
         float none = 0.f;                                                   // stays 0 while every number has its pieces
+        uint32_t rest = 0;                                                  // its low half stays 0 while every third piece is all that is left
         // the next piece of a unit: its numbers rounded, and what is left of them
         auto piece_of = [&](int u, uint32_t* h, bool first, bool last) {
 #pragma unroll
@@ -261,7 +263,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_f32_tc_kernel(const __grid_co
                 float& lo = v[u][2 * j];
                 float& hi = v[u][2 * j + 1];
                 h[j] = pack_rn(lo, hi);
-                if (last) continue;
+                if (last) { rest |= __float_as_uint(lo) | __float_as_uint(hi); continue; }
                 lo -= low_of(h[j]); hi -= high_of(h[j]);
                 if (first) { none = fmaf(0.f, lo, none); none = fmaf(0.f, hi, none); }
             }
@@ -312,7 +314,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_f32_tc_kernel(const __grid_co
             if (i > 0) ok = add(i - 1);
         }
         if (ok) ok = add(slices - 1);
-        if (none != 0.f || !ok) atomicOr(odd, ok ? 1 : 2);
+        if (none != 0.f || (rest & 0xffffu) != 0 || !ok) atomicOr(odd, ok ? 1 : 2);
         asm volatile("bar.sync 1, %0;" ::"n"(WORK_WARPS * 32) : "memory");
         const int row = (warp & 3) * 32 + lane, col0 = (warp >> 2) * COLS, m = m0 + row;
         if (p.ranks > 1) {                                                  // every MMA has read the stages: they are free

@@ -91,3 +91,11 @@ def test_rows_beside_one_without_pieces_keep_their_precision(m, n, k):
     keep = torch.arange(m, device=DEV) != 5
     assert bool(torch.isnan(got[5]).all())
     assert float((got.double() - want)[keep].norm()) <= 2e-7 * float(want[keep].norm())
+
+
+@pytest.mark.parametrize("power", [-90, -101, -110, -118, -126, -140])
+def test_numbers_whose_last_piece_bfloat16_cannot_hold(power):
+    a, w = rand(130, 192, seed=6) * 2.0 ** power, rand(70, 192, seed=7) * 2.0 ** 80
+    want = a.double() @ w.double().T
+    for got, exact in ((guarded(a, w), want), (guarded(w, a), want.T)):
+        assert float((got.double() - exact).norm()) <= 2e-7 * float(want.norm())
