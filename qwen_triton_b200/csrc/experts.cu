@@ -342,18 +342,18 @@ __global__ void __launch_bounds__(EG_WARPS * 32, 2) expert_up_groups_kernel(cons
         for (int h = 0; h < 2; ++h)
             row[r][h] = w + (size_t)(GATED ? r * p.ff + min(f0 + 8 * h + g, p.ff - 1) : min(f0 + 16 * r + 8 * h + g, p.ff - 1)) * K;
     const int turns = (K + EG_STEP - 1) / EG_STEP, mine = (turns - warp + EG_WARPS - 1) / EG_WARPS;
-    qt_few::Line<16> a[DEPTH][2][2], b[DEPTH];
+    qt_few::Line a[DEPTH][2][2], b[DEPTH];
     auto ask = [&](int slot, int i) {
         const int k = (warp + i * EG_WARPS) * EG_STEP + 16 * t;
 #pragma unroll
         for (int r = 0; r < 2; ++r)
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
-                if (k < K) a[slot][r][h] = qt_few::load_weight<16>(row[r][h] + k);
-                else a[slot][r][h] = qt_few::Line<16>{};
+                if (k < K) a[slot][r][h] = qt_few::load_weight(row[r][h] + k);
+                else a[slot][r][h] = qt_few::Line{};
             }
-        if (k < K && pair >= 0) b[slot] = qt_few::load_rows<16>(x + k);
-        else b[slot] = qt_few::Line<16>{};
+        if (k < K && pair >= 0) b[slot] = qt_few::load_rows(x + k);
+        else b[slot] = qt_few::Line{};
     };
     float c[2][4] = {};
 #pragma unroll
@@ -421,17 +421,17 @@ __global__ void __launch_bounds__(EG_WARPS * 32, 2) expert_down_groups_kernel(co
     const int first = rank + RANKS * warp, stride = RANKS * EG_WARPS;
     const int turns = (K + EG_STEP - 1) / EG_STEP, per = first < turns ? (turns - first + stride - 1) / stride : 0;   // of a group
     const int mine = per * groups.count;
-    qt_few::Line<16> a[DEPTH][1][2], b[DEPTH];
+    qt_few::Line a[DEPTH][1][2], b[DEPTH];
     auto ask = [&](int slot, int i) {                         // turns of the groups one after the other
         const int group = i / per, k = (first + (i - group * per) * stride) * EG_STEP + 16 * t, pair = groups.pair[group][g];
         const __nv_bfloat16* w = (const __nv_bfloat16*)p.down + (size_t)groups.expert[group] * p.width * K + k;
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
-            if (k < K) a[slot][0][h] = qt_few::load_weight<16>(w + (size_t)min(c0 + 8 * h + g, p.width - 1) * K);
-            else a[slot][0][h] = qt_few::Line<16>{};
+            if (k < K) a[slot][0][h] = qt_few::load_weight(w + (size_t)min(c0 + 8 * h + g, p.width - 1) * K);
+            else a[slot][0][h] = qt_few::Line{};
         }
-        if (k < K && pair >= 0) b[slot] = qt_few::load_rows<16>((const __nv_bfloat16*)p.mid + (size_t)pair * K + k);
-        else b[slot] = qt_few::Line<16>{};
+        if (k < K && pair >= 0) b[slot] = qt_few::load_rows((const __nv_bfloat16*)p.mid + (size_t)pair * K + k);
+        else b[slot] = qt_few::Line{};
     };
     float c[1][4] = {};
     auto put = [&](int group) {

@@ -4,7 +4,7 @@
 // small model, by the chain of launches it stands in: each waits for the one before it, and what it does between that moment and its
 // own end is the step's time.  So the chain is kept as short as it can be:
 //
-//   * A block holds 16 or 32 rows of W whole: its warps share K (4 E elements a warp and turn, interleaved) and add up through shared
+//   * A block holds 16 or 32 rows of W whole: its warps share K (64 elements a warp and turn, interleaved) and add up through shared
 //     memory.  No cluster, no partial sums in memory, no TMEM, no tensor maps (gemm_fused.cu has all of these between the arrival of X
 //     and its result); only q/k/v, whose heads span 128 rows, is a cluster of four blocks that hand each other finished sums.
 //   * The weight goes from memory into the registers that mma.sync reads (few_tokens.cuh).  Every warp asks for its first turns ahead of
@@ -28,10 +28,10 @@ namespace {
 
 constexpr int QKV_BLOCKS = 4;              // blocks of 32 rows that hold a 128-row group of heads
 
-// RT: tiles of 16 weight rows of a block; NT: tiles of 8 tokens; E: elements a lane loads at once; DEPTH: turns whose operands are in flight
-template <int EPI, int RT, int NT, int WARPS, int E, int DEPTH>
+// RT: tiles of 16 weight rows of a block; NT: tiles of 8 tokens; DEPTH: turns whose operands are in flight
+template <int EPI, int RT, int NT, int WARPS, int DEPTH>
 __global__ void __launch_bounds__(WARPS * 32, 16 / WARPS) gemm_few_kernel(const __nv_bfloat16* w, const __nv_bfloat16* x, int K, const __grid_constant__ EpilogueParams ep) {
-    constexpr int W = 16 * RT, LANES = W / 4, TOKENS = 8 * NT, STEP = 4 * E;
+    constexpr int W = 16 * RT, LANES = W / 4, TOKENS = 8 * NT, STEP = 4 * PIECE;
     constexpr int FINISHERS = TOKENS * LANES / 32;                  // warps that add the others' sums up
     static_assert(EPI != EPI_QKV || W * QKV_BLOCKS == TILE, "a cluster holds the 128 rows that the heads' epilogue takes");
     static_assert(FINISHERS <= WARPS, "");
@@ -50,24 +50,24 @@ __global__ void __launch_bounds__(WARPS * 32, 16 / WARPS) gemm_few_kernel(const 
     for (int r = 0; r < RT; ++r)
 #pragma unroll
         for (int h = 0; h < 2; ++h) row[r][h] = w + (size_t)min(n0 + 16 * r + 8 * h + g, ep.N - 1) * K;
-    Line<E> a[DEPTH][RT][2], b[DEPTH][NT];
+    Line a[DEPTH][RT][2], b[DEPTH][NT];
     auto ask_weight = [&](int slot, int i) {
-        const int k = (warp + i * WARPS) * STEP + E * t;
+        const int k = (warp + i * WARPS) * STEP + PIECE * t;
         const bool inside = k < K;                                  // K is a multiple of 16: a lane's elements are all in or out
 #pragma unroll
         for (int r = 0; r < RT; ++r)
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
-                if (inside) a[slot][r][h] = load_weight<E>(row[r][h] + k);
-                else a[slot][r][h] = Line<E>{};
+                if (inside) a[slot][r][h] = load_weight(row[r][h] + k);
+                else a[slot][r][h] = Line{};
             }
     };
     auto ask_rows = [&](int slot, int i) {
-        const int k = (warp + i * WARPS) * STEP + E * t;
+        const int k = (warp + i * WARPS) * STEP + PIECE * t;
 #pragma unroll
         for (int n = 0; n < NT; ++n) {
-            if (k < K && 8 * n + g < ep.M) b[slot][n] = load_rows<E>(x + (size_t)(8 * n + g) * K + k);
-            else b[slot][n] = Line<E>{};
+            if (k < K && 8 * n + g < ep.M) b[slot][n] = load_rows(x + (size_t)(8 * n + g) * K + k);
+            else b[slot][n] = Line{};
         }
     };
 #pragma unroll
@@ -95,7 +95,7 @@ __global__ void __launch_bounds__(WARPS * 32, 16 / WARPS) gemm_few_kernel(const 
         for (int u = 0; u < DEPTH; ++u) {
             if (i0 + u >= mine) break;
 #pragma unroll
-            for (int j = 0; j < E / 4; ++j)
+            for (int j = 0; j < PIECE / 4; ++j)
 #pragma unroll
                 for (int r = 0; r < RT; ++r)
 #pragma unroll
@@ -147,14 +147,14 @@ __global__ void __launch_bounds__(WARPS * 32, 16 / WARPS) gemm_few_kernel(const 
     }
 }
 
-template <int EPI, int RT, int NT, int WARPS, int E, int DEPTH>
+template <int EPI, int RT, int NT, int WARPS, int DEPTH>
 int launch(const void* w, const void* x, int K, const EpilogueParams& e, cudaStream_t stream) {
     const dim3 block(WARPS * 32);
     if (EPI == EPI_QKV)
-        launch_kernel_cluster(gemm_few_kernel<EPI, RT, NT, WARPS, E, DEPTH>, dim3((unsigned)((e.N + TILE - 1) / TILE * QKV_BLOCKS)), block, 0, stream, (unsigned)QKV_BLOCKS,
+        launch_kernel_cluster(gemm_few_kernel<EPI, RT, NT, WARPS, DEPTH>, dim3((unsigned)((e.N + TILE - 1) / TILE * QKV_BLOCKS)), block, 0, stream, (unsigned)QKV_BLOCKS,
                               (const __nv_bfloat16*)w, (const __nv_bfloat16*)x, K, e);
     else
-        launch_kernel(gemm_few_kernel<EPI, RT, NT, WARPS, E, DEPTH>, dim3((unsigned)((e.N + 16 * RT - 1) / (16 * RT))), block, 0, stream,
+        launch_kernel(gemm_few_kernel<EPI, RT, NT, WARPS, DEPTH>, dim3((unsigned)((e.N + 16 * RT - 1) / (16 * RT))), block, 0, stream,
                       (const __nv_bfloat16*)w, (const __nv_bfloat16*)x, K, e);
     QT_CHECK_LAUNCH("gemm_few");
     return QT_OK;
@@ -164,11 +164,11 @@ template <int EPI, int RT>
 int dispatch(const void* w, const void* x, int K, int warps, const EpilogueParams& e, cudaStream_t stream) {
     constexpr int DEPTH = RT == 1 ? 4 : 2, DEPTH2 = RT == 1 ? 2 : 1;
     if (e.M <= 8) {
-        if (warps == 16) return launch<EPI, RT, 1, 16, 16, DEPTH>(w, x, K, e, stream);
-        return launch<EPI, RT, 1, 8, 16, DEPTH>(w, x, K, e, stream);
+        if (warps == 16) return launch<EPI, RT, 1, 16, DEPTH>(w, x, K, e, stream);
+        return launch<EPI, RT, 1, 8, DEPTH>(w, x, K, e, stream);
     }
-    if (warps == 16) return launch<EPI, RT, 2, 16, 16, DEPTH2>(w, x, K, e, stream);
-    return launch<EPI, RT, 2, 8, 16, DEPTH2>(w, x, K, e, stream);
+    if (warps == 16) return launch<EPI, RT, 2, 16, DEPTH2>(w, x, K, e, stream);
+    return launch<EPI, RT, 2, 8, DEPTH2>(w, x, K, e, stream);
 }
 
 }  // namespace
