@@ -21,7 +21,7 @@
 // 0.84e-7 to 1.61e-7 / 0.78e-7 to 1.40e-7; operands of one sign 0.40e-7 to 0.63e-7 / 0.86e-7 to 0.98e-7, of which 0.79e-7 is the mean of the large instructions' cuts towards zero.  A factor for that
 // mean would round off sums that nothing was cut from; accumulators read back every 32 or 16 of K (0.60e-7 to 0.83e-7, 0.56e-7 to 0.91e-7) cost 10 to 25 % and 35 to 140 % of the time.
 //
-// Infinities, NaN, numbers that round to an infinite bfloat16 and those whose last piece lies below bfloat16's smallest (under 2^-110, at the earliest 2^-102) have no
+// Infinities, NaN, numbers that round to an infinite bfloat16 and those below 2^-110 with bits that no bfloat16 reaches (2^-133 is its smallest) have no
 // such pieces: a block that meets one forms its results again with FMAs (float_results:
 // 4096 x 1024, 549 rows with a NaN in each 420 us; 4096 x 12288, 4,096 rows 26 ms).
 #include "tc_common.cuh"
@@ -52,17 +52,19 @@ struct Params {
     int* status;
 };
 
-// mbar_wait without its call: the working warps hold sums and floats across their waits, which a call has them store and load again.
-__device__ __forceinline__ bool wait_here(uint32_t bar, uint32_t parity, int* status, int code) {
+// mbar_wait for a whole warp and without its call: the working warps hold sums and floats across their waits, which a call has them store and load again.
+// Lanes that leave the loop one after the other meet in the vote: what follows (tcgen05.ld, tcgen05.st) is for a warp that is together.
+__device__ __forceinline__ bool warp_wait(uint32_t bar, uint32_t parity, int* status, int code) {
     unsigned long long start = 0;
-    for (uint32_t spins = 0; !mbar_try_wait(bar, parity);) {
+    bool ok = true;
+    for (uint32_t spins = 0; ok && !mbar_try_wait(bar, parity);) {
         if ((++spins & 0x3ffu) != 0) continue;
-        if (*(volatile int*)status != 0) return false;
         const unsigned long long now = global_timer();
         if (start == 0) start = now;
-        else if (now - start > WAIT_LIMIT_NS) { atomicCAS(status, 0, code); return false; }
+        if (*(volatile int*)status != 0) ok = false;
+        else if (now - start > WAIT_LIMIT_NS) { atomicCAS(status, 0, code); ok = false; }
     }
-    return true;
+    return __all_sync(0xffffffffu, ok);
 }
 __device__ __forceinline__ uint32_t pack_rn(float lo, float hi) {
     uint32_t d;
@@ -181,7 +183,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_f32_tc_kernel(const __grid_co
             prefetch_tensor_map(&map_a);
             pdl_wait();
             for (int i = 0, s = 0, turn = 0; i < slices; ++i) {
-                if (!wait_here(taken + 8 * s, (uint32_t)turn ^ 1u, status, 1)) break;
+                if (!mbar_wait(taken + 8 * s, (uint32_t)turn ^ 1u, status, 1)) break;
                 mbar_expect_tx(arrived + 8 * s, A_STAGE_BYTES);
                 for (int h = 0; h < 2; ++h)                                 // the map counts 16-bit elements, two a float
                     tma_load_2d(a_floats + s * A_STAGE_BYTES + h * A_HALF_BYTES, &map_a, arrived + 8 * s, 2 * (k_begin + i * BK + 32 * h), m0);
@@ -195,8 +197,8 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_f32_tc_kernel(const __grid_co
             for (int i = 0; i < slices; ++i) {
                 const int s = i & 1;
                 const uint32_t turn = (uint32_t)(i >> 1) & 1u;
-                if (!wait_here(full + 8 * s, turn, status, 2)) break;
-                if (!wait_here(added + 8 * s, turn ^ 1u, status, 4)) break;
+                if (!mbar_wait(full + 8 * s, turn, status, 2)) break;
+                if (!mbar_wait(added + 8 * s, turn ^ 1u, status, 4)) break;
                 tc_fence_after();
                 const uint64_t w0 = desc0 + (uint64_t)(s * (STAGE_BYTES >> 4));
                 const uint32_t acc = tmem_base + s * TILE, a0 = tmem_base + TMEM_A + s * 3 * A_COLS;
@@ -233,7 +235,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_f32_tc_kernel(const __grid_co
         const uint32_t mine = tmem_base + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)(warp >> 2) * COLS;
         auto add = [&](int i) {
             const int s = i & 1;
-            if (!wait_here(summed + 8 * s, (uint32_t)(i >> 1) & 1u, status, 3)) return false;
+            if (!warp_wait(summed + 8 * s, (uint32_t)(i >> 1) & 1u, status, 3)) return false;
             tc_fence_after();
 #pragma unroll
             for (int part = 0; part < COLS / 16; ++part) {
@@ -271,10 +273,10 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_f32_tc_kernel(const __grid_co
         bool ok = true;
         for (int i = 0; i < slices && ok; ++i) {
             const int s = i & 1;
-            ok = wait_here(empty + 8 * s, ((uint32_t)(i >> 1) & 1u) ^ 1u, status, 1);
+            ok = warp_wait(empty + 8 * s, ((uint32_t)(i >> 1) & 1u) ^ 1u, status, 1);
             if (!ok) break;
             if (of_a) {
-                ok = wait_here(arrived + 8 * a_stage, a_turn, status, 3);
+                ok = warp_wait(arrived + 8 * a_stage, a_turn, status, 3);
                 if (!ok) break;
                 const uint8_t* floats = smem + 2 * STAGE_BYTES + a_stage * A_STAGE_BYTES + a_half * A_HALF_BYTES + a_row * 128;
 #pragma unroll
