@@ -3,7 +3,7 @@ import numpy as np
 import pytest
 import torch
 
-from qwen_triton_b200.engine.step import longest_first
+from qwen_triton_b200.engine.step import ORDERED_FROM, _DecodePlan, longest_first
 from qwen_triton_b200.ops import kernels
 from qwen_triton_b200.ops.kernels import GemmOut
 from test_gpu_kernels import DEV, PAGE, rand
@@ -67,6 +67,15 @@ def test_decode_attention_in_a_given_order(seqs, mask, splits):
         results.append(out)
     assert torch.isfinite(results[0]).all()
     assert torch.equal(results[0], results[1]) and torch.equal(results[0], results[2])
+
+
+@pytest.mark.parametrize("n, widths", [(1, (16,)), (16, (16, 3)), (ORDERED_FROM, (16, 3)), (48, (5,)), (128, (16,))])
+def test_the_order_lies_behind_the_tables_of_many_sequences(n, widths):
+    plan = _DecodePlan(torch.zeros(8192, dtype=torch.int32, device=DEV), n, widths)
+    assert (plan.order is None) is (n < ORDERED_FROM)
+    if plan.order is not None:
+        assert plan.order.shape == (n, 2) and plan.order.data_ptr() % 8 == 0
+        assert plan.order.data_ptr() >= plan.tables[len(widths) - 1].data_ptr() + 4 * n * widths[-1]
 
 
 @pytest.mark.parametrize("experts, top, width, ff, tokens, skew", [(8, 1, 1024, 2048, 8, False), (4, 2, 2048, 1040, 15, False), (3, 1, 2064, 1024, 32, True),
