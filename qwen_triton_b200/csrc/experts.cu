@@ -526,8 +526,10 @@ extern "C" int qt_experts_by_pair(const void* x, const int* token_ids, const int
         const size_t smem_up = (size_t)width * sizeof(float), smem_down = (size_t)top * ff * sizeof(float);
         const dim3 grid_up(n_tokens * top, (ff + per_block - 1) / per_block), grid_down(n_tokens, (width + per_block - 1) / per_block);
         // Per expert where the pairs are at least as many as the experts, so that some share one, and where an expert's bytes outweigh the longer way to
-        // them (groups, a cluster's sums).  Both passes, by pair / per expert: 8, 16, 32 tokens of one of 8 experts of 1,024 x 2,048 18 / 15, 33 / 25, 54 / 28 us; 8,
-        // 12, 16 tokens of 2 of 16 of 2,048 x 1,024 34 / 31, 44 / 35, 55 / 39 us; but of 1,024 x 512 10 / 14 us, 8 tokens of 4 of 32 of 2,048 x 768 48 / 54 us.
+        // them (groups, a cluster's sums).  Both passes, gated, by pair / per expert, us: 8, 16, 32 tokens of one of 8 experts of 1,024 x 2,048 18 / 15, 32 / 24, 53 / 28; of
+        // 2,048 x 2,048 29 / 24, 52 / 41, 87 / 44; of 4,096 x 1,536 44 / 29, 73 / 56, 127 / 57; 8, 12, 16 tokens of 2 of 16 of 2,048 x 1,024 33 / 30, 43 / 33, 54 / 38; but of 1,024 x 512
+        // 10 / 14, 8 tokens of 4 of 32 of 2,048 x 768 48 / 54.  Above the bound it is the slower form only where there are as many pairs as experts and few share one: 4 tokens of 2
+        // of 8 of 2,048 x 1,024 18.4 / 18.9, of 4,096 x 1,024 31 / 33, 8 tokens of 4 of 32 of 2,880 x 2,880 205 / 210.
         if (std::is_same<T, __nv_bfloat16>::value && n_tokens * top <= EG_PAIRS && n_tokens * top >= experts && (long long)width * ff >= (2ll << 20) && width % 16 == 0 && ff % 16 == 0 &&
             (((uintptr_t)up | (uintptr_t)down | (uintptr_t)x | (uintptr_t)mid) & 31) == 0) return launch_expert_groups(p, s);
         // 16-byte loads: rows of both weights, of x and of mid start on 16-byte boundaries

@@ -1,11 +1,11 @@
 // C[M, N] = A[M, K] * W[N, K]^T in true float on the FMA pipe (no tensor cores, no reduced-precision mode): the 32-bit path's
-// products of up to 32 rows wherever these are 16-byte aligned (K % 4 == 0); more rows are gemm_f32_tc.cu's.  gemm_simt.cu keeps the other alignments and
-// bfloat16 operands.
+// products of up to 32 rows wherever these are 16-byte aligned (K % 4 == 0).  More rows are gemm_f32_tc.cu's, but for a result off a 16-byte boundary
+// whose rows are multiples of 16 bytes.  gemm_simt.cu keeps the other alignments and bfloat16 operands.
 //
 // Both kernels multiply with fma.rn.f32x2 along K: a 16-byte piece of a row is two pairs of neighbouring k, which is how both
 // operands lie in memory, so no value is duplicated or repacked; the even and the odd k of a sum are added at the end.
 //
-// gemm_f32_tile_kernel   tiles of 64 x 128 (16 x 128 and 32 x 128 for few rows), 128 threads of 8 x 8 results (2 x 8, 4 x 8), K slices of 32
+// gemm_f32_tile_kernel   tiles of 16 x 128 and 32 x 128 (64 x 128 for such results), 128 threads of 2 x 8 and 4 x 8 results (8 x 8), K slices of 32
 //   through a three-stage cp.async ring, two blocks an SM.  Per 4 k a thread issues 128 packed FMAs and 16 16-byte reads, nearly free of bank
 //   conflicts (rows are 36 floats apart).  549 rows, 6144 x 1024 (ncu): the FMA pipe busy 62 % of an SM's active cycles, shared memory 50 %; the rest are
 //   fixed latencies of the two warps a scheduler that 255 registers leave.  8 x 4 results a thread (12 reads for 64

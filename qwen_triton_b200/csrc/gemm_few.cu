@@ -175,7 +175,8 @@ int dispatch(const void* w, const void* x, int K, int warps, const EpilogueParam
 
 // x [M, K] bfloat16 (M up to 16), w [N, K] bfloat16, K a multiple of 16 and both 32-byte aligned.  `epilogue` picks what is done with
 // the product and which of the pointers are read, as in qt_gemm_fused; `block_rows` (16, or 32 as q/k/v and the gate always take) is
-// how many rows of w a block holds, and the width of the tiles whose sums of squares sq_out receives; `warps` (8 or 16) share K.
+// how many rows of w a block holds, and the width of the tiles whose sums of squares sq_out receives; `warps` (8 or 16) share K.  The engine takes 16 rows with 16
+// warps, and 32 rows for heads and gates (Linear.few_plan); 16 rows with 8 warps, and 32 with the other epilogues, are for other callers.
 extern "C" int qt_gemm_few(const void* x, const void* w, int M, int N, int K, int block_rows, int warps, int epilogue,
                            const float* sq_in, int sq_tiles, int norm_width, float eps, const float* bias,
                            void* out, int out_dtype, int act, float limit,
