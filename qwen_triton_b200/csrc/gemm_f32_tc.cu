@@ -12,6 +12,9 @@
 // warps add a finished slice's accumulator up while the next one is multiplied.  Up to eight blocks of a cluster share K where the tiles do not fill
 // the SMs, and add up through distributed shared memory in the order of the ranks.
 //
+// tcgen05.ld, tcgen05.st and bar.sync are for a warp that is together: a __syncwarp stands ahead of each behind a branch of single lanes or a wait.  Without these the results
+// were right or now and then wrong by how the compiler had laid the code out.
+//
 // What bounds it now is the splitting: a slice takes 1.9 us (3,300 cycles), and with one product in the place of six 0.9 of that.
 //
 // N x K, rows, us before (gemm_f32.cu) / here, L2 flushed ahead of each: 4096 x 1024 64 27 / 21, 549 129 / 64, 4,096 807 / 236; 6144 x 1024 549 184 / 74; 1024 x 3072 549 117 / 39; 4096 x 12288
@@ -22,8 +25,8 @@
 // mean would round off sums that nothing was cut from; accumulators read back every 32 or 16 of K (0.60e-7 to 0.83e-7, 0.56e-7 to 0.91e-7) cost 10 to 25 % and 35 to 140 % of the time.
 //
 // Infinities, NaN, numbers that round to an infinite bfloat16 and those below 2^-110 with bits that no bfloat16 reaches (2^-133 is its smallest) have no
-// such pieces: a block that meets one forms its results again with FMAs (float_results:
-// 4096 x 1024, 549 rows with a NaN in each 420 us; 4096 x 12288, 4,096 rows 26 ms).
+// such pieces: a block that meets one forms its results again with FMAs, from slices of both operands in shared memory (4096 x 1024, 549 rows with a NaN in each 410 us; 4096 x 12288,
+// 4,096 rows 26 ms).
 #include "tc_common.cuh"
 
 using namespace qt;
@@ -99,6 +102,7 @@ __device__ __noinline__ void float_results(const Params& p, int m0, int n0, int 
     float sums[COLS] = {};
 #pragma unroll 1
     for (int k0 = k_begin; k0 < k_end; k0 += BK) {
+        __syncwarp();
         asm volatile("bar.sync 1, %0;" ::"n"(WORK_WARPS * 32) : "memory");
 #pragma unroll 4
         for (int i = threadIdx.x; i < 2 * TILE * BK / 4; i += WORK_WARPS * 32) {
@@ -107,6 +111,7 @@ __device__ __noinline__ void float_results(const Params& p, int m0, int n0, int 
             const float4 v = there ? load4((r < TILE ? p.a : p.w) + (size_t)at * p.K + k) : make_float4(0.f, 0.f, 0.f, 0.f);
             *reinterpret_cast<float4*>(tiles + r * FLOAT_ROW + i % (BK / 4) * 4) = v;
         }
+        __syncwarp();
         asm volatile("bar.sync 1, %0;" ::"n"(WORK_WARPS * 32) : "memory");
         const float *x = tiles + row * FLOAT_ROW, *y = tiles + (TILE + col0) * FLOAT_ROW;
 #pragma unroll
@@ -236,6 +241,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_f32_tc_kernel(const __grid_co
         auto add = [&](int i) {
             const int s = i & 1;
             if (!warp_wait(summed + 8 * s, (uint32_t)(i >> 1) & 1u, status, 3)) return false;
+            __syncwarp();
             tc_fence_after();
 #pragma unroll
             for (int part = 0; part < COLS / 16; ++part) {
@@ -285,6 +291,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_f32_tc_kernel(const __grid_co
                 __syncwarp();
                 if (lane == 0) mbar_arrive(taken + 8 * a_stage);
                 if (++a_stage == A_STAGES) { a_stage = 0; a_turn ^= 1u; }
+                __syncwarp();
                 tc_fence_after();
 #pragma unroll
                 for (int piece = 0; piece < 3; ++piece) {
@@ -293,6 +300,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_f32_tc_kernel(const __grid_co
                     for (int u = 0; u < UNITS; ++u) {
                         piece_of(u, h + 4 * u, piece == 0, piece == 2);
                     }
+                    __syncwarp();
                     store_columns(tmem_base + ((uint32_t)((warp & 3) * 32) << 16) + TMEM_A + (s * 3 + piece) * A_COLS + 16 * a_half, h);
                 }
                 tmem_wait_st();
@@ -317,6 +325,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_f32_tc_kernel(const __grid_co
         }
         if (ok) ok = add(slices - 1);
         if (none != 0.f || (rest & 0xffffu) != 0 || !ok) atomicOr(odd, ok ? 1 : 2);
+        __syncwarp();
         asm volatile("bar.sync 1, %0;" ::"n"(WORK_WARPS * 32) : "memory");
         const int row = (warp & 3) * 32 + lane, col0 = (warp >> 2) * COLS, m = m0 + row;
         if (p.ranks > 1) {                                                  // every MMA has read the stages: they are free
