@@ -12,9 +12,6 @@
 // warps add a finished slice's accumulator up while the next one is multiplied.  Up to eight blocks of a cluster share K where the tiles do not fill
 // the SMs, and add up through distributed shared memory in the order of the ranks.
 //
-// tcgen05.ld, tcgen05.st and bar.sync are for a warp that is together: a __syncwarp stands ahead of each behind a branch of single lanes or a wait.  Without these the results
-// were right or now and then wrong by how the compiler had laid the code out.
-//
 // What bounds it now is the splitting: a slice takes 1.9 us (3,300 cycles), and with one product in the place of six 0.9 of that.
 //
 // N x K, rows, us before (gemm_f32.cu) / here, L2 flushed ahead of each: 4096 x 1024 64 27 / 21, 549 129 / 64, 4,096 807 / 236; 6144 x 1024 549 184 / 74; 1024 x 3072 549 117 / 39; 4096 x 12288
@@ -24,9 +21,7 @@
 // 0.84e-7 to 1.61e-7 / 0.78e-7 to 1.40e-7; operands of one sign 0.40e-7 to 0.63e-7 / 0.86e-7 to 0.98e-7, of which 0.79e-7 is the mean of the large instructions' cuts towards zero.  A factor for that
 // mean would round off sums that nothing was cut from; accumulators read back every 32 or 16 of K (0.60e-7 to 0.83e-7, 0.56e-7 to 0.91e-7) cost 10 to 25 % and 35 to 140 % of the time.
 //
-// Infinities, NaN, numbers that round to an infinite bfloat16 and those below 2^-110 with bits that no bfloat16 reaches (2^-133 is its smallest) have no
-// such pieces: a block that meets one forms its results again with FMAs, from slices of both operands in shared memory (4096 x 1024, 549 rows with a NaN in each 410 us; 4096 x 12288,
-// 4,096 rows 26 ms).
+// Infinities, NaN and numbers that round to an infinite bfloat16 have no such pieces: a block that meets one forms its results again with FMAs.
 #include "tc_common.cuh"
 
 using namespace qt;
@@ -44,10 +39,10 @@ constexpr int A_COLS = BK / 2;                         // one piece of A in tens
 constexpr uint32_t TMEM_A = 2 * TILE, TMEM_COLS = 512; // two accumulators, two stages of A's pieces
 constexpr int UNITS = 4;                               // runs of eight elements a thread splits per slice
 constexpr int COLS = 32;                               // results a thread keeps the sums of
-constexpr int MOST_RANKS = 8, PARK_ROW = TILE + 4, FLOAT_ROW = BK + 4;
+constexpr int MOST_RANKS = 8, PARK_ROW = TILE + 4;
 constexpr uint32_t IDESC = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(TILE >> 3) << 17) | ((uint32_t)(TILE >> 4) << 24);
 static_assert(TILE * PARK_ROW * 4 <= 2 * STAGE_BYTES, "a block's part of the result is parked in the stages' memory");
-static_assert(2 * TILE * FLOAT_ROW * 4 <= A_STAGES * A_STAGE_BYTES, "a slice of both operands as floats lies in the memory of A's");
+
 
 struct Params {
     const float* a; const float* w; float* c;
@@ -55,20 +50,6 @@ struct Params {
     int* status;
 };
 
-// mbar_wait for a whole warp and without its call: the working warps hold sums and floats across their waits, which a call has them store and load again.
-// Lanes that leave the loop one after the other meet in the vote: what follows (tcgen05.ld, tcgen05.st) is for a warp that is together.
-__device__ __forceinline__ bool warp_wait(uint32_t bar, uint32_t parity, int* status, int code) {
-    unsigned long long start = 0;
-    bool ok = true;
-    for (uint32_t spins = 0; ok && !mbar_try_wait(bar, parity);) {
-        if ((++spins & 0x3ffu) != 0) continue;
-        const unsigned long long now = global_timer();
-        if (start == 0) start = now;
-        if (*(volatile int*)status != 0) ok = false;
-        else if (now - start > WAIT_LIMIT_NS) { atomicCAS(status, 0, code); ok = false; }
-    }
-    return __all_sync(0xffffffffu, ok);
-}
 __device__ __forceinline__ uint32_t pack_rn(float lo, float hi) {
     uint32_t d;
     asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(d) : "f"(hi), "f"(lo));
@@ -93,57 +74,6 @@ __device__ __forceinline__ float4 peer4(uint32_t addr) {
     float4 v;
     asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr) : "memory");
     return v;
-}
-
-// A block's results by FMAs, for numbers that are not the sum of three bfloat16 pieces, written over those of the pieces: to C, or to where a block with peers
-// parks them.  The sixteen working warps call; `tiles` receives a slice of A's rows and of W's after the other.  Sums of 16, of a slice, and of all slices.
-__device__ __noinline__ void float_results(const Params& p, int m0, int n0, int k_begin, int k_end, float* tiles, float* park) {
-    const int row = threadIdx.x & 127, col0 = (int)(threadIdx.x >> 7) * COLS;
-    float sums[COLS] = {};
-#pragma unroll 1
-    for (int k0 = k_begin; k0 < k_end; k0 += BK) {
-        __syncwarp();
-        asm volatile("bar.sync 1, %0;" ::"n"(WORK_WARPS * 32) : "memory");
-#pragma unroll 4
-        for (int i = threadIdx.x; i < 2 * TILE * BK / 4; i += WORK_WARPS * 32) {
-            const int r = i / (BK / 4), k = k0 + i % (BK / 4) * 4, at = r < TILE ? m0 + r : n0 + r - TILE;
-            const bool there = at < (r < TILE ? p.M : p.N) && k < k_end;
-            const float4 v = there ? load4((r < TILE ? p.a : p.w) + (size_t)at * p.K + k) : make_float4(0.f, 0.f, 0.f, 0.f);
-            *reinterpret_cast<float4*>(tiles + r * FLOAT_ROW + i % (BK / 4) * 4) = v;
-        }
-        __syncwarp();
-        asm volatile("bar.sync 1, %0;" ::"n"(WORK_WARPS * 32) : "memory");
-        const float *x = tiles + row * FLOAT_ROW, *y = tiles + (TILE + col0) * FLOAT_ROW;
-#pragma unroll
-        for (int j0 = 0; j0 < COLS; j0 += 16) {
-            float slice[16] = {};
-#pragma unroll 1
-            for (int k1 = 0; k1 < BK; k1 += 16) {
-                float part[16] = {};
-#pragma unroll 1
-                for (int k = k1; k < k1 + 16; k += 4) {
-                    const float4 u = *reinterpret_cast<const float4*>(x + k);
-#pragma unroll
-                    for (int j = 0; j < 16; ++j) {
-                        const float4 v = *reinterpret_cast<const float4*>(y + (j0 + j) * FLOAT_ROW + k);
-                        part[j] = fmaf(u.w, v.w, fmaf(u.z, v.z, fmaf(u.y, v.y, fmaf(u.x, v.x, part[j]))));
-                    }
-                }
-#pragma unroll
-                for (int j = 0; j < 16; ++j) slice[j] += part[j];
-            }
-#pragma unroll
-            for (int j = 0; j < 16; ++j) sums[j0 + j] += slice[j];
-        }
-    }
-    if (p.ranks > 1) {
-#pragma unroll
-        for (int j = 0; j < COLS; ++j) park[row * PARK_ROW + col0 + j] = sums[j];
-    } else if (m0 + row < p.M) {
-#pragma unroll
-        for (int j = 0; j < COLS; ++j)
-            if (n0 + col0 + j < p.N) p.c[(size_t)(m0 + row) * p.N + n0 + col0 + j] = sums[j];
-    }
 }
 
 __global__ void __launch_bounds__(THREADS, 1) gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ Params p) {
@@ -240,8 +170,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_f32_tc_kernel(const __grid_co
         const uint32_t mine = tmem_base + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)(warp >> 2) * COLS;
         auto add = [&](int i) {
             const int s = i & 1;
-            if (!warp_wait(summed + 8 * s, (uint32_t)(i >> 1) & 1u, status, 3)) return false;
-            __syncwarp();
+            if (!mbar_wait(summed + 8 * s, (uint32_t)(i >> 1) & 1u, status, 3)) return false;
             tc_fence_after();
 #pragma unroll
             for (int part = 0; part < COLS / 16; ++part) {
@@ -263,7 +192,6 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_f32_tc_kernel(const __grid_co
         int a_stage = 0;
         uint32_t a_turn = 0;
         float none = 0.f;                                                   // stays 0 while every number has its pieces
-        uint32_t rest = 0;                                                  // its low half stays 0 while every third piece is all that is left
         // the next piece of a unit: its numbers rounded, and what is left of them
         auto piece_of = [&](int u, uint32_t* h, bool first, bool last) {
 #pragma unroll
@@ -271,7 +199,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_f32_tc_kernel(const __grid_co
                 float& lo = v[u][2 * j];
                 float& hi = v[u][2 * j + 1];
                 h[j] = pack_rn(lo, hi);
-                if (last) { rest |= __float_as_uint(lo) | __float_as_uint(hi); continue; }
+                if (last) continue;
                 lo -= low_of(h[j]); hi -= high_of(h[j]);
                 if (first) { none = fmaf(0.f, lo, none); none = fmaf(0.f, hi, none); }
             }
@@ -279,10 +207,10 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_f32_tc_kernel(const __grid_co
         bool ok = true;
         for (int i = 0; i < slices && ok; ++i) {
             const int s = i & 1;
-            ok = warp_wait(empty + 8 * s, ((uint32_t)(i >> 1) & 1u) ^ 1u, status, 1);
+            ok = mbar_wait(empty + 8 * s, ((uint32_t)(i >> 1) & 1u) ^ 1u, status, 1);
             if (!ok) break;
             if (of_a) {
-                ok = warp_wait(arrived + 8 * a_stage, a_turn, status, 3);
+                ok = mbar_wait(arrived + 8 * a_stage, a_turn, status, 3);
                 if (!ok) break;
                 const uint8_t* floats = smem + 2 * STAGE_BYTES + a_stage * A_STAGE_BYTES + a_half * A_HALF_BYTES + a_row * 128;
 #pragma unroll
@@ -291,7 +219,6 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_f32_tc_kernel(const __grid_co
                 __syncwarp();
                 if (lane == 0) mbar_arrive(taken + 8 * a_stage);
                 if (++a_stage == A_STAGES) { a_stage = 0; a_turn ^= 1u; }
-                __syncwarp();
                 tc_fence_after();
 #pragma unroll
                 for (int piece = 0; piece < 3; ++piece) {
@@ -300,7 +227,6 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_f32_tc_kernel(const __grid_co
                     for (int u = 0; u < UNITS; ++u) {
                         piece_of(u, h + 4 * u, piece == 0, piece == 2);
                     }
-                    __syncwarp();
                     store_columns(tmem_base + ((uint32_t)((warp & 3) * 32) << 16) + TMEM_A + (s * 3 + piece) * A_COLS + 16 * a_half, h);
                 }
                 tmem_wait_st();
@@ -324,10 +250,20 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_f32_tc_kernel(const __grid_co
             if (i > 0) ok = add(i - 1);
         }
         if (ok) ok = add(slices - 1);
-        if (none != 0.f || (rest & 0xffffu) != 0 || !ok) atomicOr(odd, ok ? 1 : 2);
-        __syncwarp();
+        if (none != 0.f) atomicOr(odd, 1);                                  // NaN
         asm volatile("bar.sync 1, %0;" ::"n"(WORK_WARPS * 32) : "memory");
         const int row = (warp & 3) * 32 + lane, col0 = (warp >> 2) * COLS, m = m0 + row;
+        if (*(volatile int*)odd != 0) {
+            const float* x = p.a + (size_t)min(m, p.M - 1) * p.K;
+#pragma unroll 1
+            for (int j0 = 0; j0 < COLS; ++j0) {
+                const float* y = p.w + (size_t)min(n0 + col0 + j0, p.N - 1) * p.K;
+                float sum = 0.f;
+                for (int k = k_begin; k < k_end; ++k) sum = fmaf(x[k], y[k], sum);
+#pragma unroll
+                for (int j = 0; j < COLS; ++j) if (j == j0) sums[j] = sum;    // registers have no index
+            }
+        }
         if (p.ranks > 1) {                                                  // every MMA has read the stages: they are free
             float* park = reinterpret_cast<float*>(smem) + row * PARK_ROW + col0;
 #pragma unroll
@@ -347,8 +283,6 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_f32_tc_kernel(const __grid_co
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    if (warp < WORK_WARPS && *(volatile int*)odd == 1)                      // A's floats have all been read: the slices lie in their place
-        float_results(p, m0, n0, k_begin, k_end, reinterpret_cast<float*>(smem + 2 * STAGE_BYTES), reinterpret_cast<float*>(smem));
     if (*(volatile int*)status != 0) {                                      // a wait gave up: let MMAs in flight finish first
         const unsigned long long t0 = global_timer();
         while (global_timer() - t0 < 2000000ull) __nanosleep(1000);
